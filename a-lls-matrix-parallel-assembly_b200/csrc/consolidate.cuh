@@ -140,53 +140,6 @@ __global__ void __launch_bounds__(kBlockThreads) k_count_upper(ListLayout L, int
     }
 }
 
-template <int DPN>
-__global__ void __launch_bounds__(kScanThreads) k_scan_reduce_upper(const int* __restrict__ ucounts, int N,
-                                                                    long long* __restrict__ tile_sums) {
-    __shared__ long long s_warp[kScanThreads / 32 + 1];
-    const long long base = (long long)blockIdx.x * kScanTile;
-    long long sum = 0;
-#pragma unroll
-    for (int i = 0; i < kScanItems; i++) {
-        const long long n = base + (long long)i * kScanThreads + threadIdx.x;
-        if (n < N) sum += upper_node_entries<DPN>(FEM_LDG(ucounts + n));
-    }
-    long long total;
-    block_exclusive_scan(sum, s_warp, total);
-    if (threadIdx.x == 0) tile_sums[blockIdx.x] = total;
-}
-
-template <int DPN>
-__global__ void __launch_bounds__(kScanThreads) k_row_ptr_upper(const int* __restrict__ ucounts, int N,
-                                                                const long long* __restrict__ tile_offsets,
-                                                                int* __restrict__ row_ptr) {
-    __shared__ long long s_warp[kScanThreads / 32 + 1];
-    const long long base = (long long)blockIdx.x * kScanTile + (long long)threadIdx.x * kScanItems;
-    int c[kScanItems];
-    long long sum = 0;
-#pragma unroll
-    for (int i = 0; i < kScanItems; i++) {
-        const long long n = base + i;
-        c[i] = n < N ? FEM_LDG(ucounts + n) : 0;
-        sum += upper_node_entries<DPN>(c[i]);
-    }
-    long long total;
-    long long off = tile_offsets[blockIdx.x] + block_exclusive_scan(sum, s_warp, total);
-#pragma unroll
-    for (int i = 0; i < kScanItems; i++) {
-        const long long n = base + i;
-        if (n < N) {
-            long long r = off;
-#pragma unroll
-            for (int a = 0; a < DPN; a++) {
-                row_ptr[n * DPN + a] = (int)r;
-                r += upper_row_len<DPN>(c[i], a);
-            }
-        }
-        off += upper_node_entries<DPN>(c[i]);
-    }
-}
-
 // Ascending bitonic sort of G*KPL keys held as keys[i] at position lane*KPL + i
 // of a G-lane group. Every lane of the warp must call it.
 template <int G, int KPL>

@@ -112,4 +112,86 @@ __device__ __forceinline__ double ke_block_2d(const double (&xd)[NPE], const dou
     return det_out;
 }
 
+// The blocks (node 0, node b), b = 0..NPE-1, of a T3 or Q4 element whose nodes
+// are rotated so that the row node comes first (a rotation keeps the element:
+// its orientation, and the 2x2 Gauss points as a set). The same K_ab as
+// ke_block_2d with the gradients left unnormalised (X = j3 dN/dxi - j1
+// dN/deta, Y = j0 dN/deta - j2 dN/dxi, the true gradient times detJ), so one
+// division per Gauss point carries the weight and both 1/detJ factors, and a
+// T3 needs a single one. Returns detJ (Q4: the smallest over the Gauss
+// points).
+template <int NPE, typename T = double>
+__device__ __forceinline__ double ke_row_2d(const double (&xd)[NPE], const double (&yd)[NPE], double Ed, double nud,
+                                            double td, double (&kv)[NPE][4]) {
+    T x[NPE], y[NPE];
+#pragma unroll
+    for (int k = 0; k < NPE; k++) {
+        x[k] = sizeof(T) == 8 ? T(xd[k]) : T(xd[k] - xd[0]);
+        y[k] = sizeof(T) == 8 ? T(yd[k]) : T(yd[k] - yd[0]);
+    }
+    const T E = T(Ed), nu = T(nud), t = T(td);
+    const T h = T(0.5) * (T(1) - nu), one_nu2 = T(1) - nu * nu;
+    if constexpr (NPE == 3) {
+        const T X[3] = {y[1] - y[2], y[2] - y[0], y[0] - y[1]};
+        const T Y[3] = {x[2] - x[1], x[0] - x[2], x[1] - x[0]};
+        const T det = Y[2] * X[1] - Y[1] * X[2];
+        const T s = T(0.5) * t * E / (one_nu2 * det);
+        const T sx = s * X[0], sy = s * Y[0], hx = h * sx, hy = h * sy, nx = nu * sx, ny = nu * sy;
+#pragma unroll
+        for (int b = 0; b < 3; b++) {
+            kv[b][0] = double(fma(sx, X[b], hy * Y[b]));
+            kv[b][1] = double(fma(nx, Y[b], hy * X[b]));
+            kv[b][2] = double(fma(ny, X[b], hx * Y[b]));
+            kv[b][3] = double(fma(sy, Y[b], hx * X[b]));
+        }
+        return double(det);
+    } else {
+        constexpr double g = 0.577350269189626;  // Q4A:85
+        const T f = t * E / one_nu2;
+        const T lo = T(0.25 * (1.0 - g)), hi = T(0.25 * (1.0 + g));
+        // J's first row depends on eta only, its second on xi only
+        const T x10 = x[1] - x[0], x23 = x[2] - x[3], x30 = x[3] - x[0], x21 = x[2] - x[1];
+        const T y10 = y[1] - y[0], y23 = y[2] - y[3], y30 = y[3] - y[0], y21 = y[2] - y[1];
+        T k[4][4];
+#pragma unroll
+        for (int b = 0; b < 4; b++)
+#pragma unroll
+            for (int v = 0; v < 4; v++) k[b][v] = T(0);
+        T min_det = sizeof(T) == 8 ? T(1e300) : T(3.0e38f);
+#pragma unroll 1
+        for (int gi = 0; gi < 2; gi++) {      // xi = -g, g
+            const T xm = gi ? lo : hi, xp = gi ? hi : lo;  // (1 - xi) / 4, (1 + xi) / 4
+            const T j2 = fma(xm, x30, xp * x21), j3 = fma(xm, y30, xp * y21);
+#pragma unroll
+            for (int gj = 0; gj < 2; gj++) {  // eta = -g, g
+                const T em = gj ? lo : hi, ep = gj ? hi : lo;
+                const T j0 = fma(em, x10, ep * x23), j1 = fma(em, y10, ep * y23);
+                const T det = j0 * j3 - j1 * j2;
+                min_det = fmin(min_det, det);
+                const T dxi[4] = {-em, em, ep, -ep}, deta[4] = {-xm, -xp, xp, xm};
+                const T r = f / det;
+                T X[4], Y[4];
+#pragma unroll
+                for (int b = 0; b < 4; b++) {
+                    X[b] = fma(j3, dxi[b], -j1 * deta[b]);
+                    Y[b] = fma(j0, deta[b], -j2 * dxi[b]);
+                }
+                const T sx = r * X[0], sy = r * Y[0], hx = h * sx, hy = h * sy, nx = nu * sx, ny = nu * sy;
+#pragma unroll
+                for (int b = 0; b < 4; b++) {
+                    k[b][0] = fma(sx, X[b], fma(hy, Y[b], k[b][0]));
+                    k[b][1] = fma(nx, Y[b], fma(hy, X[b], k[b][1]));
+                    k[b][2] = fma(ny, X[b], fma(hx, Y[b], k[b][2]));
+                    k[b][3] = fma(sy, Y[b], fma(hx, X[b], k[b][3]));
+                }
+            }
+        }
+#pragma unroll
+        for (int b = 0; b < 4; b++)
+#pragma unroll
+            for (int v = 0; v < 4; v++) kv[b][v] = double(k[b][v]);
+        return double(min_det);
+    }
+}
+
 }  // namespace fem

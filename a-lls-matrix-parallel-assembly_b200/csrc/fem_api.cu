@@ -105,8 +105,8 @@ fem_status make_layout(const fem_mesh* m, const fem_opts* o, HostLayout& h) {
     off += align_up((size_t)h.N * sizeof(int));
     h.off_ucounts = off;  // upper-triangle column counts (fem_alls_consolidate_upper)
     off += align_up((size_t)h.N * sizeof(int));
-    h.off_tiles = off;
-    off += align_up((size_t)h.num_tiles * sizeof(long long));
+    h.off_tiles = off;  // scan partials: of kScanTile nodes in the batch, of kRowTile nodes otherwise
+    off += align_up((size_t)(h.dpn == 2 ? h.num_tiles : row_tiles(h.N)) * sizeof(long long));
     h.off_elist = off;  // visit order of the elements (perm), ranges, bucket histogram (+ bbox)
     {
         const size_t nbuckets = h.dpn == 2 ? (size_t)2 * reorder_buckets(h.N) : (size_t)1 << (3 * morton_bits(h.E));
@@ -233,16 +233,17 @@ fem_status fem_alls_scatter(const fem_mesh* mesh, const fem_opts* opts, void* wo
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     ListLayout L = device_layout(h, workspace);
     unsigned char* b = static_cast<unsigned char*>(workspace);
-    cudaError_t err = cudaMemsetAsync(b + h.off_info, 0, sizeof(DevInfo), s);
-    if (!err) err = launch_info_init(L.info, h.cap2, s);
+    MeshView m = mesh_view(mesh);
+    cudaError_t err = launch_lists_begin(L, s);
+    if (h.dpn == 2) {
+        // the long rows' queue takes the upper-triangle counts' place (written by a later call)
+        int* queue = reinterpret_cast<int*>(b + h.off_ucounts);
+        if (!err) err = launch_rows_2d(m, L, queue, h.kind, precision, ctas, s);
+        return err ? cuda_fail(err) : FEM_OK;
+    }
     if (!err) err = cudaMemsetAsync(b + h.off_meta1, 0, h.meta1_bytes, s);
-    if (!err) err = cudaMemsetAsync(b + h.off_counts, 0, (size_t)h.N * sizeof(int), s);
-    // 2-D lists accumulate every contribution with atomic adds: their first
-    // chunks' slot values start at zero (overflow chunks are zeroed when taken).
-    if (!err && h.dpn == 2) err = cudaMemsetAsync(b + h.off_vals, 0, (size_t)h.N * h.S1 * h.B * sizeof(double), s);
     if (err) return cuda_fail(err);
     if (h.E == 0) return FEM_OK;
-    MeshView m = mesh_view(mesh);
     int* perm = reinterpret_cast<int*>(b + h.off_elist);
     int* ranges = reinterpret_cast<int*>(b + h.off_elist + align_up((size_t)h.E * sizeof(int)));
     int* hist = reinterpret_cast<int*>(b + h.off_elist + align_up((size_t)h.E * sizeof(int)) + align_up(4 * sizeof(int)));
@@ -269,10 +270,6 @@ fem_status fem_alls_scatter(const fem_mesh* mesh, const fem_opts* opts, void* wo
             err = launch_claim_hex20(m, L, perm, inc_off, inc, i0, i1, map, s);
             if (!err) err = launch_values_hex20(m, L, precision, perm, i0, i1, map, stage, wait_ns, s);
         }
-    } else {
-        err = launch_reorder(m, hist, ranges, perm, sm_count(), s);
-        if (!err && h.kind != FEM_T3) err = launch_scatter_2d(m, L, 4, precision, perm, ranges + 0, ctas, s);
-        if (!err && h.kind != FEM_Q4) err = launch_scatter_2d(m, L, 3, precision, perm, ranges + 2, ctas, s);
     }
     return err ? cuda_fail(err) : FEM_OK;
 }
@@ -287,7 +284,7 @@ fem_status fem_alls_consolidate(const fem_mesh* mesh, const fem_opts* opts, void
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     ListLayout L = device_layout(h, workspace);
     long long* tiles = reinterpret_cast<long long*>(static_cast<unsigned char*>(workspace) + h.off_tiles);
-    cudaError_t err = launch_consolidate(L, h.dpn, row_ptr, col_idx, values, capacity, tiles, h.num_tiles, s);
+    cudaError_t err = launch_consolidate(L, h.dpn, row_ptr, col_idx, values, capacity, tiles, s);
     return err ? cuda_fail(err) : FEM_OK;
 }
 
@@ -304,7 +301,7 @@ fem_status fem_alls_consolidate_bsr(const fem_mesh* mesh, const fem_opts* opts, 
     ListLayout L = device_layout(h, workspace);
     long long* tiles = reinterpret_cast<long long*>(static_cast<unsigned char*>(workspace) + h.off_tiles);
     cudaError_t err = launch_consolidate_bsr(L, h.dpn, block_row_ptr, block_col_idx, block_values, capacity_blocks,
-                                             tiles, h.num_tiles, s);
+                                             tiles, s);
     return err ? cuda_fail(err) : FEM_OK;
 }
 
@@ -322,7 +319,7 @@ fem_status fem_alls_consolidate_upper(const fem_mesh* mesh, const fem_opts* opts
     long long* tiles = reinterpret_cast<long long*>(b + h.off_tiles);
     int* ucounts = reinterpret_cast<int*>(b + h.off_ucounts);
     cudaError_t err =
-        launch_consolidate_upper(L, h.dpn, ucounts, row_ptr, col_idx, values, capacity, tiles, h.num_tiles, s);
+        launch_consolidate_upper(L, h.dpn, ucounts, row_ptr, col_idx, values, capacity, tiles, s);
     return err ? cuda_fail(err) : FEM_OK;
 }
 

@@ -9,7 +9,7 @@
 // (row node, column node) pair, so the dpn rows of a node share one list.
 //
 // Chunk metadata is a row of H = S + 2 int32 words:
-//     word 0 = reserved (0)
+//     word 0 = kRowSorted for a 2-D row stored sorted and compact, else 0
 //     word 1 = next  (chunk id + 1 of the next chunk, 0 = none)
 //     word 2+s = slot s: 0 = empty, col+1 = column node col
 // Within a chunk a column's slot is found by open addressing (linear probing
@@ -34,6 +34,8 @@ namespace fem {
 
 constexpr int kBlockThreads = 256;
 constexpr int kScanTile = 4096;  // nodes per scan tile (256 threads x 16)
+constexpr int kRowTile = 1024;   // nodes per tile of the consolidation's row pointers
+inline int row_tiles(int num_nodes) { return (num_nodes + kRowTile - 1) / kRowTile; }
 
 // Device-resident info word; its first bytes are laid out exactly as fem_info.
 struct DevInfo {
@@ -43,7 +45,7 @@ struct DevInfo {
     int overflow_chunks;   // overflow-pool bump counter (may overshoot the capacity)
     int pool_chunks;
     int max_row_entries;
-    int tile_ticket;       // consolidation tile dispenser
+    int long_rows;         // 2-D: rows left to k_long_rows_2d
     int pad0;
     long long pad1[3];
 };
@@ -126,6 +128,11 @@ __device__ __forceinline__ int alloc_chunk(const ListLayout& L) {
 constexpr int kMaxChainSteps = 1 << 20;
 
 constexpr int kColMask = 0x7FFFFFFF;
+
+// Header word (word 0) of a 2-D first chunk whose row is complete in it: its
+// columns fill the first slots in increasing order (no next chunk). 0: the
+// row is hashed (fans, and the batched kernel's rows).
+constexpr int kRowSorted = 1;
 
 // Start of the probe sequence of column key `key` (col + 1) in a chunk of S slots.
 __device__ __forceinline__ int probe_start(int key, int S) {

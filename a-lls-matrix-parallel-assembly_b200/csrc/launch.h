@@ -51,11 +51,13 @@ struct MeshView {
 // 2-D chunk rows are 16 int32 words (14 slots + fill + next).
 constexpr int k2DSlots = 14;
 
-// perm: element visit order; range: device ints {begin, end} into perm;
+// Clears the per-node counters and the info word of a scatter.
+cudaError_t launch_lists_begin(const ListLayout& L, cudaStream_t s);
+// The row lists of a 2-D mesh (rows2d.cu), after launch_lists_begin;
 // precision FEM_PREC_FP64 or FEM_PREC_FP32 (the arithmetic of the Ke blocks).
-// ctas_per_sm: cap on the persistent grid's resident CTAs per SM (0 = all that fit).
-cudaError_t launch_scatter_2d(const MeshView& m, const ListLayout& L, int npe, int precision, const int* perm,
-                              const int* range, int ctas_per_sm, cudaStream_t s);
+// queue: N ints of scratch; ctas_per_sm: cap on the persistent grid's resident CTAs per SM (0 = all that fit).
+cudaError_t launch_rows_2d(const MeshView& m, const ListLayout& L, int* queue, int kind, int precision,
+                           int ctas_per_sm, cudaStream_t s);
 // Node-local element order (perm) and the element ranges {q4 begin, q4 end, t3 begin, t3 end}.
 int reorder_buckets(int num_nodes);
 cudaError_t launch_reorder(const MeshView& m, int* hist, int* ranges, int* perm, int sms, cudaStream_t s);
@@ -138,17 +140,17 @@ static_assert(kBatchHex20Wave <= kHex20Wave, "the batched ring's first map is th
 int morton_bits(int num_elems);
 cudaError_t launch_reorder_3d(const MeshView& m, int* hist, int* ranges, int* perm, unsigned long long* bbox, int sms,
                               cudaStream_t s);
+// tile_sums: row_tiles(N) partials of scratch.
 cudaError_t launch_consolidate(const ListLayout& L, int dpn, int* row_ptr, int* col_idx, double* values,
-                               long long capacity, long long* tile_sums, int num_tiles, cudaStream_t s);
+                               long long capacity, long long* tile_sums, cudaStream_t s);
 // Node-block (BSR) form of the consolidation; capacity in blocks.
 // Upper triangle (columns >= row, diagonal included) in CSR; ucounts: N ints of scratch.
 cudaError_t launch_consolidate_upper(const ListLayout& L, int dpn, int* ucounts, int* row_ptr, int* col_idx,
-                                     double* values, long long capacity, long long* tile_sums, int num_tiles,
+                                     double* values, long long capacity, long long* tile_sums,
                                      cudaStream_t s);
 cudaError_t launch_consolidate_bsr(const ListLayout& L, int dpn, int* block_row_ptr, int* block_col_idx,
                                    double* block_values, long long capacity_blocks, long long* tile_sums,
-                                   int num_tiles, cudaStream_t s);
-cudaError_t launch_info_init(DevInfo* info, int pool_chunks, cudaStream_t s);
+                                   cudaStream_t s);
 
 // ---- load vector and boundary conditions (loads.cu) ----
 // f += body-force load vector (b: device [E * dim] or NULL for the uniform b0[dim], host values).

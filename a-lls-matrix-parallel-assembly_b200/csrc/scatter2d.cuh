@@ -1,5 +1,26 @@
-// Device code of the 2-D A-LLS scatter (scatter2d.cu), shared with the
-// batched persistent kernel (batched.cu). See scatter2d.cu for the method.
+// Device code of the hashed 2-D A-LLS insertion: the long rows of rows2d.cu
+// (resolve_2d) and the scatter items of the batched persistent kernel
+// (batched.cu, scatter2d_warp).
+//
+// scatter2d_warp: one LANE serves one node block (a, b) of one element, NPE^2
+// lanes per element (T3: 9 lanes, 3 elements per warp; Q4: 16 lanes, 2 per
+// warp). It computes its 2x2 block K_ab (element2d.cuh), reads row node a's
+// 64-byte first chunk (next pointer and 14 hashed slots) with four 16-byte L2
+// loads and looks for column node b in it. An absent column is claimed with
+// atomicCAS(empty -> col) at the first empty slot of its probe sequence; a CAS
+// that meets another column marks that slot taken in the lane's view and moves
+// on along the sequence (slots are never freed, so a column is always found or
+// placed at the first empty slot of its sequence, never twice). A chunk whose
+// probe sequence is full continues in an overflow chunk (allocated from the
+// pool with zeroed values, linked by CAS). The values of every slot start at
+// zero, so the claimer and every later contributor alike add their block with
+// FP64 red.add: the claim publishes the column at once, with no pending state,
+// no fence and no waiting on another thread. The warp transposes its blocks
+// through shared memory so that each red instruction covers eight whole
+// 32-byte blocks instead of 32 scattered sectors. Claims are counted per
+// (element, row) group with one atomic per group. The reference's head insert
+// can lose a contribution or insert a column twice (Q4A:452-463); the
+// claim/publish protocol here does neither.
 #pragma once
 
 #include "element2d.cuh"
@@ -22,6 +43,8 @@ __device__ __forceinline__ unsigned rot14(unsigned m, int h) {
 // the slot's global id.
 // view: the row's first chunk, loaded by the caller (possibly some time ago:
 // a stale view only costs failed CASes, never a wrong slot).
+// kAlloc false: a column that needs a further chunk is left kUnresolved.
+template <bool kAlloc = true>
 __device__ __forceinline__ int resolve_2d(const ListLayout& L, int row, int key, const int4 (&view)[4], int& spare,
                                           unsigned& gid) {
     int c = row;
@@ -69,8 +92,13 @@ __device__ __forceinline__ int resolve_2d(const ListLayout& L, int row, int key,
             gid = slot_gid(L, c, pos);
             return state;
         }
-        c = next_chunk<true>(L, c, spare);
-        if (c < 0) return kSkip;  // pool overflow: status raised, the block is dropped
+        if constexpr (kAlloc) {
+            c = next_chunk<true>(L, c, spare);
+            if (c < 0) return kSkip;  // pool overflow: status raised, the block is dropped
+        } else {
+            c = ld_cg(meta + 1) - 1;
+            if (c < 0) return kUnresolved;
+        }
     }
     raise_status(L.info, FEM_ERR_TIMEOUT);
     return kSkip;
@@ -86,14 +114,6 @@ __device__ __forceinline__ int element_of(const MeshView& m, const int* perm, in
     if (valid && want_type >= 0) valid = FEM_LDG(m.types + e) == want_type;
     return e;
 }
-
-// Resident CTAs per SM the register budget is set for (build-time tuning knobs).
-#ifndef FEM_T3_MIN_CTAS
-#define FEM_T3_MIN_CTAS 4
-#endif
-#ifndef FEM_Q4_MIN_CTAS
-#define FEM_Q4_MIN_CTAS 2
-#endif
 
 // Warp-level shared memory of the 2-D scatter: the warp's blocks and slot ids,
 // transposed so that each red instruction covers whole 32-byte blocks.

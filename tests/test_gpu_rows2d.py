@@ -1,0 +1,87 @@
+"""The thread-per-node row lists of the 2-D kinds (rows2d.cu) at the sizes where
+they change path, through the C ABI against the oracle: rows at the limits of
+the shared-memory sums (8 columns besides the diagonal), of the chunk (14
+columns, 14 elements) and of the element list kept in the row's own storage
+(126 elements); node counts around a CTA's 64; elements with a repeated node;
+output buffers that are not aligned for the wide copy. Pattern bit for bit,
+values within 1e-12 of max(|K_ij|, sqrt(|K_ii K_jj|))."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from conftest import diag_scale
+
+pytestmark = pytest.mark.gpu
+
+RTOL = 1e-12
+
+
+def _compare(oracle_mod, m, rp, ci, v, rtol=RTOL):
+    orp, oci, ov = oracle_mod.assemble(m)
+    np.testing.assert_array_equal(rp, orp)
+    np.testing.assert_array_equal(ci, oci)
+    scale = np.maximum(np.abs(ov), diag_scale(orp, oci, ov))
+    assert np.all(np.abs(v - ov) <= rtol * scale)
+
+
+def _fan(k, closed):
+    import meshgen as mg
+    n = k if closed else k + 1
+    ang = np.linspace(0, 2 * np.pi, n, endpoint=False)
+    x = np.concatenate([[0.0], np.cos(ang)])
+    y = np.concatenate([[0.0], np.sin(ang)])
+    conn = np.array([[0, 1 + i, 1 + (i + 1) % n] for i in range(k)], np.int32)
+    conn = np.random.default_rng(k).permutation(conn)
+    return mg.Mesh(mg.T3, x, y, None, np.ascontiguousarray(conn), None, None, None, E0=1.0, nu0=0.3)
+
+
+@pytest.mark.parametrize("k", [3, 7, 8, 9, 12, 13, 14, 15, 16, 125, 126, 127, 200])
+@pytest.mark.parametrize("closed", [True, False])
+def test_fans(fem, oracle_mod, cuda_device, k, closed):
+    m = _fan(k, closed)
+    rp, ci, v, info = fem.assemble(m)
+    _compare(oracle_mod, m, rp, ci, v)
+    cols = k + 1 if closed else k + 2
+    assert info["max_row_entries"] == cols
+    assert info["overflow_chunks"] == max(0, -(-(cols - 14) // 14))
+
+
+@pytest.mark.parametrize("nx,ny", [(1, 1), (6, 8), (62, 1), (7, 7), (63, 1), (64, 1), (15, 7), (128, 3)])
+@pytest.mark.parametrize("kind", ["q4", "t3", "mixed"])
+def test_node_counts_around_a_tile(fem, oracle_mod, cuda_device, kind, nx, ny):
+    import meshgen as mg
+    m = {"q4": mg.q4_grid, "t3": mg.t3_grid, "mixed": mg.mixed_grid}[kind](nx, ny, seed=nx + ny)
+    rp, ci, v, _ = fem.assemble(m)
+    _compare(oracle_mod, m, rp, ci, v)
+
+
+@pytest.mark.parametrize("precision", [0, 3])
+def test_repeated_nodes(fem, oracle_mod, cuda_device, precision):
+    # quads collapsed to triangles at each of their four positions in turn
+    import meshgen as mg
+    m = mg.q4_grid(9, 7, seed=3)
+    conn = m.conn.copy()
+    for e in range(0, conn.shape[0], 3):
+        k = (e // 3) % 4
+        conn[e, k] = conn[e, (k + 1) % 4]
+    m.conn = conn
+    rp, ci, v, _ = fem.assemble(m, fem.opts(precision=precision))
+    _compare(oracle_mod, m, rp, ci, v, 1e-5 if precision else RTOL)
+
+
+@pytest.mark.parametrize("off_v,off_c", [(1, 0), (0, 1), (1, 1)])
+def test_outputs_off_the_wide_alignment(fem, oracle_mod, cuda_device, off_v, off_c):
+    import torch
+    import meshgen as mg
+    m = mg.by_name("mixed_small")
+    a = fem.Assembler(m)
+    nnz = int(a.assemble()[3].nnz)
+    ci = torch.full((nnz + 2,), -7, dtype=torch.int32, device="cuda")
+    v = torch.full((nnz + 2,), 7.0, dtype=torch.float64, device="cuda")
+    out = fem.FemCsr(m.num_dofs, 0, 0, nnz, a.row_ptr.data_ptr(), ci[off_c:].data_ptr(), v[off_v:].data_ptr())
+    st = fem.load().fem_assemble(C.byref(a.cm), None, C.c_void_p(a.ws_ptr), a.ws_bytes, C.byref(out), None)
+    assert st == 0 and out.nnz == nnz
+    _compare(oracle_mod, m, a.row_ptr.cpu().numpy(), ci[off_c:off_c + nnz].cpu().numpy(),
+             v[off_v:off_v + nnz].cpu().numpy())
+    assert v[off_v + nnz].item() == 7.0 and ci[off_c + nnz].item() == -7
