@@ -14,7 +14,9 @@
 //                  of the counts -> row_ptr of all dpn rows; nnz, capacity check
 //   k_write_sorted_2d  2-D CSR: the scatter's rows are sorted, so this copies
 //                  each node's blocks into its two CSR rows
-//   k_write        the other forms: a group of G lanes per row node: gather the node's non-empty
+//   k_write_hex20  Hex20: the rows are sorted, their values summed from the
+//                  elements' Ke as they are written (write_hex20.cu)
+//   k_write        the other 2-D forms: a group of G lanes per row node: gather the node's non-empty
 //                  hashed slots as 64-bit keys (col << 32 | slot), bitonic sort
 //                  across the group, then write each dof row's entries
 //                  (col*dpn + b, block value) with consecutive lanes on
@@ -227,17 +229,20 @@ long long write_grid(long long batches) {
 
 // counts: list columns per node (kOutUpper: columns >= the node); capacity in
 // scalar entries (BSR: blocks * dpn^2).
-template <int DPN, int G, int KPL, int kMode>
-cudaError_t launch_mode(const ListLayout& L, const int* counts, int* row_ptr, int* col_idx, double* values,
-                        long long capacity, long long* tile_sums, cudaStream_t s) {
+template <int DPN, int kMode>
+cudaError_t launch_mode(const ListLayout& L, const HexRows& hex, const int* counts, int* row_ptr, int* col_idx,
+                        double* values, long long capacity, long long* tile_sums, cudaStream_t s) {
     const int tiles = row_tiles(L.N);
     k_tile_entries<DPN, kMode><<<tiles, kScanThreads, 0, s>>>(counts, L.N, tile_sums);
     k_row_ptr<DPN, kMode><<<tiles, kScanThreads, 0, s>>>(counts, L.N, tile_sums, row_ptr, L.info, capacity);
-    if (capacity > 0) {
+    if (capacity <= 0) return cudaGetLastError();
+    if constexpr (DPN == 3) {
+        return launch_write_hex20(L, hex, kMode, counts, row_ptr, col_idx, values, capacity, s);
+    } else {
         // the copy kernel's 16-byte value and 8-byte column stores need outputs aligned to them (row starts are
         // multiples of 4 entries); other outputs take k_write, which stores entry by entry
         const bool wide = reinterpret_cast<uintptr_t>(values) % 16 == 0 && reinterpret_cast<uintptr_t>(col_idx) % 8 == 0;
-        if (DPN == 2 && kMode == kOutCsr && wide) {
+        if (kMode == kOutCsr && wide) {
             static DeviceCache cache;
             int per_sm = 0;
             if (per_device(cache, [](int& v) {
@@ -249,48 +254,45 @@ cudaError_t launch_mode(const ListLayout& L, const int* counts, int* row_ptr, in
             const int grid = (int)std::min<long long>(want, (long long)per_sm * sm_count());
             k_write_sorted_2d<<<grid, kBlockThreads, 0, s>>>(L, row_ptr, col_idx, values, capacity);
         } else {
-            constexpr int NPB = kBlockThreads / G;
+            constexpr int G = 8, NPB = kBlockThreads / G;
             const long long batches = ((long long)L.N + NPB - 1) / NPB;
-            k_write<DPN, G, KPL, kMode><<<(int)write_grid<DPN, G, KPL, kMode>(batches), kBlockThreads, 0, s>>>(
+            k_write<DPN, G, 2, kMode><<<(int)write_grid<DPN, G, 2, kMode>(batches), kBlockThreads, 0, s>>>(
                 L, row_ptr, col_idx, values, capacity, counts);
         }
+        return cudaGetLastError();
     }
-    return cudaGetLastError();
-}
-
-template <int DPN, int G, int KPL>
-cudaError_t launch_upper(const ListLayout& L, int* ucounts, int* row_ptr, int* col_idx, double* values,
-                         long long capacity, long long* tile_sums, cudaStream_t s) {
-    constexpr int NPB = kBlockThreads / G;
-    const long long batches = ((long long)L.N + NPB - 1) / NPB;
-    const int grid = (int)std::max<long long>(1, std::min<long long>(batches, (long long)sm_count() * 8));
-    k_count_upper<G><<<grid, kBlockThreads, 0, s>>>(L, ucounts);
-    return launch_mode<DPN, G, KPL, kOutUpper>(L, ucounts, row_ptr, col_idx, values, capacity, tile_sums, s);
 }
 
 }  // namespace
 
-cudaError_t launch_consolidate(const ListLayout& L, int dpn, int* row_ptr, int* col_idx, double* values,
-                               long long capacity, long long* tile_sums, cudaStream_t s) {
-    if (dpn == 3)
-        return launch_mode<3, 32, 4, kOutCsr>(L, L.counts, row_ptr, col_idx, values, capacity, tile_sums, s);
-    return launch_mode<2, 8, 2, kOutCsr>(L, L.counts, row_ptr, col_idx, values, capacity, tile_sums, s);
+cudaError_t launch_consolidate(const ListLayout& L, int dpn, const HexRows& hex, int* row_ptr, int* col_idx,
+                               double* values, long long capacity, long long* tile_sums, cudaStream_t s) {
+    if (dpn == 3) return launch_mode<3, kOutCsr>(L, hex, L.counts, row_ptr, col_idx, values, capacity, tile_sums, s);
+    return launch_mode<2, kOutCsr>(L, hex, L.counts, row_ptr, col_idx, values, capacity, tile_sums, s);
 }
 
-cudaError_t launch_consolidate_upper(const ListLayout& L, int dpn, int* ucounts, int* row_ptr, int* col_idx,
-                                     double* values, long long capacity, long long* tile_sums, cudaStream_t s) {
-    if (dpn == 3) return launch_upper<3, 32, 4>(L, ucounts, row_ptr, col_idx, values, capacity, tile_sums, s);
-    return launch_upper<2, 8, 2>(L, ucounts, row_ptr, col_idx, values, capacity, tile_sums, s);
+cudaError_t launch_consolidate_upper(const ListLayout& L, int dpn, const HexRows& hex, int* ucounts, int* row_ptr,
+                                     int* col_idx, double* values, long long capacity, long long* tile_sums,
+                                     cudaStream_t s) {
+    if (dpn == 3) {
+        const cudaError_t err = launch_count_upper_hex20(L, ucounts, s);
+        if (err) return err;
+        return launch_mode<3, kOutUpper>(L, hex, ucounts, row_ptr, col_idx, values, capacity, tile_sums, s);
+    }
+    constexpr int G = 8, NPB = kBlockThreads / G;
+    const long long batches = ((long long)L.N + NPB - 1) / NPB;
+    const int grid = (int)std::max<long long>(1, std::min<long long>(batches, (long long)sm_count() * 8));
+    k_count_upper<G><<<grid, kBlockThreads, 0, s>>>(L, ucounts);
+    return launch_mode<2, kOutUpper>(L, hex, ucounts, row_ptr, col_idx, values, capacity, tile_sums, s);
 }
 
-cudaError_t launch_consolidate_bsr(const ListLayout& L, int dpn, int* block_row_ptr, int* block_col_idx,
-                                   double* block_values, long long capacity_blocks, long long* tile_sums,
-                                   cudaStream_t s) {
+cudaError_t launch_consolidate_bsr(const ListLayout& L, int dpn, const HexRows& hex, int* block_row_ptr,
+                                   int* block_col_idx, double* block_values, long long capacity_blocks,
+                                   long long* tile_sums, cudaStream_t s) {
     const long long cap = capacity_blocks * dpn * dpn;
     if (dpn == 3)
-        return launch_mode<3, 32, 4, kOutBsr>(L, L.counts, block_row_ptr, block_col_idx, block_values, cap, tile_sums,
-                                              s);
-    return launch_mode<2, 8, 2, kOutBsr>(L, L.counts, block_row_ptr, block_col_idx, block_values, cap, tile_sums, s);
+        return launch_mode<3, kOutBsr>(L, hex, L.counts, block_row_ptr, block_col_idx, block_values, cap, tile_sums, s);
+    return launch_mode<2, kOutBsr>(L, hex, L.counts, block_row_ptr, block_col_idx, block_values, cap, tile_sums, s);
 }
 
 }  // namespace fem

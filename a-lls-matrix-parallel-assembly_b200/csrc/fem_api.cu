@@ -54,8 +54,8 @@ fem_status check_mesh(const fem_mesh* m, bool device_pointers_needed = true) {
     return FEM_OK;
 }
 
-// Group records of one wave (of `wave` elements) of the Hex20 scatter for a mesh of E elements.
-size_t hex20_map_bytes(int E, int wave = kHex20Wave) {
+// Group records of one wave (of `wave` elements) of the batched Hex20 scatter for a mesh of E elements.
+size_t hex20_map_bytes(int E, int wave) {
     const size_t groups = ((size_t)std::min(E, wave) + kHex20GroupSize - 1) / kHex20GroupSize;
     return groups * kHex20GroupRecWords * sizeof(unsigned);
 }
@@ -99,8 +99,12 @@ fem_status make_layout(const fem_mesh* m, const fem_opts* o, HostLayout& h) {
     off += align_up(h.meta1_bytes);
     h.off_meta2 = off;
     off += align_up((size_t)h.cap2 * h.H2 * sizeof(int));
+    // 2-D (and the batch): the slots' value blocks; a Hex20 mesh assembled on its own: the packed Ke of its
+    // elements, which take less (15.1 KB an element, about 4 nodes of 7.8 KB) unless elements overlap
     h.off_vals = off;
-    off += align_up((size_t)slots * h.B * sizeof(double));
+    size_t vals_bytes = (size_t)slots * h.B * sizeof(double);
+    if (h.kind == FEM_HEX20) vals_bytes = std::max(vals_bytes, (size_t)h.E * kPackedHex20 * sizeof(double));
+    off += align_up(vals_bytes);
     h.off_counts = off;
     off += align_up((size_t)h.N * sizeof(int));
     h.off_ucounts = off;  // upper-triangle column counts (fem_alls_consolidate_upper)
@@ -113,17 +117,14 @@ fem_status make_layout(const fem_mesh* m, const fem_opts* o, HostLayout& h) {
         off += align_up((size_t)h.E * sizeof(int)) + align_up(4 * sizeof(int)) + align_up(nbuckets * sizeof(int)) +
                align_up(6 * sizeof(unsigned long long));
     }
-    // Hex20: node -> element incidence (counts, offsets, lists), the map
-    // records of one wave of the two-pass scatter, and (tensor-core form) the
-    // staged Ke of one wave
+    // Hex20: node -> occurrences (counts, offsets, lists) and the rank map of the rows (in the batch: the group
+    // records of one wave)
     h.off_inc = off;
     if (h.kind == FEM_HEX20)
         off += 2 * align_up((size_t)(h.N + 1) * sizeof(int)) + align_up((size_t)h.E * 20 * sizeof(int));
     h.off_map = off;
-    if (h.kind == FEM_HEX20) off += align_up(hex20_map_bytes(h.E));
-    h.off_stage = off;
-    if (h.kind == FEM_HEX20 && o->precision == FEM_PREC_TC_F16X3)
-        off += align_up((size_t)std::min(h.E, kHex20Wave) * kPackedHex20 * sizeof(double));
+    if (h.kind == FEM_HEX20)
+        off += align_up(std::max(hex20_map_bytes(h.E, 32768), (size_t)h.E * 400 * sizeof(unsigned short)));
     h.total = off;
     return FEM_OK;
 }
@@ -144,6 +145,18 @@ ListLayout device_layout(const HostLayout& h, void* ws) {
     L.counts = reinterpret_cast<int*>(b + h.off_counts);
     L.info = reinterpret_cast<DevInfo*>(b + h.off_info);
     return L;
+}
+
+HexRows hex_rows(const HostLayout& h, void* ws) {
+    unsigned char* b = static_cast<unsigned char*>(ws);
+    HexRows r{};
+    if (h.kind != FEM_HEX20) return r;
+    const size_t n = align_up((size_t)(h.N + 1) * sizeof(int));
+    r.ke = reinterpret_cast<double*>(b + h.off_vals);
+    r.off = reinterpret_cast<int*>(b + h.off_inc + n);
+    r.inc = reinterpret_cast<int*>(b + h.off_inc + 2 * n);
+    r.map = reinterpret_cast<unsigned short*>(b + h.off_map);
+    return r;
 }
 
 MeshView mesh_view(const fem_mesh* m) {
@@ -235,42 +248,20 @@ fem_status fem_alls_scatter(const fem_mesh* mesh, const fem_opts* opts, void* wo
     unsigned char* b = static_cast<unsigned char*>(workspace);
     MeshView m = mesh_view(mesh);
     cudaError_t err = launch_lists_begin(L, s);
+    // the long rows' queue takes the upper-triangle counts' place (written by a later call)
+    int* queue = reinterpret_cast<int*>(b + h.off_ucounts);
     if (h.dpn == 2) {
-        // the long rows' queue takes the upper-triangle counts' place (written by a later call)
-        int* queue = reinterpret_cast<int*>(b + h.off_ucounts);
         if (!err) err = launch_rows_2d(m, L, queue, h.kind, precision, ctas, s);
         return err ? cuda_fail(err) : FEM_OK;
     }
-    if (!err) err = cudaMemsetAsync(b + h.off_meta1, 0, h.meta1_bytes, s);
-    if (err) return cuda_fail(err);
-    if (h.E == 0) return FEM_OK;
-    int* perm = reinterpret_cast<int*>(b + h.off_elist);
-    int* ranges = reinterpret_cast<int*>(b + h.off_elist + align_up((size_t)h.E * sizeof(int)));
-    int* hist = reinterpret_cast<int*>(b + h.off_elist + align_up((size_t)h.E * sizeof(int)) + align_up(4 * sizeof(int)));
-    if (h.kind == FEM_HEX20) {
-        const size_t nbuckets = (size_t)1 << (3 * morton_bits(h.E));
-        unsigned long long* bbox = reinterpret_cast<unsigned long long*>(
-            b + h.off_elist + align_up((size_t)h.E * sizeof(int)) + align_up(4 * sizeof(int)) +
-            align_up(nbuckets * sizeof(int)));
-        err = launch_reorder_3d(m, hist, ranges, perm, bbox, sm_count(), s);
-        // two-pass scatter in waves of the spatial order: a wave's claims
-        // (entries, zeroed value blocks, map records) complete before its
-        // value pass, and the blocks it touches are still in L2 when the
-        // values arrive
-        int* inc_cnt = reinterpret_cast<int*>(b + h.off_inc);
-        int* inc_off = inc_cnt + align_up((size_t)(h.N + 1) * sizeof(int)) / sizeof(int);
-        int* inc = inc_off + align_up((size_t)(h.N + 1) * sizeof(int)) / sizeof(int);
-        int* map = reinterpret_cast<int*>(b + h.off_map);
-        double* stage = reinterpret_cast<double*>(b + h.off_stage);
-        long long* tiles = reinterpret_cast<long long*>(b + h.off_tiles);  // free until the consolidation
-        const long long wait_ns = wait_ns_of(opts ? opts->wait_limit_us : 0);
-        if (!err) err = launch_incidence(m, inc_cnt, inc_off, inc, tiles, &L.info->status_bits, sm_count(), s);
-        for (int i0 = 0; i0 < h.E && !err; i0 += kHex20Wave) {
-            const int i1 = std::min(h.E, i0 + kHex20Wave);
-            err = launch_claim_hex20(m, L, perm, inc_off, inc, i0, i1, map, s);
-            if (!err) err = launch_values_hex20(m, L, precision, perm, i0, i1, map, stage, wait_ns, s);
-        }
-    }
+    const HexRows hex = hex_rows(h, workspace);
+    int* cnt = reinterpret_cast<int*>(b + h.off_inc);
+    long long* tiles = reinterpret_cast<long long*>(b + h.off_tiles);  // free until the consolidation
+    if (!err) err = launch_occurrences(m, cnt, hex.off, hex.inc, tiles, &L.info->status_bits, sm_count(), s);
+    if (!err) err = launch_rows_hex20(m, L, hex, queue, s);
+    if (!err)
+        err = launch_element_stiffness(m, FEM_HEX20, precision, hex.ke, &L.info->status_bits,
+                                       wait_ns_of(opts ? opts->wait_limit_us : 0), s);
     return err ? cuda_fail(err) : FEM_OK;
 }
 
@@ -284,7 +275,7 @@ fem_status fem_alls_consolidate(const fem_mesh* mesh, const fem_opts* opts, void
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     ListLayout L = device_layout(h, workspace);
     long long* tiles = reinterpret_cast<long long*>(static_cast<unsigned char*>(workspace) + h.off_tiles);
-    cudaError_t err = launch_consolidate(L, h.dpn, row_ptr, col_idx, values, capacity, tiles, s);
+    cudaError_t err = launch_consolidate(L, h.dpn, hex_rows(h, workspace), row_ptr, col_idx, values, capacity, tiles, s);
     return err ? cuda_fail(err) : FEM_OK;
 }
 
@@ -300,7 +291,7 @@ fem_status fem_alls_consolidate_bsr(const fem_mesh* mesh, const fem_opts* opts, 
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     ListLayout L = device_layout(h, workspace);
     long long* tiles = reinterpret_cast<long long*>(static_cast<unsigned char*>(workspace) + h.off_tiles);
-    cudaError_t err = launch_consolidate_bsr(L, h.dpn, block_row_ptr, block_col_idx, block_values, capacity_blocks,
+    cudaError_t err = launch_consolidate_bsr(L, h.dpn, hex_rows(h, workspace), block_row_ptr, block_col_idx, block_values, capacity_blocks,
                                              tiles, s);
     return err ? cuda_fail(err) : FEM_OK;
 }
@@ -319,7 +310,7 @@ fem_status fem_alls_consolidate_upper(const fem_mesh* mesh, const fem_opts* opts
     long long* tiles = reinterpret_cast<long long*>(b + h.off_tiles);
     int* ucounts = reinterpret_cast<int*>(b + h.off_ucounts);
     cudaError_t err =
-        launch_consolidate_upper(L, h.dpn, ucounts, row_ptr, col_idx, values, capacity, tiles, s);
+        launch_consolidate_upper(L, h.dpn, hex_rows(h, workspace), ucounts, row_ptr, col_idx, values, capacity, tiles, s);
     return err ? cuda_fail(err) : FEM_OK;
 }
 

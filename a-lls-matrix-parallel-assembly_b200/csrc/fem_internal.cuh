@@ -45,7 +45,7 @@ struct DevInfo {
     int overflow_chunks;   // overflow-pool bump counter (may overshoot the capacity)
     int pool_chunks;
     int max_row_entries;
-    int long_rows;         // 2-D: rows left to k_long_rows_2d
+    int long_rows;         // rows queued for the long-row kernels
     int pad0;
     long long pad1[3];
 };
@@ -168,7 +168,7 @@ struct HostLayout {
     int S1, S2, H1, H2, cap2;
     int num_tiles;  // scan tiles of kScanTile nodes
     size_t off_info, off_meta1, off_meta2, off_vals, off_counts, off_ucounts, off_tiles, off_elist, off_inc, off_map,
-        off_stage, total;
+        total;
     size_t meta1_bytes;
 };
 

@@ -57,7 +57,7 @@ static_assert(kGroupPairs <= kTabPair + 1, "pair index in 11 bits");
 static_assert(kRecCpos % 4 == 0 && kRecCofs % 4 == 0 && kRecMap % 4 == 0 && kGroupRecWords % 4 == 0, "16-byte sections");
 static_assert(kGroup * 210 <= kPosMask + 1, "block position in 11 bits");
 static_assert(kGroup == kHex20GroupSize && kGroupRecWords == kHex20GroupRecWords, "host-side sizes");
-static_assert(kHex20Wave % kGroup == 0 && kBatchHex20Wave % kGroup == 0, "waves of whole groups");
+static_assert(kBatchHex20Wave % kGroup == 0, "waves of whole groups");
 
 // Whether a map word names a slot (slot ids are below 2^31 - 1: the layout
 // keeps the slot count below 2^31).

@@ -146,19 +146,16 @@ __device__ __forceinline__ unsigned pack_half2(__half lo, __half hi) {
 // Outputs of the kernel.
 enum TcOut : int {
     kTcPacked = 0,  // the packed Ke of every element to ke_out (fem_element_stiffness)
-    kTcWave = 1,    // the packed Ke of a wave's elements perm[i0, i1) to ke_out, row q - i0 for
-                    // position q (staging of the group value pass, values_hex20.cu)
     kTcCsrMap = 2   // value-only re-assembly: Ke_IJ and its transpose added with FP64 atomics at
                     // their CSR positions (scatter map, row e)
 };
 
-// Elements and targets of the kTcWave / kTcCsrMap modes.
+// Elements and targets of the kTcCsrMap mode.
 struct SlotTarget {
-    const int* perm;     // visit order: positions [i0, i1) (kTcWave), all elements (kTcCsrMap)
-    const int* map;      // scatter map, row e (kTcCsrMap)
-    const int* row_ptr;  // the CSR (kTcCsrMap)
+    const int* perm;     // visit order
+    const int* map;      // scatter map, row e
+    const int* row_ptr;  // the CSR
     double* csr;
-    int i0, i1;
     long long wait_ns;   // bound on the wait for the products (every mode)
 };
 
@@ -168,12 +165,12 @@ __global__ void __launch_bounds__(kThreads, 4) k_hex20_ke_tc(MeshView m, double*
     extern __shared__ __align__(128) unsigned char smem_raw[];
     KeTcSmem& sm = *reinterpret_cast<KeTcSmem*>(smem_raw);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    constexpr bool kWave = kMode == kTcWave, kMap = kMode == kTcCsrMap;
-    // elements: positions q of the wave (kTcWave), of perm (kTcCsrMap) or the mesh's elements q
-    const long long count = kWave ? (long long)(tgt.i1 - tgt.i0) : (long long)m.E_count;
+    constexpr bool kMap = kMode == kTcCsrMap;
+    // elements: positions q of perm (kTcCsrMap) or the mesh's elements q
+    const long long count = m.E_count;
     const long long npairs = (count + 1) / 2;
     auto elem = [&](long long q) -> long long {
-        return kWave ? (long long)__ldg(tgt.perm + tgt.i0 + q) : (kMap ? (long long)__ldg(tgt.perm + q) : q);
+        return kMap ? (long long)__ldg(tgt.perm + q) : q;
     };
     const uint32_t bar = smem_u32(&sm.mbar);
 
@@ -523,8 +520,7 @@ cudaError_t launch_tc(const MeshView& m, double* ke_out, int* status, const Slot
         return cudaSuccess;
     }, blocks_per_sm);
     if (err) return err;
-    const long long count = kMode == kTcWave ? (long long)(tgt.i1 - tgt.i0) : (long long)m.E_count;
-    const long long npairs = (count + 1) / 2;
+    const long long npairs = ((long long)m.E_count + 1) / 2;
     const long long grid = std::max<long long>(1, std::min<long long>((long long)blocks_per_sm * sm_count(), npairs));
     const int bulk_out = kMode != kTcCsrMap && (reinterpret_cast<uintptr_t>(ke_out) & 15u) == 0;
     k_hex20_ke_tc<kMode><<<(int)grid, kThreads, smem, s>>>(m, ke_out, status, bulk_out, tgt);
@@ -540,17 +536,10 @@ cudaError_t launch_hex20_ke_tcgen05(const MeshView& m, double* ke_out, int* stat
     return launch_tc<kTcPacked>(m, ke_out, status, t, s);
 }
 
-cudaError_t launch_stage_hex20_tc(const MeshView& m, const int* perm, int i0, int i1, double* stage, int* status,
-                                  long long wait_ns, cudaStream_t s) {
-    if (i1 <= i0) return cudaSuccess;
-    return launch_tc<kTcWave>(m, stage, status, SlotTarget{perm, nullptr, nullptr, nullptr, i0, i1, wait_ns}, s);
-}
-
 cudaError_t launch_reassemble_hex20_tc(const MeshView& m, const int* perm, const MapTarget& mt, DevInfo* info,
                                        cudaStream_t s) {
     return launch_tc<kTcCsrMap>(m, nullptr, &info->status_bits,
-                                SlotTarget{perm, mt.map, mt.row_ptr, mt.values, 0, m.E_count,
-                                           wait_ns_of(0)},
+                                SlotTarget{perm, mt.map, mt.row_ptr, mt.values, wait_ns_of(0)},
                                 s);
 }
 

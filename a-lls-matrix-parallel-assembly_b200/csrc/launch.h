@@ -108,47 +108,42 @@ cudaError_t launch_colour_hex20(const MeshView& m, const int* perm, const int* r
 // scratch; status gets 1 << FEM_ERR_* bits.
 cudaError_t launch_incidence(const MeshView& m, int* cnt, int* off, int* inc, long long* tiles, int* status, int sms,
                              cudaStream_t s);
-// Two-pass Hex20 list scatter over the element groups of positions
-// perm[i0, i1) (one wave; i0 a multiple of the group size). inc_off / inc:
-// the mesh's node -> element incidence lists (launch_incidence; NULL: every
-// node pair counts as shared by several groups). Pass 1 claims the list
-// entries, zeroes the value blocks of the entries several groups add to and
-// writes the groups' records (claim_hex20.cu); pass 2 adds the Ke blocks
-// (values_hex20.cu; in the tensor-core form the wave's Ke are computed into
-// stage first, ke_tcgen05.cu). map: kHex20WaveMapWords words (the groups'
-// records, group_hex20.cuh); stage:
-// kHex20Wave * kPackedHex20 doubles (tensor-core form only). wait_ns: see
-// wait_ns_of.
-cudaError_t launch_claim_hex20(const MeshView& m, const ListLayout& L, const int* perm, const int* inc_off,
-                               const int* inc, int i0, int i1, int* map, cudaStream_t s);
-cudaError_t launch_values_hex20(const MeshView& m, const ListLayout& L, int precision, const int* perm, int i0,
-                                int i1, const int* map, double* stage, long long wait_ns, cudaStream_t s);
-// The packed Ke of the elements perm[i0, i1) on the tensor cores, row q - i0 for position q.
-cudaError_t launch_stage_hex20_tc(const MeshView& m, const int* perm, int i0, int i1, double* stage, int* status,
-                                  long long wait_ns, cudaStream_t s);
-// Elements per wave of the two-pass scatter: a multiple of the group size,
-// large enough that each pass keeps every SM busy (4,096 groups a wave);
-// the batched kernel's waves are smaller (its items interleave many meshes).
-constexpr int kHex20Wave = 32768;
+// The same lists with occurrences e * stride + k (element e, local position k) for the elements
+// without a bad node id.
+cudaError_t launch_occurrences(const MeshView& m, int* cnt, int* off, int* inc, long long* tiles, int* status, int sms,
+                               cudaStream_t s);
+// What a Hex20 scatter leaves besides the list chunks (rows_hex20.cuh).
+struct HexRows {
+    double* ke;           // [E * kPackedHex20] packed element stiffness
+    int* off;             // [N + 1] node -> occurrences
+    int* inc;             // occurrences 20 e + a
+    unsigned short* map;  // [E * 400] rank of column node b in row node a's list, at 20 (20 e + a) + b
+};
+// The sorted row lists and the rank map; queue: N ints of scratch.
+cudaError_t launch_rows_hex20(const MeshView& m, const ListLayout& L, const HexRows& h, int* queue, cudaStream_t s);
+// Row lists -> CSR / BSR / upper triangle (mode: consolidate.cuh's kOut*; row_ptr already written).
+cudaError_t launch_count_upper_hex20(const ListLayout& L, int* ucounts, cudaStream_t s);
+cudaError_t launch_write_hex20(const ListLayout& L, const HexRows& h, int mode, const int* ucounts, const int* row_ptr,
+                               int* col_idx, double* values, long long capacity, cudaStream_t s);
+// Elements per wave of the batched kernel's claims and values: a multiple of the group size.
 constexpr int kBatchHex20Wave = 4096;
 constexpr int kHex20GroupSize = 8;            // elements per group (group_hex20.cuh)
 constexpr int kHex20GroupRecWords = 5220;     // record words per group (header, nodes, blocks by pair, slots)
-constexpr size_t kHex20WaveMapWords = (size_t)kHex20Wave / kHex20GroupSize * kHex20GroupRecWords;
-static_assert(kBatchHex20Wave <= kHex20Wave, "the batched ring's first map is the single-mesh one");
 
 // Spatial (3-D Morton bucket) element order; hist needs 1 << (3 * morton_bits(E)) ints, bbox 6 words.
 int morton_bits(int num_elems);
 cudaError_t launch_reorder_3d(const MeshView& m, int* hist, int* ranges, int* perm, unsigned long long* bbox, int sms,
                               cudaStream_t s);
 // tile_sums: row_tiles(N) partials of scratch.
-cudaError_t launch_consolidate(const ListLayout& L, int dpn, int* row_ptr, int* col_idx, double* values,
+cudaError_t launch_consolidate(const ListLayout& L, int dpn, const HexRows& hex, int* row_ptr, int* col_idx, double* values,
                                long long capacity, long long* tile_sums, cudaStream_t s);
 // Node-block (BSR) form of the consolidation; capacity in blocks.
 // Upper triangle (columns >= row, diagonal included) in CSR; ucounts: N ints of scratch.
-cudaError_t launch_consolidate_upper(const ListLayout& L, int dpn, int* ucounts, int* row_ptr, int* col_idx,
-                                     double* values, long long capacity, long long* tile_sums,
+cudaError_t launch_consolidate_upper(const ListLayout& L, int dpn, const HexRows& hex, int* ucounts, int* row_ptr,
+                                     int* col_idx, double* values, long long capacity, long long* tile_sums,
                                      cudaStream_t s);
-cudaError_t launch_consolidate_bsr(const ListLayout& L, int dpn, int* block_row_ptr, int* block_col_idx,
+cudaError_t launch_consolidate_bsr(const ListLayout& L, int dpn, const HexRows& hex, int* block_row_ptr,
+                                   int* block_col_idx,
                                    double* block_values, long long capacity_blocks, long long* tile_sums,
                                    cudaStream_t s);
 

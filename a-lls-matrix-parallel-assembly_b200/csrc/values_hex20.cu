@@ -1,13 +1,9 @@
-// Hex20 A-LLS scatter, pass 2 of 2: element stiffness in FP64 and the
-// accumulation of its blocks into the list entries that pass 1
-// (claim_hex20.cu) claimed and recorded in the groups' map records; also the
-// CTA-cooperative element pass of the value-only re-assembly and of the
-// colouring baseline.
+// The CTA-cooperative Hex20 element pass (values_hex20.cuh): FP64 element
+// stiffness added into a CSR, for the value-only re-assembly and the colouring
+// baseline (and, in the batched kernel, into list slots).
 //
-// Replaces the value half of assembleGlobalStiffnessKernelALLSFixedArray
-// (ALLS_Hex20_3D_Assembly_Performance.cu:212-256: one thread per element with
-// its 60x60 FP32 Ke in 14.9 KB of local memory, atomicAdd(float) per entry)
-// and its element routine computeElementStiffnessHex20 (H20:130-195).
+// Replaces the element routine computeElementStiffnessHex20
+// (ALLS_Hex20_3D_Assembly_Performance.cu:130-195).
 //
 // Element stiffness in direction-major form. With G_a (20 x 27) the physical
 // shape-function gradients along direction a at the Gauss points and
@@ -22,24 +18,6 @@
 // lane holds, for its two (I, J) node pairs of a tile, all nine M^{ab}_IJ and
 // forms Ke_IJ without exchanging anything with other lanes.
 //
-// Group value pass (k_values_group): one CTA of kGroup warps per element
-// group, persistent over the wave's groups. Warp w computes the Ke of the
-// group's element w alone: the lanes' gradients G_a(n, g) for the fragment
-// rows n = 8 t + lane / 4 and k-columns g = 4 s + lane % 4 are the same
-// values for the A and the B operands, so they stay in registers (63 per
-// lane) and all six tile positions run from registers. Each of the 210 upper
-// blocks is stored, already oriented as it adds to its node pair (the block,
-// its transpose, or block + transpose for a repeated node), at its position
-// in the group's pair-major block order (from the claim pass's record): one
-// writer per position, plain shared stores. After a barrier, three threads
-// per node pair sum the pair's contiguous blocks, one row each, so a pair
-// that several of the group's elements share leaves the CTA once, and write
-// the sum to the slot of (row u, column v) and its transpose to (row v,
-// column u): a plain store for a pair only this group has (its slots were
-// not zeroed), an FP64 atomic add for a shared pair (zeroed by its claimer).
-// The tensor-core form computes the wave's Ke in ke_tcgen05.cu into a staging
-// buffer first, and the same kernel stages those blocks instead.
-//
 // Element pass (k_values_hex20, kToCsrMap / kToCsrColour): one 6-warp CTA
 // per element at a time, warp w owning tile position w; the shape-function
 // derivatives at the 27 Gauss points (H20:95-128) are tabulated once per CTA
@@ -47,7 +25,7 @@
 // current one is computed.
 #include <algorithm>
 
-#include "values_group.cuh"
+#include "values_hex20.cuh"
 
 namespace fem {
 namespace {
@@ -93,45 +71,7 @@ cudaError_t launch_values(const MeshView& m, const int* perm, int i0, int i1, co
     return cudaGetLastError();
 }
 
-constexpr int kGroupThreads = kGroup * 32;
-
-__global__ void __launch_bounds__(kGroupThreads, 1)
-    k_values_group(MeshView m, int i0, int i1, const int* __restrict__ recs, const double* __restrict__ stage,
-                   double* vals, DevInfo* info) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    GroupValuesSmem& sm = *reinterpret_cast<GroupValuesSmem*>(smem_raw);
-    values_group_init(sm);
-    values_group(m, i0, i1, recs, stage, vals, info, sm);
-}
-
-cudaError_t launch_group_values(const MeshView& m, const ListLayout& L, int i0, int i1, const int* recs,
-                                const double* stage, cudaStream_t s) {
-    static DeviceCache cache;
-    const size_t smem = sizeof(GroupValuesSmem);
-    int per_sm = 0;
-    const cudaError_t err = per_device(cache, [&](int& v) {
-        cudaError_t e = cudaFuncSetAttribute(k_values_group, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (!e) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, k_values_group, kGroupThreads, smem);
-        return e;
-    }, per_sm);
-    if (err) return err;
-    const long long groups = (i1 - i0 + kGroup - 1) / kGroup;
-    const long long grid = std::max<long long>(1, std::min<long long>(groups, (long long)per_sm * sm_count()));
-    k_values_group<<<(int)grid, kGroupThreads, smem, s>>>(m, i0, i1, recs, stage, L.vals, L.info);
-    return cudaGetLastError();
-}
-
 }  // namespace
-
-cudaError_t launch_values_hex20(const MeshView& m, const ListLayout& L, int precision, const int* perm, int i0,
-                                int i1, const int* map, double* stage, long long wait_ns, cudaStream_t s) {
-    if (i1 <= i0) return cudaSuccess;
-    if (precision == FEM_PREC_TC_F16X3) {
-        cudaError_t err = launch_stage_hex20_tc(m, perm, i0, i1, stage, &L.info->status_bits, wait_ns, s);
-        return err ? err : launch_group_values(m, L, i0, i1, map, stage, s);
-    }
-    return launch_group_values(m, L, i0, i1, map, nullptr, s);
-}
 
 cudaError_t launch_reassemble_hex20(const MeshView& m, int precision, const int* perm, const MapTarget& mt,
                                     DevInfo* info, cudaStream_t s) {
