@@ -12,20 +12,19 @@
 // 2-D (k_ke_2d): one lane per node block, as the A-LLS scatter computes it
 // (FP64, or FP32 blocks with FEM_PREC_FP32).
 //
-// Hex20 (k_hex20_ke): one CTA (4 warps) per element at a time, persistent:
+// Hex20: FEM_PREC_FP64 runs the FP64 tensor-core kernel of ke_hex20.cu,
+// FEM_PREC_TC_F16X3 the tcgen05 kernel of ke_tcgen05.cu. k_hex20_ke is the
+// plain FP64 form without tensor cores (FEM_PREC_FP64_SIMT), the comparison
+// point: one CTA (4 warps) per element at a time, persistent:
 //   Jacobians at the 27 Gauss points (243 entries), their inverses and
 //   w_g = weight * detJ_g (27 threads; a non-positive detJ raises
-//   FEM_ERR_DETJ), physical gradients P[3n+a][g] (540 items), then
-//   M = P diag(w) P^T on the FP64 tensor cores with mma.sync.m8n8k4.f64
-//   (36 upper 8x8 tiles of the 64x64 padded product x 7 k-steps); each upper
-//   entry of M is written to its upper 3x3 node block (so Ke is exactly
-//   symmetric), and the 210 Ke blocks
+//   FEM_ERR_DETJ), physical gradients P[3n+a][g] (540 items), then every upper
+//   entry of M = P diag(w) P^T as a dot product, written to its upper 3x3 node
+//   block (so Ke is exactly symmetric), and the 210 Ke blocks
 //       Ke_IJ[a][b] = lambda M_IJ[a][b] + mu M_IJ[b][a] + mu delta_ab tr(M_IJ)
-//   are written with coalesced stores. With FEM_PREC_FP64_SIMT the contraction
-//   is plain FP64 dot products instead; FEM_PREC_TC_F16X3 runs the tcgen05
-//   kernel of ke_tcgen05.cu. The Gauss-point shape derivatives
-//   (H20:95-128) are tabulated once per CTA; the next element's nodes and
-//   coordinates are loaded while the current one is computed.
+//   with coalesced stores. The Gauss-point shape derivatives (H20:95-128) are
+//   tabulated once per CTA; the next element's nodes and coordinates are
+//   loaded while the current one is computed.
 #include <algorithm>
 
 #include "element2d.cuh"
@@ -37,15 +36,7 @@ namespace {
 using namespace hex20;
 
 constexpr int kThreads = 128;  // small CTAs: several elements' phases overlap on an SM
-constexpr int kWarps = kThreads / 32;
-constexpr int kTilesPerWarp = (36 + kWarps - 1) / kWarps;
-constexpr int PS = 28;  // row stride of P (doubles): conflict-free m8n8k4 fragment loads
-
-// The 36 upper 8x8 tiles (mt <= nt) of the 64x64 node-pair matrix.
-__constant__ unsigned char c_tile_m[36] = {0, 0, 0, 0, 0, 0, 0, 0, 1, 1, 1, 1, 1, 1, 1, 2, 2, 2,
-                                           2, 2, 2, 3, 3, 3, 3, 3, 4, 4, 4, 4, 5, 5, 5, 6, 6, 7};
-__constant__ unsigned char c_tile_n[36] = {0, 1, 2, 3, 4, 5, 6, 7, 1, 2, 3, 4, 5, 6, 7, 2, 3, 4,
-                                           5, 6, 7, 3, 4, 5, 6, 7, 4, 5, 6, 7, 5, 6, 7, 6, 7, 7};
+constexpr int PS = 28;  // row stride of P (doubles)
 
 struct KeSmem {
     double dN[27][3][20];  // shape derivatives at the Gauss points
@@ -61,21 +52,11 @@ struct KeSmem {
 };
 static_assert(offsetof(KeSmem, Mb) % 16 == 0, "16-byte copies out of Mb");
 
-__device__ __forceinline__ void dmma_8x8x4(double& c0, double& c1, double a, double b) {
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
-                 : "+d"(c0), "+d"(c1)
-                 : "d"(a), "d"(b));
-}
-
-// kPrec: the node-pair contraction on the FP64 tensor cores (FEM_PREC_FP64)
-// or as plain FP64 dot products on the CUDA cores (FEM_PREC_FP64_SIMT, the
-// reference's arithmetic without tensor cores).
-template <int kPrec>
 __global__ void __launch_bounds__(kThreads, 5) k_hex20_ke(MeshView m, double* __restrict__ ke_out,
                                                           int* __restrict__ status) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     KeSmem& sm = *reinterpret_cast<KeSmem*>(smem_raw);
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x;
 
     for (int idx = tid; idx < 27 * 20; idx += kThreads) {
         const int g = idx / 20, n = idx % 20;
@@ -179,7 +160,7 @@ __global__ void __launch_bounds__(kThreads, 5) k_hex20_ke(MeshView m, double* __
             for (int a = 0; a < 3; a++) sm.P[3 * n + a][g] = fma(iJ[3 * a], d0, fma(iJ[3 * a + 1], d1, iJ[3 * a + 2] * d2));
         }
         __syncthreads();
-        if (kPrec == FEM_PREC_FP64_SIMT) {
+        {
             // every upper entry (r <= c < 60) of M as a plain FP64 dot product
             // over the 27 Gauss points; kept in registers until every thread
             // has read P, whose storage then takes the M blocks
@@ -212,45 +193,6 @@ __global__ void __launch_bounds__(kThreads, 5) k_hex20_ke(MeshView m, double* __
                 sm.Mb[pair_index(I, J)][3 * a + b] = mv[k];
                 if (I == J) sm.Mb[pair_index(I, I)][3 * b + a] = mv[k];
             }
-        } else {
-        // M = (P diag(w)) P^T on the FP64 tensor cores, upper 8x8 tiles only
-        // (M is symmetric): the 36 tiles (mt <= nt) are dealt round-robin to the
-        // warps.
-        double acc[kTilesPerWarp][2];
-#pragma unroll
-        for (int q = 0; q < kTilesPerWarp; q++) acc[q][0] = acc[q][1] = 0.0;
-        const int fr = lane >> 2, fc = lane & 3;
-#pragma unroll
-        for (int q = 0; q < kTilesPerWarp; q++) {
-            const int t = warp + q * kWarps;
-            if (t < 36) {
-                const int mt = c_tile_m[t], nt = c_tile_n[t];
-#pragma unroll
-                for (int ks = 0; ks < 7; ks++) {
-                    const int k = 4 * ks + fc;
-                    dmma_8x8x4(acc[q][0], acc[q][1], sm.w[k] * sm.P[8 * mt + fr][k], sm.P[8 * nt + fr][k]);
-                }
-            }
-        }
-        __syncthreads();  // every warp has read P: its storage now takes the M blocks
-#pragma unroll
-        for (int q = 0; q < kTilesPerWarp; q++) {
-            const int t = warp + q * kWarps;
-            if (t < 36) {
-                const int mt = c_tile_m[t], nt = c_tile_n[t];
-#pragma unroll
-                for (int h = 0; h < 2; h++) {
-                    const int r = 8 * mt + fr, c = 8 * nt + 2 * fc + h;
-                    // entry (r, c) stands for itself and, by symmetry, for (c, r);
-                    // in a diagonal tile only r <= c writes (its mirror is in the tile)
-                    if (r < 60 && c < 60 && (mt < nt || r <= c)) {
-                        const int I = r / 3, a = r - 3 * I, J = c / 3, b = c - 3 * J;
-                        if (I <= J) sm.Mb[pair_index(I, J)][3 * a + b] = acc[q][h];
-                        if (J <= I) sm.Mb[pair_index(J, I)][3 * b + a] = acc[q][h];
-                    }
-                }
-            }
-        }
         }
         __syncthreads();
         // Ke upper blocks, consecutive threads on consecutive entries
@@ -329,19 +271,18 @@ __global__ void __launch_bounds__(kThreads2D) k_ke_2d(MeshView m, double* __rest
     }
 }
 
-template <int kPrec>
-cudaError_t launch_hex20_ke(const MeshView& m, double* ke_out, int* status, cudaStream_t s) {
+cudaError_t launch_hex20_ke_simt(const MeshView& m, double* ke_out, int* status, cudaStream_t s) {
     static DeviceCache cache;
     const size_t smem = sizeof(KeSmem);
     int blocks_per_sm = 0;
     const cudaError_t err = per_device(cache, [&](int& v) {
-        cudaError_t e = cudaFuncSetAttribute(k_hex20_ke<kPrec>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (!e) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, k_hex20_ke<kPrec>, kThreads, smem);
+        cudaError_t e = cudaFuncSetAttribute(k_hex20_ke, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (!e) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, k_hex20_ke, kThreads, smem);
         return e;
     }, blocks_per_sm);
     if (err) return err;
     const long long grid = std::min<long long>((long long)blocks_per_sm * sm_count(), m.E_count);
-    k_hex20_ke<kPrec><<<(int)grid, kThreads, smem, s>>>(m, ke_out, status);
+    k_hex20_ke<<<(int)grid, kThreads, smem, s>>>(m, ke_out, status);
     return cudaGetLastError();
 }
 
@@ -352,8 +293,8 @@ cudaError_t launch_element_stiffness(const MeshView& m, int kind, int precision,
     if (m.E_count <= 0) return cudaSuccess;
     if (kind == FEM_HEX20) {
         if (precision == FEM_PREC_TC_F16X3) return launch_hex20_ke_tcgen05(m, ke_out, status, wait_ns, s);
-        if (precision == FEM_PREC_FP64_SIMT) return launch_hex20_ke<FEM_PREC_FP64_SIMT>(m, ke_out, status, s);
-        return launch_hex20_ke<FEM_PREC_FP64>(m, ke_out, status, s);
+        if (precision == FEM_PREC_FP64_SIMT) return launch_hex20_ke_simt(m, ke_out, status, s);
+        return launch_hex20_ke_dmma(m, ke_out, status, s);
     } else {
         const long long warps = ((long long)m.E_count + 1) / 2;  // two elements per warp
         const int grid = (int)std::min<long long>((warps * 32 + kThreads2D - 1) / kThreads2D, (long long)sm_count() * 8);

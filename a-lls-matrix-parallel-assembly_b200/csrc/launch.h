@@ -69,6 +69,8 @@ constexpr int kPacked2D_T3 = 6 * 4;
 // Element stiffness of every element, natural order; status gets 1 << FEM_ERR_* bits.
 cudaError_t launch_element_stiffness(const MeshView& m, int kind, int precision, double* ke_out, int* status,
                                      long long wait_ns, cudaStream_t s);
+// Hex20 element stiffness on the FP64 tensor cores, one warp per element (ke_hex20.cu).
+cudaError_t launch_hex20_ke_dmma(const MeshView& m, double* ke_out, int* status, cudaStream_t s);
 // Hex20 element stiffness with the contraction on the tcgen05 tensor cores
 // (FEM_PREC_TC_F16X3), two elements per CTA step.
 // wait_ns: bound on a CTA's wait for its products (< 0: no wait), see fem_opts.wait_limit_us.
