@@ -118,6 +118,7 @@ __global__ void __launch_bounds__(kScanThreads) k_row_ptr(const int* __restrict_
         info->nnz = nnz;
         info->list_entries = 0;
         info->max_row_entries = 0;
+        info->ticket = 0;
         row_ptr[(long long)N * R] = (int)(nnz / (kMode == kOutBsr ? B : 1));
     }
 }

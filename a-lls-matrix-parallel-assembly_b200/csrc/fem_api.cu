@@ -147,6 +147,10 @@ ListLayout device_layout(const HostLayout& h, void* ws) {
     return L;
 }
 
+// Hex20 meshes of at least this many elements are consolidated in a spatial node order: the packed Ke of
+// smaller ones (46 MB) stays in L2 whatever the order.
+constexpr int kOrderedElems = 3072;
+
 HexRows hex_rows(const HostLayout& h, void* ws) {
     unsigned char* b = static_cast<unsigned char*>(ws);
     HexRows r{};
@@ -156,6 +160,8 @@ HexRows hex_rows(const HostLayout& h, void* ws) {
     r.off = reinterpret_cast<int*>(b + h.off_inc + n);
     r.inc = reinterpret_cast<int*>(b + h.off_inc + 2 * n);
     r.map = reinterpret_cast<unsigned short*>(b + h.off_map);
+    // the occurrence counts' place, free once the occurrences are filled
+    if (h.E >= kOrderedElems) r.order = reinterpret_cast<const int*>(b + h.off_inc);
     return r;
 }
 
@@ -259,6 +265,12 @@ fem_status fem_alls_scatter(const fem_mesh* mesh, const fem_opts* opts, void* wo
     long long* tiles = reinterpret_cast<long long*>(b + h.off_tiles);  // free until the consolidation
     if (!err) err = launch_occurrences(m, cnt, hex.off, hex.inc, tiles, &L.info->status_bits, sm_count(), s);
     if (!err) err = launch_rows_hex20(m, L, hex, queue, s);
+    if (!err && hex.order) {
+        int* ranges = reinterpret_cast<int*>(b + h.off_elist);
+        int* hist = ranges + kAlign / sizeof(int);
+        unsigned long long* bbox = reinterpret_cast<unsigned long long*>(hist + (1 << (3 * kNodeOrderBits)));
+        err = launch_node_order(m, hist, ranges, cnt, bbox, sm_count(), s);
+    }
     if (!err)
         err = launch_element_stiffness(m, FEM_HEX20, precision, hex.ke, &L.info->status_bits,
                                        wait_ns_of(opts ? opts->wait_limit_us : 0), s);

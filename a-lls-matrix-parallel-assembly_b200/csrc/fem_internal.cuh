@@ -46,7 +46,7 @@ struct DevInfo {
     int pool_chunks;
     int max_row_entries;
     int long_rows;         // rows queued for the long-row kernels
-    int pad0;
+    int ticket;            // consolidation: next row node to write
     long long pad1[3];
 };
 static_assert(sizeof(DevInfo) == 64, "DevInfo size");

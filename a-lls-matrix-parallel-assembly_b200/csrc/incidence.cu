@@ -23,7 +23,20 @@ __device__ __forceinline__ int elem_npe(const MeshView& m, int e) {
     return m.stride;
 }
 
-// kOcc (Hex20 rows): an element with a bad node id has no occurrence at all.
+// kOcc (Hex20 rows): an element with a bad node id has no occurrence at all;
+// the occurrences of an element that repeats a node carry kOccRepeats.
+__device__ __forceinline__ unsigned repeats_flag(const MeshView& m, int e) {
+    int n[20];
+    bool rep = false;
+#pragma unroll
+    for (int k = 0; k < 20; k++) n[k] = __ldg(m.conn + (size_t)e * 20 + k);
+#pragma unroll
+    for (int k = 1; k < 20; k++)
+#pragma unroll
+        for (int j = 0; j < k; j++) rep |= n[j] == n[k];
+    return rep ? kOccRepeats : 0u;
+}
+
 __device__ __forceinline__ bool bad_element(const MeshView& m, int e) {
     bool bad = false;
     for (int k = 0; k < m.stride; k++) {
@@ -116,10 +129,11 @@ __global__ void k_inc_fill(MeshView m, const int* __restrict__ off, int* __restr
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < m.E_count; e += gridDim.x * blockDim.x) {
         const int npe = elem_npe(m, e);
         if (kOcc && bad_element(m, e)) continue;
+        const unsigned flag = kOcc ? repeats_flag(m, e) : 0u;
         for (int k = 0; k < npe; k++) {
             const int n = __ldg(m.conn + (size_t)e * m.stride + k);
             if (n < 0 || n >= m.N) continue;
-            inc[off[n] + atomicAdd(cursor + n, 1)] = kOcc ? e * m.stride + k : e;
+            inc[off[n] + atomicAdd(cursor + n, 1)] = kOcc ? (int)((unsigned)(e * 20 + k) | flag) : e;
         }
     }
 }

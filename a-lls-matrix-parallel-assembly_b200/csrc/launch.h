@@ -110,15 +110,18 @@ cudaError_t launch_colour_hex20(const MeshView& m, const int* perm, const int* r
 // scratch; status gets 1 << FEM_ERR_* bits.
 cudaError_t launch_incidence(const MeshView& m, int* cnt, int* off, int* inc, long long* tiles, int* status, int sms,
                              cudaStream_t s);
-// The same lists with occurrences e * stride + k (element e, local position k) for the elements
-// without a bad node id.
+// The same lists for Hex20 with occurrences 20 e + a (element e, local position a) for the elements
+// without a bad node id; bit 31 marks the elements that repeat a node (the count of occurrences stays
+// below 2^31, else FEM_ERR_RANGE).
+constexpr unsigned kOccRepeats = 0x80000000u;
 cudaError_t launch_occurrences(const MeshView& m, int* cnt, int* off, int* inc, long long* tiles, int* status, int sms,
                                cudaStream_t s);
 // What a Hex20 scatter leaves besides the list chunks (rows_hex20.cuh).
 struct HexRows {
     double* ke;           // [E * kPackedHex20] packed element stiffness
     int* off;             // [N + 1] node -> occurrences
-    int* inc;             // occurrences 20 e + a
+    int* inc;             // occurrences 20 e + a (bit 31: kOccRepeats)
+    const int* order;     // [N] node visit order of the consolidation, or NULL: as numbered
     unsigned short* map;  // [E * 400] rank of column node b in row node a's list, at 20 (20 e + a) + b
 };
 // The sorted row lists and the rank map; queue: N ints of scratch.
@@ -134,6 +137,10 @@ constexpr int kHex20GroupRecWords = 5220;     // record words per group (header,
 
 // Spatial (3-D Morton bucket) element order; hist needs 1 << (3 * morton_bits(E)) ints, bbox 6 words.
 int morton_bits(int num_elems);
+// Nodes by the Morton code of their cell on a 2^kNodeOrderBits grid per axis (hist: one int per cell).
+constexpr int kNodeOrderBits = 4;
+cudaError_t launch_node_order(const MeshView& m, int* hist, int* ranges, int* order, unsigned long long* bbox, int sms,
+                              cudaStream_t s);
 cudaError_t launch_reorder_3d(const MeshView& m, int* hist, int* ranges, int* perm, unsigned long long* bbox, int sms,
                               cudaStream_t s);
 // tile_sums: row_tiles(N) partials of scratch.

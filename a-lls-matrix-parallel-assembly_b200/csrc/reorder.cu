@@ -21,7 +21,10 @@
 // from L2 between their visits (in natural x-y-z order they are a whole z-layer
 // of elements apart). The key is the 3-D Morton code of the midpoint of each
 // element's corner diagonal (nodes 0 and 6), quantized on a 2^b grid over the
-// node bounding box (k_bbox), counting-sorted the same way.
+// node bounding box (k_bbox), counting-sorted the same way. The consolidation of
+// a large Hex20 mesh visits its nodes by the Morton code of their cell on a
+// 16^3 grid (launch_node_order), so that the rows that read an element's Ke are
+// written close together in time, whatever the numbering.
 #include <algorithm>
 
 #include "launch.h"
@@ -140,12 +143,24 @@ __global__ void k_bbox(MeshView m, unsigned long long* bbox) {
             hi[d] = h2 > hi[d] ? h2 : hi[d];
         }
     }
+    // one set of atomics per CTA
+    __shared__ unsigned long long s_lo[kThreads / 32][3], s_hi[kThreads / 32][3];
     if ((threadIdx.x & 31) == 0) {
 #pragma unroll
         for (int d = 0; d < 3; d++) {
-            atomicMin(bbox + d, lo[d]);
-            atomicMax(bbox + 3 + d, hi[d]);
+            s_lo[threadIdx.x >> 5][d] = lo[d];
+            s_hi[threadIdx.x >> 5][d] = hi[d];
         }
+    }
+    __syncthreads();
+    if (threadIdx.x < 3) {
+        unsigned long long l = ~0ull, h = 0ull;
+        for (int w = 0; w < kThreads / 32; w++) {
+            l = s_lo[w][threadIdx.x] < l ? s_lo[w][threadIdx.x] : l;
+            h = s_hi[w][threadIdx.x] > h ? s_hi[w][threadIdx.x] : h;
+        }
+        atomicMin(bbox + threadIdx.x, l);
+        atomicMax(bbox + 3 + threadIdx.x, h);
     }
 }
 
@@ -159,13 +174,8 @@ __device__ __forceinline__ unsigned spread3(unsigned v) {
     return v;
 }
 
-__device__ __forceinline__ int morton_key(const MeshView& m, int e, const unsigned long long* bbox, int bits) {
-    const int* c = m.conn + (size_t)e * m.stride;
-    int n0 = __ldg(c + 0), n6 = __ldg(c + 6);
-    n0 = (n0 >= 0 && n0 < m.N) ? n0 : 0;  // bad ids are reported by the scatter
-    n6 = (n6 >= 0 && n6 < m.N) ? n6 : 0;
-    const double p[3] = {0.5 * (__ldg(m.x + n0) + __ldg(m.x + n6)), 0.5 * (__ldg(m.y + n0) + __ldg(m.y + n6)),
-                         0.5 * (__ldg(m.z + n0) + __ldg(m.z + n6))};
+// Morton code of point p on the 2^bits grid over the bounding box.
+__device__ __forceinline__ int morton_of(const double (&p)[3], const unsigned long long* bbox, int bits) {
     const int cells = 1 << bits;
     unsigned q[3];
 #pragma unroll
@@ -176,6 +186,16 @@ __device__ __forceinline__ int morton_key(const MeshView& m, int e, const unsign
         q[d] = (unsigned)min(max(qi, 0), cells - 1);
     }
     return (int)(spread3(q[0]) | (spread3(q[1]) << 1) | (spread3(q[2]) << 2));
+}
+
+__device__ __forceinline__ int morton_key(const MeshView& m, int e, const unsigned long long* bbox, int bits) {
+    const int* c = m.conn + (size_t)e * m.stride;
+    int n0 = __ldg(c + 0), n6 = __ldg(c + 6);
+    n0 = (n0 >= 0 && n0 < m.N) ? n0 : 0;  // bad ids are reported by the scatter
+    n6 = (n6 >= 0 && n6 < m.N) ? n6 : 0;
+    const double p[3] = {0.5 * (__ldg(m.x + n0) + __ldg(m.x + n6)), 0.5 * (__ldg(m.y + n0) + __ldg(m.y + n6)),
+                         0.5 * (__ldg(m.z + n0) + __ldg(m.z + n6))};
+    return morton_of(p, bbox, bits);
 }
 
 __global__ void k_morton_count(MeshView m, const unsigned long long* bbox, int bits, int* __restrict__ hist) {
@@ -194,6 +214,15 @@ struct BucketKey {
     MeshView m;
     int NB;
     __device__ __forceinline__ int operator()(int e) const { return element_key(m, e, NB); }
+};
+struct NodeMortonKey {
+    MeshView m;
+    const unsigned long long* bbox;
+    int bits;
+    __device__ __forceinline__ int operator()(int n) const {
+        const double p[3] = {__ldg(m.x + n), __ldg(m.y + n), __ldg(m.z + n)};
+        return morton_of(p, bbox, bits);
+    }
 };
 struct MortonKey {
     MeshView m;
@@ -283,6 +312,8 @@ cudaError_t counting_sort(const Key& key, int E, int nkeys, int NB, int mixed, i
 
 }  // namespace
 
+static_assert((1 << (3 * kNodeOrderBits)) <= kMaxSmemKeys, "the node order always sorts in shared memory");
+
 int reorder_buckets(int num_nodes) { return (num_nodes >> kBucketShift) + 1; }
 
 int morton_bits(int num_elems) {
@@ -304,6 +335,18 @@ cudaError_t launch_reorder_3d(const MeshView& m, int* hist, int* ranges, int* pe
         MortonKey{m, bbox, bits}, m.E_count, nkeys, nkeys, 0, hist, ranges, perm, sms,
         [&](int grid) { k_morton_count<<<grid, kThreads, 0, s>>>(m, bbox, bits, hist); },
         [&](int grid) { k_morton_scatter<<<grid, kThreads, 0, s>>>(m, bbox, bits, hist, perm); }, s);
+}
+
+cudaError_t launch_node_order(const MeshView& m, int* hist, int* ranges, int* order, unsigned long long* bbox, int sms,
+                              cudaStream_t s) {
+    constexpr int nkeys = 1 << (3 * kNodeOrderBits);
+    cudaError_t err = cudaMemsetAsync(hist, 0, (size_t)nkeys * sizeof(int), s);
+    if (err) return err;
+    k_bbox_init<<<1, 32, 0, s>>>(bbox);
+    const long long wn = ((long long)m.N + kThreads - 1) / kThreads;
+    k_bbox<<<(int)std::min<long long>(wn > 0 ? wn : 1, (long long)sms * 4), kThreads, 0, s>>>(m, bbox);
+    return counting_sort(NodeMortonKey{m, bbox, kNodeOrderBits}, m.N, nkeys, nkeys, 0, hist, ranges, order, sms,
+                         [](int) {}, [](int) {}, s);
 }
 
 cudaError_t launch_reorder(const MeshView& m, int* hist, int* ranges, int* perm, int sms, cudaStream_t s) {

@@ -44,7 +44,6 @@ constexpr unsigned kFull = 0xFFFFFFFFu;
 struct RowSmem {
     int table[kTable];                 // distinct column nodes, -1 = empty
     int uniq[kTable];                  // compacted, then sorted
-    unsigned seen[kMaxElems][5];       // ranks met per element (repeated nodes)
     unsigned short rank[kTable];       // rank of a table entry
 };
 
@@ -127,7 +126,7 @@ __global__ void __launch_bounds__(kThreads, FEM_HEXR_CTAS) k_rows_hex20(const in
             if (lane == 0) queue[atomicAdd(&L.info->long_rows, 1)] = n;
             continue;
         }
-        const int o = lane < d ? __ldg(inc + lo + lane) : 0;
+        const int o = lane < d ? (int)occ_of(__ldg(inc + lo + lane)) : 0;
         int node[kCand], slot[kCand];
 #pragma unroll
         for (int q = 0; q < kCand; q++) {
@@ -137,8 +136,6 @@ __global__ void __launch_bounds__(kThreads, FEM_HEXR_CTAS) k_rows_hex20(const in
         }
         reinterpret_cast<int4*>(sm.table)[lane] = make_int4(-1, -1, -1, -1);
         reinterpret_cast<int4*>(sm.table)[lane + 32] = make_int4(-1, -1, -1, -1);
-        (&sm.seen[0][0])[lane] = 0u;
-        if (lane < kMaxElems * 5 - 32) (&sm.seen[0][0])[lane + 32] = 0u;
         __syncwarp();
 #pragma unroll
         for (int q = 0; q < kCand; q++) {
@@ -184,22 +181,10 @@ __global__ void __launch_bounds__(kThreads, FEM_HEXR_CTAS) k_rows_hex20(const in
         for (int q = 0; q < kCand; q++) {
             const int j = lane + 32 * q, t = j / 20, b = j - 20 * t;
             const int ot = __shfl_sync(kFull, o, t & 31);
-            if (node[q] >= 0) {
-                const unsigned r = sm.rank[slot[q]], bit = 1u << (r & 31);
-                const bool dup = atomicOr(&sm.seen[t][r >> 5], bit) & bit;
-                map[(size_t)ot * 20 + b] = (unsigned short)(r | (dup ? kRankDup : 0u));
-            }
+            if (node[q] >= 0) map[(size_t)ot * 20 + b] = sm.rank[slot[q]];
         }
         __syncwarp();
     }
-}
-
-// Whether position b of the element at conn row `row` repeats an earlier position's node.
-__device__ __forceinline__ bool repeats(const int* row, int b) {
-    const int n = __ldg(row + b);
-    bool r = false;
-    for (int k = 0; k < b; k++) r |= __ldg(row + k) == n;
-    return r;
 }
 
 __global__ void __launch_bounds__(32) k_wide_rows_hex20(const int* __restrict__ conn, ListLayout L,
@@ -211,7 +196,7 @@ __global__ void __launch_bounds__(32) k_wide_rows_hex20(const int* __restrict__ 
     for (int k = blockIdx.x; k < count; k += gridDim.x) {
         const int n = __ldg(queue + k), lo = __ldg(off + n), d = __ldg(off + n + 1) - lo;
         if (d > kWideElems) continue;  // k_long_rows_hex20's
-        const int o = lane < d ? __ldg(inc + lo + lane) : 0;
+        const int o = lane < d ? (int)occ_of(__ldg(inc + lo + lane)) : 0;
         int node[kWideCand];
 #pragma unroll
         for (int q = 0; q < kWideCand; q++) {
@@ -230,9 +215,7 @@ __global__ void __launch_bounds__(32) k_wide_rows_hex20(const int* __restrict__ 
             for (int q = 0; q < kWideCand; q++) {
                 const int j = lane + 32 * q, t = j / 20, b = j - 20 * t;
                 const int ot = __shfl_sync(kFull, o, t);
-                if (node[q] == m)
-                    map[(size_t)ot * 20 + b] =
-                        (unsigned short)(u | (repeats(conn + (size_t)(ot / 20) * 20, b) ? kRankDup : 0u));
+                if (node[q] == m) map[(size_t)ot * 20 + b] = (unsigned short)u;
             }
             if (lane == 0) s_uniq[u] = m;
             u++;
@@ -270,13 +253,11 @@ __global__ void __launch_bounds__(kThreads) k_long_rows_hex20(const int* __restr
                 __syncthreads();
                 int m = 0x7FFFFFFF;
                 for (long long j = tid; j < cand; j += kThreads) {
-                    const int ot = __ldg(inc + lo + (int)(j / 20)), b = (int)(j % 20);
-                    const int* row = conn + (size_t)(ot / 20) * 20;
-                    const int x = __ldg(row + b);
+                    const unsigned ot = occ_of(__ldg(inc + lo + (int)(j / 20)));
+                    const int b = (int)(j % 20), x = __ldg(conn + (size_t)(ot / 20) * 20 + b);
                     if (x > last) m = min(m, x);
                     // the previous column's rank, met again on the way
-                    if (pass == 1 && u > 0 && x == last)
-                        map[(size_t)ot * 20 + b] = (unsigned short)((u - 1) | (repeats(row, b) ? kRankDup : 0u));
+                    if (pass == 1 && u > 0 && x == last) map[(size_t)ot * 20 + b] = (unsigned short)(u - 1);
                 }
                 m = __reduce_min_sync(kFull, m);
                 if ((tid & 31) == 0) atomicMin(&s_min[u & 1], m);
@@ -287,9 +268,9 @@ __global__ void __launch_bounds__(kThreads) k_long_rows_hex20(const int* __restr
                 last = m;
             }
             if (pass == 0 && tid == 0) {
-                if (u > (int)kRankMask) {  // past the rank map's range
+                if (u > kMaxRank) {  // past the rank map's range
                     raise_status(L.info, FEM_ERR_RANGE);
-                    u = (int)kRankMask;
+                    u = kMaxRank;
                 }
                 s_next = take_chunks(L, u);
                 s_kept = u;

@@ -14,8 +14,9 @@
 namespace fem {
 namespace {
 
-constexpr unsigned kRankMask = 0x7FFFu;  // rank in the row; bit 15: the element has the column node at an
-constexpr unsigned kRankDup = 0x8000u;   // earlier position too (a repeated node)
+constexpr int kMaxRank = 0xFFFF;  // columns of a row that the rank map can number
+
+__device__ __forceinline__ unsigned occ_of(int word) { return (unsigned)word & ~kOccRepeats; }
 
 // Column word (column node + 1) k of row node n: the first chunk's slots, then
 // the row's overflow chunks, which are consecutive from chunk id `next` - 1 on.
