@@ -1,88 +1,58 @@
 // Batched assembly: many independent meshes of uneven sizes and element kinds
-// in one persistent launch (graph-capturable).
+// in one stream-ordered, graph-capturable call.
 //
 // The reference assembles one mesh per program run (each driver's main, e.g.
-// ALLS_Q4_T3_Mixed_Elements_Assembly_Performance.cu:742-854). Here the host
-// turns the batch into a schedule: for each mesh its phases (list reset,
-// 2-D scatter or Hex20 claim / value waves of element groups, consolidation
-// scan, row pointers,
-// sorted write, completion) as segments of work items, the meshes in rounds
-// of `slots` (the workspace holds that many meshes' lists at once), each
-// round phase by phase. One persistent kernel then runs the whole schedule:
-// every CTA takes the next ticket from one counter, finds its segment, waits
-// (bounded) until the mesh's phase counters say the items it depends on are
-// finished, runs the item with the same device code as the single-mesh
-// kernels (claim_hex20.cuh, values_hex20.cuh, scatter2d.cuh, consolidate.cuh)
-// and counts it done. An item only ever depends on items with smaller
-// tickets, which CTAs already running have taken, so the kernel always makes
-// progress. A mesh's last item copies its info word into the caller's array
-// and stamps its completion with the GPU global timer.
+// ALLS_Q4_T3_Mixed_Elements_Assembly_Performance.cu:742-854). Here the meshes
+// are assembled in rounds of `slots` (the workspace holds that many meshes'
+// lists at once), and a round runs phase by phase: one launch per phase covers
+// all of the round's meshes (begin; 2-D fill and Hex20 occurrences; rows; Hex20
+// Ke; row pointers; writes; finish), its blocks dealt to the meshes in
+// proportion to their work, each block running the device code of the
+// single-mesh kernels. Phases follow each other in stream order, so nothing
+// waits inside a kernel, small meshes share their launches, and large ones get
+// the same kernels as on their own. A round's mesh descriptors travel as kernel
+// parameters, so a captured CUDA graph holds them.
 //
-// The mesh descriptors and the schedule travel as kernel parameters of small
-// copy kernels into the workspace, so a captured CUDA graph holds them; the
-// counters and the ticket are zeroed by a kernel of the same sequence.
-#define FEM_LDG(p) __ldcg(p)  // items read what earlier items of the launch wrote
-
+// What bounds it: the single-mesh kernels; a round costs up to 18 launches
+// whatever its number of meshes. B200, 16 meshes of 1,000 to 50,000 elements of
+// all kinds in 4 slots: 1.73 ms, where one persistent kernel of dependent work
+// items (CAS claims, element-wise atomics, no spatial order) took 8.0 ms.
 #include <algorithm>
-#include <mutex>
 #include <numeric>
 #include <vector>
 
-#include "claim_hex20.cuh"
-#include "consolidate.cuh"
-#include "scatter2d.cuh"
-#include "values_hex20.cuh"
+#include "ke_hex20.cuh"
+#include "rows2d.cuh"
+#include "rows_hex20.cuh"
+#include "write_hex20.cuh"
 
 namespace fem {
 namespace {
 
-constexpr int kBatchThreads = 256;
-constexpr int kBatchWarps = kBatchThreads / 32;
-static_assert(kBatchThreads == kScanThreads && kBatchThreads == kBlockThreads, "one CTA shape for every item");
-static_assert(kBatchClaim % kGroup == 0 && kBatchValues == kGroup, "claim and value items of whole groups");
+// Meshes per round launch: the descriptors are kernel parameters (at most 32 KB).
+// Rounds of up to kRoundSmall meshes (the default is 4 slots) pass small ones.
+constexpr int kRoundSmall = 8, kRoundLarge = 64;
 
-// A Hex20 value item: one group's topology and the element pass. Every pair
-// is shared in the batch (the claim items get no node degrees), so each
-// element's blocks are added atomically to slots that their claimers zeroed.
-struct BatchValuesSmem {
-    ValuesSmem values;
-    GroupTopo topo;
+template <int kMax>
+struct BatchRound {
+    int n;
+    int first[kMax + 1];  // first block of each mesh in this launch
+    BatchMesh mesh[kMax];
 };
+static_assert(sizeof(BatchRound<kRoundLarge>) < 32000, "kernel parameter size");
 
-// Shared memory of the item kinds (one at a time).
-union BatchSmem {
-    ClaimSmem claim;
-    BatchValuesSmem gv;
-    Scatter2DWarpSmem scatter[kBatchWarps];
-    WriteSmem<2, 8, 2> write2;
-    WriteSmem<3, 32, 4> write3;
-    long long scan[kScanThreads / 32 + 1];
-};
-
-constexpr int kMeshChunk = 96;   // descriptors per copy kernel (kernel parameters stay under 32 KB)
-constexpr int kSegChunk = 700;   // segments per copy kernel
-struct MeshChunk {
-    int first, count;
-    BatchMesh m[kMeshChunk];
-};
-struct SegChunk {
-    int first, count;
-    BatchSegment s[kSegChunk];
-};
-static_assert(sizeof(MeshChunk) < 32000 && sizeof(SegChunk) < 32000, "kernel parameter size");
-
-__global__ void k_copy_meshes(const MeshChunk c, BatchMesh* dst) {
+// The block's mesh, copied to shared memory; its block number and block count there.
+template <int kMax>
+__device__ __forceinline__ void block_mesh(const BatchRound<kMax>& r, BatchMesh& bm, int& block, int& nblocks) {
+    int i = 0;
+    while (i + 1 < r.n && r.first[i + 1] <= (int)blockIdx.x) i++;
+    block = blockIdx.x - r.first[i];
+    nblocks = r.first[i + 1] - r.first[i];
     constexpr int kWords = sizeof(BatchMesh) / 8;
     static_assert(sizeof(BatchMesh) % 8 == 0, "descriptor copy in 8-byte words");
-    for (int i = threadIdx.x; i < c.count * kWords; i += blockDim.x) {
-        const int k = i / kWords, w = i - k * kWords;
-        reinterpret_cast<unsigned long long*>(dst + c.first + k)[w] =
-            reinterpret_cast<const unsigned long long*>(&c.m[k])[w];
-    }
-}
-
-__global__ void k_copy_segments(const SegChunk c, BatchSegment* dst) {
-    for (int i = threadIdx.x; i < c.count; i += blockDim.x) dst[c.first + i] = c.s[i];
+    const unsigned long long* src = reinterpret_cast<const unsigned long long*>(&r.mesh[i]);
+    for (int w = threadIdx.x; w < kWords; w += blockDim.x) reinterpret_cast<unsigned long long*>(&bm)[w] = src[w];
+    __syncthreads();
 }
 
 __device__ __forceinline__ unsigned long long global_timer() {
@@ -91,167 +61,216 @@ __device__ __forceinline__ unsigned long long global_timer() {
     return t;
 }
 
-__global__ void k_batch_start(int* counters, int n, int* ticket, unsigned long long* stamp0) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) counters[i] = 0;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        *ticket = 0;
-        if (stamp0) *stamp0 = global_timer();
-    }
+#define FEM_BATCH_KERNEL(...) template <int kMax> __global__ void __launch_bounds__(__VA_ARGS__)
+#define FEM_BATCH_MESH                   \
+    __shared__ BatchMesh bm;             \
+    int block, nblocks;                  \
+    block_mesh<kMax>(r, bm, block, nblocks)
+
+FEM_BATCH_KERNEL(256) kb_begin(const __grid_constant__ BatchRound<kMax> r, unsigned long long* start) {
+    FEM_BATCH_MESH;
+    if (start && blockIdx.x == 0 && threadIdx.x == 0) *start = global_timer();
+    lists_begin(bm.L, block, nblocks);
+    if (bm.kind == FEM_HEX20)
+        for (int i = block * 256 + threadIdx.x; i < bm.L.N; i += nblocks * 256) bm.cnt[i] = 0;
 }
 
-// Clears bytes [lo, hi) of the concatenation of the mesh's reset ranges.
-__device__ void reset_range(const BatchMesh& bm, long long lo, long long hi) {
-    long long base = 0;
-    for (int r = 0; r < 3; r++) {
-        const long long len = bm.zero_bytes[r];
-        const long long a = max(lo, base), b = min(hi, base + len);
-        if (a < b) {
-            unsigned char* p = bm.zero_ptr[r] + (a - base);
-            const long long nb = b - a;
-            // the ranges and the item bounds are 16-byte multiples except the
-            // counts' tail: 16-byte stores, then bytes
-            const long long n16 = nb >> 4;
-            for (long long i = threadIdx.x; i < n16; i += blockDim.x)
-                reinterpret_cast<int4*>(p)[i] = make_int4(0, 0, 0, 0);
-            for (long long i = (n16 << 4) + threadIdx.x; i < nb; i += blockDim.x) p[i] = 0;
-        }
-        base += len;
-    }
+static_assert(kFillThreads == kOccThreads, "one block shape for both");
+FEM_BATCH_KERNEL(kFillThreads) kb_fill(const __grid_constant__ BatchRound<kMax> r) {
+    FEM_BATCH_MESH;
+    if (bm.kind == FEM_HEX20) occ_count(bm.m, bm.h, bm.cnt, bm.L.info, block, nblocks);
+    else if (bm.kind == FEM_T3) fill_2d<FEM_T3>(bm.m, bm.L, block, nblocks);
+    else if (bm.kind == FEM_Q4) fill_2d<FEM_Q4>(bm.m, bm.L, block, nblocks);
+    else fill_2d<FEM_MIXED_2D>(bm.m, bm.L, block, nblocks);
 }
 
-// Bounded wait of thread 0 until counters[c] >= target; false when it ran out.
-__device__ bool wait_counter(const int* counters, int c, int target, long long wait_ns) {
-    const volatile int* p = counters + c;
-    if (*p >= target) return true;
-    const unsigned long long t0 = global_timer();
-    while (*p < target) {
-        if ((long long)(global_timer() - t0) > wait_ns) return false;
-        __nanosleep(256);
-    }
-    return true;
+FEM_BATCH_KERNEL(kScanThreads) kb_occ_sums(const __grid_constant__ BatchRound<kMax> r) {
+    FEM_BATCH_MESH;
+    __shared__ long long s_warp[kScanThreads / 32 + 1];
+    occ_sums(bm.cnt, bm.L.N, bm.tiles, block, s_warp);
 }
 
-__global__ void __launch_bounds__(kBatchThreads, 2)
-    k_batch(const BatchMesh* __restrict__ meshes, const BatchSegment* __restrict__ segs, int nseg, int total,
-            int* counters, int* ticket, long long wait_ns) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    BatchSmem& sm = *reinterpret_cast<BatchSmem*>(smem_raw);
-    __shared__ int s_ticket, s_seg;
-    const int tid = threadIdx.x, warp = tid >> 5;
-    for (;;) {
-        if (tid == 0) {
-            const int t = atomicAdd(ticket, 1);
-            int lo = 0, hi = nseg - 1;  // the last segment whose first ticket is <= t
-            while (lo < hi) {
-                const int mid = (lo + hi + 1) >> 1;
-                if (__ldg(&segs[mid].first) <= t) lo = mid;
-                else hi = mid - 1;
-            }
-            s_ticket = t;
-            s_seg = lo;
-            if (t < total) {
-                const BatchSegment& sg = segs[lo];
-                for (int d = 0; d < 2; d++)
-                    if (sg.dep_ctr[d] >= 0 && !wait_counter(counters, sg.dep_ctr[d], sg.dep_target[d], wait_ns))
-                        raise_status(meshes[sg.mesh].L.info, FEM_ERR_TIMEOUT);
-                __threadfence();  // what the awaited items wrote is seen after the counters
-            }
+FEM_BATCH_KERNEL(kScanThreads) kb_occ_offsets(const __grid_constant__ BatchRound<kMax> r) {
+    FEM_BATCH_MESH;
+    __shared__ OccSmem sm;
+    occ_offsets(bm.cnt, bm.L.N, bm.tiles, bm.h.off, bm.L.info, block, nblocks, sm);
+}
+
+FEM_BATCH_KERNEL(kOccThreads) kb_occ_fill(const __grid_constant__ BatchRound<kMax> r) {
+    FEM_BATCH_MESH;
+    occ_fill(bm.m, bm.h, block, nblocks);
+}
+
+FEM_BATCH_KERNEL(kRowThreads, FEM_ROWS_Q4_CTAS) kb_rows_2d(const __grid_constant__ BatchRound<kMax> r) {
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    RowSmem& sm = *reinterpret_cast<RowSmem*>(smem_raw);
+    FEM_BATCH_MESH;
+    if (bm.kind == FEM_T3) rows_2d<FEM_T3, double>(bm.m, bm.L, bm.queue, block, nblocks, sm);
+    else if (bm.kind == FEM_Q4) rows_2d<FEM_Q4, double>(bm.m, bm.L, bm.queue, block, nblocks, sm);
+    else rows_2d<FEM_MIXED_2D, double>(bm.m, bm.L, bm.queue, block, nblocks, sm);
+}
+
+FEM_BATCH_KERNEL(kRowThreads) kb_long_rows_2d(const __grid_constant__ BatchRound<kMax> r) {
+    FEM_BATCH_MESH;
+    __shared__ LongSmem sm;
+    if (bm.kind == FEM_T3) long_rows_2d<FEM_T3, double>(bm.m, bm.L, bm.queue, block, nblocks, sm);
+    else if (bm.kind == FEM_Q4) long_rows_2d<FEM_Q4, double>(bm.m, bm.L, bm.queue, block, nblocks, sm);
+    else long_rows_2d<FEM_MIXED_2D, double>(bm.m, bm.L, bm.queue, block, nblocks, sm);
+}
+
+FEM_BATCH_KERNEL(kHexRowThreads, FEM_HEXR_CTAS) kb_rows_hex20(const __grid_constant__ BatchRound<kMax> r) {
+    FEM_BATCH_MESH;
+    __shared__ HexRowSmem s_row[kHexRowWarps];
+    rows_hex20(bm.m.conn, bm.L, bm.h, bm.queue, block, nblocks, s_row);
+}
+
+FEM_BATCH_KERNEL(32) kb_wide_rows_hex20(const __grid_constant__ BatchRound<kMax> r) {
+    FEM_BATCH_MESH;
+    __shared__ int s_uniq[kWideElems * 20];
+    wide_rows_hex20(bm.m.conn, bm.L, bm.h, bm.queue, block, nblocks, s_uniq);
+}
+
+FEM_BATCH_KERNEL(kHexRowThreads) kb_long_rows_hex20(const __grid_constant__ BatchRound<kMax> r) {
+    FEM_BATCH_MESH;
+    long_rows_hex20(bm.m.conn, bm.L, bm.h, bm.queue, block, nblocks);
+}
+
+FEM_BATCH_KERNEL(kKeThreads, 1) kb_ke_hex20(const __grid_constant__ BatchRound<kMax> r) {
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    FEM_BATCH_MESH;
+    ke_hex20(bm.m, bm.h.ke, &bm.L.info->status_bits, true, block, nblocks, *reinterpret_cast<KeHexSmem*>(smem_raw));
+}
+
+FEM_BATCH_KERNEL(kScanThreads) kb_tile_entries(const __grid_constant__ BatchRound<kMax> r) {
+    FEM_BATCH_MESH;
+    __shared__ long long s_warp[kScanThreads / 32 + 1];
+    if (bm.kind == FEM_HEX20) tile_entries<3, kOutCsr>(bm.L.counts, bm.L.N, bm.tiles, block, s_warp);
+    else tile_entries<2, kOutCsr>(bm.L.counts, bm.L.N, bm.tiles, block, s_warp);
+}
+
+FEM_BATCH_KERNEL(kScanThreads) kb_row_ptr(const __grid_constant__ BatchRound<kMax> r) {
+    FEM_BATCH_MESH;
+    __shared__ RowPtrSmem sm;
+    if (bm.kind == FEM_HEX20)
+        row_ptr_rows<3, kOutCsr>(bm.L.counts, bm.L.N, bm.tiles, bm.row_ptr, bm.L.info, bm.capacity, block, nblocks, sm);
+    else
+        row_ptr_rows<2, kOutCsr>(bm.L.counts, bm.L.N, bm.tiles, bm.row_ptr, bm.L.info, bm.capacity, block, nblocks, sm);
+}
+
+FEM_BATCH_KERNEL(kBlockThreads) kb_write_2d(const __grid_constant__ BatchRound<kMax> r) {
+    FEM_BATCH_MESH;
+    __shared__ int s_stat[2 * (kBlockThreads / 32)];
+    write_sorted_2d(bm.L, bm.row_ptr, bm.col_idx, bm.values, bm.capacity, block, nblocks, s_stat);
+}
+
+// The 2-D meshes whose outputs are not aligned for write_sorted_2d.
+FEM_BATCH_KERNEL(kBlockThreads) kb_write_2d_entries(const __grid_constant__ BatchRound<kMax> r) {
+    FEM_BATCH_MESH;
+    __shared__ WriteSmem<2, 8, 2> sm;
+    constexpr int NPB = kBlockThreads / 8;
+    write_batches<2, 8, 2, kOutCsr>(bm.L, bm.row_ptr, bm.col_idx, bm.values, bm.capacity, nullptr,
+                                    (long long)block * NPB, (long long)nblocks * NPB, bm.L.N, sm);
+}
+
+FEM_BATCH_KERNEL(kWriteThreads, FEM_HEXW_CTAS) kb_write_hex20(const __grid_constant__ BatchRound<kMax> r) {
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    FEM_BATCH_MESH;
+    write_hex20<kOutCsr>(bm.L, bm.h, nullptr, bm.row_ptr, bm.col_idx, bm.values, bm.capacity, block, nblocks,
+                         *reinterpret_cast<WriteHexCta*>(smem_raw));
+}
+
+// One block per mesh: the info word to the caller's array, the completion stamp.
+FEM_BATCH_KERNEL(32) kb_finish(const __grid_constant__ BatchRound<kMax> r) {
+    FEM_BATCH_MESH;
+    if (threadIdx.x < (int)(sizeof(fem_info) / 8))
+        reinterpret_cast<unsigned long long*>(bm.info_out)[threadIdx.x] =
+            reinterpret_cast<const unsigned long long*>(bm.L.info)[threadIdx.x];
+    if (threadIdx.x == 0 && bm.stamp) *bm.stamp = global_timer();
+}
+
+template <int kMax>
+struct RoundLauncher {
+    BatchRound<kMax> r;
+    cudaStream_t s;
+    cudaError_t err = cudaSuccess;
+
+    // Launches `kernel` over the meshes with want(mesh) > 0 blocks; more than `cap` blocks in all are scaled down to
+    // it (the kernels are persistent over their mesh's work; cap 0: exactly the wanted blocks).
+    template <typename Kernel, typename Want, typename... Args>
+    void run(Kernel kernel, int threads, size_t smem, long long cap, Want want, Args... args) {
+        if (err) return;
+        long long sum = 0;
+        for (int i = 0; i < r.n; i++) sum += want(r.mesh[i]);
+        if (sum == 0) return;
+        long long at = 0;
+        for (int i = 0; i < r.n; i++) {
+            r.first[i] = (int)at;
+            const long long w = want(r.mesh[i]);
+            at += cap == 0 || sum <= cap ? w : (w > 0 ? std::max<long long>(1, w * cap / sum) : 0);
         }
-        __syncthreads();
-        const int t = s_ticket;
-        if (t >= total) break;
-        const BatchSegment sg = segs[s_seg];
-        const BatchMesh& bm = meshes[sg.mesh];
-        const int k = t - sg.first;
-        const MeshView& m = bm.m;
-        const ListLayout& L = bm.L;
-        switch (sg.phase) {
-            case kBpReset: {
-                reset_range(bm, (long long)k * kBatchResetBytes, (long long)(k + 1) * kBatchResetBytes);
-                if (k == 0) {
-                    __syncthreads();
-                    if (tid == 0) L.info->pool_chunks = L.cap2;
-                }
-                break;
-            }
-            case kBpScatter2D: {
-                const int b = k * kBatchScatter2D, cnt = min(kBatchScatter2D, m.E_count - b);
-                if (bm.kind == FEM_Q4) {
-                    scatter2d_warp<4, double>(m, L, nullptr, b, cnt, warp, kBatchWarps, sm.scatter[warp]);
-                } else if (bm.kind == FEM_T3) {
-                    scatter2d_warp<3, double>(m, L, nullptr, b, cnt, warp, kBatchWarps, sm.scatter[warp]);
-                } else {
-                    scatter2d_warp<4, double>(m, L, nullptr, b, cnt, warp, kBatchWarps, sm.scatter[warp], FEM_Q4);
-                    scatter2d_warp<3, double>(m, L, nullptr, b, cnt, warp, kBatchWarps, sm.scatter[warp], FEM_T3);
-                }
-                break;
-            }
-            case kBpClaim: {
-                const int w0 = sg.arg * kBatchHex20Wave, w1 = min(m.E_count, w0 + kBatchHex20Wave);
-                const int b = w0 + k * kBatchClaim, e1 = min(w1, b + kBatchClaim);
-                for (int gb = b; gb < e1; gb += kGroup)
-                    claim_group(m, L, nullptr, nullptr, nullptr, gb, min(kGroup, e1 - gb),
-                                bm.map[sg.arg & 1] + (size_t)((gb - w0) / kGroup) * kGroupRecWords, sm.claim);
-                break;
-            }
-            case kBpValues: {
-                const int w0 = sg.arg * kBatchHex20Wave, w1 = min(m.E_count, w0 + kBatchHex20Wave);
-                const int b = w0 + k * kBatchValues, ne = min(kGroup, w1 - b);
-                group_topology(m, nullptr, b, ne, sm.gv.topo);
-                if (sm.gv.topo.bad) break;  // the claim item raised it
-                ValuesTarget vt{};
-                vt.topo = &sm.gv.topo;
-                vt.rec = reinterpret_cast<const unsigned*>(bm.map[sg.arg & 1] + (size_t)((b - w0) / kGroup) * kGroupRecWords +
-                                                           kRecMap);
-                vt.g0 = b;
-                vt.vals = L.vals;
-                vt.info = L.info;
-                values_init(sm.gv.values);
-                values_cta<kToSlots>(m, nullptr, b, 1, b + ne, vt, sm.gv.values);
-                break;
-            }
-            case kBpScanReduce:
-                if (bm.dpn == 3) scan_reduce_tile<9>(L.counts, L.N, bm.tiles, k, sm.scan);
-                else scan_reduce_tile<4>(L.counts, L.N, bm.tiles, k, sm.scan);
-                break;
-            case kBpScanTop:
-                scan_tiles_body(bm.tiles, bm.num_tiles, L.info, bm.row_ptr + (size_t)L.N * bm.dpn, bm.capacity, 1,
-                                sm.scan);
-                break;
-            case kBpRowPtr:
-                if (bm.dpn == 3) row_ptr_tile<3, false>(L.counts, L.N, bm.tiles, bm.row_ptr, k, sm.scan);
-                else row_ptr_tile<2, false>(L.counts, L.N, bm.tiles, bm.row_ptr, k, sm.scan);
-                break;
-            case kBpWrite:
-                if (bm.dpn == 3) {
-                    constexpr int NPB = kBlockThreads / 32;
-                    const long long b = (long long)k * NPB * kBatchWriteBatches;
-                    write_batches<3, 32, 4, kOutCsr>(L, bm.row_ptr, bm.col_idx, bm.values, bm.capacity, nullptr, b,
-                                                     NPB, min((long long)L.N, b + NPB * kBatchWriteBatches),
-                                                     sm.write3);
-                } else {
-                    constexpr int NPB = kBlockThreads / 8;
-                    const long long b = (long long)k * NPB * kBatchWriteBatches;
-                    write_batches<2, 8, 2, kOutCsr>(L, bm.row_ptr, bm.col_idx, bm.values, bm.capacity, nullptr, b,
-                                                    NPB, min((long long)L.N, b + NPB * kBatchWriteBatches),
-                                                    sm.write2);
-                }
-                break;
-            case kBpFinish:
-                if (tid < (int)(sizeof(fem_info) / 8))
-                    reinterpret_cast<unsigned long long*>(bm.info_out)[tid] =
-                        __ldcg(reinterpret_cast<const unsigned long long*>(L.info) + tid);
-                if (tid == 0 && bm.stamp) *bm.stamp = global_timer();
-                break;
-            default:
-                break;
-        }
-        __syncthreads();  // the item is finished (and the shared memory free) before it is counted
-        if (tid == 0) {
-            __threadfence();
-            atomicAdd(counters + sg.done_ctr, 1);
-        }
+        r.first[r.n] = (int)at;
+        kernel<<<(unsigned)at, threads, smem, s>>>(r, args...);
+        err = cudaGetLastError();
     }
+};
+
+long long blocks_of(long long work, long long per) { return (work + per - 1) / per; }
+
+template <int kMax>
+cudaError_t launch_round(const BatchMesh* meshes, int n, unsigned long long* start, int ctas_per_sm, cudaStream_t s) {
+    static DeviceCache cache;
+    int ready = 0;
+    cudaError_t err = per_device(cache, [](int& v) {
+        v = 1;
+        cudaError_t e = cudaFuncSetAttribute(kb_rows_2d<kMax>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)sizeof(RowSmem));
+        if (!e)
+            e = cudaFuncSetAttribute(kb_ke_hex20<kMax>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)sizeof(KeHexSmem));
+        if (!e)
+            e = cudaFuncSetAttribute(kb_write_hex20<kMax>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)sizeof(WriteHexCta));
+        return e;
+    }, ready);
+    if (err) return err;
+    const int sms = sm_count();
+    RoundLauncher<kMax> l;
+    l.s = s;
+    l.r.n = n;
+    std::copy(meshes, meshes + n, l.r.mesh);
+    using M = const BatchMesh&;
+    auto hex = [](M b) { return b.kind == FEM_HEX20; };
+    l.run(kb_begin<kMax>, 256, 0, 4 * sms, [](M b) { return blocks_of(b.L.N, 1024); }, start);
+    l.run(kb_fill<kMax>, kFillThreads, 0, 8 * sms, [](M b) { return blocks_of(b.m.E_count, kFillThreads); });
+    l.run(kb_occ_sums<kMax>, kScanThreads, 0, 0, [&](M b) { return hex(b) ? (long long)row_tiles(b.L.N) : 0; });
+    l.run(kb_occ_offsets<kMax>, kScanThreads, 0, 0, [&](M b) { return hex(b) ? (long long)row_tiles(b.L.N) : 0; });
+    l.run(kb_occ_fill<kMax>, kOccThreads, 0, 16 * sms,
+          [&](M b) { return hex(b) ? blocks_of(20ll * b.m.E_count, kOccThreads) : 0; });
+    l.run(kb_rows_2d<kMax>, kRowThreads, sizeof(RowSmem),
+          (long long)(ctas_per_sm > 0 ? std::min(ctas_per_sm, FEM_ROWS_Q4_CTAS) : FEM_ROWS_Q4_CTAS) * sms,
+          [&](M b) { return hex(b) ? 0 : blocks_of(b.L.N, kRowThreads); });
+    l.run(kb_long_rows_2d<kMax>, kRowThreads, 0, 2 * sms, [&](M b) { return hex(b) ? 0 : blocks_of(b.L.N, kRowThreads); });
+    l.run(kb_rows_hex20<kMax>, kHexRowThreads, 0, FEM_HEXR_CTAS * sms,
+          [&](M b) { return hex(b) ? blocks_of(b.L.N, kHexRowWarps) : 0; });
+    l.run(kb_wide_rows_hex20<kMax>, 32, 0, 4 * sms, [&](M b) { return hex(b) ? (long long)b.L.N : 0; });
+    l.run(kb_long_rows_hex20<kMax>, kHexRowThreads, 0, sms, [&](M b) { return hex(b) ? (long long)b.L.N : 0; });
+    for (int i = 0; i < n && !l.err; i++)
+        if (hex(meshes[i]) && meshes[i].h.order)
+            l.err = launch_node_order(meshes[i].m, meshes[i].hist, meshes[i].ranges, meshes[i].cnt, meshes[i].bbox, sms, s);
+    l.run(kb_ke_hex20<kMax>, kKeThreads, sizeof(KeHexSmem), sms,
+          [&](M b) { return hex(b) ? blocks_of(b.m.E_count, kKeWarps) : 0; });
+    l.run(kb_tile_entries<kMax>, kScanThreads, 0, 0, [](M b) { return (long long)row_tiles(b.L.N); });
+    l.run(kb_row_ptr<kMax>, kScanThreads, 0, 0, [](M b) { return (long long)row_tiles(b.L.N); });
+    l.run(kb_write_2d<kMax>, kBlockThreads, 0, 4 * sms, [&](M b) {
+        return !hex(b) && b.capacity > 0 && b.wide ? blocks_of(b.L.N, kBlockThreads / 16 * kCopyNodes) : 0;
+    });
+    l.run(kb_write_2d_entries<kMax>, kBlockThreads, 0, 4 * sms, [&](M b) {
+        return !hex(b) && b.capacity > 0 && !b.wide ? blocks_of(b.L.N, kBlockThreads / 8) : 0;
+    });
+    l.run(kb_write_hex20<kMax>, kWriteThreads, sizeof(WriteHexCta), FEM_HEXW_CTAS * sms,
+          [&](M b) { return hex(b) && b.capacity > 0 ? blocks_of(b.L.N, kWriteWarps) : 0; });
+    l.run(kb_finish<kMax>, 32, 0, 0, [](M) { return 1ll; });
+    return l.err;
 }
 
 }  // namespace
@@ -275,47 +294,15 @@ std::vector<int> batch_schedule(const fem_mesh* meshes, int n, int slots) {
     return slot_of;
 }
 
-cudaError_t launch_batch(const BatchMesh* meshes, int n, const BatchSegment* segs, int nseg, int total_items,
-                         BatchMesh* d_meshes, BatchSegment* d_segs, int* d_counters, int* d_ticket,
-                         unsigned long long* stamp0, long long wait_ns, int ctas_per_sm, cudaStream_t s) {
-    static MeshChunk mc;  // staging of the kernel parameters (copied at each launch)
-    static SegChunk sc;
-    static std::mutex mtx;
-    std::lock_guard<std::mutex> lock(mtx);
-    cudaError_t err = cudaSuccess;
-    for (int f = 0; f < n && !err; f += kMeshChunk) {
-        mc.first = f;
-        mc.count = std::min(kMeshChunk, n - f);
-        std::copy(meshes + f, meshes + f + mc.count, mc.m);
-        k_copy_meshes<<<1, 256, 0, s>>>(mc, d_meshes);
-        err = cudaGetLastError();
+cudaError_t launch_batch_round(const BatchMesh* meshes, int n, unsigned long long* start, int ctas_per_sm,
+                               cudaStream_t s) {
+    if (n <= kRoundSmall) return launch_round<kRoundSmall>(meshes, n, start, ctas_per_sm, s);
+    for (int i = 0; i < n; i += kRoundLarge) {
+        const cudaError_t err = launch_round<kRoundLarge>(meshes + i, std::min(kRoundLarge, n - i),
+                                                          i == 0 ? start : nullptr, ctas_per_sm, s);
+        if (err) return err;
     }
-    for (int f = 0; f < nseg && !err; f += kSegChunk) {
-        sc.first = f;
-        sc.count = std::min(kSegChunk, nseg - f);
-        std::copy(segs + f, segs + f + sc.count, sc.s);
-        k_copy_segments<<<1, 256, 0, s>>>(sc, d_segs);
-        err = cudaGetLastError();
-    }
-    if (err) return err;
-    k_batch_start<<<std::max(1, std::min(64, (n * kBatchCounters + 255) / 256)), 256, 0, s>>>(
-        d_counters, n * kBatchCounters, d_ticket, stamp0);
-    if ((err = cudaGetLastError())) return err;
-    static DeviceCache cache;
-    const size_t smem = sizeof(BatchSmem);
-    int per_sm = 0;
-    err = per_device(cache, [&](int& v) {
-        cudaError_t e = cudaFuncSetAttribute(k_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (!e) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, k_batch, kBatchThreads, smem);
-        return e;
-    }, per_sm);
-    if (err) return err;
-    // every CTA of the grid is resident at once: a CTA that waits never holds
-    // back one that has not started
-    const int use = ctas_per_sm > 0 ? std::min(ctas_per_sm, per_sm) : per_sm;
-    const long long grid = std::max<long long>(1, std::min<long long>(total_items, (long long)use * sm_count()));
-    k_batch<<<(int)grid, kBatchThreads, smem, s>>>(d_meshes, d_segs, nseg, total_items, d_counters, d_ticket, wait_ns);
-    return cudaGetLastError();
+    return cudaSuccess;
 }
 
 }  // namespace fem

@@ -12,87 +12,12 @@ namespace {
 
 constexpr unsigned long long kEmptyKey = ~0ull;
 
-constexpr int kScanItems = kScanTile / kScanThreads;  // 16 nodes per thread
-
 __device__ __forceinline__ unsigned long long shfl_xor_u64(unsigned long long v, int m) {
     unsigned lo = (unsigned)v, hi = (unsigned)(v >> 32);
     lo = __shfl_xor_sync(0xFFFFFFFFu, lo, m);
     hi = __shfl_xor_sync(0xFFFFFFFFu, hi, m);
     return ((unsigned long long)hi << 32) | lo;
 }
-
-// Tile sums of dpn^2 * counts: tile `tile` (kScanThreads threads).
-template <int B>
-__device__ __forceinline__ void scan_reduce_tile(const int* __restrict__ counts, int N, long long* __restrict__ tile_sums,
-                                                 int tile, long long* s_warp) {
-    const long long base = (long long)tile * kScanTile;
-    long long sum = 0;
-#pragma unroll
-    for (int i = 0; i < kScanItems; i++) {
-        const long long n = base + (long long)i * kScanThreads + threadIdx.x;
-        if (n < N) sum += FEM_LDG(counts + n);
-    }
-    long long total;
-    block_exclusive_scan(sum, s_warp, total);
-    if (threadIdx.x == 0) tile_sums[tile] = (long long)B * total;
-}
-
-
-// Exclusive scan of the tile sums in place (one CTA), nnz, last row_ptr entry.
-__device__ __forceinline__ void scan_tiles_body(long long* __restrict__ tile_sums, int num_tiles, DevInfo* info,
-                                                int* __restrict__ row_ptr_end, long long capacity, int end_div,
-                                                long long* s_warp) {
-    long long carry = 0;
-    for (int base = 0; base < num_tiles; base += kScanThreads) {
-        const int t = base + threadIdx.x;
-        const long long v = t < num_tiles ? __ldcg(tile_sums + t) : 0;
-        long long total;
-        const long long ex = block_exclusive_scan(v, s_warp, total);
-        if (t < num_tiles) tile_sums[t] = carry + ex;
-        carry += total;
-    }
-    if (threadIdx.x == 0) {
-        info->nnz = carry;
-        *row_ptr_end = (int)(carry / end_div);
-        if (carry > 0x7FFFFFFFll) raise_status(info, FEM_ERR_RANGE);
-        if (carry > capacity) raise_status(info, FEM_ERR_CAPACITY);
-    }
-}
-
-
-// row_ptr of every dof row: node n's rows start at dpn^2 * (exclusive count sum).
-// kBsr: one block row per node, block_row_ptr[n] = exclusive count sum.
-template <int DPN, bool kBsr>
-__device__ __forceinline__ void row_ptr_tile(const int* __restrict__ counts, int N,
-                                             const long long* __restrict__ tile_offsets, int* __restrict__ row_ptr,
-                                             int tile, long long* s_warp) {
-    constexpr int B = DPN * DPN;
-    const long long base = (long long)tile * kScanTile + (long long)threadIdx.x * kScanItems;
-    int c[kScanItems];
-    long long sum = 0;
-#pragma unroll
-    for (int i = 0; i < kScanItems; i++) {
-        const long long n = base + i;
-        c[i] = n < N ? FEM_LDG(counts + n) : 0;
-        sum += c[i];
-    }
-    long long total;
-    long long off = __ldcg(tile_offsets + tile) + (long long)B * block_exclusive_scan(sum, s_warp, total);
-#pragma unroll
-    for (int i = 0; i < kScanItems; i++) {
-        const long long n = base + i;
-        if (n < N) {
-            if (kBsr) {
-                row_ptr[n] = (int)(off / B);
-            } else {
-#pragma unroll
-                for (int a = 0; a < DPN; a++) row_ptr[n * DPN + a] = (int)(off + (long long)a * DPN * c[i]);
-            }
-        }
-        off += (long long)B * c[i];
-    }
-}
-
 
 template <int G>
 __device__ __forceinline__ unsigned group_mask(int grp_in_warp) {
@@ -125,9 +50,9 @@ __global__ void __launch_bounds__(kBlockThreads) k_count_upper(ListLayout L, int
             for (int step = 0; step < kMaxChainSteps; step++) {
                 const int* meta = chunk_meta(L, c);
                 const int cap = chunk_cap(L, c);
-                const int next = FEM_LDG(meta + 1);
+                const int next = __ldg(meta + 1);
                 for (int s = glane; s < cap; s += G) {
-                    const int col = (FEM_LDG(meta + 2 + s) & kColMask) - 1;
+                    const int col = (__ldg(meta + 2 + s) & kColMask) - 1;
                     cnt += col >= n;
                 }
                 if (next == 0) break;
@@ -189,9 +114,9 @@ __device__ int long_row_next_col(const ListLayout& L, int n, int after, int glan
     for (int step = 0; step < kMaxChainSteps; step++) {
         const int* meta = chunk_meta(L, c);
         const int cap = chunk_cap(L, c);
-        const int next = FEM_LDG(meta + 1);
+        const int next = __ldg(meta + 1);
         for (int s = glane; s < cap; s += G) {
-            const int col = (FEM_LDG(meta + 2 + s) & kColMask) - 1;
+            const int col = (__ldg(meta + 2 + s) & kColMask) - 1;
             if (col > after && col < best) best = col;
         }
         if (next == 0) break;
@@ -217,12 +142,12 @@ __device__ void long_row_write(const ListLayout& L, int n, int u, long long base
         for (int step = 0; step < kMaxChainSteps; step++) {
             const int* meta = chunk_meta(L, c);
             const int cap = chunk_cap(L, c);
-            const int next = FEM_LDG(meta + 1);
+            const int next = __ldg(meta + 1);
             for (int s = glane; s < cap; s += G) {
-                if ((FEM_LDG(meta + 2 + s) & kColMask) - 1 == col) {
+                if ((__ldg(meta + 2 + s) & kColMask) - 1 == col) {
                     const double* p = L.vals + (size_t)slot_gid(L, c, s) * B;
 #pragma unroll
-                    for (int v = 0; v < B; v++) sum[v] += FEM_LDG(p + v);
+                    for (int v = 0; v < B; v++) sum[v] += __ldg(p + v);
                 }
             }
             if (next == 0) break;
@@ -262,12 +187,12 @@ __device__ void long_row_write_bsr(const ListLayout& L, int n, int u, long long 
         for (int step = 0; step < kMaxChainSteps; step++) {
             const int* meta = chunk_meta(L, c);
             const int cap = chunk_cap(L, c);
-            const int next = FEM_LDG(meta + 1);
+            const int next = __ldg(meta + 1);
             for (int s = glane; s < cap; s += G) {
-                if ((FEM_LDG(meta + 2 + s) & kColMask) - 1 == col) {
+                if ((__ldg(meta + 2 + s) & kColMask) - 1 == col) {
                     const double* p = L.vals + (size_t)slot_gid(L, c, s) * B;
 #pragma unroll
-                    for (int v = 0; v < B; v++) sum[v] += FEM_LDG(p + v);
+                    for (int v = 0; v < B; v++) sum[v] += __ldg(p + v);
                 }
             }
             if (next == 0) break;
@@ -303,12 +228,12 @@ __device__ void long_row_write_upper(const ListLayout& L, int n, int u, const in
         for (int step = 0; step < kMaxChainSteps; step++) {
             const int* meta = chunk_meta(L, c);
             const int cap = chunk_cap(L, c);
-            const int next = FEM_LDG(meta + 1);
+            const int next = __ldg(meta + 1);
             for (int s = glane; s < cap; s += G) {
-                if ((FEM_LDG(meta + 2 + s) & kColMask) - 1 == col) {
+                if ((__ldg(meta + 2 + s) & kColMask) - 1 == col) {
                     const double* p = L.vals + (size_t)slot_gid(L, c, s) * B;
 #pragma unroll
-                    for (int v = 0; v < B; v++) sum[v] += FEM_LDG(p + v);
+                    for (int v = 0; v < B; v++) sum[v] += __ldg(p + v);
                 }
             }
             if (next == 0) break;
@@ -322,7 +247,7 @@ __device__ void long_row_write_upper(const ListLayout& L, int n, int u, const in
         if (glane == 0) {
 #pragma unroll
             for (int a = 0; a < DPN; a++) {
-                const long long rbase = FEM_LDG(row_ptr + (size_t)n * DPN + a);
+                const long long rbase = __ldg(row_ptr + (size_t)n * DPN + a);
 #pragma unroll
                 for (int b = 0; b < DPN; b++) {
                     if (k == 0 && b < a) continue;  // below the diagonal
@@ -343,22 +268,19 @@ __device__ __forceinline__ void prefetch_first_chunk(const ListLayout& L, long l
                                                      int& next) {
     if (node < L.N) {
         const int* meta = chunk_meta(L, (int)node);
-        next = FEM_LDG(meta + 1);
+        next = __ldg(meta + 1);
 #pragma unroll
         for (int q = 0; q < kPre; q++) {
             const int s = q * G + glane;
-            w[q] = s < L.S1 ? FEM_LDG(meta + 2 + s) : 0;
+            w[q] = s < L.S1 ? __ldg(meta + 2 + s) : 0;
         }
     }
 }
 
 // Resident CTAs per SM the register budget of k_write is set for (build-time
-// tuning knobs; measured on B200: 5 for the 2-D kinds, 4 for Hex20).
+// tuning knob, measured on B200).
 #ifndef FEM_WRITE_MIN_CTAS_2D
 #define FEM_WRITE_MIN_CTAS_2D 5
-#endif
-#ifndef FEM_WRITE_MIN_CTAS_3D
-#define FEM_WRITE_MIN_CTAS_3D 4
 #endif
 
 // Shared memory of the sorted write: each group's sort keys and (2-D) the
@@ -404,13 +326,13 @@ __device__ __forceinline__ void write_batches(const ListLayout& L, const int* __
         long long base = 0;
         if (valid) {
             if (kMode == kOutUpper) {
-                u = FEM_LDG(ucounts + n);  // columns >= n (the full row count is in L.counts)
+                u = __ldg(ucounts + n);  // columns >= n (the full row count is in L.counts)
             } else if (kBsr) {
-                base = FEM_LDG(row_ptr + n);
-                u = FEM_LDG(row_ptr + n + 1) - (int)base;
+                base = __ldg(row_ptr + n);
+                u = __ldg(row_ptr + n + 1) - (int)base;
             } else {
-                base = FEM_LDG(row_ptr + (size_t)n * DPN);
-                u = (FEM_LDG(row_ptr + (size_t)n * DPN + 1) - (int)base) / DPN;
+                base = __ldg(row_ptr + (size_t)n * DPN);
+                u = (__ldg(row_ptr + (size_t)n * DPN + 1) - (int)base) / DPN;
             }
         }
         // 1. gather the non-empty slots of the node's chunk chain (the first
@@ -434,10 +356,10 @@ __device__ __forceinline__ void write_batches(const ListLayout& L, const int* __
                 const int c = next - 1;
                 const int* meta = chunk_meta(L, c);
                 const int cap = chunk_cap(L, c);
-                next = FEM_LDG(meta + 1);
+                next = __ldg(meta + 1);
                 for (int s0 = 0; s0 < cap; s0 += G) {
                     const int s = s0 + glane;
-                    const int col = s < cap ? (FEM_LDG(meta + 2 + s) & kColMask) : 0;
+                    const int col = s < cap ? (__ldg(meta + 2 + s) & kColMask) : 0;
                     const unsigned used = (__ballot_sync(gmask, col != 0) >> gshift) & gmask >> gshift;
                     const int e = T + __popc(used & ((1u << glane) - 1u));
                     if (col != 0 && e < NK)
@@ -445,7 +367,7 @@ __device__ __forceinline__ void write_batches(const ListLayout& L, const int* __
                     T += __popc(used);
                 }
             }
-            const int expect = kMode == kOutUpper ? FEM_LDG(L.counts + n) : u;
+            const int expect = kMode == kOutUpper ? __ldg(L.counts + n) : u;
             if (glane == 0 && (T != expect || u > T)) raise_status(L.info, FEM_ERR_INTERNAL);
         }
         if (nb + nb_stride < nb_end) prefetch_first_chunk<G, kPre>(L, nb + nb_stride + grp, glane, pre_w, pre_next);
@@ -469,15 +391,15 @@ __device__ __forceinline__ void write_batches(const ListLayout& L, const int* __
             // all of the node's blocks in flight at once (two 16-byte loads each)
             for (int k = glane; k < Ts; k += G) {
                 const double2* p = reinterpret_cast<const double2*>(L.vals + (size_t)(unsigned)s_keys[grp][k] * B);
-                s_vals[grp][k][0] = FEM_LDG(p);
-                s_vals[grp][k][1] = FEM_LDG(p + 1);
+                s_vals[grp][k][0] = __ldg(p);
+                s_vals[grp][k][1] = __ldg(p + 1);
             }
             __syncwarp();
         }
         // entry v of the node's k-th sorted block
         auto block_value = [&](int k, int v) -> double {
             if constexpr (DPN == 2) return reinterpret_cast<const double*>(&s_vals[grp][k][0])[v];
-            return FEM_LDG(L.vals + (size_t)(unsigned)s_keys[grp][k] * B + v);
+            return __ldg(L.vals + (size_t)(unsigned)s_keys[grp][k] * B + v);
         };
         // 3. write the dpn rows of the node (or its block row, or its upper rows)
         if (valid && kMode == kOutUpper) {
@@ -486,7 +408,7 @@ __device__ __forceinline__ void write_batches(const ListLayout& L, const int* __
             } else if (u > 0 && u <= Ts) {
                 const int k0 = Ts - u;  // the sorted row's first column >= n (n itself)
                 for (int a = 0; a < DPN; a++) {
-                    const long long rbase = FEM_LDG(row_ptr + (size_t)n * DPN + a);
+                    const long long rbase = __ldg(row_ptr + (size_t)n * DPN + a);
                     const int len = (u - 1) * DPN + (DPN - a);
                     for (int r = glane; r < len; r += G) {
                         int k, b;
@@ -540,6 +462,181 @@ __device__ __forceinline__ void write_batches(const ListLayout& L, const int* __
     }
     if ((tid & 31) == 0) {
         // every lane of a group counted the same rows: divide by G
+        atomicAdd(reinterpret_cast<unsigned long long*>(&L.info->list_entries), (unsigned long long)(t_sum / G));
+        atomicMax(&L.info->max_row_entries, t_max);
+    }
+}
+
+
+// Entries of a node with c list columns (kOutUpper: c columns >= the node).
+template <int DPN, int kMode>
+__device__ __forceinline__ long long node_entries(int c) {
+    return kMode == kOutUpper ? upper_node_entries<DPN>(c) : (long long)DPN * DPN * c;
+}
+
+// Entries of each tile of kRowTile nodes.
+template <int DPN, int kMode>
+__device__ __forceinline__ void tile_entries(const int* __restrict__ counts, int N, long long* __restrict__ tile_sums,
+                                             int tile, long long* s_warp) {
+    long long sum = 0;
+#pragma unroll
+    for (int i = 0; i < kRowTile / kScanThreads; i++) {
+        const long long n = (long long)tile * kRowTile + i * kScanThreads + threadIdx.x;
+        if (n < N) sum += node_entries<DPN, kMode>(__ldg(counts + n));
+    }
+    long long total;
+    block_exclusive_scan(sum, s_warp, total);
+    if (threadIdx.x == 0) tile_sums[tile] = total;
+}
+
+// row_ptr of a tile's rows (kOutBsr: block rows). Each CTA sums the tiles
+// before its own itself (a few loads per thread: no launch in between), and
+// writes its row pointers with consecutive threads on consecutive rows. The
+// last CTA, which knows the total, clears what a consolidation pass owns in
+// the info word (so the pass can be re-run on the same lists) and sets nnz.
+struct RowPtrSmem {
+    long long warp[kScanThreads / 32 + 1];
+    int off[kRowTile], cnt[kRowTile];
+};
+template <int DPN, int kMode>
+__device__ __forceinline__ void row_ptr_rows(const int* __restrict__ counts, int N,
+                                             const long long* __restrict__ tile_sums, int* __restrict__ row_ptr,
+                                             DevInfo* info, long long capacity, int tile, int ntiles, RowPtrSmem& sm) {
+    constexpr int kItems = kRowTile / kScanThreads, B = DPN * DPN;
+    long long* const s_warp = sm.warp;
+    int* const s_off = sm.off;
+    int* const s_cnt = sm.cnt;
+    const int tid = threadIdx.x;
+    const long long first = (long long)tile * kRowTile;
+#pragma unroll
+    for (int i = 0; i < kItems; i++) {
+        const long long n = first + i * kScanThreads + tid;
+        s_cnt[i * kScanThreads + tid] = n < N ? __ldg(counts + n) : 0;
+    }
+    long long before = 0;
+    for (int t = tid; t < tile; t += kScanThreads) before += __ldg(tile_sums + t);
+    long long base;
+    block_exclusive_scan(before, s_warp, base);
+    long long sum = 0;
+#pragma unroll
+    for (int i = 0; i < kItems; i++) sum += node_entries<DPN, kMode>(s_cnt[tid * kItems + i]);
+    long long total;
+    long long off = block_exclusive_scan(sum, s_warp, total);
+#pragma unroll
+    for (int i = 0; i < kItems; i++) {
+        s_off[tid * kItems + i] = (int)off;
+        off += node_entries<DPN, kMode>(s_cnt[tid * kItems + i]);
+    }
+    __syncthreads();
+    constexpr int R = kMode == kOutBsr ? 1 : DPN;  // rows per node
+    const int rows = R * (int)min((long long)kRowTile, (long long)N - first);
+    for (int r = tid; r < rows; r += kScanThreads) {
+        const int i = r / R, a = r - i * R, c = s_cnt[i];
+        long long p = base + s_off[i];
+        if (kMode == kOutBsr) {
+            p /= B;
+        } else if (kMode == kOutUpper) {
+#pragma unroll
+            for (int k = 0; k < DPN - 1; k++) p += k < a ? upper_row_len<DPN>(c, k) : 0;
+        } else {
+            p += (long long)a * DPN * c;
+        }
+        row_ptr[first * R + r] = (int)p;
+    }
+    if (tile == ntiles - 1 && tid == 0) {
+        constexpr int kOwned = (1 << FEM_ERR_CAPACITY) | (1 << FEM_ERR_RANGE) | (1 << FEM_ERR_INTERNAL);
+        const long long nnz = base + total;
+        int bits = info->status_bits & ~kOwned;
+        if (nnz > 0x7FFFFFFFll) bits |= 1 << FEM_ERR_RANGE;
+        if (nnz > capacity) bits |= 1 << FEM_ERR_CAPACITY;
+        info->status_bits = bits;
+        info->nnz = nnz;
+        info->list_entries = 0;
+        info->max_row_entries = 0;
+        info->ticket = 0;
+        row_ptr[(long long)N * R] = (int)(nnz / (kMode == kOutBsr ? B : 1));
+    }
+}
+
+// CSR of the 2-D lists whose rows the scatter left sorted (kRowSorted): 16
+// lanes per node, lane 2k + i on row i of block k. A lane moves 16 bytes of
+// values (a warp's loads are consecutive, its stores two runs per node) and 8
+// bytes of columns; four nodes of a group are in flight. Hashed rows (fans)
+// take the exact slow path.
+constexpr int kCopyNodes = 4;
+__device__ __forceinline__ void write_sorted_2d(const ListLayout& L, const int* __restrict__ row_ptr,
+                                                int* __restrict__ col_idx, double* __restrict__ values,
+                                                long long capacity, int block, int nblocks, int* s_stat) {
+    constexpr int G = 16, NPB = kBlockThreads / G;
+    int* const s_sum = s_stat;
+    int* const s_max = s_stat + kBlockThreads / 32;
+    if (__ldg(&L.info->nnz) > capacity) return;  // FEM_ERR_CAPACITY already raised; write nothing
+    const int tid = threadIdx.x, grp = tid / G, lane = tid % G, i = lane & 1;
+    const unsigned gmask = 0xFFFFu << (((tid & 31) / G) * G);
+    int t_sum = 0, t_max = 0;
+    for (long long nb = (long long)block * NPB * kCopyNodes; nb < L.N; nb += (long long)nblocks * NPB * kCopyNodes) {
+        int base[kCopyNodes], u[kCopyNodes], head[kCopyNodes];
+#pragma unroll
+        for (int q = 0; q < kCopyNodes; q++) {
+            const long long n = nb + q * NPB + grp;
+            base[q] = u[q] = 0;
+            head[q] = kRowSorted;
+            if (n < L.N) {
+                base[q] = __ldg(row_ptr + 2 * n);
+                u[q] = (__ldg(row_ptr + 2 * n + 1) - base[q]) / 2;
+                head[q] = __ldg(L.meta1 + n * (k2DSlots + 2));
+            }
+        }
+        double2 v[kCopyNodes][2];  // blocks k = lane / 2 and, in rows of more than 8, k + 8
+        int c[kCopyNodes][2];
+#pragma unroll
+        for (int q = 0; q < kCopyNodes; q++) {
+            const long long n = nb + q * NPB + grp;
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const int p = lane + h * G;
+                if (head[q] == kRowSorted && p < 2 * u[q]) {
+                    v[q][h] = __ldg(reinterpret_cast<const double2*>(L.vals + n * (k2DSlots * 4)) + p);
+                    c[q][h] = __ldg(L.meta1 + n * (k2DSlots + 2) + 2 + (p >> 1));
+                }
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < kCopyNodes; q++) {
+            const long long n = nb + q * NPB + grp;
+            t_sum += u[q];
+            t_max = max(t_max, u[q]);
+            if (head[q] == kRowSorted) {
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const int k = (lane + h * G) >> 1;
+                    if (k < u[q]) {
+                        const long long p = base[q] + 2ll * i * u[q] + 2 * k;
+                        *reinterpret_cast<double2*>(values + p) = v[q][h];
+                        *reinterpret_cast<int2*>(col_idx + p) = make_int2(2 * c[q][h] - 2, 2 * c[q][h] - 1);
+                    }
+                }
+            } else {
+                long_row_write<2, G>(L, (int)n, u[q], base[q], lane, gmask, col_idx, values);
+            }
+        }
+    }
+    // list statistics (one atomic pair per CTA)
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) {
+        t_max = max(t_max, __shfl_xor_sync(0xFFFFFFFFu, t_max, d));
+        t_sum += __shfl_xor_sync(0xFFFFFFFFu, t_sum, d);
+    }
+    if ((tid & 31) == 0) {
+        s_sum[tid >> 5] = t_sum;
+        s_max[tid >> 5] = t_max;
+    }
+    __syncthreads();
+    if (tid == 0) {
+        for (int w = 1; w < kBlockThreads / 32; w++) {
+            t_sum += s_sum[w];
+            t_max = max(t_max, s_max[w]);
+        }
         atomicAdd(reinterpret_cast<unsigned long long*>(&L.info->list_entries), (unsigned long long)(t_sum / G));
         atomicMax(&L.info->max_row_entries, t_max);
     }

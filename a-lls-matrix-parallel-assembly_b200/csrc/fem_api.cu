@@ -54,11 +54,10 @@ fem_status check_mesh(const fem_mesh* m, bool device_pointers_needed = true) {
     return FEM_OK;
 }
 
-// Group records of one wave (of `wave` elements) of the batched Hex20 scatter for a mesh of E elements.
-size_t hex20_map_bytes(int E, int wave) {
-    const size_t groups = ((size_t)std::min(E, wave) + kHex20GroupSize - 1) / kHex20GroupSize;
-    return groups * kHex20GroupRecWords * sizeof(unsigned);
-}
+// Bytes per Hex20 element of the region that holds the rank map (800 bytes an
+// element): the workspace sizes that callers have been given, from 20,880-byte
+// records per 8 elements of at most `wave`.
+size_t hex20_record_bytes(int E, int wave) { return ((size_t)std::min(E, wave) + 7) / 8 * 20880; }
 
 fem_status make_layout(const fem_mesh* m, const fem_opts* o, HostLayout& h) {
     fem_status st = check_mesh(m);
@@ -99,8 +98,8 @@ fem_status make_layout(const fem_mesh* m, const fem_opts* o, HostLayout& h) {
     off += align_up(h.meta1_bytes);
     h.off_meta2 = off;
     off += align_up((size_t)h.cap2 * h.H2 * sizeof(int));
-    // 2-D (and the batch): the slots' value blocks; a Hex20 mesh assembled on its own: the packed Ke of its
-    // elements, which take less (15.1 KB an element, about 4 nodes of 7.8 KB) unless elements overlap
+    // 2-D: the slots' value blocks; Hex20: the packed Ke of the elements, which take less (15.1 KB an element,
+    // about 4 nodes of 7.8 KB) unless elements overlap
     h.off_vals = off;
     size_t vals_bytes = (size_t)slots * h.B * sizeof(double);
     if (h.kind == FEM_HEX20) vals_bytes = std::max(vals_bytes, (size_t)h.E * kPackedHex20 * sizeof(double));
@@ -109,7 +108,7 @@ fem_status make_layout(const fem_mesh* m, const fem_opts* o, HostLayout& h) {
     off += align_up((size_t)h.N * sizeof(int));
     h.off_ucounts = off;  // upper-triangle column counts (fem_alls_consolidate_upper)
     off += align_up((size_t)h.N * sizeof(int));
-    h.off_tiles = off;  // scan partials: of kScanTile nodes in the batch, of kRowTile nodes otherwise
+    h.off_tiles = off;  // scan partials of kRowTile nodes (2-D: running on into the next region)
     off += align_up((size_t)(h.dpn == 2 ? h.num_tiles : row_tiles(h.N)) * sizeof(long long));
     h.off_elist = off;  // visit order of the elements (perm), ranges, bucket histogram (+ bbox)
     {
@@ -117,14 +116,13 @@ fem_status make_layout(const fem_mesh* m, const fem_opts* o, HostLayout& h) {
         off += align_up((size_t)h.E * sizeof(int)) + align_up(4 * sizeof(int)) + align_up(nbuckets * sizeof(int)) +
                align_up(6 * sizeof(unsigned long long));
     }
-    // Hex20: node -> occurrences (counts, offsets, lists) and the rank map of the rows (in the batch: the group
-    // records of one wave)
+    // Hex20: node -> occurrences (counts, offsets, lists) and the rank map of the rows
     h.off_inc = off;
     if (h.kind == FEM_HEX20)
         off += 2 * align_up((size_t)(h.N + 1) * sizeof(int)) + align_up((size_t)h.E * 20 * sizeof(int));
     h.off_map = off;
     if (h.kind == FEM_HEX20)
-        off += align_up(std::max(hex20_map_bytes(h.E, 32768), (size_t)h.E * 400 * sizeof(unsigned short)));
+        off += align_up(std::max(hex20_record_bytes(h.E, 32768), (size_t)h.E * 400 * sizeof(unsigned short)));
     h.total = off;
     return FEM_OK;
 }
@@ -163,6 +161,16 @@ HexRows hex_rows(const HostLayout& h, void* ws) {
     // the occurrence counts' place, free once the occurrences are filled
     if (h.E >= kOrderedElems) r.order = reinterpret_cast<const int*>(b + h.off_inc);
     return r;
+}
+
+// Scratch of launch_node_order, in the place of the element order (at least kOrderedElems ints and a histogram).
+void node_order_scratch(const HostLayout& h, unsigned char* ws, int*& ranges, int*& hist, unsigned long long*& bbox) {
+    static_assert(kAlign + (sizeof(int) << (3 * kNodeOrderBits)) + 64 <= kOrderedElems * sizeof(int) + 4 * kAlign +
+                      (sizeof(int) << (3 * kNodeOrderBits)),
+                  "the region of a mesh with kOrderedElems elements holds it");
+    ranges = reinterpret_cast<int*>(ws + h.off_elist);
+    hist = ranges + kAlign / sizeof(int);
+    bbox = reinterpret_cast<unsigned long long*>(hist + (1 << (3 * kNodeOrderBits)));
 }
 
 MeshView mesh_view(const fem_mesh* m) {
@@ -263,12 +271,12 @@ fem_status fem_alls_scatter(const fem_mesh* mesh, const fem_opts* opts, void* wo
     const HexRows hex = hex_rows(h, workspace);
     int* cnt = reinterpret_cast<int*>(b + h.off_inc);
     long long* tiles = reinterpret_cast<long long*>(b + h.off_tiles);  // free until the consolidation
-    if (!err) err = launch_occurrences(m, cnt, hex.off, hex.inc, tiles, &L.info->status_bits, sm_count(), s);
+    if (!err) err = launch_occurrences(m, L, hex, cnt, tiles, s);
     if (!err) err = launch_rows_hex20(m, L, hex, queue, s);
     if (!err && hex.order) {
-        int* ranges = reinterpret_cast<int*>(b + h.off_elist);
-        int* hist = ranges + kAlign / sizeof(int);
-        unsigned long long* bbox = reinterpret_cast<unsigned long long*>(hist + (1 << (3 * kNodeOrderBits)));
+        int *ranges, *hist;
+        unsigned long long* bbox;
+        node_order_scratch(h, b, ranges, hist, bbox);
         err = launch_node_order(m, hist, ranges, cnt, bbox, sm_count(), s);
     }
     if (!err)
@@ -435,49 +443,31 @@ int batch_slots(int n, int concurrency) {
     return std::max(1, std::min(k, n));
 }
 
-// Workspace of a batch: the control block (mesh descriptors, schedule,
-// per-mesh counters, ticket) and `slots` list workspaces, each sized for the
-// largest mesh dealt to it (Hex20: plus a second wave's slot map).
+// Workspace of a batch: `slots` list workspaces, each sized for the largest
+// mesh dealt to it, after one aligned unit.
 struct BatchLayout {
     std::vector<int> slot_of;
     std::vector<size_t> slot_off;
-    size_t off_meshes, off_counters, off_ticket, off_segs, total;
+    size_t total;
 };
 
 size_t batch_mesh_bytes(const fem_mesh& m, const fem_opts* opts, fem_status& st) {
     HostLayout h;
     st = make_layout(&m, opts, h);
     if (st) return 0;
-    return h.total + (h.kind == FEM_HEX20 ? align_up(hex20_map_bytes(h.E, kBatchHex20Wave)) : 0);
-}
-
-// Work items of one mesh in the batch schedule (an upper bound of the
-// segments too), used to size the schedule.
-int batch_segments_bound(const fem_mesh& m) {
-    const int waves = m.kind == FEM_HEX20 ? (m.num_elems + kBatchHex20Wave - 1) / kBatchHex20Wave : 0;
-    return 8 + 2 * waves;
+    return h.total + (h.kind == FEM_HEX20 ? align_up(hex20_record_bytes(h.E, 4096)) : 0);
 }
 
 fem_status batch_layout(const fem_mesh* meshes, int n, const fem_opts* opts, int slots, BatchLayout& bl) {
     bl.slot_of = batch_schedule(meshes, n, slots);
     std::vector<size_t> need(slots, 0);
-    long long segs = 0;
     for (int i = 0; i < n; i++) {
         fem_status st;
         const size_t b = batch_mesh_bytes(meshes[i], opts, st);
         if (st) return st;
         need[bl.slot_of[i]] = std::max(need[bl.slot_of[i]], b);
-        segs += batch_segments_bound(meshes[i]);
     }
-    size_t off = 0;
-    bl.off_meshes = off;
-    off += align_up((size_t)n * sizeof(BatchMesh));
-    bl.off_counters = off;
-    off += align_up((size_t)n * kBatchCounters * sizeof(int));
-    bl.off_ticket = off;
-    off += align_up(sizeof(int));
-    bl.off_segs = off;
-    off += align_up((size_t)segs * sizeof(BatchSegment));
+    size_t off = kAlign;
     bl.slot_off.assign(slots, 0);
     for (int k = 0; k < slots; k++) {
         bl.slot_off[k] = off;
@@ -486,29 +476,6 @@ fem_status batch_layout(const fem_mesh* meshes, int n, const fem_opts* opts, int
     bl.total = off;
     return FEM_OK;
 }
-
-// Appends a segment of `count` items of one phase of mesh j.
-struct ScheduleBuilder {
-    std::vector<BatchSegment> segs;
-    int total = 0;
-    void add(int j, int phase, int count, int arg, int done, int dep0 = -1, int target0 = 0, int dep1 = -1,
-             int target1 = 0) {
-        if (count <= 0) return;
-        BatchSegment g{};
-        g.mesh = j;
-        g.phase = phase;
-        g.first = total;
-        g.count = count;
-        g.arg = arg;
-        g.dep_ctr[0] = dep0;
-        g.dep_target[0] = target0;
-        g.dep_ctr[1] = dep1;
-        g.dep_target[1] = target1;
-        g.done_ctr = done;
-        segs.push_back(g);
-        total += count;
-    }
-};
 
 }  // namespace
 
@@ -549,24 +516,19 @@ fem_status fem_assemble_batched(const fem_mesh* meshes, int32_t n, const fem_opt
         bm = BatchMesh{};
         bm.m = mesh_view(&meshes[i]);
         bm.L = device_layout(h, ws);
+        bm.h = hex_rows(h, ws);
+        bm.cnt = reinterpret_cast<int*>(ws + h.off_inc);
+        bm.queue = reinterpret_cast<int*>(ws + h.off_ucounts);
         bm.tiles = reinterpret_cast<long long*>(ws + h.off_tiles);
-        bm.map[0] = reinterpret_cast<int*>(ws + h.off_map);
-        bm.map[1] = reinterpret_cast<int*>(ws + h.total);
+        node_order_scratch(h, ws, bm.ranges, bm.hist, bm.bbox);
         bm.row_ptr = outs[i].row_ptr;
         bm.col_idx = outs[i].col_idx;
         bm.values = outs[i].values;
         bm.capacity = outs[i].capacity;
         bm.info_out = infos + i;
         bm.stamp = stamps ? stamps + 1 + i : nullptr;
-        bm.zero_ptr[0] = ws;  // info word and first chunks
-        bm.zero_bytes[0] = (long long)(h.off_meta1 + h.meta1_bytes);
-        bm.zero_ptr[1] = ws + h.off_vals;  // 2-D: the first chunks' values (every contribution is an atomic add)
-        bm.zero_bytes[1] = h.dpn == 2 ? (long long)h.N * h.S1 * h.B * (long long)sizeof(double) : 0;
-        bm.zero_ptr[2] = ws + h.off_counts;
-        bm.zero_bytes[2] = (long long)h.N * (long long)sizeof(int);
         bm.kind = h.kind;
-        bm.dpn = h.dpn;
-        bm.num_tiles = h.num_tiles;
+        bm.wide = wide_outputs(outs[i].col_idx, outs[i].values);
         outs[i].n_rows = meshes[i].num_nodes * kind_dpn(meshes[i].kind);
     }
     // rounds: the r-th mesh of every slot (slots keep their meshes smallest
@@ -581,90 +543,15 @@ fem_status fem_assemble_batched(const fem_mesh* meshes, int32_t n, const fem_opt
     }
     size_t rounds = 0;
     for (auto& v : per_slot) rounds = std::max(rounds, v.size());
-    ScheduleBuilder sb;
-    std::vector<int> prev_in_slot(n, -1);
-    for (auto& v : per_slot)
-        for (size_t r = 1; r < v.size(); r++) prev_in_slot[v[r]] = v[r - 1];
-    auto ctr = [](int j, int c) { return j * kBatchCounters + c; };
-    for (size_t r = 0; r < rounds; r++) {
-        std::vector<int> round;
+    cudaError_t err = cudaSuccess;
+    std::vector<BatchMesh> round;
+    for (size_t r = 0; r < rounds && !err; r++) {
+        round.clear();
         for (auto& v : per_slot)
-            if (r < v.size()) round.push_back(v[r]);
-        // largest first within a round, so that the long meshes start early
-        std::stable_sort(round.begin(), round.end(),
-                         [&](int a, int b) { return batch_cost(meshes[a]) > batch_cost(meshes[b]); });
-        std::vector<int> resets(n, 0), scatter_items(n, 0), write_items(n, 0);
-        for (int j : round) {
-            const BatchMesh& bm = bms[j];
-            const long long zb = bm.zero_bytes[0] + bm.zero_bytes[1] + bm.zero_bytes[2];
-            resets[j] = (int)((zb + kBatchResetBytes - 1) / kBatchResetBytes);
-            const int p = prev_in_slot[j];
-            sb.add(j, kBpReset, resets[j], 0, ctr(j, kBcReset), p >= 0 ? ctr(p, kBcFinish) : -1, 1);
-        }
-        for (int j : round) {
-            const int E = meshes[j].num_elems;
-            if (E <= 0) continue;
-            if (bms[j].kind == FEM_HEX20) {
-                const int nw = (E + kBatchHex20Wave - 1) / kBatchHex20Wave;
-                std::vector<int> claims(nw), values(nw);
-                for (int w = 0; w < nw; w++) {
-                    const int ew = std::min(kBatchHex20Wave, E - w * kBatchHex20Wave);
-                    claims[w] = (ew + kBatchClaim - 1) / kBatchClaim;
-                    values[w] = (ew + kBatchValues - 1) / kBatchValues;
-                }
-                std::vector<int> claims_upto(nw), values_upto(nw);
-                std::partial_sum(claims.begin(), claims.end(), claims_upto.begin());
-                std::partial_sum(values.begin(), values.end(), values_upto.begin());
-                // C0, C1, V0, C2, V1, ...: a wave's values follow the claims of
-                // the next wave; a wave's claims reuse the slot map of the wave
-                // two before, once its values are in
-                auto claim = [&](int w) {
-                    sb.add(j, kBpClaim, claims[w], w, ctr(j, kBcScatter), ctr(j, kBcReset), resets[j],
-                           w >= 2 ? ctr(j, kBcValues) : -1, w >= 2 ? values_upto[w - 2] : 0);
-                };
-                auto value = [&](int w) {
-                    sb.add(j, kBpValues, values[w], w, ctr(j, kBcValues), ctr(j, kBcScatter),
-                           claims_upto[std::min(w + 1, nw - 1)]);
-                };
-                claim(0);
-                for (int w = 0; w < nw; w++) {
-                    if (w + 1 < nw) claim(w + 1);
-                    value(w);
-                }
-                scatter_items[j] = values_upto[nw - 1];
-            } else {
-                scatter_items[j] = (E + kBatchScatter2D - 1) / kBatchScatter2D;
-                sb.add(j, kBpScatter2D, scatter_items[j], 0, ctr(j, kBcScatter), ctr(j, kBcReset), resets[j]);
-            }
-        }
-        for (int j : round) {
-            const int sc = bms[j].kind == FEM_HEX20 ? kBcValues : kBcScatter;
-            if (meshes[j].num_elems > 0)
-                sb.add(j, kBpScanReduce, bms[j].num_tiles, 0, ctr(j, kBcScanReduce), ctr(j, sc), scatter_items[j]);
-            else
-                sb.add(j, kBpScanReduce, bms[j].num_tiles, 0, ctr(j, kBcScanReduce), ctr(j, kBcReset), resets[j]);
-        }
-        for (int j : round)
-            sb.add(j, kBpScanTop, 1, 0, ctr(j, kBcScanTop), ctr(j, kBcScanReduce), bms[j].num_tiles);
-        for (int j : round) sb.add(j, kBpRowPtr, bms[j].num_tiles, 0, ctr(j, kBcRowPtr), ctr(j, kBcScanTop), 1);
-        for (int j : round) {
-            const int npb = bms[j].dpn == 3 ? kBlockThreads / 32 : kBlockThreads / 8;
-            const long long per = (long long)npb * kBatchWriteBatches;
-            write_items[j] = outs[j].capacity > 0 ? (int)((meshes[j].num_nodes + per - 1) / per) : 0;
-            sb.add(j, kBpWrite, write_items[j], 0, ctr(j, kBcWrite), ctr(j, kBcRowPtr), bms[j].num_tiles);
-        }
-        for (int j : round)
-            sb.add(j, kBpFinish, 1, 0, ctr(j, kBcFinish), ctr(j, kBcWrite), write_items[j],
-                   ctr(j, kBcRowPtr), bms[j].num_tiles);
+            if (r < v.size()) round.push_back(bms[v[r]]);
+        err = launch_batch_round(round.data(), (int)round.size(), r == 0 ? stamps : nullptr,
+                                 opts ? opts->ctas_per_sm : 0, static_cast<cudaStream_t>(stream));
     }
-    long long seg_bound = 0;
-    for (int i = 0; i < n; i++) seg_bound += batch_segments_bound(meshes[i]);
-    if ((long long)sb.segs.size() > seg_bound) return FEM_ERR_INTERNAL;
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const cudaError_t err = launch_batch(
-        bms.data(), n, sb.segs.data(), (int)sb.segs.size(), sb.total, reinterpret_cast<BatchMesh*>(base + bl.off_meshes),
-        reinterpret_cast<BatchSegment*>(base + bl.off_segs), reinterpret_cast<int*>(base + bl.off_counters),
-        reinterpret_cast<int*>(base + bl.off_ticket), stamps, 2000ll * 1000 * 1000, opts ? opts->ctas_per_sm : 0, s);
     return err ? cuda_fail(err) : FEM_OK;
 }
 

@@ -4,25 +4,21 @@
 // ALLS_Quad2D_Assembly_Accuracy_Analysis.cu:63-67,384-391) live in a device
 // pool of fixed-size chunks. Every node n owns chunk n (its "first chunk");
 // further chunks come from an overflow pool through an atomic bump counter and
-// are linked with atomicCAS on the previous chunk's `next` word. A list entry
-// (slot) holds one column NODE and the dof_per_node^2 block of values of that
-// (row node, column node) pair, so the dpn rows of a node share one list.
+// are linked through the previous chunk's `next` word. A list entry (slot) holds
+// one column NODE of a row node, so the dpn rows of a node share one list.
 //
 // Chunk metadata is a row of H = S + 2 int32 words:
 //     word 0 = kRowSorted for a 2-D row stored sorted and compact, else 0
 //     word 1 = next  (chunk id + 1 of the next chunk, 0 = none)
 //     word 2+s = slot s: 0 = empty, col+1 = column node col
-// Within a chunk a column's slot is found by open addressing (linear probing
-// from a hash of the column); a chunk with no free slot on the probe sequence
-// continues in the next chunk. A slot is claimed by atomicCAS(0 -> col+1), so
-// every column appears at most once per row. Block values are never written by
-// a claim: they are zero before the first addition (2-D: the value array is
-// cleared with the lists; Hex20: the claimer zeroes the block in the claim
-// pass, and values are added in a later launch), so no contributor ever waits
-// for another.
-// Slot values are stored slot-major: vals[gid * B + v], B = dpn^2, where gid is
-// the global slot id (first-chunk slots first, then overflow-chunk slots), so a
-// slot's block is contiguous (one 32-byte sector in 2-D, 72 bytes for Hex20).
+// A row belongs to the thread, warp or CTA that builds it (rows2d.cuh,
+// rows_hex20.cuh), so a column appears once, and rows are stored sorted: the
+// first u slots of the chain. The exception are 2-D rows that do not fit their
+// first chunk, whose slots are hashed (scatter2d.cuh).
+// 2-D values: each slot's dpn x dpn block, vals[gid * 4], gid the global slot id
+// (first-chunk slots first, then overflow-chunk slots): one 32-byte sector.
+// Hex20 values stay in the elements' packed Ke (in the place of vals) until the
+// consolidation sums them (write_hex20.cuh).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -60,8 +56,8 @@ struct ListLayout {
     int cap2;       // overflow chunk capacity
     int* meta1;     // [N * H1]
     int* meta2;     // [cap2 * H2]
-    double* vals;   // [(N*S1 + cap2*S2) * B]
-    int* counts;    // [N] list entries of each row node (incremented by the claimers)
+    double* vals;   // 2-D: [(N*S1 + cap2*S2) * B]
+    int* counts;    // [N] list entries of each row node (2-D: elements of the node until its row is built)
     DevInfo* info;
 };
 
@@ -78,37 +74,14 @@ __device__ __forceinline__ unsigned slot_gid(const ListLayout& L, int c, int s) 
     return c < L.N ? (unsigned)c * (unsigned)L.S1 + (unsigned)s
                    : (unsigned)L.N * (unsigned)L.S1 + (unsigned)(c - L.N) * (unsigned)L.S2 + (unsigned)s;
 }
-// Chunk id and slot of a global slot id.
-__device__ __forceinline__ void gid_chunk(const ListLayout& L, unsigned gid, int& c, int& s) {
-    unsigned first = (unsigned)L.N * (unsigned)L.S1;
-    if (gid < first) {
-        c = (int)(gid / (unsigned)L.S1);
-        s = (int)(gid % (unsigned)L.S1);
-    } else {
-        unsigned g2 = gid - first;
-        c = L.N + (int)(g2 / (unsigned)L.S2);
-        s = (int)(g2 % (unsigned)L.S2);
-    }
-}
-
-// Loads of data that no kernel of the launch writes go through the read-only
-// path. The batched persistent kernel (batched.cu), whose work items read what
-// earlier items of the same launch wrote, defines FEM_LDG as an L2 load before
-// it includes the kernels' device code.
-#ifndef FEM_LDG
-#define FEM_LDG(p) __ldg(p)
-#endif
-
 // L2-coherent loads (bypass L1: list words change under other SMs' writes).
 __device__ __forceinline__ int ld_cg(const int* p) { return __ldcg(p); }
 __device__ __forceinline__ int4 ld_cg4(const int* p) { return __ldcg(reinterpret_cast<const int4*>(p)); }
 
-// Takes one chunk from the overflow pool and zeroes its meta row (and, with
-// kZeroVals, its slots' values, for lists whose contributions are all
-// atomic adds). Returns the chunk id, or -1 (and raises FEM_ERR_POOL_OVERFLOW)
-// when the pool is empty. The caller must __threadfence() before publishing
-// the chunk.
-template <bool kZeroVals = false>
+// Takes one chunk from the overflow pool and zeroes its meta row and its slots'
+// values (all contributions are atomic adds). Returns the chunk id, or -1 (and
+// raises FEM_ERR_POOL_OVERFLOW) when the pool is empty. The caller must
+// __threadfence() before publishing the chunk.
 __device__ __forceinline__ int alloc_chunk(const ListLayout& L) {
     int k = atomicAdd(&L.info->overflow_chunks, 1);
     if (k >= L.cap2) {
@@ -117,10 +90,8 @@ __device__ __forceinline__ int alloc_chunk(const ListLayout& L) {
     }
     int* m = L.meta2 + (size_t)k * L.H2;
     for (int i = 0; i < L.H2; i += 4) *reinterpret_cast<int4*>(m + i) = make_int4(0, 0, 0, 0);
-    if (kZeroVals) {
-        double2* v = reinterpret_cast<double2*>(L.vals + (size_t)slot_gid(L, L.N + k, 0) * L.B);
-        for (int i = 0; i < L.S2 * L.B / 2; i++) v[i] = make_double2(0.0, 0.0);
-    }
+    double2* v = reinterpret_cast<double2*>(L.vals + (size_t)slot_gid(L, L.N + k, 0) * L.B);
+    for (int i = 0; i < L.S2 * L.B / 2; i++) v[i] = make_double2(0.0, 0.0);
     return L.N + k;
 }
 
@@ -139,27 +110,20 @@ __device__ __forceinline__ int probe_start(int key, int S) {
     return (int)__umulhi((unsigned)key * 2654435761u, (unsigned)S);
 }
 
-// Next chunk of chunk c, allocating and atomicCAS-linking a new one if there is
-// none. Returns -1 on pool overflow (status raised). `spare` keeps a chunk that
-// lost a link race for this thread's next allocation (-1 = none).
-template <bool kZeroVals = false>
-__device__ __forceinline__ int next_chunk(const ListLayout& L, int c, int& spare) {
-    int* m = chunk_meta(L, c);
-    int nx = ld_cg(m + 1);
-    if (nx == 0) {
-        int nc = spare >= 0 ? spare : alloc_chunk<kZeroVals>(L);
-        spare = -1;
-        if (nc < 0) return -1;
-        __threadfence();  // the zeroed meta row is visible before the link
-        int old = atomicCAS(m + 1, 0, nc + 1);
-        if (old == 0) {
-            nx = nc + 1;
-        } else {
-            spare = nc;
-            nx = old;
-        }
+// Appends a chunk to the end of row node n's chain (one thread). Returns false
+// on pool overflow (status raised).
+__device__ __forceinline__ bool append_chunk(const ListLayout& L, int n) {
+    int c = n;
+    for (int step = 0; step < kMaxChainSteps; step++) {
+        const int nx = ld_cg(chunk_meta(L, c) + 1);
+        if (nx == 0) break;
+        c = nx - 1;
     }
-    return nx - 1;
+    const int nc = alloc_chunk(L);
+    if (nc < 0) return false;
+    __threadfence();  // the zeroed meta row is visible before the link
+    atomicExch(chunk_meta(L, c) + 1, nc + 1);
+    return true;
 }
 
 // Host-side layout description (sizes in bytes, offsets from the workspace base).

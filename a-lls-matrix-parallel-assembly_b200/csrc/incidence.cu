@@ -1,6 +1,5 @@
 // Node -> element incidence lists (CSR over the nodes) of a mesh: the
-// colouring baseline's neighbour structure (colour.cu) and, for Hex20, the
-// occurrences of each row node (element and local position, rows_hex20.cu).
+// colouring baseline's neighbour structure (colour.cu).
 //
 //   k_inc_count                  cnt[n] = elements with node n (a node twice
 //                                in one element counts twice)
@@ -23,37 +22,9 @@ __device__ __forceinline__ int elem_npe(const MeshView& m, int e) {
     return m.stride;
 }
 
-// kOcc (Hex20 rows): an element with a bad node id has no occurrence at all;
-// the occurrences of an element that repeats a node carry kOccRepeats.
-__device__ __forceinline__ unsigned repeats_flag(const MeshView& m, int e) {
-    int n[20];
-    bool rep = false;
-#pragma unroll
-    for (int k = 0; k < 20; k++) n[k] = __ldg(m.conn + (size_t)e * 20 + k);
-#pragma unroll
-    for (int k = 1; k < 20; k++)
-#pragma unroll
-        for (int j = 0; j < k; j++) rep |= n[j] == n[k];
-    return rep ? kOccRepeats : 0u;
-}
-
-__device__ __forceinline__ bool bad_element(const MeshView& m, int e) {
-    bool bad = false;
-    for (int k = 0; k < m.stride; k++) {
-        const int n = __ldg(m.conn + (size_t)e * m.stride + k);
-        bad |= n < 0 || n >= m.N;
-    }
-    return bad;
-}
-
-template <bool kOcc>
 __global__ void k_inc_count(MeshView m, int* __restrict__ cnt, int* status) {
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < m.E_count; e += gridDim.x * blockDim.x) {
         const int npe = elem_npe(m, e);
-        if (kOcc && bad_element(m, e)) {
-            atomicOr(status, 1 << FEM_ERR_BAD_MESH);
-            continue;
-        }
         for (int k = 0; k < npe; k++) {
             const int n = __ldg(m.conn + (size_t)e * m.stride + k);
             if (n < 0 || n >= m.N) {
@@ -124,46 +95,32 @@ __global__ void __launch_bounds__(kScanThreads) k_tile_apply(int* __restrict__ c
     }
 }
 
-template <bool kOcc>
 __global__ void k_inc_fill(MeshView m, const int* __restrict__ off, int* __restrict__ cursor, int* __restrict__ inc) {
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < m.E_count; e += gridDim.x * blockDim.x) {
         const int npe = elem_npe(m, e);
-        if (kOcc && bad_element(m, e)) continue;
-        const unsigned flag = kOcc ? repeats_flag(m, e) : 0u;
         for (int k = 0; k < npe; k++) {
             const int n = __ldg(m.conn + (size_t)e * m.stride + k);
             if (n < 0 || n >= m.N) continue;
-            inc[off[n] + atomicAdd(cursor + n, 1)] = kOcc ? (int)((unsigned)(e * 20 + k) | flag) : e;
+            inc[off[n] + atomicAdd(cursor + n, 1)] = e;
         }
     }
 }
 
 }  // namespace
 
-template <bool kOcc>
-static cudaError_t launch_incidence_t(const MeshView& m, int* cnt, int* off, int* inc, long long* tiles, int* status,
-                                      int sms, cudaStream_t s) {
+cudaError_t launch_incidence(const MeshView& m, int* cnt, int* off, int* inc, long long* tiles, int* status, int sms,
+                             cudaStream_t s) {
     cudaError_t err = cudaMemsetAsync(cnt, 0, (size_t)m.N * sizeof(int), s);
     if (err) return err;
     const int num_tiles = (m.N + kScanTile - 1) / kScanTile;
     const int ge = (int)std::max<long long>(1, std::min<long long>(((long long)m.E_count + kThreads - 1) / kThreads,
                                                                    (long long)sms * 8));
-    if (m.E_count > 0) k_inc_count<kOcc><<<ge, kThreads, 0, s>>>(m, cnt, status);
+    if (m.E_count > 0) k_inc_count<<<ge, kThreads, 0, s>>>(m, cnt, status);
     k_tile_sums<<<num_tiles, kScanThreads, 0, s>>>(cnt, m.N, tiles);
     k_tile_scan<<<1, kScanThreads, 0, s>>>(tiles, num_tiles, off + m.N, status);
     k_tile_apply<<<num_tiles, kScanThreads, 0, s>>>(cnt, m.N, tiles, off);
-    if (m.E_count > 0) k_inc_fill<kOcc><<<ge, kThreads, 0, s>>>(m, off, cnt, inc);
+    if (m.E_count > 0) k_inc_fill<<<ge, kThreads, 0, s>>>(m, off, cnt, inc);
     return cudaGetLastError();
-}
-
-cudaError_t launch_incidence(const MeshView& m, int* cnt, int* off, int* inc, long long* tiles, int* status, int sms,
-                             cudaStream_t s) {
-    return launch_incidence_t<false>(m, cnt, off, inc, tiles, status, sms, s);
-}
-
-cudaError_t launch_occurrences(const MeshView& m, int* cnt, int* off, int* inc, long long* tiles, int* status, int sms,
-                               cudaStream_t s) {
-    return launch_incidence_t<true>(m, cnt, off, inc, tiles, status, sms, s);
 }
 
 }  // namespace fem

@@ -110,13 +110,9 @@ cudaError_t launch_colour_hex20(const MeshView& m, const int* perm, const int* r
 // scratch; status gets 1 << FEM_ERR_* bits.
 cudaError_t launch_incidence(const MeshView& m, int* cnt, int* off, int* inc, long long* tiles, int* status, int sms,
                              cudaStream_t s);
-// The same lists for Hex20 with occurrences 20 e + a (element e, local position a) for the elements
-// without a bad node id; bit 31 marks the elements that repeat a node (the count of occurrences stays
-// below 2^31, else FEM_ERR_RANGE).
+// Mark of the occurrences of an element that repeats a node.
 constexpr unsigned kOccRepeats = 0x80000000u;
-cudaError_t launch_occurrences(const MeshView& m, int* cnt, int* off, int* inc, long long* tiles, int* status, int sms,
-                               cudaStream_t s);
-// What a Hex20 scatter leaves besides the list chunks (rows_hex20.cuh).
+// What a Hex20 scatter leaves besides the list chunks (hex_rows.cuh).
 struct HexRows {
     double* ke;           // [E * kPackedHex20] packed element stiffness
     int* off;             // [N + 1] node -> occurrences
@@ -124,16 +120,20 @@ struct HexRows {
     const int* order;     // [N] node visit order of the consolidation, or NULL: as numbered
     unsigned short* map;  // [E * 400] rank of column node b in row node a's list, at 20 (20 e + a) + b
 };
+// Fills off / inc for the elements without a bad node id; cnt: N ints, tiles: row_tiles(N) partials of scratch.
+cudaError_t launch_occurrences(const MeshView& m, const ListLayout& L, const HexRows& h, int* cnt, long long* tiles,
+                               cudaStream_t s);
 // The sorted row lists and the rank map; queue: N ints of scratch.
 cudaError_t launch_rows_hex20(const MeshView& m, const ListLayout& L, const HexRows& h, int* queue, cudaStream_t s);
 // Row lists -> CSR / BSR / upper triangle (mode: consolidate.cuh's kOut*; row_ptr already written).
 cudaError_t launch_count_upper_hex20(const ListLayout& L, int* ucounts, cudaStream_t s);
 cudaError_t launch_write_hex20(const ListLayout& L, const HexRows& h, int mode, const int* ucounts, const int* row_ptr,
                                int* col_idx, double* values, long long capacity, cudaStream_t s);
-// Elements per wave of the batched kernel's claims and values: a multiple of the group size.
-constexpr int kBatchHex20Wave = 4096;
-constexpr int kHex20GroupSize = 8;            // elements per group (group_hex20.cuh)
-constexpr int kHex20GroupRecWords = 5220;     // record words per group (header, nodes, blocks by pair, slots)
+// Whether CSR outputs are aligned for the 2-D copy kernel's 16-byte value and 8-byte column stores (row starts are
+// multiples of 4 entries); other outputs are stored entry by entry.
+inline bool wide_outputs(const int* col_idx, const double* values) {
+    return reinterpret_cast<uintptr_t>(values) % 16 == 0 && reinterpret_cast<uintptr_t>(col_idx) % 8 == 0;
+}
 
 // Spatial (3-D Morton bucket) element order; hist needs 1 << (3 * morton_bits(E)) ints, bbox 6 words.
 int morton_bits(int num_elems);
@@ -165,61 +165,37 @@ cudaError_t launch_dirichlet(int n_rows, const int* row_ptr, const int* col_idx,
                              const unsigned char* fixed, const double* u, cudaStream_t s);
 
 // ---- batched assembly (batched.cu) ----
-// One persistent kernel assembles every mesh of a batch: its CTAs take work
-// items from one ticket counter in a fixed order (the schedule) and wait,
-// bounded, on per-mesh phase counters for the items an item depends on.
 constexpr int kMaxBatchConcurrency = 256;  // meshes whose lists are live at once (workspace slots)
 // Estimated work of a mesh (elements weighted by kind) and the slot of each
 // mesh (largest first onto the least loaded slot).
 double batch_cost(const fem_mesh& m);
 std::vector<int> batch_schedule(const fem_mesh* meshes, int n, int slots);
 
-// Everything the batched kernel needs to know about one mesh (device copy).
+// Everything the batched kernels need to know about one mesh (a kernel parameter).
 struct BatchMesh {
     MeshView m;
     ListLayout L;
+    HexRows h;
+    int* cnt;                  // Hex20: occurrence counts, then the node order
+    int* queue;                // long rows
     long long* tiles;          // scan partials
-    int* map[2];               // Hex20: group records of even / odd waves
+    int* hist;                 // Hex20: scratch of the node order
+    int* ranges;
+    unsigned long long* bbox;
     int* row_ptr;              // the caller's CSR
     int* col_idx;
     double* values;
     long long capacity;
     fem_info* info_out;        // the caller's info array entry
     unsigned long long* stamp; // completion stamp (may be NULL)
-    unsigned char* zero_ptr[3];  // what the reset clears: info + first chunks, 2-D first-chunk values, counts
-    long long zero_bytes[3];
-    int kind, dpn, num_tiles, pad;
+    int kind;
+    int wide;                  // 2-D: the outputs are aligned for the copy kernel
 };
 
-// Phases of a mesh (work item kinds); a segment is a run of consecutive
-// tickets of one phase of one mesh.
-enum BatchPhase : int {
-    kBpReset = 0, kBpScatter2D, kBpClaim, kBpValues, kBpScanReduce, kBpScanTop, kBpRowPtr, kBpWrite, kBpFinish
-};
-// Per-mesh completion counters (index within the mesh's group of kBatchCounters).
-enum BatchCounter : int {
-    kBcReset = 0, kBcScatter, kBcValues, kBcScanReduce, kBcScanTop, kBcRowPtr, kBcWrite, kBcFinish
-};
-constexpr int kBatchCounters = 8;
-struct BatchSegment {
-    int mesh, phase, first, count;
-    int arg;                 // Hex20 claim / value items: the wave
-    int dep_ctr[2];          // counter indices (-1: none) and the values they must reach first
-    int dep_target[2];
-    int done_ctr;            // the counter each finished item increments
-};
-// Work item sizes.
-constexpr int kBatchResetBytes = 1 << 20;  // bytes cleared per reset item
-constexpr int kBatchScatter2D = 2048;      // 2-D elements per scatter item
-constexpr int kBatchClaim = 8;             // Hex20 elements per claim item (one element group)
-constexpr int kBatchValues = 8;            // Hex20 elements per value item (one group, one element at a time)
-constexpr int kBatchWriteBatches = 16;     // node batches per write item
-
-// Copies the tables into the workspace and zeroes the counters and the
-// ticket (with the start stamp), then launches the persistent kernel.
-cudaError_t launch_batch(const BatchMesh* meshes, int n, const BatchSegment* segs, int nseg, int total_items,
-                         BatchMesh* d_meshes, BatchSegment* d_segs, int* d_counters, int* d_ticket,
-                         unsigned long long* stamp0, long long wait_ns, int ctas_per_sm, cudaStream_t s);
+// Assembles the meshes of one round (each in its own workspace slot), phase by
+// phase on the stream; start: optional start stamp.
+cudaError_t launch_batch_round(const BatchMesh* meshes, int n, unsigned long long* start, int ctas_per_sm,
+                               cudaStream_t s);
 
 // ---- element-colouring baseline (colour.cu) ----
 constexpr int kMaxColours = 64;         // colours per mesh (a 64-bit mask of neighbour colours)

@@ -1,26 +1,4 @@
-// Row lists of a Hex20 mesh: the pattern half of the A-LLS scatter.
-//
-// Replaces the insert half of assembleGlobalStiffnessKernelALLSFixedArray
-// (ALLS_Hex20_3D_Assembly_Performance.cu:226-256: a linear scan of the row's
-// columns, a slot claimed with atomicAdd on the row count, no fence), whose
-// racing inserts duplicate or drop columns. Here a row belongs to the warp
-// that builds it, from the node's occurrences (incidence.cu), so nothing
-// races, and the row comes out sorted:
-//   k_rows_hex20       one warp per node with at most 8 elements (every inner
-//                      node of a regular mesh): its elements' up to 160 node
-//                      ids are loaded, five per lane, and inserted into a
-//                      256-entry hash table in shared memory; the distinct
-//                      ones are compacted and sorted (bitonic, in registers:
-//                      64, 128 or 256 keys), written to the list chunks, and
-//                      their ranks go back through the table to the rank map.
-//   k_wide_rows_hex20  nodes with up to 32 elements, one warp each: repeated
-//                      minimum over the candidates, which stay in registers.
-//   k_long_rows_hex20  longer rows, one CTA each: the same over memory.
-// A row past its first chunk takes consecutive overflow chunks from the pool.
-//
-// What bounds it: instruction issue (hash, sort, rank look-ups) and the latency
-// of occurrence -> connectivity. B200, 64^3 (1.09 M nodes): 1.18 ms, where the
-// CAS claims of element groups took 4.36 ms; 9^3: 8 against 141 us.
+// Launches of the Hex20 row-list kernels (rows_hex20.cuh).
 #include <algorithm>
 
 #include "rows_hex20.cuh"
@@ -28,276 +6,74 @@
 namespace fem {
 namespace {
 
-// Resident CTAs per SM that the registers are set for.
-#ifndef FEM_HEXR_CTAS
-#define FEM_HEXR_CTAS 4
-#endif
-constexpr int kWarps = 8;
-constexpr int kThreads = kWarps * 32;
-constexpr int kMaxElems = 8;               // elements of a node in the main pass
-constexpr int kCand = kMaxElems * 20 / 32; // candidates per lane
-constexpr int kTable = 256;
-constexpr int kWideElems = 32;
-constexpr int kWideCand = kWideElems * 20 / 32;
-constexpr unsigned kFull = 0xFFFFFFFFu;
-
-struct RowSmem {
-    int table[kTable];                 // distinct column nodes, -1 = empty
-    int uniq[kTable];                  // compacted, then sorted
-    unsigned short rank[kTable];       // rank of a table entry
-};
-
-// Overflow chunks of a row of u columns (called by one lane): returns the
-// chain's first chunk id + 1 (0: none needed); a pool that is out cuts the row
-// at its first chunk (FEM_ERR_POOL_OVERFLOW).
-__device__ __forceinline__ int take_chunks(const ListLayout& L, int& u) {
-    if (u <= L.S1) return 0;
-    const int need = (u - L.S1 + L.S2 - 1) / L.S2;
-    const int k = atomicAdd(&L.info->overflow_chunks, need);
-    if (k < 0 || k + need > L.cap2) {
-        raise_status(L.info, FEM_ERR_POOL_OVERFLOW);
-        u = L.S1;
-        return 0;
-    }
-    for (int i = 0; i < need; i++) {
-        int* m = L.meta2 + (size_t)(k + i) * L.H2;
-        m[0] = 0;
-        m[1] = i + 1 < need ? L.N + k + i + 2 : 0;
-    }
-    return L.N + k + 1;
+__global__ void __launch_bounds__(kOccThreads) k_occ_count(MeshView m, HexRows h, int* __restrict__ cnt, DevInfo* info) {
+    occ_count(m, h, cnt, info, blockIdx.x, gridDim.x);
 }
 
-// Header of row n's first chunk and its column count.
-__device__ __forceinline__ void finish_row(const ListLayout& L, int n, int u, int next) {
-    *reinterpret_cast<int2*>(L.meta1 + (size_t)n * L.H1) = make_int2(0, next);
-    L.counts[n] = u;
+__global__ void __launch_bounds__(kScanThreads) k_occ_sums(const int* __restrict__ cnt, int N,
+                                                           long long* __restrict__ tiles) {
+    __shared__ long long s_warp[kScanThreads / 32 + 1];
+    occ_sums(cnt, N, tiles, blockIdx.x, s_warp);
 }
 
-__device__ __forceinline__ int table_slot(int node) { return (int)(((unsigned)node * 2654435761u) >> 24); }
-
-// Sorts the u keys of uniq (KPL per lane, padded) by a bitonic network.
-template <int KPL>
-__device__ __forceinline__ void sort_keys(int* uniq, int u, int lane) {
-    int key[KPL];
-#pragma unroll
-    for (int i = 0; i < KPL; i++) key[i] = lane * KPL + i < u ? uniq[lane * KPL + i] : 0x7FFFFFFF;
-#pragma unroll
-    for (int size = 2; size <= 32 * KPL; size <<= 1) {
-#pragma unroll
-        for (int stride = size >> 1; stride > 0; stride >>= 1) {
-            if (stride >= KPL) {
-                const bool lower = ((lane * KPL) & stride) == 0;
-#pragma unroll
-                for (int i = 0; i < KPL; i++) {
-                    const bool up = ((lane * KPL + i) & size) == 0;
-                    const int o = __shfl_xor_sync(kFull, key[i], stride / KPL);
-                    key[i] = lower == up ? min(key[i], o) : max(key[i], o);
-                }
-            } else {
-#pragma unroll
-                for (int i = 0; i < KPL; i++) {
-                    const int j = i ^ stride;
-                    if (j > i) {
-                        const bool up = ((lane * KPL + i) & size) == 0;
-                        const int lo = min(key[i], key[j]), hi = max(key[i], key[j]);
-                        key[i] = up ? lo : hi;
-                        key[j] = up ? hi : lo;
-                    }
-                }
-            }
-        }
-    }
-    __syncwarp();
-#pragma unroll
-    for (int i = 0; i < KPL; i++)
-        if (lane * KPL + i < u) uniq[lane * KPL + i] = key[i];
-    __syncwarp();
+__global__ void __launch_bounds__(kScanThreads) k_occ_offsets(const int* __restrict__ cnt, int N,
+                                                              const long long* __restrict__ tiles,
+                                                              int* __restrict__ off, DevInfo* info) {
+    __shared__ OccSmem sm;
+    occ_offsets(cnt, N, tiles, off, info, blockIdx.x, gridDim.x, sm);
 }
 
-__global__ void __launch_bounds__(kThreads, FEM_HEXR_CTAS) k_rows_hex20(const int* __restrict__ conn, ListLayout L,
-                                                         const int* __restrict__ off, const int* __restrict__ inc,
-                                                         unsigned short* __restrict__ map, int* __restrict__ queue) {
-    __shared__ RowSmem s_row[kWarps];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    RowSmem& sm = s_row[warp];
-    for (long long nn = (long long)blockIdx.x * kWarps + warp; nn < L.N; nn += (long long)gridDim.x * kWarps) {
-        const int n = (int)nn, lo = __ldg(off + n), d = __ldg(off + n + 1) - lo;
-        if (d > kMaxElems) {
-            if (lane == 0) queue[atomicAdd(&L.info->long_rows, 1)] = n;
-            continue;
-        }
-        const int o = lane < d ? (int)occ_of(__ldg(inc + lo + lane)) : 0;
-        int node[kCand], slot[kCand];
-#pragma unroll
-        for (int q = 0; q < kCand; q++) {
-            const int j = lane + 32 * q, t = j / 20, b = j - 20 * t;
-            const int e = __shfl_sync(kFull, o, t & 31) / 20;
-            node[q] = j < 20 * d ? __ldg(conn + (size_t)e * 20 + b) : -1;
-        }
-        reinterpret_cast<int4*>(sm.table)[lane] = make_int4(-1, -1, -1, -1);
-        reinterpret_cast<int4*>(sm.table)[lane + 32] = make_int4(-1, -1, -1, -1);
-        __syncwarp();
-#pragma unroll
-        for (int q = 0; q < kCand; q++) {
-            int h = table_slot(node[q]);
-            if (node[q] >= 0) {
-                for (int i = 0; i < kTable; i++) {  // at most 160 of the 256 entries fill
-                    const int old = atomicCAS(&sm.table[h], -1, node[q]);
-                    if (old == -1 || old == node[q]) break;
-                    h = (h + 1) & (kTable - 1);
-                }
-            }
-            slot[q] = h;
-        }
-        __syncwarp();
-        int u = 0;
-#pragma unroll
-        for (int q = 0; q < kTable / 32; q++) {
-            const int k = sm.table[lane + 32 * q];
-            const unsigned used = __ballot_sync(kFull, k >= 0);
-            if (k >= 0) sm.uniq[u + __popc(used & ((1u << lane) - 1u))] = k;
-            u += __popc(used);
-        }
-        __syncwarp();
-        if (u <= 64) sort_keys<2>(sm.uniq, u, lane);
-        else if (u <= 128) sort_keys<4>(sm.uniq, u, lane);
-        else sort_keys<8>(sm.uniq, u, lane);
-        int kept = u, next = 0;
-        if (u > L.S1) {
-            if (lane == 0) next = take_chunks(L, kept);
-            next = __shfl_sync(kFull, next, 0);
-            kept = __shfl_sync(kFull, kept, 0);
-        }
-        for (int p = lane; p < u; p += 32) {
-            const int k = sm.uniq[p];
-            int h = table_slot(k);
-            while (sm.table[h] != k) h = (h + 1) & (kTable - 1);
-            sm.rank[h] = (unsigned short)p;
-            if (p < kept) *hex_col_word(L, n, next, p) = k + 1;
-        }
-        if (lane == 0) finish_row(L, n, kept, next);
-        __syncwarp();
-#pragma unroll
-        for (int q = 0; q < kCand; q++) {
-            const int j = lane + 32 * q, t = j / 20, b = j - 20 * t;
-            const int ot = __shfl_sync(kFull, o, t & 31);
-            if (node[q] >= 0) map[(size_t)ot * 20 + b] = sm.rank[slot[q]];
-        }
-        __syncwarp();
-    }
+__global__ void __launch_bounds__(kOccThreads) k_occ_fill(MeshView m, HexRows h) {
+    occ_fill(m, h, blockIdx.x, gridDim.x);
 }
 
-__global__ void __launch_bounds__(32) k_wide_rows_hex20(const int* __restrict__ conn, ListLayout L,
-                                                        const int* __restrict__ off, const int* __restrict__ inc,
-                                                        unsigned short* __restrict__ map,
+__global__ void __launch_bounds__(kHexRowThreads, FEM_HEXR_CTAS)
+    k_rows_hex20(const int* __restrict__ conn, ListLayout L, HexRows h, int* __restrict__ queue) {
+    __shared__ HexRowSmem s_row[kHexRowWarps];
+    rows_hex20(conn, L, h, queue, blockIdx.x, gridDim.x, s_row);
+}
+
+__global__ void __launch_bounds__(32) k_wide_rows_hex20(const int* __restrict__ conn, ListLayout L, HexRows h,
                                                         const int* __restrict__ queue) {
     __shared__ int s_uniq[kWideElems * 20];
-    const int lane = threadIdx.x, count = __ldg(&L.info->long_rows);
-    for (int k = blockIdx.x; k < count; k += gridDim.x) {
-        const int n = __ldg(queue + k), lo = __ldg(off + n), d = __ldg(off + n + 1) - lo;
-        if (d > kWideElems) continue;  // k_long_rows_hex20's
-        const int o = lane < d ? (int)occ_of(__ldg(inc + lo + lane)) : 0;
-        int node[kWideCand];
-#pragma unroll
-        for (int q = 0; q < kWideCand; q++) {
-            const int j = lane + 32 * q, t = j / 20, b = j - 20 * t;
-            const int e = __shfl_sync(kFull, o, t) / 20;
-            node[q] = j < 20 * d ? __ldg(conn + (size_t)e * 20 + b) : 0x7FFFFFFF;
-        }
-        int u = 0;
-        for (int last = -1;;) {
-            int m = 0x7FFFFFFF;
-#pragma unroll
-            for (int q = 0; q < kWideCand; q++) m = node[q] > last ? min(m, node[q]) : m;
-            m = __reduce_min_sync(kFull, m);
-            if (m == 0x7FFFFFFF) break;
-#pragma unroll
-            for (int q = 0; q < kWideCand; q++) {
-                const int j = lane + 32 * q, t = j / 20, b = j - 20 * t;
-                const int ot = __shfl_sync(kFull, o, t);
-                if (node[q] == m) map[(size_t)ot * 20 + b] = (unsigned short)u;
-            }
-            if (lane == 0) s_uniq[u] = m;
-            u++;
-            last = m;
-        }
-        int kept = u, next = 0;
-        if (lane == 0) next = take_chunks(L, kept);
-        next = __shfl_sync(kFull, next, 0);
-        kept = __shfl_sync(kFull, kept, 0);
-        __syncwarp();
-        for (int p = lane; p < kept; p += 32) *hex_col_word(L, n, next, p) = s_uniq[p] + 1;
-        if (lane == 0) finish_row(L, n, kept, next);
-        __syncwarp();
-    }
+    wide_rows_hex20(conn, L, h, queue, blockIdx.x, gridDim.x, s_uniq);
 }
 
-__global__ void __launch_bounds__(kThreads) k_long_rows_hex20(const int* __restrict__ conn, ListLayout L,
-                                                              const int* __restrict__ off,
-                                                              const int* __restrict__ inc,
-                                                              unsigned short* __restrict__ map,
-                                                              const int* __restrict__ queue) {
-    __shared__ int s_min[2], s_kept, s_next;
-    const int tid = threadIdx.x, count = __ldg(&L.info->long_rows);
-    for (int k = blockIdx.x; k < count; k += gridDim.x) {
-        const int n = __ldg(queue + k), lo = __ldg(off + n), d = __ldg(off + n + 1) - lo;
-        if (d <= kWideElems) continue;
-        const long long cand = 20ll * d;
-        // two passes over the row's columns in increasing order: count, then write
-        int kept = 0, next = 0;
-        for (int pass = 0; pass < 2; pass++) {
-            int u = 0;
-            for (int last = -1;; u++) {
-                __syncthreads();
-                if (tid == 0) s_min[u & 1] = 0x7FFFFFFF;
-                __syncthreads();
-                int m = 0x7FFFFFFF;
-                for (long long j = tid; j < cand; j += kThreads) {
-                    const unsigned ot = occ_of(__ldg(inc + lo + (int)(j / 20)));
-                    const int b = (int)(j % 20), x = __ldg(conn + (size_t)(ot / 20) * 20 + b);
-                    if (x > last) m = min(m, x);
-                    // the previous column's rank, met again on the way
-                    if (pass == 1 && u > 0 && x == last) map[(size_t)ot * 20 + b] = (unsigned short)(u - 1);
-                }
-                m = __reduce_min_sync(kFull, m);
-                if ((tid & 31) == 0) atomicMin(&s_min[u & 1], m);
-                __syncthreads();
-                m = s_min[u & 1];
-                if (m == 0x7FFFFFFF) break;
-                if (pass == 1 && tid == 0 && u < kept) *hex_col_word(L, n, next, u) = m + 1;
-                last = m;
-            }
-            if (pass == 0 && tid == 0) {
-                if (u > kMaxRank) {  // past the rank map's range
-                    raise_status(L.info, FEM_ERR_RANGE);
-                    u = kMaxRank;
-                }
-                s_next = take_chunks(L, u);
-                s_kept = u;
-                finish_row(L, n, s_kept, s_next);
-            }
-            __syncthreads();
-            kept = s_kept;
-            next = s_next;
-        }
-    }
+__global__ void __launch_bounds__(kHexRowThreads) k_long_rows_hex20(const int* __restrict__ conn, ListLayout L,
+                                                                    HexRows h, const int* __restrict__ queue) {
+    long_rows_hex20(conn, L, h, queue, blockIdx.x, gridDim.x);
 }
 
 }  // namespace
+
+cudaError_t launch_occurrences(const MeshView& m, const ListLayout& L, const HexRows& h, int* cnt, long long* tiles,
+                               cudaStream_t s) {
+    const cudaError_t err = cudaMemsetAsync(cnt, 0, (size_t)m.N * sizeof(int), s);
+    if (err) return err;
+    const int ntiles = row_tiles(m.N), sms = sm_count();
+    auto blocks = [&](long long work, int per_sm) {
+        return (int)std::min<long long>((work + kOccThreads - 1) / kOccThreads, (long long)sms * per_sm);
+    };
+    if (m.E_count > 0) k_occ_count<<<blocks(m.E_count, 8), kOccThreads, 0, s>>>(m, h, cnt, L.info);
+    k_occ_sums<<<ntiles, kScanThreads, 0, s>>>(cnt, m.N, tiles);
+    k_occ_offsets<<<ntiles, kScanThreads, 0, s>>>(cnt, m.N, tiles, h.off, L.info);
+    if (m.E_count > 0) k_occ_fill<<<blocks(20ll * m.E_count, 16), kOccThreads, 0, s>>>(m, h);
+    return cudaGetLastError();
+}
 
 cudaError_t launch_rows_hex20(const MeshView& m, const ListLayout& L, const HexRows& h, int* queue, cudaStream_t s) {
     static DeviceCache cache;
     int per_sm = 0;
     const cudaError_t err = per_device(cache, [](int& v) {
-        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, k_rows_hex20, kThreads, 0);
+        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, k_rows_hex20, kHexRowThreads, 0);
     }, per_sm);
     if (err) return err;
-    const long long want = ((long long)L.N + kWarps - 1) / kWarps;
-    k_rows_hex20<<<(int)std::min<long long>(want, (long long)per_sm * sm_count()), kThreads, 0, s>>>(
-        m.conn, L, h.off, h.inc, h.map, queue);
+    const long long want = ((long long)L.N + kHexRowWarps - 1) / kHexRowWarps;
+    k_rows_hex20<<<(int)std::min<long long>(want, (long long)per_sm * sm_count()), kHexRowThreads, 0, s>>>(
+        m.conn, L, h, queue);
     const int few = (int)std::min<long long>(L.N, 4 * sm_count());
-    k_wide_rows_hex20<<<few, 32, 0, s>>>(m.conn, L, h.off, h.inc, h.map, queue);
-    k_long_rows_hex20<<<std::min(few, sm_count()), kThreads, 0, s>>>(m.conn, L, h.off, h.inc, h.map, queue);
+    k_wide_rows_hex20<<<few, 32, 0, s>>>(m.conn, L, h, queue);
+    k_long_rows_hex20<<<std::min(few, sm_count()), kHexRowThreads, 0, s>>>(m.conn, L, h, queue);
     return cudaGetLastError();
 }
 

@@ -1,29 +1,397 @@
-// Row lists of a Hex20 mesh (rows_hex20.cu) and their gather into CSR / BSR /
-// upper-triangle CSR (write_hex20.cu).
+// Device code of the Hex20 row lists (rows_hex20.cu, and the batch, batched.cu):
+// the pattern half of the A-LLS scatter.
 //
-// A Hex20 scatter leaves, per row node, its sorted column nodes in the list
-// chunks, and the packed Ke of every element (fem_element_stiffness's layout);
-// the consolidation sums each row's element blocks where it writes them. An
-// element's block (a, b) meets its row through two tables: the node's
-// occurrences (node -> element e and local position a, as o = 20 e + a) and
-// the rank of column node b in row node a's sorted list, map[20 o + b].
+// Replaces the insert half of assembleGlobalStiffnessKernelALLSFixedArray
+// (ALLS_Hex20_3D_Assembly_Performance.cu:226-256: a linear scan of the row's
+// columns, a slot claimed with atomicAdd on the row count, no fence), whose
+// racing inserts duplicate or drop columns. Here a row belongs to the warp
+// that builds it, from the node's occurrences (occ_* below), so nothing
+// races, and the row comes out sorted:
+//   k_rows_hex20       one warp per node with at most 8 elements (every inner
+//                      node of a regular mesh): its elements' up to 160 node
+//                      ids are loaded, five per lane, and inserted into a
+//                      256-entry hash table in shared memory; the distinct
+//                      ones are compacted and sorted (bitonic, in registers:
+//                      64, 128 or 256 keys), written to the list chunks, and
+//                      their ranks go back through the table to the rank map.
+//   k_wide_rows_hex20  nodes with up to 32 elements, one warp each: repeated
+//                      minimum over the candidates, which stay in registers.
+//   k_long_rows_hex20  longer rows, one CTA each: the same over memory.
+// A row past its first chunk takes consecutive overflow chunks from the pool.
+//
+// What bounds it: instruction issue (hash, sort, rank look-ups) and the latency
+// of occurrence -> connectivity. B200, 64^3 (1.09 M nodes): 1.18 ms, where the
+// CAS claims of element groups took 4.36 ms; 9^3: 8 against 141 us.
 #pragma once
 
-#include "launch.h"
+#include "hex_rows.cuh"
+#include "scan.cuh"
 
 namespace fem {
 namespace {
 
-constexpr int kMaxRank = 0xFFFF;  // columns of a row that the rank map can number
+// ---- occurrences: node -> (element, position) lists -----------------------------
+//   occ_count  thread per element: one counter atomic per node; the position it
+//              returns is kept (pos), so the fill needs no atomics. An element
+//              with a bad node id has no occurrence (pos kNoOcc); the
+//              occurrences of an element that repeats a node carry kOccRepeats.
+//   occ_sums   sum of the counts per tile of kRowTile nodes
+//   occ_offsets  exclusive prefix: each tile sums the tiles before it
+//   occ_fill   thread per occurrence: inc[off[node] + pos] = 20 e + a
 
-__device__ __forceinline__ unsigned occ_of(int word) { return (unsigned)word & ~kOccRepeats; }
+constexpr int kOccThreads = 256;
+constexpr int kNoOcc = 0x7FFFFFFF;
 
-// Column word (column node + 1) k of row node n: the first chunk's slots, then
-// the row's overflow chunks, which are consecutive from chunk id `next` - 1 on.
-__device__ __forceinline__ int* hex_col_word(const ListLayout& L, int n, int next, int k) {
-    if (k < L.S1) return L.meta1 + (size_t)n * L.H1 + 2 + k;
-    const int q = k - L.S1, c = next - 1 - L.N + q / L.S2;
-    return L.meta2 + (size_t)c * L.H2 + 2 + q % L.S2;
+__device__ __forceinline__ int* occ_pos(const HexRows& h) { return reinterpret_cast<int*>(h.map); }  // 80 of 800 bytes an element
+
+__device__ __forceinline__ void occ_count(const MeshView& m, const HexRows& h, int* __restrict__ cnt, DevInfo* info,
+                                          int block, int nblocks) {
+    int* pos = occ_pos(h);
+    for (int e = block * kOccThreads + threadIdx.x; e < m.E_count; e += nblocks * kOccThreads) {
+        const size_t o = (size_t)e * 20;
+        int n[20];
+        bool bad = false, rep = false;
+#pragma unroll
+        for (int k = 0; k < 20; k++) {
+            n[k] = __ldg(m.conn + o + k);
+            bad |= n[k] < 0 || n[k] >= m.N;
+#pragma unroll
+            for (int j = 0; j < k; j++) rep |= n[j] == n[k];
+        }
+        if (bad) raise_status(info, FEM_ERR_BAD_MESH);
+        int p[20];
+#pragma unroll
+        for (int k = 0; k < 20; k++) p[k] = bad ? kNoOcc : atomicAdd(cnt + n[k], 1);
+#pragma unroll
+        for (int k = 0; k < 20; k++) pos[o + k] = rep && !bad ? (int)((unsigned)p[k] | kOccRepeats) : p[k];
+    }
+}
+
+__device__ __forceinline__ void occ_sums(const int* __restrict__ cnt, int N, long long* __restrict__ tiles, int tile,
+                                         long long* s_warp) {
+    long long sum = 0;
+#pragma unroll
+    for (int i = 0; i < kRowTile / kScanThreads; i++) {
+        const long long n = (long long)tile * kRowTile + i * kScanThreads + threadIdx.x;
+        if (n < N) sum += __ldg(cnt + n);
+    }
+    long long total;
+    block_exclusive_scan(sum, s_warp, total);
+    if (threadIdx.x == 0) tiles[tile] = total;
+}
+
+struct OccSmem {
+    long long warp[kScanThreads / 32 + 1];
+    int cnt[kRowTile];
+};
+
+__device__ __forceinline__ void occ_offsets(const int* __restrict__ cnt, int N, const long long* __restrict__ tiles,
+                                            int* __restrict__ off, DevInfo* info, int tile, int ntiles, OccSmem& sm) {
+    constexpr int kItems = kRowTile / kScanThreads;
+    const int tid = threadIdx.x;
+    const long long first = (long long)tile * kRowTile;
+#pragma unroll
+    for (int i = 0; i < kItems; i++) {
+        const long long n = first + i * kScanThreads + tid;
+        sm.cnt[i * kScanThreads + tid] = n < N ? __ldg(cnt + n) : 0;
+    }
+    long long before = 0, base, total;
+    for (int t = tid; t < tile; t += kScanThreads) before += __ldg(tiles + t);
+    block_exclusive_scan(before, sm.warp, base);
+    int c[kItems];
+    long long sum = 0;
+#pragma unroll
+    for (int i = 0; i < kItems; i++) {
+        c[i] = sm.cnt[tid * kItems + i];
+        sum += c[i];
+    }
+    long long o = base + block_exclusive_scan(sum, sm.warp, total);
+#pragma unroll
+    for (int i = 0; i < kItems; i++) {
+        sm.cnt[tid * kItems + i] = (int)o;
+        o += c[i];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < kItems; i++) {
+        const long long n = first + i * kScanThreads + tid;
+        if (n < N) off[n] = sm.cnt[i * kScanThreads + tid];
+    }
+    if (tile == ntiles - 1 && tid == 0) {
+        off[N] = (int)(base + total);
+        if (base + total > 0x7FFFFFFFll) raise_status(info, FEM_ERR_RANGE);
+    }
+}
+
+__device__ __forceinline__ void occ_fill(const MeshView& m, const HexRows& h, int block, int nblocks) {
+    const int* pos = occ_pos(h);
+    const long long count = 20ll * m.E_count;
+    for (long long o = (long long)block * kOccThreads + threadIdx.x; o < count; o += (long long)nblocks * kOccThreads) {
+        const int p = pos[o];
+        if (p == kNoOcc) continue;
+        const unsigned flag = (unsigned)p & kOccRepeats;
+        h.inc[__ldg(h.off + __ldg(m.conn + o)) + (int)((unsigned)p & ~kOccRepeats)] = (int)((unsigned)o | flag);
+    }
+}
+
+// ---- rows -------------------------------------------------------------------------
+
+// Resident CTAs per SM that the registers are set for.
+#ifndef FEM_HEXR_CTAS
+#define FEM_HEXR_CTAS 4
+#endif
+constexpr int kHexRowWarps = 8;
+constexpr int kHexRowThreads = kHexRowWarps * 32;
+constexpr int kMaxElems = 8;               // elements of a node in the main pass
+constexpr int kCand = kMaxElems * 20 / 32; // candidates per lane
+constexpr int kTable = 256;
+constexpr int kWideElems = 32;
+constexpr int kWideCand = kWideElems * 20 / 32;
+
+struct alignas(16) HexRowSmem {  // cleared with 16-byte stores
+    int table[kTable];                 // distinct column nodes, -1 = empty
+    int uniq[kTable];                  // compacted, then sorted
+    unsigned short rank[kTable];       // rank of a table entry
+};
+
+// Overflow chunks of a row of u columns (called by one lane): returns the
+// chain's first chunk id + 1 (0: none needed); a pool that is out cuts the row
+// at its first chunk (FEM_ERR_POOL_OVERFLOW).
+__device__ __forceinline__ int take_chunks(const ListLayout& L, int& u) {
+    if (u <= L.S1) return 0;
+    const int need = (u - L.S1 + L.S2 - 1) / L.S2;
+    const int k = atomicAdd(&L.info->overflow_chunks, need);
+    if (k < 0 || k + need > L.cap2) {
+        raise_status(L.info, FEM_ERR_POOL_OVERFLOW);
+        u = L.S1;
+        return 0;
+    }
+    for (int i = 0; i < need; i++) {
+        int* m = L.meta2 + (size_t)(k + i) * L.H2;
+        m[0] = 0;
+        m[1] = i + 1 < need ? L.N + k + i + 2 : 0;
+    }
+    return L.N + k + 1;
+}
+
+// Header of row n's first chunk and its column count.
+__device__ __forceinline__ void finish_row(const ListLayout& L, int n, int u, int next) {
+    *reinterpret_cast<int2*>(L.meta1 + (size_t)n * L.H1) = make_int2(0, next);
+    L.counts[n] = u;
+}
+
+__device__ __forceinline__ int table_slot(int node) { return (int)(((unsigned)node * 2654435761u) >> 24); }
+
+// Sorts the u keys of uniq (KPL per lane, padded) by a bitonic network.
+template <int KPL>
+__device__ __forceinline__ void sort_keys(int* uniq, int u, int lane) {
+    int key[KPL];
+#pragma unroll
+    for (int i = 0; i < KPL; i++) key[i] = lane * KPL + i < u ? uniq[lane * KPL + i] : 0x7FFFFFFF;
+#pragma unroll
+    for (int size = 2; size <= 32 * KPL; size <<= 1) {
+#pragma unroll
+        for (int stride = size >> 1; stride > 0; stride >>= 1) {
+            if (stride >= KPL) {
+                const bool lower = ((lane * KPL) & stride) == 0;
+#pragma unroll
+                for (int i = 0; i < KPL; i++) {
+                    const bool up = ((lane * KPL + i) & size) == 0;
+                    const int o = __shfl_xor_sync(0xFFFFFFFFu, key[i], stride / KPL);
+                    key[i] = lower == up ? min(key[i], o) : max(key[i], o);
+                }
+            } else {
+#pragma unroll
+                for (int i = 0; i < KPL; i++) {
+                    const int j = i ^ stride;
+                    if (j > i) {
+                        const bool up = ((lane * KPL + i) & size) == 0;
+                        const int lo = min(key[i], key[j]), hi = max(key[i], key[j]);
+                        key[i] = up ? lo : hi;
+                        key[j] = up ? hi : lo;
+                    }
+                }
+            }
+        }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < KPL; i++)
+        if (lane * KPL + i < u) uniq[lane * KPL + i] = key[i];
+    __syncwarp();
+}
+
+// The bodies below run as block `block` of `nblocks` of their launch.
+__device__ __forceinline__ void rows_hex20(const int* __restrict__ conn, const ListLayout& L, const HexRows& h,
+                                           int* __restrict__ queue, int block, int nblocks,
+                                           HexRowSmem (&s_row)[kHexRowWarps]) {
+    const int* __restrict__ off = h.off;
+    const int* __restrict__ inc = h.inc;
+    unsigned short* __restrict__ map = h.map;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    HexRowSmem& sm = s_row[warp];
+    for (long long nn = (long long)block * kHexRowWarps + warp; nn < L.N; nn += (long long)nblocks * kHexRowWarps) {
+        const int n = (int)nn, lo = __ldg(off + n), d = __ldg(off + n + 1) - lo;
+        if (d > kMaxElems) {
+            if (lane == 0) queue[atomicAdd(&L.info->long_rows, 1)] = n;
+            continue;
+        }
+        const int o = lane < d ? (int)occ_of(__ldg(inc + lo + lane)) : 0;
+        int node[kCand], slot[kCand];
+#pragma unroll
+        for (int q = 0; q < kCand; q++) {
+            const int j = lane + 32 * q, t = j / 20, b = j - 20 * t;
+            const int e = __shfl_sync(0xFFFFFFFFu, o, t & 31) / 20;
+            node[q] = j < 20 * d ? __ldg(conn + (size_t)e * 20 + b) : -1;
+        }
+        reinterpret_cast<int4*>(sm.table)[lane] = make_int4(-1, -1, -1, -1);
+        reinterpret_cast<int4*>(sm.table)[lane + 32] = make_int4(-1, -1, -1, -1);
+        __syncwarp();
+#pragma unroll
+        for (int q = 0; q < kCand; q++) {
+            int h = table_slot(node[q]);
+            if (node[q] >= 0) {
+                for (int i = 0; i < kTable; i++) {  // at most 160 of the 256 entries fill
+                    const int old = atomicCAS(&sm.table[h], -1, node[q]);
+                    if (old == -1 || old == node[q]) break;
+                    h = (h + 1) & (kTable - 1);
+                }
+            }
+            slot[q] = h;
+        }
+        __syncwarp();
+        int u = 0;
+#pragma unroll
+        for (int q = 0; q < kTable / 32; q++) {
+            const int k = sm.table[lane + 32 * q];
+            const unsigned used = __ballot_sync(0xFFFFFFFFu, k >= 0);
+            if (k >= 0) sm.uniq[u + __popc(used & ((1u << lane) - 1u))] = k;
+            u += __popc(used);
+        }
+        __syncwarp();
+        if (u <= 64) sort_keys<2>(sm.uniq, u, lane);
+        else if (u <= 128) sort_keys<4>(sm.uniq, u, lane);
+        else sort_keys<8>(sm.uniq, u, lane);
+        int kept = u, next = 0;
+        if (u > L.S1) {
+            if (lane == 0) next = take_chunks(L, kept);
+            next = __shfl_sync(0xFFFFFFFFu, next, 0);
+            kept = __shfl_sync(0xFFFFFFFFu, kept, 0);
+        }
+        for (int p = lane; p < u; p += 32) {
+            const int k = sm.uniq[p];
+            int h = table_slot(k);
+            while (sm.table[h] != k) h = (h + 1) & (kTable - 1);
+            sm.rank[h] = (unsigned short)p;
+            if (p < kept) *hex_col_word(L, n, next, p) = k + 1;
+        }
+        if (lane == 0) finish_row(L, n, kept, next);
+        __syncwarp();
+#pragma unroll
+        for (int q = 0; q < kCand; q++) {
+            const int j = lane + 32 * q, t = j / 20, b = j - 20 * t;
+            const int ot = __shfl_sync(0xFFFFFFFFu, o, t & 31);
+            if (node[q] >= 0) map[(size_t)ot * 20 + b] = sm.rank[slot[q]];
+        }
+        __syncwarp();
+    }
+}
+
+__device__ __forceinline__ void wide_rows_hex20(const int* __restrict__ conn, const ListLayout& L, const HexRows& h,
+                                                const int* __restrict__ queue, int block, int nblocks,
+                                                int (&s_uniq)[kWideElems * 20]) {
+    const int* __restrict__ off = h.off;
+    const int* __restrict__ inc = h.inc;
+    unsigned short* __restrict__ map = h.map;
+    const int lane = threadIdx.x, count = __ldg(&L.info->long_rows);
+    for (int k = block; k < count; k += nblocks) {
+        const int n = __ldg(queue + k), lo = __ldg(off + n), d = __ldg(off + n + 1) - lo;
+        if (d > kWideElems) continue;  // k_long_rows_hex20's
+        const int o = lane < d ? (int)occ_of(__ldg(inc + lo + lane)) : 0;
+        int node[kWideCand];
+#pragma unroll
+        for (int q = 0; q < kWideCand; q++) {
+            const int j = lane + 32 * q, t = j / 20, b = j - 20 * t;
+            const int e = __shfl_sync(0xFFFFFFFFu, o, t) / 20;
+            node[q] = j < 20 * d ? __ldg(conn + (size_t)e * 20 + b) : 0x7FFFFFFF;
+        }
+        int u = 0;
+        for (int last = -1;;) {
+            int m = 0x7FFFFFFF;
+#pragma unroll
+            for (int q = 0; q < kWideCand; q++) m = node[q] > last ? min(m, node[q]) : m;
+            m = __reduce_min_sync(0xFFFFFFFFu, m);
+            if (m == 0x7FFFFFFF) break;
+#pragma unroll
+            for (int q = 0; q < kWideCand; q++) {
+                const int j = lane + 32 * q, t = j / 20, b = j - 20 * t;
+                const int ot = __shfl_sync(0xFFFFFFFFu, o, t);
+                if (node[q] == m) map[(size_t)ot * 20 + b] = (unsigned short)u;
+            }
+            if (lane == 0) s_uniq[u] = m;
+            u++;
+            last = m;
+        }
+        int kept = u, next = 0;
+        if (lane == 0) next = take_chunks(L, kept);
+        next = __shfl_sync(0xFFFFFFFFu, next, 0);
+        kept = __shfl_sync(0xFFFFFFFFu, kept, 0);
+        __syncwarp();
+        for (int p = lane; p < kept; p += 32) *hex_col_word(L, n, next, p) = s_uniq[p] + 1;
+        if (lane == 0) finish_row(L, n, kept, next);
+        __syncwarp();
+    }
+}
+
+__device__ __forceinline__ void long_rows_hex20(const int* __restrict__ conn, const ListLayout& L, const HexRows& h,
+                                                const int* __restrict__ queue, int block, int nblocks) {
+    const int* __restrict__ off = h.off;
+    const int* __restrict__ inc = h.inc;
+    unsigned short* __restrict__ map = h.map;
+    __shared__ int s_min[2], s_kept, s_next;
+    const int tid = threadIdx.x, count = __ldg(&L.info->long_rows);
+    for (int k = block; k < count; k += nblocks) {
+        const int n = __ldg(queue + k), lo = __ldg(off + n), d = __ldg(off + n + 1) - lo;
+        if (d <= kWideElems) continue;
+        const long long cand = 20ll * d;
+        // two passes over the row's columns in increasing order: count, then write
+        int kept = 0, next = 0;
+        for (int pass = 0; pass < 2; pass++) {
+            int u = 0;
+            for (int last = -1;; u++) {
+                __syncthreads();
+                if (tid == 0) s_min[u & 1] = 0x7FFFFFFF;
+                __syncthreads();
+                int m = 0x7FFFFFFF;
+                for (long long j = tid; j < cand; j += kHexRowThreads) {
+                    const unsigned ot = occ_of(__ldg(inc + lo + (int)(j / 20)));
+                    const int b = (int)(j % 20), x = __ldg(conn + (size_t)(ot / 20) * 20 + b);
+                    if (x > last) m = min(m, x);
+                    // the previous column's rank, met again on the way
+                    if (pass == 1 && u > 0 && x == last) map[(size_t)ot * 20 + b] = (unsigned short)(u - 1);
+                }
+                m = __reduce_min_sync(0xFFFFFFFFu, m);
+                if ((tid & 31) == 0) atomicMin(&s_min[u & 1], m);
+                __syncthreads();
+                m = s_min[u & 1];
+                if (m == 0x7FFFFFFF) break;
+                if (pass == 1 && tid == 0 && u < kept) *hex_col_word(L, n, next, u) = m + 1;
+                last = m;
+            }
+            if (pass == 0 && tid == 0) {
+                if (u > kMaxRank) {  // past the rank map's range
+                    raise_status(L.info, FEM_ERR_RANGE);
+                    u = kMaxRank;
+                }
+                s_next = take_chunks(L, u);
+                s_kept = u;
+                finish_row(L, n, s_kept, s_next);
+            }
+            __syncthreads();
+            kept = s_kept;
+            next = s_next;
+        }
+    }
 }
 
 }  // namespace

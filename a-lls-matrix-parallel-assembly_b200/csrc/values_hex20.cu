@@ -1,6 +1,6 @@
 // The CTA-cooperative Hex20 element pass (values_hex20.cuh): FP64 element
 // stiffness added into a CSR, for the value-only re-assembly and the colouring
-// baseline (and, in the batched kernel, into list slots).
+// baseline.
 //
 // Replaces the element routine computeElementStiffnessHex20
 // (ALLS_Hex20_3D_Assembly_Performance.cu:130-195).

@@ -1,11 +1,9 @@
 // Device code of the CTA-cooperative Hex20 FP64 element pass: the value-only
-// re-assembly and the colouring baseline (values_hex20.cu), and the value
-// items of the batched persistent kernel (batched.cu). See values_hex20.cu for
-// the method.
+// re-assembly and the colouring baseline. See values_hex20.cu for the method.
 #pragma once
 
-#include "group_hex20.cuh"
 #include "hex20.cuh"
+#include "launch.h"
 
 namespace fem {
 namespace {
@@ -15,7 +13,6 @@ constexpr int KS = 28;  // Gauss points padded to 7 k-steps of 4; row stride of 
 
 // Where the value pass puts an element's Ke blocks.
 enum ValueOut : int {
-    kToSlots = 0,   // FP64 atomics into the list slots of a group's map record (both orientations)
     kToCsrMap = 1,  // FP64 atomics into a CSR at the positions of a scatter map (both triangles)
     kToCsrColour = 2  // plain adds into a CSR at binary-searched positions (one colour: no two
                       // elements share a node)
@@ -23,10 +20,6 @@ enum ValueOut : int {
 
 struct ValuesTarget {
     const int* map;          // kToCsrMap: CSR positions, row e
-    const GroupTopo* topo;   // kToSlots: topology of the group of the elements
-    const unsigned* rec;     // kToSlots: the slot words of the group's record
-    long long g0;            // kToSlots: position of the group's first element
-    double* vals;            // kToSlots: list values
     const int* row_ptr;   // kToCsr*: the CSR
     const int* col_idx;
     double* csr;
@@ -46,9 +39,6 @@ struct ValuesSmem {
     int nodes[20];
     double lam, mu;
     int bad;
-    // per tile warp: its node-pair blocks, compacted, before they are added
-    double stage[kValueWarps][64][9];
-    int stage_gid[kValueWarps][64];
 };
 
 __device__ __forceinline__ void dmma(double& c0, double& c1, double a, double b) {
@@ -78,8 +68,7 @@ __device__ __forceinline__ void values_init(ValuesSmem& sm) {
 // The value pass of the elements at positions i = i_first, i_first +
 // i_stride, ... below i1 of the visit order perm (perm NULL: element i) by
 // one CTA of at least kValueWarps warps (warps beyond them help with the
-// per-element tables only); the slot ids of position i are map row
-// i - map_origin. Every thread of the CTA calls it.
+// per-element tables only). Every thread of the CTA calls it.
 template <int kOut>
 __device__ __forceinline__ void values_cta(const MeshView& m, const int* __restrict__ perm, long long i_first,
                                            long long i_stride, int i1, const ValuesTarget& t, ValuesSmem& sm) {
@@ -87,16 +76,16 @@ __device__ __forceinline__ void values_cta(const MeshView& m, const int* __restr
     const bool tile_warp = warp < kValueWarps;
     const int ti = tile_ti(warp), tj = tile_tj(warp);
     const int fr = lane >> 2, fc = lane & 3;
-    auto elem = [&](long long i) -> int { return perm ? FEM_LDG(perm + i) : (int)i; };
+    auto elem = [&](long long i) -> int { return perm ? __ldg(perm + i) : (int)i; };
     // node id and coordinates of the next element
     int pre_n = 0;
     double pre_x = 0.0, pre_y = 0.0, pre_z = 0.0;
     if (tid < 20 && i_first < i1) {
-        pre_n = FEM_LDG(m.conn + (size_t)elem(i_first) * 20 + tid);
+        pre_n = __ldg(m.conn + (size_t)elem(i_first) * 20 + tid);
         if (pre_n >= 0 && pre_n < m.N) {
-            pre_x = FEM_LDG(m.x + pre_n);
-            pre_y = FEM_LDG(m.y + pre_n);
-            pre_z = FEM_LDG(m.z + pre_n);
+            pre_x = __ldg(m.x + pre_n);
+            pre_y = __ldg(m.y + pre_n);
+            pre_z = __ldg(m.z + pre_n);
         }
     }
     __syncthreads();
@@ -116,20 +105,20 @@ __device__ __forceinline__ void values_cta(const MeshView& m, const int* __restr
             }
         }
         if (tid == 32) {
-            const double E = m.E ? FEM_LDG(m.E + e) : m.E0;
-            const double nu = m.nu ? FEM_LDG(m.nu + e) : m.nu0;
+            const double E = m.E ? __ldg(m.E + e) : m.E0;
+            const double nu = m.nu ? __ldg(m.nu + e) : m.nu0;
             sm.lam = E * nu / ((1.0 + nu) * (1.0 - 2.0 * nu));
             sm.mu = E / (2.0 * (1.0 + nu));
         }
         __syncthreads();
         const long long i_next = i + i_stride;
-        if (tid < 20 && i_next < i1) pre_n = FEM_LDG(m.conn + (size_t)elem(i_next) * 20 + tid);
+        if (tid < 20 && i_next < i1) pre_n = __ldg(m.conn + (size_t)elem(i_next) * 20 + tid);
         if (sm.bad) {  // nothing to add
-            if (tid == 0 && kOut != kToSlots) raise_status(t.info, FEM_ERR_BAD_MESH);  // else the claim pass did
+            if (tid == 0) raise_status(t.info, FEM_ERR_BAD_MESH);
             if (tid < 20 && i_next < i1 && pre_n >= 0 && pre_n < m.N) {
-                pre_x = FEM_LDG(m.x + pre_n);
-                pre_y = FEM_LDG(m.y + pre_n);
-                pre_z = FEM_LDG(m.z + pre_n);
+                pre_x = __ldg(m.x + pre_n);
+                pre_y = __ldg(m.y + pre_n);
+                pre_z = __ldg(m.z + pre_n);
             }
             __syncthreads();  // uniform: every thread has read the flag before it is reset
             continue;
@@ -175,9 +164,9 @@ __device__ __forceinline__ void values_cta(const MeshView& m, const int* __restr
         __syncthreads();
         // the coordinates of the next element arrive during the contraction
         if (tid < 20 && i_next < i1 && pre_n >= 0 && pre_n < m.N) {
-            pre_x = FEM_LDG(m.x + pre_n);
-            pre_y = FEM_LDG(m.y + pre_n);
-            pre_z = FEM_LDG(m.z + pre_n);
+            pre_x = __ldg(m.x + pre_n);
+            pre_y = __ldg(m.y + pre_n);
+            pre_z = __ldg(m.z + pre_n);
         }
         if (!tile_warp) continue;  // the remaining warps wait at the next element's first barrier
         // M^{ab} tiles (ti, tj): A[r][k] = w_k G[a][8 ti + r][k], B[k][c] = G[b][8 tj + c][k]
@@ -203,65 +192,7 @@ __device__ __forceinline__ void values_cta(const MeshView& m, const int* __restr
         }
         const double lam = sm.lam, mu = sm.mu;
         const int I = 8 * ti + fr;
-        if constexpr (kOut == kToSlots) {
-            // Ke block of each of this lane's node pairs {I, J}, staged for two
-            // atomic passes: Ke_IJ to the slot of (row node I, column node J),
-            // then its transpose to the slot of (row J, column I), the slots
-            // from the group's map record
-            const GroupTopo& T = *t.topo;
-            const int w = (int)(i - t.g0);
-            unsigned tgt[2][2];
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const int Jn = 8 * tj + 2 * fc + h;
-                tgt[h][0] = tgt[h][1] = kMapNone;
-                if (I < 20 && Jn < 20 && (ti != tj || Jn >= I)) {
-                    const int u = T.lidx[20 * w + I], v = T.lidx[20 * w + Jn];
-                    if (u <= v) {
-                        const int p = pair_index(T, u, v);
-                        tgt[h][0] = FEM_LDG(t.rec + 2 * p);
-                        // a repeated node of one element: both orientations on one block
-                        tgt[h][1] = u == v ? (I != Jn ? tgt[h][0] : kMapNone) : FEM_LDG(t.rec + 2 * p + 1);
-                    } else {
-                        const int p = pair_index(T, v, u);
-                        tgt[h][0] = FEM_LDG(t.rec + 2 * p + 1);
-                        tgt[h][1] = FEM_LDG(t.rec + 2 * p);
-                    }
-                }
-            }
-#pragma unroll
-            for (int o = 0; o < 2; o++) {
-                int base = 0;
-#pragma unroll
-                for (int h = 0; h < 2; h++) {
-                    const unsigned g = tgt[h][o];
-                    const bool ok = map_has_slot(g);
-                    const unsigned have = __ballot_sync(0xFFFFFFFFu, ok);
-                    if (ok) {
-                        const int slot = base + __popc(have & ((1u << lane) - 1u));
-                        const double mtr = mu * (acc[0][0][h] + acc[1][1][h] + acc[2][2][h]);
-#pragma unroll
-                        for (int a = 0; a < 3; a++)
-#pragma unroll
-                            for (int b = 0; b < 3; b++) {
-                                const double k = fma(lam, acc[a][b][h], fma(mu, acc[b][a][h], a == b ? mtr : 0.0));
-                                sm.stage[warp][slot][o ? 3 * b + a : 3 * a + b] = k;
-                            }
-                        sm.stage_gid[warp][slot] = (int)(g & ~kPairShared);
-                    }
-                    base += __popc(have);
-                }
-                __syncwarp();
-                // nine consecutive lanes per block, three blocks per instruction:
-                // each block's 72 bytes are one atomic pass over its three sectors
-                if (lane < 27) {
-                    const int q = lane / 9, v = lane - 9 * q;
-                    for (int blk = q; blk < base; blk += 3)
-                        atomicAdd(t.vals + (size_t)(unsigned)sm.stage_gid[warp][blk] * 9 + v, sm.stage[warp][blk][v]);
-                }
-                __syncwarp();
-            }
-        } else {
+        {
             // CSR targets hold both triangles: Ke_IJ at block (I, J) and its
             // transpose at (J, I)
 #pragma unroll
@@ -277,15 +208,15 @@ __device__ __forceinline__ void values_cta(const MeshView& m, const int* __restr
                 for (int o = 0; o < (I == Jn ? 1 : 2); o++) {
                     const int R = o ? Jn : I, Cn = o ? I : Jn;  // block (R, Cn) of the element
                     const int r0 = 3 * sm.nodes[R], c0 = 3 * sm.nodes[Cn];
-                    const int lo = FEM_LDG(t.row_ptr + r0), len = FEM_LDG(t.row_ptr + r0 + 1) - lo;
+                    const int lo = __ldg(t.row_ptr + r0), len = __ldg(t.row_ptr + r0 + 1) - lo;
                     int p = -1;
                     if constexpr (kOut == kToCsrMap) {
-                        p = FEM_LDG(t.map + (size_t)e * 400 + R * 20 + Cn);
+                        p = __ldg(t.map + (size_t)e * 400 + R * 20 + Cn);
                     } else {
                         int a0 = lo, a1 = lo + len - 1;
                         while (a0 <= a1) {
                             const int mid = (a0 + a1) >> 1;
-                            const int c = FEM_LDG(t.col_idx + mid);
+                            const int c = __ldg(t.col_idx + mid);
                             if (c == c0) {
                                 p = mid;
                                 break;

@@ -259,16 +259,15 @@ FEM_API fem_status fem_apply_dirichlet(int32_t n_rows, const int32_t* row_ptr, c
  * Many independent meshes (any element kinds, uneven sizes) in one
  * stream-ordered call; the reference assembles one mesh per program run
  * (its drivers' main, e.g. ALLS_Q4_T3_Mixed_Elements_Assembly_Performance.cu:742-854).
- * One persistent kernel assembles the whole batch from a schedule of work
- * items (list resets, 2-D scatter tiles, Hex20 claim and value tiles in
- * waves, scan tiles, row pointers, sorted-write tiles, completion), which
- * its CTAs take in order and run once the items they depend on are done.
+ * The meshes of a round are assembled phase by phase, one launch per phase over
+ * all of them (the single-mesh kernels' device code, blocks dealt in proportion
+ * to the work).
  * The meshes are dealt (largest first, to the least loaded) to `concurrency`
  * workspace slots (0 = 4, at most 256): a slot holds one mesh's lists at a
- * time, so the meshes are assembled in rounds of `concurrency`. The call is a
- * few small copy kernels and the persistent kernel on `stream`; it can be
- * captured into a CUDA graph, and calls on different streams are independent
- * (each uses only its own workspace). FP64 (opts->precision FEM_PREC_FP64). */
+ * time, so the meshes are assembled in rounds of `concurrency`. The call only
+ * queues kernels on `stream`; it can be captured into a CUDA graph, and calls
+ * on different streams are independent (each uses only its own workspace).
+ * FP64 (opts->precision FEM_PREC_FP64). */
 
 /* Bytes of workspace for this batch (the slots are sized for their largest mesh). */
 FEM_API fem_status fem_batched_workspace_size(const fem_mesh* meshes, int32_t n, const fem_opts* opts,
@@ -279,9 +278,7 @@ FEM_API fem_status fem_batched_workspace_size(const fem_mesh* meshes, int32_t n,
  * row_ptr and FEM_ERR_CAPACITY in its info). infos: DEVICE array [n] that
  * receives each mesh's fem_info (nnz, status bits, ...). stamps: optional
  * DEVICE array [n + 1] of GPU global-timer nanoseconds: stamps[0] at the start,
- * stamps[1 + i] when mesh i is done. outs[i].n_rows is set. Asynchronous.
- * A wait inside the kernel that runs out (2 s) raises FEM_ERR_TIMEOUT in the
- * info of the mesh whose item waited. */
+ * stamps[1 + i] when mesh i's round is done. outs[i].n_rows is set. Asynchronous. */
 FEM_API fem_status fem_assemble_batched(const fem_mesh* meshes, int32_t n, const fem_opts* opts,
                                         int32_t concurrency, void* workspace, size_t workspace_bytes,
                                         fem_csr* outs, fem_info* infos, unsigned long long* stamps, void* stream);

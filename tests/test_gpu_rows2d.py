@@ -85,3 +85,22 @@ def test_outputs_off_the_wide_alignment(fem, oracle_mod, cuda_device, off_v, off
     _compare(oracle_mod, m, a.row_ptr.cpu().numpy(), ci[off_c:off_c + nnz].cpu().numpy(),
              v[off_v:off_v + nnz].cpu().numpy())
     assert v[off_v + nnz].item() == 7.0 and ci[off_c + nnz].item() == -7
+
+
+def test_batch_of_many_slots_and_unaligned_outputs(fem, oracle_mod, cuda_device):
+    # 70 slots: a round of more meshes than one launch's descriptors hold; every
+    # third mesh's outputs off the wide alignment (and all kinds in a round)
+    import torch
+    import meshgen as mg
+    meshes = mg.batch_meshes(70, seed=11, emin=1, emax=120)
+    b = fem.Batch(meshes, concurrency=70)
+    nnz = b.sizes()
+    for i in range(0, 70, 3):
+        b.col_idx[i] = torch.empty(nnz[i] + 1, dtype=torch.int32, device="cuda")[1:]
+        b.values[i] = torch.empty(nnz[i] + 1, dtype=torch.float64, device="cuda")[1:]
+    b._set_outs(capacity=True)
+    b.run()
+    torch.cuda.synchronize()
+    assert all(s == 0 for s in b.statuses())
+    for i, m in enumerate(meshes):
+        _compare(oracle_mod, m, *b.result(i))
