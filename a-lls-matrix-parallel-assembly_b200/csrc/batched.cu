@@ -13,7 +13,7 @@
 // the same kernels as on their own. A round's mesh descriptors travel as kernel
 // parameters, so a captured CUDA graph holds them.
 //
-// What bounds it: the single-mesh kernels; a round costs up to 18 launches
+// What bounds it: the single-mesh kernels; a round costs up to 15 launches
 // whatever its number of meshes. B200, 16 meshes of 1,000 to 50,000 elements of
 // all kinds in 4 slots: 1.73 ms, where one persistent kernel of dependent work
 // items (CAS claims, element-wise atomics, no spatial order) took 8.0 ms.
@@ -70,9 +70,8 @@ __device__ __forceinline__ unsigned long long global_timer() {
 FEM_BATCH_KERNEL(256) kb_begin(const __grid_constant__ BatchRound<kMax> r, unsigned long long* start) {
     FEM_BATCH_MESH;
     if (start && blockIdx.x == 0 && threadIdx.x == 0) *start = global_timer();
-    lists_begin(bm.L, block, nblocks);
-    if (bm.kind == FEM_HEX20)
-        for (int i = block * 256 + threadIdx.x; i < bm.L.N; i += nblocks * 256) bm.cnt[i] = 0;
+    if (bm.kind == FEM_HEX20) lists_begin_hex20(bm.L, bm.cnt, block, nblocks);
+    else lists_begin(bm.L, block, nblocks);
 }
 
 static_assert(kFillThreads == kOccThreads, "one block shape for both");
@@ -124,14 +123,11 @@ FEM_BATCH_KERNEL(kHexRowThreads, FEM_HEXR_CTAS) kb_rows_hex20(const __grid_const
     rows_hex20(bm.m.conn, bm.L, bm.h, bm.queue, block, nblocks, s_row);
 }
 
-FEM_BATCH_KERNEL(32) kb_wide_rows_hex20(const __grid_constant__ BatchRound<kMax> r) {
-    FEM_BATCH_MESH;
-    __shared__ int s_uniq[kWideElems * 20];
-    wide_rows_hex20(bm.m.conn, bm.L, bm.h, bm.queue, block, nblocks, s_uniq);
-}
-
 FEM_BATCH_KERNEL(kHexRowThreads) kb_long_rows_hex20(const __grid_constant__ BatchRound<kMax> r) {
     FEM_BATCH_MESH;
+    __shared__ int s_uniq[kHexRowWarps][kWideElems * 20];
+    const int warp = threadIdx.x >> 5;
+    wide_rows_hex20(bm.m.conn, bm.L, bm.h, bm.queue, block * kHexRowWarps + warp, nblocks * kHexRowWarps, s_uniq[warp]);
     long_rows_hex20(bm.m.conn, bm.L, bm.h, bm.queue, block, nblocks);
 }
 
@@ -252,8 +248,8 @@ cudaError_t launch_round(const BatchMesh* meshes, int n, unsigned long long* sta
     l.run(kb_long_rows_2d<kMax>, kRowThreads, 0, 2 * sms, [&](M b) { return hex(b) ? 0 : blocks_of(b.L.N, kRowThreads); });
     l.run(kb_rows_hex20<kMax>, kHexRowThreads, 0, FEM_HEXR_CTAS * sms,
           [&](M b) { return hex(b) ? blocks_of(b.L.N, kHexRowWarps) : 0; });
-    l.run(kb_wide_rows_hex20<kMax>, 32, 0, 4 * sms, [&](M b) { return hex(b) ? (long long)b.L.N : 0; });
-    l.run(kb_long_rows_hex20<kMax>, kHexRowThreads, 0, sms, [&](M b) { return hex(b) ? (long long)b.L.N : 0; });
+    l.run(kb_long_rows_hex20<kMax>, kHexRowThreads, 0, sms,
+          [&](M b) { return hex(b) ? blocks_of(b.L.N, kHexRowWarps) : 0; });
     for (int i = 0; i < n && !l.err; i++)
         if (hex(meshes[i]) && meshes[i].h.order)
             l.err = launch_node_order(meshes[i].m, meshes[i].hist, meshes[i].ranges, meshes[i].cnt, meshes[i].bbox, sms, s);

@@ -87,7 +87,8 @@ template <int DPN, int kMode>
 cudaError_t launch_mode(const ListLayout& L, const HexRows& hex, const int* counts, int* row_ptr, int* col_idx,
                         double* values, long long capacity, long long* tile_sums, cudaStream_t s) {
     const int tiles = row_tiles(L.N);
-    k_tile_entries<DPN, kMode><<<tiles, kScanThreads, 0, s>>>(counts, L.N, tile_sums);
+    if (L.N <= kSmallNodes) tile_sums = nullptr;
+    else k_tile_entries<DPN, kMode><<<tiles, kScanThreads, 0, s>>>(counts, L.N, tile_sums);
     k_row_ptr<DPN, kMode><<<tiles, kScanThreads, 0, s>>>(counts, L.N, tile_sums, row_ptr, L.info, capacity);
     if (capacity <= 0) return cudaGetLastError();
     if constexpr (DPN == 3) {

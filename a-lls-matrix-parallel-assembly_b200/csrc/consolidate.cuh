@@ -514,7 +514,12 @@ __device__ __forceinline__ void row_ptr_rows(const int* __restrict__ counts, int
         s_cnt[i * kScanThreads + tid] = n < N ? __ldg(counts + n) : 0;
     }
     long long before = 0;
-    for (int t = tid; t < tile; t += kScanThreads) before += __ldg(tile_sums + t);
+    if (tile_sums) {
+        for (int t = tid; t < tile; t += kScanThreads) before += __ldg(tile_sums + t);
+    } else {  // a small mesh: the nodes before the tile
+#pragma unroll 8
+        for (int n = tid; n < (int)first; n += kScanThreads) before += node_entries<DPN, kMode>(__ldg(counts + n));
+    }
     long long base;
     block_exclusive_scan(before, s_warp, base);
     long long sum = 0;

@@ -261,18 +261,17 @@ fem_status fem_alls_scatter(const fem_mesh* mesh, const fem_opts* opts, void* wo
     ListLayout L = device_layout(h, workspace);
     unsigned char* b = static_cast<unsigned char*>(workspace);
     MeshView m = mesh_view(mesh);
-    cudaError_t err = launch_lists_begin(L, s);
+    cudaError_t err = cudaSuccess;
     // the long rows' queue takes the upper-triangle counts' place (written by a later call)
     int* queue = reinterpret_cast<int*>(b + h.off_ucounts);
     if (h.dpn == 2) {
-        if (!err) err = launch_rows_2d(m, L, queue, h.kind, precision, ctas, s);
+        err = launch_rows_2d(m, L, queue, h.kind, precision, ctas, s);
         return err ? cuda_fail(err) : FEM_OK;
     }
     const HexRows hex = hex_rows(h, workspace);
     int* cnt = reinterpret_cast<int*>(b + h.off_inc);
     long long* tiles = reinterpret_cast<long long*>(b + h.off_tiles);  // free until the consolidation
-    if (!err) err = launch_occurrences(m, L, hex, cnt, tiles, s);
-    if (!err) err = launch_rows_hex20(m, L, hex, queue, s);
+    err = launch_rows_hex20(m, L, hex, cnt, tiles, queue, s);
     if (!err && hex.order) {
         int *ranges, *hist;
         unsigned long long* bbox;

@@ -51,9 +51,10 @@ struct MeshView {
 // 2-D chunk rows are 16 int32 words (14 slots + fill + next).
 constexpr int k2DSlots = 14;
 
-// Clears the per-node counters and the info word of a scatter.
-cudaError_t launch_lists_begin(const ListLayout& L, cudaStream_t s);
-// The row lists of a 2-D mesh (rows2d.cu), after launch_lists_begin;
+// Meshes of at most this many nodes (and 2-D: 4 times as many elements) are scattered by one cooperative launch and
+// scanned without a tile pass: their time is the launches'.
+constexpr int kSmallNodes = 16384;
+// The info word, counters and row lists of a 2-D mesh (rows2d.cu);
 // precision FEM_PREC_FP64 or FEM_PREC_FP32 (the arithmetic of the Ke blocks).
 // queue: N ints of scratch; ctas_per_sm: cap on the persistent grid's resident CTAs per SM (0 = all that fit).
 cudaError_t launch_rows_2d(const MeshView& m, const ListLayout& L, int* queue, int kind, int precision,
@@ -120,11 +121,10 @@ struct HexRows {
     const int* order;     // [N] node visit order of the consolidation, or NULL: as numbered
     unsigned short* map;  // [E * 400] rank of column node b in row node a's list, at 20 (20 e + a) + b
 };
-// Fills off / inc for the elements without a bad node id; cnt: N ints, tiles: row_tiles(N) partials of scratch.
-cudaError_t launch_occurrences(const MeshView& m, const ListLayout& L, const HexRows& h, int* cnt, long long* tiles,
-                               cudaStream_t s);
-// The sorted row lists and the rank map; queue: N ints of scratch.
-cudaError_t launch_rows_hex20(const MeshView& m, const ListLayout& L, const HexRows& h, int* queue, cudaStream_t s);
+// The info word, the occurrences (off / inc, of the elements without a bad node id), the sorted row lists and the
+// rank map; cnt, queue: N ints, tiles: row_tiles(N) partials of scratch.
+cudaError_t launch_rows_hex20(const MeshView& m, const ListLayout& L, const HexRows& h, int* cnt, long long* tiles,
+                              int* queue, cudaStream_t s);
 // Row lists -> CSR / BSR / upper triangle (mode: consolidate.cuh's kOut*; row_ptr already written).
 cudaError_t launch_count_upper_hex20(const ListLayout& L, int* ucounts, cudaStream_t s);
 cudaError_t launch_write_hex20(const ListLayout& L, const HexRows& h, int mode, const int* ucounts, const int* row_ptr,

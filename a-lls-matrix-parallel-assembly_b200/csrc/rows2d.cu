@@ -1,4 +1,6 @@
 // K1 for 2-D meshes: launches of the row-list kernels (rows2d.cuh).
+#include <cooperative_groups.h>
+
 #include <algorithm>
 
 #include "rows2d.cuh"
@@ -26,8 +28,57 @@ __global__ void __launch_bounds__(kRowThreads) k_long_rows_2d(MeshView m, ListLa
     long_rows_2d<KIND, T>(m, L, queue, blockIdx.x, gridDim.x, sm);
 }
 
+// The whole scatter of a small mesh (launch.h's kSmallNodes) in one cooperative
+// launch: a launch costs the caller about 4 us, a grid barrier 1 to 2 us, and
+// the phases of such a mesh take 1 to 10 us each. The long rows' registers slow
+// the rows down here (rows2d.cuh), by less than a launch.
+template <int KIND, typename T>
+__global__ void __launch_bounds__(kRowThreads, FEM_ROWS_Q4_CTAS)
+    k_small_2d(MeshView m, ListLayout L, int* __restrict__ queue) {
+    __shared__ union {
+        RowSmem rows;
+        LongSmem longs;
+    } sm;
+    const cooperative_groups::grid_group grid = cooperative_groups::this_grid();
+    lists_begin(L, blockIdx.x, gridDim.x);
+    grid.sync();
+    fill_2d<KIND>(m, L, blockIdx.x, gridDim.x);
+    grid.sync();
+    rows_2d<KIND, T>(m, L, queue, blockIdx.x, gridDim.x, sm.rows);
+    grid.sync();
+    long_rows_2d<KIND, T>(m, L, queue, blockIdx.x, gridDim.x, sm.longs);
+}
+
+template <int KIND, typename T>
+cudaError_t launch_small_t(const MeshView& m, const ListLayout& L, int* queue, int ctas_per_sm, cudaStream_t s) {
+    static DeviceCache cache;
+    int per_sm = 0;
+    cudaError_t err = per_device(cache, [](int& v) {
+        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, k_small_2d<KIND, T>, kRowThreads, 0);
+    }, per_sm);
+    if (err) return err;
+    const int use = ctas_per_sm > 0 ? std::min(ctas_per_sm, per_sm) : per_sm;
+    const long long want = std::max(((long long)m.N + kRowThreads - 1) / kRowThreads,
+                                    ((long long)m.E_count + kRowThreads - 1) / kRowThreads);
+    const int grid = (int)std::min<long long>(want, (long long)use * sm_count());
+    MeshView mv = m;
+    ListLayout lv = L;
+    void* args[] = {&mv, &lv, &queue};
+    return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_small_2d<KIND, T>), dim3(grid), dim3(kRowThreads),
+                                       args, 0, s);
+}
+
+cudaError_t launch_lists_begin(const ListLayout& L, cudaStream_t s) {
+    const int grid = (int)std::max<long long>(1, std::min<long long>(((long long)L.N + 1023) / 1024, sm_count() * 4));
+    k_lists_begin<<<grid, 256, 0, s>>>(L);
+    return cudaGetLastError();
+}
+
 template <int KIND, typename T>
 cudaError_t launch_rows_t(const MeshView& m, const ListLayout& L, int* queue, int ctas_per_sm, cudaStream_t s) {
+    if (m.N <= kSmallNodes && m.E_count <= 4 * kSmallNodes) return launch_small_t<KIND, T>(m, L, queue, ctas_per_sm, s);
+    cudaError_t err0 = launch_lists_begin(L, s);
+    if (err0) return err0;
     static DeviceCache cache;
     const size_t smem = sizeof(RowSmem);
     int per_sm = 0;
@@ -56,12 +107,6 @@ cudaError_t launch_rows_kind(const MeshView& m, const ListLayout& L, int* queue,
 }
 
 }  // namespace
-
-cudaError_t launch_lists_begin(const ListLayout& L, cudaStream_t s) {
-    const int grid = (int)std::max<long long>(1, std::min<long long>(((long long)L.N + 1023) / 1024, sm_count() * 4));
-    k_lists_begin<<<grid, 256, 0, s>>>(L);
-    return cudaGetLastError();
-}
 
 cudaError_t launch_rows_2d(const MeshView& m, const ListLayout& L, int* queue, int kind, int precision,
                            int ctas_per_sm, cudaStream_t s) {

@@ -76,7 +76,7 @@ __device__ __forceinline__ int elem_nodes(const MeshView& m, int e) {
 template <int KIND>
 __device__ __forceinline__ void fill_2d(const MeshView& m, const ListLayout& L, int block, int nblocks) {
     constexpr int NPE = KIND == FEM_T3 ? 3 : 4;
-    for (int e = block * kFillThreads + threadIdx.x; e < m.E_count; e += nblocks * kFillThreads) {
+    for (int e = block * blockDim.x + threadIdx.x; e < m.E_count; e += nblocks * blockDim.x) {
         const int npe = elem_nodes<KIND>(m, e);
         int n[NPE];
         bool bad = false;
@@ -359,9 +359,9 @@ __device__ __forceinline__ void long_row_2d(const MeshView& m, const ListLayout&
 template <int KIND, typename T>
 __device__ __forceinline__ void long_rows_2d(const MeshView& m, const ListLayout& L, const int* __restrict__ queue,
                                              int block, int nblocks, LongSmem& sm) {
-    const int count = __ldg(&L.info->long_rows);
+    const int count = __ldcg(&L.info->long_rows);
     for (int k = block; k < count; k += nblocks) {
-        const int n = __ldg(queue + k);
+        const int n = __ldcg(queue + k);
         long_row_2d<KIND, T>(m, L, n, __ldcg(L.counts + n), sm);
     }
 }

@@ -44,6 +44,16 @@ constexpr int kNoOcc = 0x7FFFFFFF;
 
 __device__ __forceinline__ int* occ_pos(const HexRows& h) { return reinterpret_cast<int*>(h.map); }  // 80 of 800 bytes an element
 
+// Clears a scatter's info word and occurrence counters.
+__device__ __forceinline__ void lists_begin_hex20(const ListLayout& L, int* __restrict__ cnt, int block, int nblocks) {
+    for (int i = block * blockDim.x + threadIdx.x; i < L.N; i += nblocks * blockDim.x) cnt[i] = 0;
+    if (block == 0 && threadIdx.x == 0) {
+        DevInfo d{};
+        d.pool_chunks = L.cap2;
+        *L.info = d;
+    }
+}
+
 __device__ __forceinline__ void occ_count(const MeshView& m, const HexRows& h, int* __restrict__ cnt, DevInfo* info,
                                           int block, int nblocks) {
     int* pos = occ_pos(h);
@@ -73,7 +83,7 @@ __device__ __forceinline__ void occ_sums(const int* __restrict__ cnt, int N, lon
 #pragma unroll
     for (int i = 0; i < kRowTile / kScanThreads; i++) {
         const long long n = (long long)tile * kRowTile + i * kScanThreads + threadIdx.x;
-        if (n < N) sum += __ldg(cnt + n);
+        if (n < N) sum += __ldcg(cnt + n);
     }
     long long total;
     block_exclusive_scan(sum, s_warp, total);
@@ -85,6 +95,7 @@ struct OccSmem {
     int cnt[kRowTile];
 };
 
+// tiles NULL (small meshes): the counts before the tile are summed directly.
 __device__ __forceinline__ void occ_offsets(const int* __restrict__ cnt, int N, const long long* __restrict__ tiles,
                                             int* __restrict__ off, DevInfo* info, int tile, int ntiles, OccSmem& sm) {
     constexpr int kItems = kRowTile / kScanThreads;
@@ -93,10 +104,15 @@ __device__ __forceinline__ void occ_offsets(const int* __restrict__ cnt, int N, 
 #pragma unroll
     for (int i = 0; i < kItems; i++) {
         const long long n = first + i * kScanThreads + tid;
-        sm.cnt[i * kScanThreads + tid] = n < N ? __ldg(cnt + n) : 0;
+        sm.cnt[i * kScanThreads + tid] = n < N ? __ldcg(cnt + n) : 0;
     }
     long long before = 0, base, total;
-    for (int t = tid; t < tile; t += kScanThreads) before += __ldg(tiles + t);
+    if (tiles) {
+        for (int t = tid; t < tile; t += kScanThreads) before += __ldcg(tiles + t);
+    } else {
+#pragma unroll 8
+        for (int n = tid; n < (int)first; n += kScanThreads) before += __ldcg(cnt + n);
+    }
     block_exclusive_scan(before, sm.warp, base);
     int c[kItems];
     long long sum = 0;
@@ -127,10 +143,10 @@ __device__ __forceinline__ void occ_fill(const MeshView& m, const HexRows& h, in
     const int* pos = occ_pos(h);
     const long long count = 20ll * m.E_count;
     for (long long o = (long long)block * kOccThreads + threadIdx.x; o < count; o += (long long)nblocks * kOccThreads) {
-        const int p = pos[o];
+        const int p = __ldcg(pos + o);
         if (p == kNoOcc) continue;
         const unsigned flag = (unsigned)p & kOccRepeats;
-        h.inc[__ldg(h.off + __ldg(m.conn + o)) + (int)((unsigned)p & ~kOccRepeats)] = (int)((unsigned)o | flag);
+        h.inc[__ldcg(h.off + __ldg(m.conn + o)) + (int)((unsigned)p & ~kOccRepeats)] = (int)((unsigned)o | flag);
     }
 }
 
@@ -231,12 +247,12 @@ __device__ __forceinline__ void rows_hex20(const int* __restrict__ conn, const L
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     HexRowSmem& sm = s_row[warp];
     for (long long nn = (long long)block * kHexRowWarps + warp; nn < L.N; nn += (long long)nblocks * kHexRowWarps) {
-        const int n = (int)nn, lo = __ldg(off + n), d = __ldg(off + n + 1) - lo;
+        const int n = (int)nn, lo = __ldcg(off + n), d = __ldcg(off + n + 1) - lo;
         if (d > kMaxElems) {
             if (lane == 0) queue[atomicAdd(&L.info->long_rows, 1)] = n;
             continue;
         }
-        const int o = lane < d ? (int)occ_of(__ldg(inc + lo + lane)) : 0;
+        const int o = lane < d ? (int)occ_of(__ldcg(inc + lo + lane)) : 0;
         int node[kCand], slot[kCand];
 #pragma unroll
         for (int q = 0; q < kCand; q++) {
@@ -297,17 +313,17 @@ __device__ __forceinline__ void rows_hex20(const int* __restrict__ conn, const L
     }
 }
 
+// warp `warp` of `nwarps`; s_uniq: the warp's kWideElems * 20 words.
 __device__ __forceinline__ void wide_rows_hex20(const int* __restrict__ conn, const ListLayout& L, const HexRows& h,
-                                                const int* __restrict__ queue, int block, int nblocks,
-                                                int (&s_uniq)[kWideElems * 20]) {
+                                                const int* __restrict__ queue, int warp, int nwarps, int* s_uniq) {
     const int* __restrict__ off = h.off;
     const int* __restrict__ inc = h.inc;
     unsigned short* __restrict__ map = h.map;
-    const int lane = threadIdx.x, count = __ldg(&L.info->long_rows);
-    for (int k = block; k < count; k += nblocks) {
-        const int n = __ldg(queue + k), lo = __ldg(off + n), d = __ldg(off + n + 1) - lo;
+    const int lane = threadIdx.x & 31, count = __ldcg(&L.info->long_rows);
+    for (int k = warp; k < count; k += nwarps) {
+        const int n = __ldcg(queue + k), lo = __ldcg(off + n), d = __ldcg(off + n + 1) - lo;
         if (d > kWideElems) continue;  // k_long_rows_hex20's
-        const int o = lane < d ? (int)occ_of(__ldg(inc + lo + lane)) : 0;
+        const int o = lane < d ? (int)occ_of(__ldcg(inc + lo + lane)) : 0;
         int node[kWideCand];
 #pragma unroll
         for (int q = 0; q < kWideCand; q++) {
@@ -349,9 +365,9 @@ __device__ __forceinline__ void long_rows_hex20(const int* __restrict__ conn, co
     const int* __restrict__ inc = h.inc;
     unsigned short* __restrict__ map = h.map;
     __shared__ int s_min[2], s_kept, s_next;
-    const int tid = threadIdx.x, count = __ldg(&L.info->long_rows);
+    const int tid = threadIdx.x, count = __ldcg(&L.info->long_rows);
     for (int k = block; k < count; k += nblocks) {
-        const int n = __ldg(queue + k), lo = __ldg(off + n), d = __ldg(off + n + 1) - lo;
+        const int n = __ldcg(queue + k), lo = __ldcg(off + n), d = __ldcg(off + n + 1) - lo;
         if (d <= kWideElems) continue;
         const long long cand = 20ll * d;
         // two passes over the row's columns in increasing order: count, then write
@@ -364,7 +380,7 @@ __device__ __forceinline__ void long_rows_hex20(const int* __restrict__ conn, co
                 __syncthreads();
                 int m = 0x7FFFFFFF;
                 for (long long j = tid; j < cand; j += kHexRowThreads) {
-                    const unsigned ot = occ_of(__ldg(inc + lo + (int)(j / 20)));
+                    const unsigned ot = occ_of(__ldcg(inc + lo + (int)(j / 20)));
                     const int b = (int)(j % 20), x = __ldg(conn + (size_t)(ot / 20) * 20 + b);
                     if (x > last) m = min(m, x);
                     // the previous column's rank, met again on the way
