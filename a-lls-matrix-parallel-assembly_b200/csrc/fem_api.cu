@@ -718,6 +718,9 @@ namespace {
 struct MapHostLayout {
     int G;  // map entries per element
     size_t off_info, off_pos, off_perm, off_ranges, off_hist, off_bbox, total;
+    // 2-D meshes whose occurrences fit in the same bytes (all but mostly unconnected triangles): by row nodes instead
+    bool rows;
+    size_t off_off, off_occ, off_ranks;
 };
 
 MapHostLayout map_layout(const fem_mesh* m) {
@@ -741,7 +744,22 @@ MapHostLayout map_layout(const fem_mesh* m) {
     h.off_bbox = off;
     off += align_up(6 * sizeof(unsigned long long));
     h.total = off;
+    if (m->kind != FEM_HEX20) {
+        const size_t N = (size_t)m->num_nodes;
+        h.off_off = h.off_pos;
+        h.off_occ = h.off_off + align_up((N + 1) * sizeof(int));
+        h.off_ranks = h.off_occ + align_up(E * npe * sizeof(unsigned));
+        // the ranks, or, while the map is built, the counters and scan partials in their place
+        const size_t end = h.off_ranks + std::max(align_up(E * npe * npe * sizeof(unsigned short)),
+                                                  align_up(N * sizeof(int)) + row_tiles(m->num_nodes) * sizeof(long long));
+        h.rows = end <= h.total && E < ((size_t)1 << 29) && E > 0;
+    }
     return h;
+}
+
+RowsMap rows_map(const MapHostLayout& h, unsigned char* b) {
+    return RowsMap{reinterpret_cast<int*>(b + h.off_off), reinterpret_cast<unsigned*>(b + h.off_occ),
+                   reinterpret_cast<unsigned short*>(b + h.off_ranks)};
 }
 
 fem_status check_map(const fem_mesh* mesh, const void* map, size_t map_bytes, MapHostLayout& h) {
@@ -778,7 +796,11 @@ fem_status fem_scatter_map_build(const fem_mesh* mesh, const int32_t* row_ptr, c
     int* ranges = reinterpret_cast<int*>(b + h.off_ranges);
     int* hist = reinterpret_cast<int*>(b + h.off_hist);
     cudaError_t err = cudaMemsetAsync(info, 0, sizeof(DevInfo), s);
-    if (!err && mesh->num_elems > 0) {
+    if (!err && h.rows) {
+        int* cnt = reinterpret_cast<int*>(b + h.off_ranks);
+        long long* tiles = reinterpret_cast<long long*>(b + h.off_ranks + align_up((size_t)m.N * sizeof(int)));
+        err = launch_build_rows_map(m, mesh->kind, row_ptr, col_idx, rows_map(h, b), cnt, tiles, info, s);
+    } else if (!err && mesh->num_elems > 0) {
         err = launch_build_map(m, mesh->kind, row_ptr, col_idx, reinterpret_cast<int*>(b + h.off_pos),
                                &info->status_bits, s);
         // the element visit order of the A-LLS scatter, for the locality of the adds
@@ -806,11 +828,13 @@ fem_status fem_reassemble_values(const fem_mesh* mesh, const fem_opts* opts, con
     const int* pos = reinterpret_cast<const int*>(b + h.off_pos);
     const int* perm = reinterpret_cast<const int*>(b + h.off_perm);
     const int* ranges = reinterpret_cast<const int*>(b + h.off_ranges);
-    cudaError_t err = cudaMemsetAsync(&info->status_bits, 0, sizeof(int), s);
-    if (!err && nnz > 0) err = cudaMemsetAsync(values, 0, (size_t)nnz * sizeof(double), s);
+    cudaError_t err = cudaMemsetAsync(info, 0, sizeof(DevInfo), s);
+    if (!err && nnz > 0 && !h.rows) err = cudaMemsetAsync(values, 0, (size_t)nnz * sizeof(double), s);
     if (!err && mesh->num_elems > 0) {
         const MeshView m = mesh_view(mesh);
-        if (mesh->kind == FEM_HEX20)
+        if (h.rows)
+            err = launch_rows_values_2d(m, mesh->kind, precision, rows_map(h, b), row_ptr, values, &info->status_bits, s);
+        else if (mesh->kind == FEM_HEX20)
             err = launch_reassemble_hex20(m, precision, perm, MapTarget{pos, row_ptr, values, nullptr}, info, s);
         else
             err = launch_reassemble_2d(m, precision, pos, h.G, perm, ranges, row_ptr, values, &info->status_bits, s);

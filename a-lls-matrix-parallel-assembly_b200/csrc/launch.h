@@ -96,6 +96,17 @@ cudaError_t launch_build_map(const MeshView& m, int kind, const int* row_ptr, co
 // {q4 begin, q4 end, t3 begin, t3 end}; Hex20 over perm (status bits in info).
 cudaError_t launch_reassemble_2d(const MeshView& m, int precision, const int* map, int G, const int* perm,
                                  const int* ranges, const int* row_ptr, double* values, int* status, cudaStream_t s);
+// The same by row nodes (2-D): each node's occurrences (element << 2 | position) and the ranks of their nodes in its row.
+struct RowsMap {
+    int* off;               // [N + 1]
+    unsigned* occ;          // [npe * E]
+    unsigned short* ranks;  // [npe * npe * E]
+};
+// cnt (N ints) and tiles (row_tiles(N) partials): scratch.
+cudaError_t launch_build_rows_map(const MeshView& m, int kind, const int* row_ptr, const int* col_idx, const RowsMap& r,
+                                  int* cnt, long long* tiles, DevInfo* info, cudaStream_t s);
+cudaError_t launch_rows_values_2d(const MeshView& m, int kind, int precision, const RowsMap& r, const int* row_ptr,
+                                  double* values, int* status, cudaStream_t s);
 // The tensor-core form of the Hex20 value-only re-assembly (ke_tcgen05.cu).
 cudaError_t launch_reassemble_hex20_tc(const MeshView& m, const int* perm, const MapTarget& t, DevInfo* info,
                                        cudaStream_t s);

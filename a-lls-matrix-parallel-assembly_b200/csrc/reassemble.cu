@@ -1,25 +1,37 @@
 // Value-only re-assembly: a mesh whose connectivity is unchanged (new
 // coordinates, E or nu, as in nonlinear or time-stepping solvers) is
 // re-assembled into the CSR pattern of an earlier assembly without building
-// any list: a scatter map records, for every element node block (a, b), the
-// CSR position of its first entry, and the element blocks are added there
-// with FP64 atomics.
+// any list.
 //
 // The reference has no such path: every assembly repeats the list build
 // (assembleGlobalStiffnessKernelALLS, ALLS_Quad2D_Assembly_Accuracy_Analysis.cu:394-468)
 // and, on the host, the pattern (buildCSRStructure, Q4A:605-645).
 //
-// Map layout (int32): [E * G] block positions, G = npe^2 (Q4 and mixed 16,
-// T3 9, Hex20 400), position of block (a, b) of element e at e * G + a * npe + b;
-// then the element visit order [E] and its scratch (element-type ranges,
-// bucket histogram, bounding box), built with the same element order as the
-// A-LLS scatter. Entry (i, j) of block (a, b) lies at p + i * rowlen + j,
-// rowlen being the length of the block's first CSR row (the dpn rows of a node
-// have the same columns).
+// 2-D kinds (k_rows_values_2d): the map holds, node by node, the node's
+// occurrences (element e, local position a) and the ranks of the element's
+// nodes in the node's sorted row. A thread owns a node: it computes the node's
+// row of each of its elements' Ke and sums the blocks at their ranks in shared
+// memory; the warp then writes its nodes' two CSR rows with consecutive lanes
+// on consecutive entries. No zeroing, no atomics, and nothing is searched. Rows
+// of more than 14 columns are added with FP64 atomics by their warp. What
+// bounds it: the gathered loads (element -> nodes -> coordinates) and the
+// instructions of the element rows. B200, T3 1001x699 (shuffled elements): 177
+// us, where the block-position form took 301 us plus 28 us of zeroing.
+//
+// Block positions (Hex20, and 2-D meshes whose occurrences do not fit, mostly
+// unconnected triangles): the map records, for every element node block (a, b),
+// the CSR position of its first entry, position of block (a, b) of element e at
+// e * G + a * npe + b, G = npe^2; the element blocks are added there with FP64
+// atomics, in the element order of reorder.cu, which the map holds too. Entry
+// (i, j) of block (a, b) lies at p + i * rowlen + j, rowlen being the length of
+// the block's first CSR row (the dpn rows of a node have the same columns).
+// Bound by the L2's FP64 atomics (about 180 G/s measured; adding the entries of
+// a block row by neighbouring lanes changes little: 301 against 281 us).
 #include <algorithm>
 
 #include "element2d.cuh"
 #include "launch.h"
+#include "rows_hex20.cuh"
 
 namespace fem {
 namespace {
@@ -113,6 +125,326 @@ __global__ void __launch_bounds__(kThreads) k_reassemble_2d(MeshView m, const in
     }
 }
 
+// ---- 2-D rows ---------------------------------------------------------------------
+
+template <int KIND>
+__device__ __forceinline__ int elem_nodes(const MeshView& m, int e) {
+    if (KIND == FEM_T3) return 3;
+    if (KIND == FEM_Q4) return 4;
+    return __ldg(m.types + e) == FEM_Q4 ? 4 : 3;
+}
+
+template <int KIND>
+__device__ __forceinline__ bool bad_nodes(const MeshView& m, int e, int npe) {
+    bool bad = false;
+    for (int k = 0; k < npe; k++) {
+        const int n = __ldg(m.conn + (size_t)e * m.stride + k);
+        bad |= n < 0 || n >= m.N;
+    }
+    return bad;
+}
+
+template <int KIND>
+__global__ void __launch_bounds__(kThreads) k_map_count(MeshView m, int* __restrict__ cnt, int* __restrict__ status) {
+    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < m.E_count; e += gridDim.x * blockDim.x) {
+        const int npe = elem_nodes<KIND>(m, e);
+        if (bad_nodes<KIND>(m, e, npe)) {
+            atomicOr(status, 1 << FEM_ERR_BAD_MESH);
+            continue;
+        }
+        for (int k = 0; k < npe; k++) atomicAdd(cnt + __ldg(m.conn + (size_t)e * m.stride + k), 1);
+    }
+}
+
+__global__ void __launch_bounds__(kScanThreads) k_map_sums(const int* __restrict__ cnt, int N,
+                                                           long long* __restrict__ tiles) {
+    __shared__ long long s_warp[kScanThreads / 32 + 1];
+    occ_sums(cnt, N, tiles, blockIdx.x, s_warp);
+}
+
+__global__ void __launch_bounds__(kScanThreads) k_map_offsets(const int* __restrict__ cnt, int N,
+                                                              const long long* __restrict__ tiles,
+                                                              int* __restrict__ off, DevInfo* info) {
+    __shared__ OccSmem sm;
+    occ_offsets(cnt, N, tiles, off, info, blockIdx.x, gridDim.x, sm);
+}
+
+// The occurrences of every node (cnt counts down to zero).
+template <int KIND>
+__global__ void __launch_bounds__(kThreads) k_map_fill(MeshView m, const int* __restrict__ off, int* __restrict__ cnt,
+                                                       unsigned* __restrict__ occ) {
+    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < m.E_count; e += gridDim.x * blockDim.x) {
+        const int npe = elem_nodes<KIND>(m, e);
+        if (bad_nodes<KIND>(m, e, npe)) continue;
+        for (int k = 0; k < npe; k++) {
+            const int n = __ldg(m.conn + (size_t)e * m.stride + k);
+            occ[__ldg(off + n) + atomicSub(cnt + n, 1) - 1] = ((unsigned)e << 2) | k;
+        }
+    }
+}
+
+// ranks[NPE * j + k]: rank in the row of occurrence j's node of the element's node k positions after it.
+template <int KIND>
+__global__ void __launch_bounds__(kThreads) k_map_ranks(MeshView m, const int* __restrict__ off,
+                                                        const unsigned* __restrict__ occ,
+                                                        const int* __restrict__ row_ptr,
+                                                        const int* __restrict__ col_idx,
+                                                        unsigned short* __restrict__ ranks, int* __restrict__ status) {
+    constexpr int NPE = KIND == FEM_T3 ? 3 : 4;
+    const int total = __ldg(off + m.N);
+    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < total; j += gridDim.x * blockDim.x) {
+        const unsigned w = __ldg(occ + j);
+        const int e = (int)(w >> 2), a = (int)(w & 3u), npe = elem_nodes<KIND>(m, e);
+        const int n = __ldg(m.conn + (size_t)e * m.stride + a);
+        for (int k = 0; k < npe; k++) {
+            const int b = a + k < npe ? a + k : a + k - npe;
+            const int p = find_col(row_ptr, col_idx, 2 * n, 2 * __ldg(m.conn + (size_t)e * m.stride + b));
+            if (p < 0) atomicOr(status, 1 << FEM_ERR_INTERNAL);  // the pattern lacks the block
+            const int r = p < 0 ? 0 : (p - __ldg(row_ptr + 2 * n)) / 2;
+            if (r > 0xFFFF) atomicOr(status, 1 << FEM_ERR_RANGE);
+            ranks[(size_t)NPE * j + k] = (unsigned short)r;
+        }
+    }
+}
+
+constexpr int kRowThreads = 64;
+constexpr int kRowPad = kRowThreads + 1;  // a node's entries on different banks, and a warp's nodes too
+// Columns of a row summed in shared memory (T3 nodes of up to 9 triangles, quadrilateral nodes of up to 6), and the
+// resident CTAs the registers are set for. T3: 8 CTAs of 21 KB leave L1 60 KB for the gathered loads (9 CTAs 223, 10
+// CTAs 217 us; 14 columns, 7 CTAs 232 us).
+#ifndef FEM_REROWS_T3
+#define FEM_REROWS_T3 10
+#define FEM_REROWS_T3_CTAS 8
+#endif
+#ifndef FEM_REROWS_Q4
+#define FEM_REROWS_Q4 14
+#define FEM_REROWS_Q4_CTAS 6
+#endif
+template <int KIND>
+struct RowsShape {
+    static constexpr int kCols = KIND == FEM_T3 ? FEM_REROWS_T3 : FEM_REROWS_Q4;
+    static constexpr int kCtas = KIND == FEM_T3 ? FEM_REROWS_T3_CTAS : FEM_REROWS_Q4_CTAS;
+};
+
+template <int NPE>
+struct OccData {
+    int e, npe;
+    int nodes[NPE];  // [0]: unused (the row node)
+    double x[NPE], y[NPE], E, nu;
+    unsigned short rank[NPE];
+};
+
+template <int KIND, int NPE>
+__device__ __forceinline__ void load_occ(const MeshView& m, unsigned w, const unsigned short* ranks, int j,
+                                         OccData<NPE>& d) {
+    d.e = (int)(w >> 2);
+    d.npe = elem_nodes<KIND>(m, d.e);
+    const int a = (int)(w & 3u);
+#pragma unroll
+    for (int k = 1; k < NPE; k++) {
+        const int b = a + k < d.npe ? a + k : a + k - d.npe;
+        d.nodes[k] = __ldg(m.conn + (size_t)d.e * m.stride + (k < d.npe ? b : a));
+    }
+#pragma unroll
+    for (int k = 0; k < NPE; k++) d.rank[k] = __ldg(ranks + (size_t)NPE * j + k);
+}
+
+template <int NPE>
+__device__ __forceinline__ void load_geometry(const MeshView& m, OccData<NPE>& d) {
+#pragma unroll
+    for (int k = 1; k < NPE; k++) {
+        d.x[k] = __ldg(m.x + d.nodes[k]);
+        d.y[k] = __ldg(m.y + d.nodes[k]);
+    }
+    d.E = m.E ? __ldg(m.E + d.e) : m.E0;
+    d.nu = m.nu ? __ldg(m.nu + d.e) : m.nu0;
+}
+
+// Blocks (row node, node k positions after it) of an occurrence, k < npe. Returns detJ.
+template <int KIND, typename T, int NPE>
+__device__ __forceinline__ double occ_blocks(const OccData<NPE>& d, double t, double (&k)[NPE][4]) {
+    if constexpr (KIND != FEM_MIXED_2D) {
+        return ke_row_2d<NPE, T>(d.x, d.y, d.E, d.nu, t, k);
+    } else {
+        if (d.npe == 4) return ke_row_2d<4, T>(d.x, d.y, d.E, d.nu, t, k);
+        const double x3[3] = {d.x[0], d.x[1], d.x[2]}, y3[3] = {d.y[0], d.y[1], d.y[2]};
+        double k3[3][4];
+        const double det = ke_row_2d<3, T>(x3, y3, d.E, d.nu, t, k3);
+#pragma unroll
+        for (int b = 0; b < 3; b++)
+#pragma unroll
+            for (int v = 0; v < 4; v++) k[b][v] = k3[b][v];
+        return det;
+    }
+}
+
+template <int KIND, typename T>
+__global__ void __launch_bounds__(kRowThreads, RowsShape<KIND>::kCtas)
+    k_rows_values_2d(MeshView m, const int* __restrict__ off, const unsigned* __restrict__ occ,
+                     const unsigned short* __restrict__ ranks, const int* __restrict__ row_ptr,
+                     double* __restrict__ values, bool wide, int* __restrict__ status) {
+    constexpr int NPE = KIND == FEM_T3 ? 3 : 4, kRowCols = RowsShape<KIND>::kCols;
+    constexpr unsigned kFull = 0xFFFFFFFFu;
+    __shared__ double acc[kRowCols][4][kRowPad];
+    const int tid = threadIdx.x, lane = tid & 31, warp0 = tid & ~31;
+    for (long long tile = blockIdx.x; tile * kRowThreads < m.N; tile += gridDim.x) {
+        const long long n = tile * kRowThreads + tid;
+        int base = 0, u = 0, lo = 0, d = 0;
+        if (n < m.N) {
+            base = __ldg(row_ptr + 2 * n);
+            u = (__ldg(row_ptr + 2 * n + 1) - base) / 2;
+            lo = __ldg(off + n);
+            d = __ldg(off + n + 1) - lo;
+        }
+        const bool fits = u <= kRowCols;
+        if (fits) {
+            for (int q = 0; q < u; q++)
+#pragma unroll
+                for (int v = 0; v < 4; v++) acc[q][v][tid] = 0.0;
+        }
+        if (fits && d > 0) {
+            OccData<NPE> cur, nxt;
+            const double xn = __ldg(m.x + n), yn = __ldg(m.y + n);
+            double dg[4] = {0.0, 0.0, 0.0, 0.0};
+            load_occ<KIND>(m, __ldg(occ + lo), ranks, lo, cur);
+            unsigned w1 = d > 1 ? __ldg(occ + lo + 1) : 0;
+            load_geometry(m, cur);
+            int diag = 0;
+            for (int i = 0; i < d; i++) {
+                // the next occurrence's nodes and the one after's word are in flight
+                if (i + 1 < d) load_occ<KIND>(m, w1, ranks, lo + i + 1, nxt);
+                if (i + 2 < d) w1 = __ldg(occ + lo + i + 2);
+                cur.x[0] = xn;
+                cur.y[0] = yn;
+                double kb[NPE][4];
+                if (!(occ_blocks<KIND, T>(cur, m.t, kb) > 0.0)) atomicOr(status, 1 << FEM_ERR_DETJ);
+                if (i + 1 < d) load_geometry(m, nxt);
+                diag = cur.rank[0];
+#pragma unroll
+                for (int v = 0; v < 4; v++) dg[v] += kb[0][v];
+                bool same = false;  // a repeated node
+#pragma unroll
+                for (int b = 2; b < NPE; b++)
+#pragma unroll
+                    for (int q = 1; q < b; q++) same |= b < cur.npe && cur.rank[b] == cur.rank[q];
+                if (!same) {
+                    double old[NPE][4];
+#pragma unroll
+                    for (int b = 1; b < NPE; b++)
+                        if (b < cur.npe)
+#pragma unroll
+                            for (int v = 0; v < 4; v++) old[b][v] = acc[cur.rank[b]][v][tid];
+#pragma unroll
+                    for (int b = 1; b < NPE; b++)
+                        if (b < cur.npe)
+#pragma unroll
+                            for (int v = 0; v < 4; v++) acc[cur.rank[b]][v][tid] = old[b][v] + kb[b][v];
+                } else {
+#pragma unroll
+                    for (int b = 1; b < NPE; b++)
+                        if (b < cur.npe)
+#pragma unroll
+                            for (int v = 0; v < 4; v++) acc[cur.rank[b]][v][tid] += kb[b][v];
+                }
+                cur = nxt;
+            }
+#pragma unroll
+            for (int v = 0; v < 4; v++) acc[diag][v][tid] += dg[v];
+        }
+        __syncwarp();
+        // the warp's nodes: 2 rows of 2 u entries each
+        if (wide) {  // two nodes at a time, 16 lanes each, two entries per lane and store
+            const int half = lane >> 4, hl = lane & 15;
+#pragma unroll 4
+            for (int j = 0; j < 32; j += 2) {
+                const int uj = __shfl_sync(kFull, fits ? u : 0, j + half), bj = __shfl_sync(kFull, base, j + half);
+                for (int x = hl; x < 2 * uj; x += 16) {
+                    const int i = x >= uj, q = x - (i ? uj : 0);
+                    const double* a = &acc[q][2 * i][warp0 + j + half];
+                    *reinterpret_cast<double2*>(values + (long long)bj + 2 * x) = make_double2(a[0], a[kRowPad]);
+                }
+            }
+        } else {
+            for (int j = 0; j < 32; j++) {
+                const int uj = __shfl_sync(kFull, fits ? u : 0, j), bj = __shfl_sync(kFull, base, j);
+                for (int x = lane; x < 4 * uj; x += 32) {
+                    const int i = x >= 2 * uj, c = x - i * 2 * uj;
+                    values[(long long)bj + x] = acc[c >> 1][2 * i + (c & 1)][warp0 + j];
+                }
+            }
+        }
+        // rows too long for the shared memory: the warp's lanes on the node's occurrences
+        for (unsigned longs = __ballot_sync(kFull, !fits); longs; longs &= longs - 1) {
+            const int src = __ffs(longs) - 1;
+            const long long nl = tile * kRowThreads + warp0 + src;
+            const int ul = __shfl_sync(kFull, u, src), bl = __shfl_sync(kFull, base, src);
+            const int ll = __shfl_sync(kFull, lo, src), dl = __shfl_sync(kFull, d, src);
+            for (int x = lane; x < 4 * ul; x += 32) values[(long long)bl + x] = 0.0;
+            __syncwarp();
+            for (int i = lane; i < dl; i += 32) {
+                OccData<NPE> el;
+                load_occ<KIND>(m, __ldg(occ + ll + i), ranks, ll + i, el);
+                load_geometry(m, el);
+                el.x[0] = __ldg(m.x + nl);
+                el.y[0] = __ldg(m.y + nl);
+                double kb[NPE][4];
+                if (!(occ_blocks<KIND, T>(el, m.t, kb) > 0.0)) atomicOr(status, 1 << FEM_ERR_DETJ);
+#pragma unroll
+                for (int b = 0; b < NPE; b++) {
+                    if (b >= el.npe) continue;
+                    double* p = values + bl + 2 * el.rank[b];
+                    atomicAdd(p, kb[b][0]);
+                    atomicAdd(p + 1, kb[b][1]);
+                    atomicAdd(p + 2 * ul, kb[b][2]);
+                    atomicAdd(p + 2 * ul + 1, kb[b][3]);
+                }
+            }
+            __syncwarp();
+        }
+        __syncwarp();
+    }
+}
+
+template <int KIND>
+cudaError_t build_rows_map(const MeshView& m, const int* row_ptr, const int* col_idx, const RowsMap& r, int* cnt,
+                           long long* tiles, DevInfo* info, cudaStream_t s) {
+    const cudaError_t err = cudaMemsetAsync(cnt, 0, (size_t)m.N * sizeof(int), s);
+    if (err) return err;
+    const int ntiles = row_tiles(m.N);
+    const int grid = (int)std::min<long long>(((long long)m.E_count + kThreads - 1) / kThreads, (long long)sm_count() * 8);
+    int* status = &info->status_bits;
+    k_map_count<KIND><<<grid, kThreads, 0, s>>>(m, cnt, status);
+    k_map_sums<<<ntiles, kScanThreads, 0, s>>>(cnt, m.N, tiles);
+    k_map_offsets<<<ntiles, kScanThreads, 0, s>>>(cnt, m.N, tiles, r.off, info);
+    k_map_fill<KIND><<<grid, kThreads, 0, s>>>(m, r.off, cnt, r.occ);
+    k_map_ranks<KIND><<<(int)std::min<long long>(3ll * grid, (long long)sm_count() * 16), kThreads, 0, s>>>(
+        m, r.off, r.occ, row_ptr, col_idx, r.ranks, status);
+    return cudaGetLastError();
+}
+
+template <int KIND, typename T>
+cudaError_t rows_values(const MeshView& m, const RowsMap& r, const int* row_ptr, double* values, int* status,
+                        cudaStream_t s) {
+    static DeviceCache cache;
+    int per_sm = 0;
+    const cudaError_t err = per_device(cache, [](int& v) {
+        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, k_rows_values_2d<KIND, T>, kRowThreads, 0);
+    }, per_sm);
+    if (err) return err;
+    const long long tiles = ((long long)m.N + kRowThreads - 1) / kRowThreads;
+    k_rows_values_2d<KIND, T><<<(int)std::min<long long>(tiles, (long long)per_sm * sm_count()), kRowThreads, 0, s>>>(
+        m, r.off, r.occ, r.ranks, row_ptr, values, reinterpret_cast<uintptr_t>(values) % 16 == 0, status);
+    return cudaGetLastError();
+}
+
+template <typename T>
+cudaError_t rows_values_kind(const MeshView& m, int kind, const RowsMap& r, const int* row_ptr, double* values,
+                             int* status, cudaStream_t s) {
+    if (kind == FEM_T3) return rows_values<FEM_T3, T>(m, r, row_ptr, values, status, s);
+    if (kind == FEM_Q4) return rows_values<FEM_Q4, T>(m, r, row_ptr, values, status, s);
+    return rows_values<FEM_MIXED_2D, T>(m, r, row_ptr, values, status, s);
+}
+
 }  // namespace
 
 cudaError_t launch_build_map(const MeshView& m, int kind, const int* row_ptr, const int* col_idx, int* map,
@@ -147,6 +479,19 @@ cudaError_t launch_reassemble_2d(const MeshView& m, int precision, const int* ma
     else
         reassemble_2d_t<double>(m, map, G, perm, ranges, row_ptr, values, status, s);
     return cudaGetLastError();
+}
+
+cudaError_t launch_build_rows_map(const MeshView& m, int kind, const int* row_ptr, const int* col_idx, const RowsMap& r,
+                                  int* cnt, long long* tiles, DevInfo* info, cudaStream_t s) {
+    if (kind == FEM_T3) return build_rows_map<FEM_T3>(m, row_ptr, col_idx, r, cnt, tiles, info, s);
+    if (kind == FEM_Q4) return build_rows_map<FEM_Q4>(m, row_ptr, col_idx, r, cnt, tiles, info, s);
+    return build_rows_map<FEM_MIXED_2D>(m, row_ptr, col_idx, r, cnt, tiles, info, s);
+}
+
+cudaError_t launch_rows_values_2d(const MeshView& m, int kind, int precision, const RowsMap& r, const int* row_ptr,
+                                  double* values, int* status, cudaStream_t s) {
+    return precision == FEM_PREC_FP32 ? rows_values_kind<float>(m, kind, r, row_ptr, values, status, s)
+                                      : rows_values_kind<double>(m, kind, r, row_ptr, values, status, s);
 }
 
 }  // namespace fem

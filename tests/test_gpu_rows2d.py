@@ -104,3 +104,34 @@ def test_batch_of_many_slots_and_unaligned_outputs(fem, oracle_mod, cuda_device)
     assert all(s == 0 for s in b.statuses())
     for i, m in enumerate(meshes):
         _compare(oracle_mod, m, *b.result(i))
+
+
+@pytest.mark.parametrize("name", ["fan5", "fan13", "fan14", "fan40", "wedge", "q4_7x9", "mixed_33x2", "loose"])
+def test_reassembly_rows(fem, oracle_mod, cuda_device, name):
+    # rows at the limit of the shared-memory sums (14 columns) and past it,
+    # repeated nodes, and mostly unconnected triangles (the block-position map)
+    import torch
+    import meshgen as mg
+    if name.startswith("fan"):
+        m = _fan(int(name[3:]), True)
+    elif name == "wedge":
+        m = mg.q4_grid(9, 7, seed=3)
+        conn = m.conn.copy()
+        conn[::3, 1] = conn[::3, 2]
+        m.conn = conn
+    elif name == "loose":
+        g = mg.t3_grid(40, 40, seed=2)
+        m = mg.Mesh(mg.T3, g.x[g.conn].ravel(), g.y[g.conn].ravel(), None,
+                    np.arange(3 * g.num_elems, dtype=np.int32).reshape(-1, 3), None, None, None)
+    else:
+        m = {"q4_7x9": lambda: mg.q4_grid(7, 9, seed=1), "mixed_33x2": lambda: mg.mixed_grid(33, 2, seed=1)}[name]()
+    asm = fem.Assembler(m)
+    rp, ci, v, info = asm.assemble()
+    re = fem.Reassembler(asm)
+    re.build(int(info.nnz))
+    vals = torch.full((int(info.nnz) + 1,), 7.0, dtype=torch.float64, device="cuda")
+    for _ in range(2):
+        re.reassemble(vals)
+        assert re.read_info() == 0
+        _compare(oracle_mod, m, rp.cpu().numpy(), ci.cpu().numpy(), vals[:-1].cpu().numpy())
+        assert vals[-1].item() == 7.0
