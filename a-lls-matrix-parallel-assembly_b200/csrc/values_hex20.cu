@@ -23,6 +23,19 @@
 // derivatives at the 27 Gauss points (H20:95-128) are tabulated once per CTA
 // and the next element's node ids and coordinates are loaded while the
 // current one is computed.
+//
+// What bounds the re-assembly is the L2's FP64 atomics: 3,600 additions per
+// element, 230 M for 40x40x40 elements, 1.28 ms of the 1.43 ms call (the
+// clear of the values is the rest). The elements are drawn one by one from a
+// counter (two ahead, so the draw is never waited for). At a fixed stride over the grid the
+// CTAs drift apart in the visit order, so additions to the same rows no longer meet in
+// L2 and the lines go to memory and back; drawn, the elements in flight stay
+// together. Call, 40x40x40: fixed stride 1733 us, drawn with 1 / 2 / 3 / 4 CTAs per
+// SM 2544 / 1645 / 1467 / 1430 us (20x20x20: 203 us with 3, 196 with 4).
+// One warp per element with its blocks staged in shared memory
+// (ke_hex20.cuh's pass with additions in place of the packed store) has no
+// barriers, but only 8 elements per SM in flight behind their additions: 1969 us.
+// The colouring keeps the fixed stride and 3 CTAs: its elements share no rows.
 #include <algorithm>
 
 #include "values_hex20.cuh"
@@ -30,15 +43,15 @@
 namespace fem {
 namespace {
 
-#ifndef FEM_VALUES_MIN_CTAS
-#define FEM_VALUES_MIN_CTAS 3
+#ifndef FEM_MAP_CTAS
+#define FEM_MAP_CTAS 4
 #endif
 constexpr int kThreads = kValueWarps * 32;
 
 // kOut as values_cta (kToCsrMap: all elements in the order perm, scatter map
 // row e; kToCsrColour: the elements perm[range[0], range[1]) of one colour).
 template <int kOut>
-__global__ void __launch_bounds__(kThreads, FEM_VALUES_MIN_CTAS)
+__global__ void __launch_bounds__(kThreads, kOut == kToCsrMap ? FEM_MAP_CTAS : 3)
     k_values_hex20(MeshView m, const int* __restrict__ perm, int i0, int i1, const int* __restrict__ range,
                    ValuesTarget t) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -82,6 +95,7 @@ cudaError_t launch_reassemble_hex20(const MeshView& m, int precision, const int*
     t.row_ptr = mt.row_ptr;
     t.csr = mt.values;
     t.info = info;
+    t.ticket = &info->ticket;
     return launch_values<kToCsrMap>(m, perm, 0, m.E_count, nullptr, t, 0, s);
 }
 

@@ -76,3 +76,39 @@ def test_fp32_reassembly(fem, oracle_mod, cuda_device, name):
     rel, scaled = value_errors(orp, oci, ov, vals.cpu().numpy())
     print(f"{name}: FP32 re-assembly max scaled error {scaled:.2e}")
     assert scaled <= 1e-5, scaled
+
+
+@pytest.mark.parametrize("count", [1, 591, 592, 593, 800])
+def test_hex20_drawn_elements(fem, oracle_mod, cuda_device, count):
+    # around the launch's first elements (4 CTAs on each of 148 SMs), past which they are drawn from a counter;
+    # a second call draws again, and elements that went bad (the first, one of the middle, the last) add nothing
+    import copy
+    import torch
+    import meshgen as mg
+    m = mg.hex20_grid(10, 10, 8, seed=9)
+    m.conn = m.conn[:count].copy()
+    r = np.random.default_rng(9)
+    m.E, m.nu = r.lognormal(0, 0.5, count), r.uniform(0.1, 0.45, count)
+    asm = fem.Assembler(m)
+    rp, ci, v, info = asm.assemble()
+    re = fem.Reassembler(asm)
+    re.build(int(info.nnz))
+    vals = torch.full((int(info.nnz) + 1,), 7.0, dtype=torch.float64, device="cuda")
+    orp, oci, ov = oracle_mod.assemble(m)
+    for _ in range(2):
+        re.reassemble(vals[:-1])
+        assert re.read_info() == 0
+        assert value_errors(orp, oci, ov, vals[:-1].cpu().numpy())[1] <= RTOL
+        assert vals[-1].item() == 7.0
+    bad = sorted({0, count // 2, count - 1})
+    for k, e in enumerate(bad):
+        asm.dev["conn"][e, 5 * k] = m.num_nodes if k % 2 else -1
+    re.reassemble(vals[:-1])
+    assert re.read_info() == 2  # FEM_ERR_BAD_MESH
+    m2 = copy.copy(m)
+    m2.E = m.E.copy()
+    m2.E[bad] = 0.0
+    orp, oci, ov2 = oracle_mod.assemble(m2)
+    got = vals[:-1].cpu().numpy()
+    scale = value_errors(orp, oci, ov, ov + (got - ov2))[1]  # on the scale of the whole matrix
+    assert scale <= RTOL
