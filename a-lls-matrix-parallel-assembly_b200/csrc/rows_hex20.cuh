@@ -9,19 +9,30 @@
 // races, and the row comes out sorted:
 //   k_rows_hex20       one warp per node with at most 8 elements (every inner
 //                      node of a regular mesh): its elements' up to 160 node
-//                      ids are loaded, five per lane, and inserted into a
-//                      256-entry hash table in shared memory; the distinct
-//                      ones are compacted and sorted (bitonic, in registers:
-//                      64, 128 or 256 keys), written to the list chunks, and
-//                      their ranks go back through the table to the rank map.
+//                      ids are loaded, up to five per lane, and inserted into
+//                      a hash table in shared memory (128 entries for up to 4
+//                      elements, the nodes inside an edge, 256 for 5 to 8);
+//                      the distinct ones are compacted and sorted (bitonic, in
+//                      registers: 64, 128 or 256 keys), written to the list
+//                      chunks, and their ranks go back through the table to
+//                      the rank map.
 //   k_wide_rows_hex20  nodes with up to 32 elements, one warp each: repeated
 //                      minimum over the candidates, which stay in registers.
 //   k_long_rows_hex20  longer rows, one CTA each: the same over memory.
 // A row past its first chunk takes consecutive overflow chunks from the pool.
 //
-// What bounds it: instruction issue (hash, sort, rank look-ups) and the latency
-// of occurrence -> connectivity. B200, 64^3 (1.09 M nodes): 1.18 ms, where the
-// CAS claims of element groups took 4.36 ms; 9^3: 8 against 141 us.
+// What bounds it: instruction issue (660 warp instructions a node in hash, sort
+// and rank look-ups; ALU 58 %, 2.5 instructions per cycle) and waits for
+// instructions and shared memory; DRAM is at 2 %. B200, 64^3 (1.09 M nodes):
+// 1.02 ms, where five single-word loads per lane and a 256-entry table for
+// every node took 1.13 ms, and the CAS claims of element groups 4.36 ms.
+// CTAs per SM: 4 / 5 / 6 1.03 / 1.02 / 1.01 ms at 64^3, 9^3 call 70.7 / 70.9 /
+// 73.6 us, batch of 16 meshes 1.73 / 1.69 / 1.73 ms. Listing new nodes as they
+// are inserted, with the table entry packed into the sort key (no table scan,
+// no second look-up), is 1.34 ms: the ballots after each insertion make the
+// warps wait out each other's probes and the code no longer fits the
+// instruction cache; so does a copy of the sorts for each of the two forms
+// (batch 1.73 ms).
 #pragma once
 
 #include "hex_rows.cuh"
@@ -154,12 +165,11 @@ __device__ __forceinline__ void occ_fill(const MeshView& m, const HexRows& h, in
 
 // Resident CTAs per SM that the registers are set for.
 #ifndef FEM_HEXR_CTAS
-#define FEM_HEXR_CTAS 4
+#define FEM_HEXR_CTAS 5
 #endif
 constexpr int kHexRowWarps = 8;
 constexpr int kHexRowThreads = kHexRowWarps * 32;
 constexpr int kMaxElems = 8;               // elements of a node in the main pass
-constexpr int kCand = kMaxElems * 20 / 32; // candidates per lane
 constexpr int kTable = 256;
 constexpr int kWideElems = 32;
 constexpr int kWideCand = kWideElems * 20 / 32;
@@ -195,8 +205,6 @@ __device__ __forceinline__ void finish_row(const ListLayout& L, int n, int u, in
     *reinterpret_cast<int2*>(L.meta1 + (size_t)n * L.H1) = make_int2(0, next);
     L.counts[n] = u;
 }
-
-__device__ __forceinline__ int table_slot(int node) { return (int)(((unsigned)node * 2654435761u) >> 24); }
 
 // Sorts the u keys of uniq (KPL per lane, padded) by a bitonic network.
 template <int KPL>
@@ -237,79 +245,115 @@ __device__ __forceinline__ void sort_keys(int* uniq, int u, int lane) {
     __syncwarp();
 }
 
+// The row of node n with d <= 8 elements; o: lane t < d holds its occurrence t.
+// Four lanes take an element's node ids (up to 4 elements: eight lanes): 16 in
+// one load of four (two) words each, and the last four. conn16: conn is 16-byte
+// aligned. The sorts are shared by both forms: at twice the code the warps wait for instructions.
+__device__ __forceinline__ void row_hex20(const int* __restrict__ conn, bool conn16, const ListLayout& L,
+                                          unsigned short* __restrict__ map, int n, int d, int o, HexRowSmem& sm) {
+    const bool many = d > 4;
+    const int lane = threadIdx.x & 31, t = many ? lane >> 2 : lane >> 3, sub = many ? lane & 3 : lane & 7;
+    const int tab = many ? kTable : kTable / 2, shift = many ? 24 : 25;  // at most 20/32 of the table fills
+    auto start = [&](int node) { return (int)(((unsigned)node * 2654435761u) >> shift); };
+    const bool has = t < d, last = has && sub < 4;
+    const int ot = __shfl_sync(0xFFFFFFFFu, o, t);
+    const int* src = conn + (size_t)(ot / 20) * 20;
+    int node[5] = {-1, -1, -1, -1, -1}, slot[5];
+    if (last) node[4] = __ldg(src + 16 + sub);
+    if (has && many) {
+        if (conn16) {
+            const int4 v = __ldg(reinterpret_cast<const int4*>(src) + sub);
+            node[0] = v.x, node[1] = v.y, node[2] = v.z, node[3] = v.w;
+        } else {
+#pragma unroll
+            for (int i = 0; i < 4; i++) node[i] = __ldg(src + 4 * sub + i);
+        }
+    } else if (has) {
+        if (conn16) {
+            const int2 v = __ldg(reinterpret_cast<const int2*>(src) + sub);
+            node[0] = v.x, node[1] = v.y;
+        } else {
+            node[0] = __ldg(src + 2 * sub), node[1] = __ldg(src + 2 * sub + 1);
+        }
+    }
+    reinterpret_cast<int4*>(sm.table)[lane] = make_int4(-1, -1, -1, -1);
+    if (many) reinterpret_cast<int4*>(sm.table)[lane + 32] = make_int4(-1, -1, -1, -1);
+    __syncwarp();
+    auto insert = [&](int i) {
+        int at = start(node[i]);
+        if (node[i] >= 0) {
+            for (int k = 0; k < kTable; k++) {
+                const int old = atomicCAS(&sm.table[at], -1, node[i]);
+                if (old == -1 || old == node[i]) break;
+                at = (at + 1) & (tab - 1);
+            }
+        }
+        slot[i] = at;
+    };
+    insert(4), insert(0), insert(1);
+    if (many) insert(2), insert(3);
+    __syncwarp();
+    int u = 0;
+#pragma unroll 4
+    for (int q = 0; q < tab; q += 32) {
+        const int k = sm.table[lane + q];
+        const unsigned used = __ballot_sync(0xFFFFFFFFu, k >= 0);
+        if (k >= 0) sm.uniq[u + __popc(used & ((1u << lane) - 1u))] = k;
+        u += __popc(used);
+    }
+    __syncwarp();
+    if (u <= 64) sort_keys<2>(sm.uniq, u, lane);
+    else if (u <= 128) sort_keys<4>(sm.uniq, u, lane);
+    else sort_keys<8>(sm.uniq, u, lane);
+    int kept = u, next = 0;
+    if (u > L.S1) {
+        if (lane == 0) next = take_chunks(L, kept);
+        next = __shfl_sync(0xFFFFFFFFu, next, 0);
+        kept = __shfl_sync(0xFFFFFFFFu, kept, 0);
+    }
+    for (int p = lane; p < u; p += 32) {
+        const int k = sm.uniq[p];
+        int at = start(k);
+        while (sm.table[at] != k) at = (at + 1) & (tab - 1);
+        sm.rank[at] = (unsigned short)p;
+        if (p < kept) *hex_col_word(L, n, next, p) = k + 1;
+    }
+    if (lane == 0) finish_row(L, n, kept, next);
+    __syncwarp();
+    unsigned short* dst = map + (size_t)ot * 20;
+    if (has && many)
+        reinterpret_cast<ushort4*>(dst)[sub] =
+            make_ushort4(sm.rank[slot[0]], sm.rank[slot[1]], sm.rank[slot[2]], sm.rank[slot[3]]);
+    else if (has)
+        reinterpret_cast<ushort2*>(dst)[sub] = make_ushort2(sm.rank[slot[0]], sm.rank[slot[1]]);
+    if (last) dst[16 + sub] = sm.rank[slot[4]];
+    __syncwarp();
+}
+
 // The bodies below run as block `block` of `nblocks` of their launch.
 __device__ __forceinline__ void rows_hex20(const int* __restrict__ conn, const ListLayout& L, const HexRows& h,
                                            int* __restrict__ queue, int block, int nblocks,
                                            HexRowSmem (&s_row)[kHexRowWarps]) {
-    const int* __restrict__ off = h.off;
-    const int* __restrict__ inc = h.inc;
-    unsigned short* __restrict__ map = h.map;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const bool conn16 = (reinterpret_cast<uintptr_t>(conn) & 15) == 0;
     HexRowSmem& sm = s_row[warp];
-    for (long long nn = (long long)block * kHexRowWarps + warp; nn < L.N; nn += (long long)nblocks * kHexRowWarps) {
-        const int n = (int)nn, lo = __ldcg(off + n), d = __ldcg(off + n + 1) - lo;
+    const long long step = (long long)nblocks * kHexRowWarps;
+    // the next node's occurrences are loaded while the current row is built
+    auto bounds = [&](long long nn) { return nn < L.N ? make_int2(__ldcg(h.off + nn), __ldcg(h.off + nn + 1)) : make_int2(0, 0); };
+    auto occ = [&](int2 r) { return lane < min(r.y - r.x, kMaxElems) ? (int)occ_of(__ldcg(h.inc + r.x + lane)) : 0; };
+    long long nn = (long long)block * kHexRowWarps + warp;
+    int2 r = bounds(nn), r1 = bounds(nn + step);
+    int o = occ(r);
+    for (; nn < L.N; nn += step) {
+        const int n = (int)nn, d = r.y - r.x, o1 = occ(r1);
+        r = r1;
+        r1 = bounds(nn + 2 * step);
         if (d > kMaxElems) {
             if (lane == 0) queue[atomicAdd(&L.info->long_rows, 1)] = n;
-            continue;
+        } else {
+            row_hex20(conn, conn16, L, h.map, n, d, o, sm);
         }
-        const int o = lane < d ? (int)occ_of(__ldcg(inc + lo + lane)) : 0;
-        int node[kCand], slot[kCand];
-#pragma unroll
-        for (int q = 0; q < kCand; q++) {
-            const int j = lane + 32 * q, t = j / 20, b = j - 20 * t;
-            const int e = __shfl_sync(0xFFFFFFFFu, o, t & 31) / 20;
-            node[q] = j < 20 * d ? __ldg(conn + (size_t)e * 20 + b) : -1;
-        }
-        reinterpret_cast<int4*>(sm.table)[lane] = make_int4(-1, -1, -1, -1);
-        reinterpret_cast<int4*>(sm.table)[lane + 32] = make_int4(-1, -1, -1, -1);
-        __syncwarp();
-#pragma unroll
-        for (int q = 0; q < kCand; q++) {
-            int h = table_slot(node[q]);
-            if (node[q] >= 0) {
-                for (int i = 0; i < kTable; i++) {  // at most 160 of the 256 entries fill
-                    const int old = atomicCAS(&sm.table[h], -1, node[q]);
-                    if (old == -1 || old == node[q]) break;
-                    h = (h + 1) & (kTable - 1);
-                }
-            }
-            slot[q] = h;
-        }
-        __syncwarp();
-        int u = 0;
-#pragma unroll
-        for (int q = 0; q < kTable / 32; q++) {
-            const int k = sm.table[lane + 32 * q];
-            const unsigned used = __ballot_sync(0xFFFFFFFFu, k >= 0);
-            if (k >= 0) sm.uniq[u + __popc(used & ((1u << lane) - 1u))] = k;
-            u += __popc(used);
-        }
-        __syncwarp();
-        if (u <= 64) sort_keys<2>(sm.uniq, u, lane);
-        else if (u <= 128) sort_keys<4>(sm.uniq, u, lane);
-        else sort_keys<8>(sm.uniq, u, lane);
-        int kept = u, next = 0;
-        if (u > L.S1) {
-            if (lane == 0) next = take_chunks(L, kept);
-            next = __shfl_sync(0xFFFFFFFFu, next, 0);
-            kept = __shfl_sync(0xFFFFFFFFu, kept, 0);
-        }
-        for (int p = lane; p < u; p += 32) {
-            const int k = sm.uniq[p];
-            int h = table_slot(k);
-            while (sm.table[h] != k) h = (h + 1) & (kTable - 1);
-            sm.rank[h] = (unsigned short)p;
-            if (p < kept) *hex_col_word(L, n, next, p) = k + 1;
-        }
-        if (lane == 0) finish_row(L, n, kept, next);
-        __syncwarp();
-#pragma unroll
-        for (int q = 0; q < kCand; q++) {
-            const int j = lane + 32 * q, t = j / 20, b = j - 20 * t;
-            const int ot = __shfl_sync(0xFFFFFFFFu, o, t & 31);
-            if (node[q] >= 0) map[(size_t)ot * 20 + b] = sm.rank[slot[q]];
-        }
-        __syncwarp();
+        o = o1;
     }
 }
 

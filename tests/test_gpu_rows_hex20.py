@@ -128,3 +128,25 @@ def test_bad_element_leaves_the_others(fem, oracle_mod, cuda_device):
     np.testing.assert_array_equal(asm.col_idx[:n].cpu().numpy(), oci)
     scale = np.maximum(np.abs(ov), diag_scale(orp, oci, ov))
     assert np.all(np.abs(asm.values[:n].cpu().numpy() - ov) <= RTOL * scale)
+
+
+@pytest.mark.parametrize("name", ["grid", "star4", "star5", "star8", "wedges"])
+@pytest.mark.parametrize("offset", [0, 1, 2])
+def test_connectivity_alignment(fem, oracle_mod, cuda_device, name, offset):
+    # node ids are read four or two at a time when conn is 16-byte aligned; nodes of up to 4 elements take eight
+    # lanes an element and half the table, nodes of 5 to 8 four lanes and the whole one
+    import torch
+    import meshgen as mg
+    m = mg.hex20_grid(4, 3, 3, seed=6) if name == "grid" else _wedges() if name == "wedges" else _star(int(name[4:]))
+    asm = fem.Assembler(m)
+    buf = torch.empty(m.conn.size + 4, dtype=torch.int32, device="cuda")
+    conn = buf[offset:offset + m.conn.size]
+    conn.copy_(torch.from_numpy(m.conn.ravel()))
+    asm.cm.conn = conn.data_ptr()
+    rp, ci, v, info = asm.assemble()
+    orp, oci, ov = oracle_mod.assemble(m)
+    rp, ci, v = rp.cpu().numpy(), ci.cpu().numpy()[:len(oci)], v.cpu().numpy()[:len(oci)]
+    np.testing.assert_array_equal(rp, orp)
+    np.testing.assert_array_equal(ci, oci)
+    sc = diag_scale(orp, oci, ov)
+    assert np.all(np.abs(v - ov) <= RTOL * np.maximum(np.abs(ov), sc))
