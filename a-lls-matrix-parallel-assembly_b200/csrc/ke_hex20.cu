@@ -24,8 +24,7 @@ cudaError_t launch_hex20_ke_dmma(const MeshView& m, double* ke_out, int* status,
         return e;
     }, per_sm);
     if (err) return err;
-    const long long want = ((long long)m.E_count + kKeWarps - 1) / kKeWarps;
-    const int grid = (int)std::min<long long>(want, (long long)per_sm * sm_count());
+    const int grid = (int)std::min<long long>(m.E_count, (long long)per_sm * sm_count());
     const int bulk = (reinterpret_cast<uintptr_t>(ke_out) & 15u) == 0;
     k_ke_hex20<<<grid, kKeThreads, smem, s>>>(m, ke_out, status, bulk);
     return cudaGetLastError();

@@ -32,8 +32,12 @@
 // gradients and blocks per element and quarter: 1.3 ms for 64^3), then the
 // output (0.61 ms at the measured copy rate). B200, 64^3: 1.67 ms, where one
 // 4-warp CTA per element with its fragments and products in shared memory took
-// 3.65 ms; 39x41x40: 440 against 897 us. 10 warps 2.01 ms, two CTAs of 4 warps
-// 1.73 ms.
+// 3.65 ms; 39x41x40: 437 against 910 us. 10 warps 2.01 ms, two CTAs of 4 warps
+// 1.73 ms. Warps of one CTA take elements a grid apart, so that few elements
+// spread over all SMs, and the first element's loads are in flight while the
+// derivative table is built: 8 elements 7.9 us (8.7 us by CTAs of 4 warps; 13.0
+// us with a CTA's warps on consecutive elements), 512 9.3 (14.3; 13.4), 1,728
+// 18.0 (33.4; 22.5).
 #pragma once
 
 #include "hex20.cuh"
@@ -84,19 +88,8 @@ __device__ __forceinline__ void ke_hex20(const MeshView& m, double* __restrict__
                                          bool bulk, int block, int nblocks, KeHexSmem& sm) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, fr = lane >> 2, fc = lane & 3;
     KeWarpSmem& ws = sm.w[warp];
-    for (int idx = tid; idx < 27 * 20; idx += kKeThreads) {
-        const int g = idx / 20, n = idx - 20 * g;
-        double dx, dy, dz;
-        hex20::dshape_node(n, hex20::gauss3(g / 9), hex20::gauss3((g / 3) % 3), hex20::gauss3(g % 3), dx, dy, dz);
-        sm.dN[0][n][g] = dx;
-        sm.dN[1][n][g] = dy;
-        sm.dN[2][n][g] = dz;
-    }
-    for (int idx = tid; idx < 3 * 20; idx += kKeThreads) sm.dN[idx / 20][idx % 20][27] = 0.0;
-    for (int k = lane; k < 10; k += 32) ws.iJw[27][k] = 0.0;
-    __syncthreads();
     const long long stride = (long long)nblocks * kKeWarps;
-    long long e = (long long)block * kKeWarps + warp;
+    long long e = (long long)warp * nblocks + block;  // few elements: spread over the SMs
     // the next element's nodes, then its coordinates and material, are loaded ahead
     auto load_node = [&](long long el) { return el < m.E_count && lane < 20 ? __ldg(m.conn + el * 20 + lane) : 0; };
     double px = 0.0, py = 0.0, pz = 0.0;
@@ -118,6 +111,17 @@ __device__ __forceinline__ void ke_hex20(const MeshView& m, double* __restrict__
     };
     load_coords(e, load_node(e));
     int pnode = load_node(e + stride);
+    for (int idx = tid; idx < 27 * 20; idx += kKeThreads) {
+        const int g = idx / 20, n = idx - 20 * g;
+        double dx, dy, dz;
+        hex20::dshape_node(n, hex20::gauss3(g / 9), hex20::gauss3((g / 3) % 3), hex20::gauss3(g % 3), dx, dy, dz);
+        sm.dN[0][n][g] = dx;
+        sm.dN[1][n][g] = dy;
+        sm.dN[2][n][g] = dz;
+    }
+    for (int idx = tid; idx < 3 * 20; idx += kKeThreads) sm.dN[idx / 20][idx % 20][27] = 0.0;
+    for (int k = lane; k < 10; k += 32) ws.iJw[27][k] = 0.0;
+    __syncthreads();
     for (; e < m.E_count; e += stride) {
         const bool bad = __any_sync(kKeFull, pbad);
         if (lane < 20) {
