@@ -718,10 +718,17 @@ namespace {
 struct MapHostLayout {
     int G;  // map entries per element
     size_t off_info, off_pos, off_perm, off_ranges, off_hist, off_bbox, total;
-    // 2-D meshes whose occurrences fit in the same bytes (all but mostly unconnected triangles): by row nodes instead
+    // 2-D meshes of at least min_row_nodes nodes, whose occurrences fit in the same bytes (all but mostly unconnected
+    // triangles): by row nodes instead
     bool rows;
     size_t off_off, off_occ, off_ranks;
 };
+
+// Nodes from which a 2-D map is by row nodes. A row node's thread goes through its 4 (Q4) to 6 (T3) elements one after
+// another, 10 to 20 us however few there are, so small meshes add element blocks. Call by blocks / by rows, us:
+// Q4 60^2 14.9 / 15.5, 100^2 16.0 / 15.7, 200^2 30.9 / 18.7; T3 60^2 14.6 / 20.4, 150^2 21.5 / 21.8, 200^2 25.7 / 23.8;
+// mixed 100^2 18.7 / 25.7, 150^2 25.6 / 29.4, 200^2 32.6 / 31.3.
+size_t min_row_nodes(int kind) { return kind == FEM_Q4 ? 8192 : 32768; }
 
 MapHostLayout map_layout(const fem_mesh* m) {
     MapHostLayout h{};
@@ -752,7 +759,7 @@ MapHostLayout map_layout(const fem_mesh* m) {
         // the ranks, or, while the map is built, the counters and scan partials in their place
         const size_t end = h.off_ranks + std::max(align_up(E * npe * npe * sizeof(unsigned short)),
                                                   align_up(N * sizeof(int)) + row_tiles(m->num_nodes) * sizeof(long long));
-        h.rows = end <= h.total && E < ((size_t)1 << 29) && E > 0;
+        h.rows = N >= min_row_nodes(m->kind) && end <= h.total && E < ((size_t)1 << 29) && E > 0;
     }
     return h;
 }

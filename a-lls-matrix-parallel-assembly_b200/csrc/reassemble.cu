@@ -18,8 +18,9 @@
 // instructions of the element rows. B200, T3 1001x699 (shuffled elements): 177
 // us, where the block-position form took 301 us plus 28 us of zeroing.
 //
-// Block positions (Hex20, and 2-D meshes whose occurrences do not fit, mostly
-// unconnected triangles): the map records, for every element node block (a, b),
+// Block positions (Hex20, small 2-D meshes, whose time is the serial walk over a
+// node's elements above (min_row_nodes in fem_api.cu), and 2-D meshes whose
+// occurrences do not fit, mostly unconnected triangles): the map records, for every element node block (a, b),
 // the CSR position of its first entry, position of block (a, b) of element e at
 // e * G + a * npe + b, G = npe^2; the element blocks are added there with FP64
 // atomics, in the element order of reorder.cu, which the map holds too. Entry

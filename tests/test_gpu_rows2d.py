@@ -135,3 +135,39 @@ def test_reassembly_rows(fem, oracle_mod, cuda_device, name):
         assert re.read_info() == 0
         _compare(oracle_mod, m, rp.cpu().numpy(), ci.cpu().numpy(), vals[:-1].cpu().numpy())
         assert vals[-1].item() == 7.0
+
+
+@pytest.mark.parametrize("name", ["fan5", "fan13", "fan14", "fan40", "wedge", "mixed", "q4_89", "q4_90", "t3_180", "t3_181"])
+def test_reassembly_rows_larger(fem, oracle_mod, cuda_device, name):
+    # the map by row nodes starts at 8,192 nodes (Q4) and 32,768 (T3, mixed): grids on both sides of the line, and odd
+    # pieces beside a grid past it
+    import torch
+    import meshgen as mg
+
+    def beside(m, g):
+        g.conn = np.ascontiguousarray(np.concatenate([g.conn, m.conn + g.num_nodes]).astype(np.int32))
+        return mg.Mesh(m.kind, np.concatenate([g.x, m.x + 10.0]), np.concatenate([g.y, m.y]), None, g.conn, None, None,
+                       None, E0=1.0, nu0=0.3)
+
+    if name.startswith("fan"):
+        m = beside(_fan(int(name[3:]), True), mg.t3_grid(185, 185, seed=2))
+    elif name == "wedge":
+        w = mg.q4_grid(9, 7, seed=3)
+        w.conn = w.conn.copy()
+        w.conn[::3, 1] = w.conn[::3, 2]
+        m = beside(w, mg.q4_grid(95, 95, seed=2))
+    elif name == "mixed":
+        m = mg.mixed_grid(200, 180, seed=1)
+    else:
+        k, n = name.split("_")
+        m = (mg.q4_grid if k == "q4" else mg.t3_grid)(int(n), int(n), seed=4)
+    asm = fem.Assembler(m)
+    rp, ci, v, info = asm.assemble()
+    re = fem.Reassembler(asm)
+    re.build(int(info.nnz))
+    vals = torch.full((int(info.nnz) + 1,), 7.0, dtype=torch.float64, device="cuda")
+    for _ in range(2):
+        re.reassemble(vals)
+        assert re.read_info() == 0
+        _compare(oracle_mod, m, rp.cpu().numpy(), ci.cpu().numpy(), vals[:-1].cpu().numpy())
+        assert vals[-1].item() == 7.0
