@@ -24,7 +24,7 @@ struct ValuesTarget {
     const int* col_idx;
     double* csr;
     DevInfo* info;        // status bits
-    int* ticket;          // positions drawn past the first gridDim.x, 0 at the launch (NULL: fixed stride)
+    int* ticket;          // kToCsrMap: positions drawn past the first gridDim.x, 0 at the launch
 };
 
 // The six 8x8 tile positions (ti <= tj) of the upper triangle of the 24 x 24 node grid.
@@ -91,8 +91,8 @@ __device__ __forceinline__ void values_cta(const MeshView& m, const int* __restr
     }
     __syncthreads();
 
-    // the elements come at a fixed stride, or (t.ticket) are drawn from a counter, two ahead
-    const bool drawn = t.ticket != nullptr;
+    // the elements come at a fixed stride, or (kToCsrMap) are drawn from a counter, two ahead
+    const bool drawn = kOut == kToCsrMap;
     if (drawn) {
         if (tid == 0) sm.next = (int)i_stride + atomicAdd(t.ticket, 1);
         __syncthreads();
