@@ -56,10 +56,11 @@ WORKLOADS = {
 DEFAULT_WORKLOAD = "hex20"
 L2_BYTES = 126 * 2 ** 20
 L2_NOTE = ("a buffer of 2x L2 (252 MB) is zeroed between timed steps, outside the step events; the Hex20 64^3 "
-           "step also moves 24.6 GB of algorithmic traffic, far above L2")
+           "step also moves 15.6 GB of algorithmic traffic, far above L2")
 METRIC = "elements/s (device FP64 A-LLS assembly: element stiffness, list scatter, CSR pattern + values)"
-SCATTER_KERNEL = {"q4": "k_scatter_2d<4>", "t3": "k_scatter_2d<3>", "mixed": "k_scatter_2d<4> + k_scatter_2d<3>",
-                  "hex20": "k_claim_hex20 + k_values_group (two-pass list scatter by element groups, in waves)"}
+SCATTER_KERNEL = {"q4": "k_small_2d", "t3": "k_fill_2d + k_rows_2d", "mixed": "k_fill_2d + k_rows_2d",
+                  "hex20": "k_occ_* + k_rows_hex20 (row lists) + k_ke_hex20 (packed element matrices)"}
+ROUND_LARGE, ORDERED_ELEMS, SMALL_NODES = 64, 3072, 16384  # as in the library (batched.cu, fem_api.cu, launch.h)
 
 
 def make_mesh(workload: str, size: int = 0, **kw):
@@ -87,13 +88,15 @@ def workload_config(workload: str, mesh, nnz: int, world: int, sized: bool = Fal
 
 
 def algorithmic_bytes(mesh, nnz: int) -> dict:
-    """Algorithmic bytes of one assembly: inputs, CSR output and the A-LLS list
-    entries written once and read once (16 B each way per nnz)."""
+    """Algorithmic bytes of one assembly: inputs, CSR output, and what the scatter
+    hands to the consolidation, written once and read once: 2-D, each node
+    pair's column and 2x2 block (36 B, 9 per nnz); Hex20, the packed element
+    matrices (15,120 B), the rank map (800 B per element) and each node pair's column (4 B)."""
     dim = 3 if mesh.z is not None else 2
     conn = int(np.sum(mesh.nodes_per_elem())) * 4
     b_in = mesh.num_nodes * dim * 8 + conn + mesh.num_elems * 16 + (mesh.num_elems if mesh.types is not None else 0)
     b_out = 4 * (mesh.num_dofs + 1) + 12 * nnz
-    b_list = 32 * nnz
+    b_list = 2 * (mesh.num_elems * 15920 + 4 * nnz // 9 if mesh.z is not None else 9 * nnz)
     return {"in": b_in, "out": b_out, "list": b_list, "total": b_in + b_out + b_list}
 
 
@@ -299,8 +302,8 @@ def run_batched(args, rank: int, world: int, local_rank: int, compact: bool = Fa
     """The batched configuration: 256 meshes assembled by fem_assemble_batched
     (one call per step, graph-captured), concurrency picked by the library's
     autotuner (fem_autotune_batched: 1/2/4/8/16 slots timed on this batch);
-    concurrency 1 is the sequential baseline (the same per-mesh launches one
-    after another on one stream). value = elements/s of the whole batch.
+    concurrency 1 is the sequential baseline (one mesh's launches after
+    another's on one stream). value = elements/s of the whole batch.
     compact: return the fields as a dict (the default line's batched field)."""
     import torch
     import fem_alls as fem
@@ -384,7 +387,7 @@ def run_batched(args, rank: int, world: int, local_rank: int, compact: bool = Fa
         "speedup_vs_sequential": seq["ms"] / ms,
         "meshes": len(meshes), "elements": elems, "nnz": int(sum(nnz)),
         "kinds": {k: sum(1 for m in meshes if m.kind == k) for k in range(4)}, "mesh_generation_s": gen_s,
-        "clocks": clk.summary(), "gpu_launches": args.steps * batch_launches(meshes),
+        "clocks": clk.summary(), "gpu_launches": args.steps * batch_launches(meshes, best),
         "api": "fem_assemble_batched, captured in one CUDA graph",
     }
     if compact:
@@ -446,8 +449,8 @@ def assembly_leg(torch, fem, mesh, dev, stream, flush, steps: int, warmup: int, 
 def rooflines(mesh, nnz: int, t: dict, peak: dict, workload: str) -> dict:
     ab = algorithmic_bytes(mesh, nnz)
     hbm = peak["hbm_gbs"]
-    # scatter phase: reads the inputs, writes every list entry once (16 B per
-    # CSR nonzero); consolidation reads the entries back and writes the CSR
+    # scatter phase: reads the inputs, writes what the consolidation reads;
+    # consolidation reads it and writes the CSR
     scatter_bytes = ab["in"] + ab["list"] // 2
     consolidate_bytes = ab["list"] // 2 + ab["out"]
     sg = scatter_bytes / (t["scatter_ms"] / 1e3) / 1e9
@@ -456,12 +459,13 @@ def rooflines(mesh, nnz: int, t: dict, peak: dict, workload: str) -> dict:
     return {
         "roofline": {"bound": "hbm", "achieved": sg, "peak": hbm, "unit": "GB/s", "frac": sg / hbm,
                      "traffic": read_profile_traffic(workload), "peak_kind": peak["kind"],
-                     "kernel": SCATTER_KERNEL.get(workload, "") + " (scatter phase: list reset, element order, scatter)",
+                     "kernel": SCATTER_KERNEL.get(workload, "") + " (scatter phase)",
                      "algorithmic_bytes_per_launch": scatter_bytes,
                      "algorithmic_bytes_per_element": scatter_bytes / max(mesh.num_elems, 1),
                      "ms_per_launch": t["scatter_ms"]},
         "consolidate_roofline": {"bound": "hbm", "achieved": cg, "peak": hbm, "unit": "GB/s", "frac": cg / hbm,
-                                 "kernel": "k_write (consolidation phase: count, scan, sorted write)",
+                                 "kernel": "consolidation phase (" + ("k_write_hex20: node order, scan, gather of the element blocks"
+                                               if mesh.z is not None else "k_write_sorted_2d: scan, sorted write") + ")",
                                  "algorithmic_bytes_per_launch": consolidate_bytes, "ms_per_launch": t["consolidate_ms"]},
         "step_roofline": {"achieved": step, "frac": step / hbm, "algorithmic_bytes": ab,
                           "frac_nominal_8tbs": step / 8000.0,
@@ -774,25 +778,36 @@ def run_ours(args, rank: int, world: int, local_rank: int):
 
 def kernels_per_step(workload: str, mesh) -> int:
     """Library kernels launched by one assembly step."""
+    small = mesh.num_nodes <= SMALL_NODES
     if workload == "hex20":
-        waves = (mesh.num_elems + 32767) // 32768
-        # k_info_init, k_bbox_init, k_bbox, Morton key count / bucket scan / scatter;
-        # node -> element incidence (count, tile sums, tile scan, tile apply, fill);
-        # claim + value pass per wave; k_consolidate_reset, k_scan_reduce,
-        # k_scan_tiles, k_row_ptr, k_write (the launch list of one step)
-        return 6 + 5 + 2 * waves + 5
-    return {"q4": 10, "t3": 10, "mixed": 11}[workload]
+        # lists (k_begin, k_occ_count, _sums, _offsets, _fill, k_rows, k_long_rows, or one cooperative launch), k_ke,
+        # node order (box twice, key count, scan, scatter), k_tile_entries (not small), k_row_ptr, k_write_hex20
+        lists = 1 if small and mesh.num_elems <= SMALL_NODES else 7
+        return lists + 1 + 5 * (mesh.num_elems >= ORDERED_ELEMS) + (2 if small else 3)
+    # k_lists_begin, k_fill_2d, k_rows_2d, k_long_rows_2d, or one cooperative launch; k_tile_entries (not small),
+    # k_row_ptr, k_write_sorted_2d
+    return (1 if small and mesh.num_elems <= 4 * SMALL_NODES else 4) + (2 if small else 3)
 
 
-def batch_launches(meshes) -> int:
-    """Library kernels of one fem_assemble_batched call: the copies of the mesh
-    descriptors (96 a launch) and of the schedule (700 segments a launch; a
-    mesh's segments: reset, 2-D scatter or a claim and a value segment per
-    4,096-element Hex20 wave, scan tiles, top scan, row pointers, write,
-    finish), the start kernel (counters, ticket, start stamp) and the
-    persistent kernel."""
-    segs = sum(6 + 2 * ((m.num_elems + 4095) // 4096) if m.kind == 2 else 7 for m in meshes)
-    return -(-len(meshes) // 96) + -(-segs // 700) + 2
+def batch_launches(meshes, slots: int) -> int:
+    """Library kernels of one fem_assemble_batched call: the meshes are dealt to
+    the slots, largest first, and run in rounds (the r-th smallest mesh of every slot) of merged launches."""
+    cost = [(60.0 if m.kind == 2 else 1.0 if m.kind == 1 else 1.4) * m.num_elems + 1e3 for m in meshes]
+    load, dealt = [0.0] * slots, [[] for _ in range(slots)]
+    for i in sorted(range(len(meshes)), key=lambda i: -cost[i]):
+        k = load.index(min(load))
+        load[k] += cost[i]
+        dealt[k].insert(0, meshes[i])
+    total = 0
+    for r in range(max(len(d) for d in dealt)):
+        part = [d[r] for d in dealt if r < len(d)]
+        for i in range(0, len(part), ROUND_LARGE):
+            ms = part[i:i + ROUND_LARGE]
+            hexes = [m for m in ms if m.kind == 2]
+            # begin, fill, tile entries, row pointers, finish; occurrences (3), rows (2), Ke, write; 2-D rows (2), write
+            total += 5 + 7 * bool(hexes) + 3 * (len(hexes) < len(ms))
+            total += 5 * sum(m.num_elems >= ORDERED_ELEMS for m in hexes)
+    return total
 
 
 def read_profile_traffic(workload: str):
