@@ -25,16 +25,19 @@
 // current one is computed.
 //
 // What bounds the re-assembly is the L2's FP64 atomics: 3,600 additions per
-// element, 230 M for 40x40x40 elements, 1.28 ms of the 1.43 ms call (the
-// clear of the values is the rest). The elements are drawn one by one from a
-// counter (two ahead, so the draw is never waited for). At a fixed stride over the grid the
-// CTAs drift apart in the visit order, so additions to the same rows no longer meet in
-// L2 and the lines go to memory and back; drawn, the elements in flight stay
-// together. Call, 40x40x40: fixed stride 1733 us, drawn with 1 / 2 / 3 / 4 CTAs per
-// SM 2544 / 1645 / 1467 / 1430 us (20x20x20: 203 us with 3, 196 with 4).
-// One warp per element with its blocks staged in shared memory
-// (ke_hex20.cuh's pass with additions in place of the packed store) has no
-// barriers, but only 8 elements per SM in flight behind their additions: 1969 us.
+// element, 230 M for 40x40x40 elements, 1.33 ms of the 1.49 ms call (the
+// clear of the values is the rest). At one fixed stride over the grid the CTAs drift
+// apart in the visit order, so additions to the same rows no longer meet in L2 and
+// the lines go to memory and back. So the CTAs take at most kMapRun elements
+// each, a wave of resident CTAs sharing a stretch of the order, and the next
+// CTAs start where the last ones end: the drift is bounded without any shared
+// state (a map may be in use on several streams). Call, 40x40x40, at 4 CTAs per
+// SM: one stride 1722 us; 2 / 4 / 8 / 16 elements 1538 / 1506 / 1487 / 1513;
+// 20x20x20 215 (one stride), 211 / 202 / 210 / 212; a run of 4 consecutive
+// elements per CTA 1506. One warp per element with its
+// blocks staged in shared memory (ke_hex20.cuh's pass with additions in place of
+// the packed store) has no barriers, but only 8 elements per SM in flight behind
+// their additions: 1969 us.
 // The colouring keeps the fixed stride (its elements share no rows): 32^3 with 2 / 3 / 4
 // CTAs per SM 4.91 / 3.83 / 3.07 ms; 5.49 ms when the choice of the stride is made at run time.
 #include <algorithm>
@@ -44,6 +47,7 @@
 namespace fem {
 namespace {
 
+constexpr int kMapRun = 8;  // elements of one CTA of the re-assembly, at most
 #ifndef FEM_VALUES_CTAS
 #define FEM_VALUES_CTAS 4
 #endif
@@ -54,7 +58,7 @@ constexpr int kThreads = kValueWarps * 32;
 template <int kOut>
 __global__ void __launch_bounds__(kThreads, FEM_VALUES_CTAS)
     k_values_hex20(MeshView m, const int* __restrict__ perm, int i0, int i1, const int* __restrict__ range,
-                   ValuesTarget t) {
+                   ValuesTarget t, int group, int run) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     ValuesSmem& sm = *reinterpret_cast<ValuesSmem*>(smem_raw);
     if (range) {
@@ -62,12 +66,18 @@ __global__ void __launch_bounds__(kThreads, FEM_VALUES_CTAS)
         i1 = range[1];
     }
     values_init(sm);
-    values_cta<kOut>(m, perm, (long long)i0 + blockIdx.x, gridDim.x, i1, t, sm);
+    if constexpr (kOut == kToCsrMap) {
+        const long long chunk = blockIdx.x / group * ((long long)group * run);
+        values_cta<kOut>(m, perm, chunk + blockIdx.x % group, group, (int)min((long long)i1, chunk + (long long)group * run),
+                         t, sm);
+    } else {
+        values_cta<kOut>(m, perm, (long long)i0 + blockIdx.x, gridDim.x, i1, t, sm);
+    }
 }
 
 template <int kOut>
 cudaError_t launch_values(const MeshView& m, const int* perm, int i0, int i1, const int* range, const ValuesTarget& t,
-                          int ctas_per_sm, cudaStream_t s) {
+                          cudaStream_t s) {
     static DeviceCache cache;
     const size_t smem = sizeof(ValuesSmem);
     int per_sm = 0;
@@ -78,10 +88,16 @@ cudaError_t launch_values(const MeshView& m, const int* perm, int i0, int i1, co
         return e;
     }, per_sm);
     if (err) return err;
-    const int use = ctas_per_sm > 0 ? std::min(ctas_per_sm, per_sm) : per_sm;
     const long long count = range ? m.E_count : i1 - i0;  // a colour's size is on the device: bound by E
-    const long long grid = std::max<long long>(1, std::min<long long>(count, (long long)use * sm_count()));
-    k_values_hex20<kOut><<<(int)grid, kThreads, smem, s>>>(m, perm, i0, i1, range, t);
+    const long long fit = (long long)per_sm * sm_count();
+    long long grid = std::max<long long>(1, std::min(count, fit));
+    int run = 1;
+    if (kOut == kToCsrMap && count > fit) {
+        const long long waves = (count + fit * kMapRun - 1) / (fit * kMapRun);
+        run = (int)((count + fit * waves - 1) / (fit * waves));
+        grid = waves * fit;
+    }
+    k_values_hex20<kOut><<<(int)grid, kThreads, smem, s>>>(m, perm, i0, i1, range, t, (int)fit, run);
     return cudaGetLastError();
 }
 
@@ -96,8 +112,7 @@ cudaError_t launch_reassemble_hex20(const MeshView& m, int precision, const int*
     t.row_ptr = mt.row_ptr;
     t.csr = mt.values;
     t.info = info;
-    t.ticket = &info->ticket;
-    return launch_values<kToCsrMap>(m, perm, 0, m.E_count, nullptr, t, 0, s);
+    return launch_values<kToCsrMap>(m, perm, 0, m.E_count, nullptr, t, s);
 }
 
 cudaError_t launch_colour_hex20(const MeshView& m, const int* perm, const int* range, const MapTarget& mt,
@@ -107,7 +122,7 @@ cudaError_t launch_colour_hex20(const MeshView& m, const int* perm, const int* r
     t.col_idx = mt.col_idx;
     t.csr = mt.values;
     t.info = info;
-    return launch_values<kToCsrColour>(m, perm, 0, 0, range, t, 0, s);
+    return launch_values<kToCsrColour>(m, perm, 0, 0, range, t, s);
 }
 
 }  // namespace fem

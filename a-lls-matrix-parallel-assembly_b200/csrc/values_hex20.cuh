@@ -24,7 +24,6 @@ struct ValuesTarget {
     const int* col_idx;
     double* csr;
     DevInfo* info;        // status bits
-    int* ticket;          // kToCsrMap: positions drawn past the first gridDim.x, 0 at the launch
 };
 
 // The six 8x8 tile positions (ti <= tj) of the upper triangle of the 24 x 24 node grid.
@@ -39,7 +38,7 @@ struct ValuesSmem {
     double w[KS];          // gauss weight * detJ (w[27] = 0)
     int nodes[20];
     double lam, mu;
-    int bad, next;
+    int bad;
 };
 
 __device__ __forceinline__ void dmma(double& c0, double& c1, double a, double b) {
@@ -91,16 +90,8 @@ __device__ __forceinline__ void values_cta(const MeshView& m, const int* __restr
     }
     __syncthreads();
 
-    // the elements come at a fixed stride, or (kToCsrMap) are drawn from a counter, two ahead
-    const bool drawn = kOut == kToCsrMap;
-    if (drawn) {
-        if (tid == 0) sm.next = (int)i_stride + atomicAdd(t.ticket, 1);
-        __syncthreads();
-    }
-    long long i_next = drawn ? sm.next : i_first + i_stride;
-    for (long long i = i_first; i < i1;) {
+    for (long long i = i_first; i < i1; i += i_stride) {
         const int e = elem(i);
-        const int draw = drawn && tid == 0 ? (int)i_stride + atomicAdd(t.ticket, 1) : 0;
         if (tid == 0) sm.bad = 0;
         __syncthreads();  // the previous element's G, w, lam/mu and flag are no longer read
         if (tid < 20) {
@@ -120,6 +111,7 @@ __device__ __forceinline__ void values_cta(const MeshView& m, const int* __restr
             sm.mu = E / (2.0 * (1.0 + nu));
         }
         __syncthreads();
+        const long long i_next = i + i_stride;
         if (tid < 20 && i_next < i1) pre_n = __ldg(m.conn + (size_t)elem(i_next) * 20 + tid);
         if (sm.bad) {  // nothing to add
             if (tid == 0) raise_status(t.info, FEM_ERR_BAD_MESH);
@@ -128,10 +120,7 @@ __device__ __forceinline__ void values_cta(const MeshView& m, const int* __restr
                 pre_y = __ldg(m.y + pre_n);
                 pre_z = __ldg(m.z + pre_n);
             }
-            if (tid == 0) sm.next = draw;
             __syncthreads();  // uniform: every thread has read the flag before it is reset
-            i = i_next;
-            i_next = drawn ? sm.next : i + i_stride;
             continue;
         }
         // Jacobians J[g][3i + j] = sum_n dN[i][n][g] X[n][j]
@@ -163,9 +152,7 @@ __device__ __forceinline__ void values_cta(const MeshView& m, const int* __restr
             for (int k = 0; k < 9; k++) J[k] = iJ[k];
             sm.w[tid] = hex20::weight3(tid / 9) * hex20::weight3((tid / 3) % 3) * hex20::weight3(tid % 3) * det;
         }
-        if (tid == 0) sm.next = draw;
         __syncthreads();
-        const long long i_after = drawn ? sm.next : i_next + i_stride;
         // physical gradients G[a][n][g] = sum_i iJ[g][3a + i] dN[i][n][g]
         for (int idx = tid; idx < 20 * 27; idx += nt) {
             const int n = idx / 27, g = idx - 27 * n;
@@ -181,8 +168,6 @@ __device__ __forceinline__ void values_cta(const MeshView& m, const int* __restr
             pre_y = __ldg(m.y + pre_n);
             pre_z = __ldg(m.z + pre_n);
         }
-        i = i_next;
-        i_next = i_after;
         if (!tile_warp) continue;  // the remaining warps wait at the next element's first barrier
         // M^{ab} tiles (ti, tj): A[r][k] = w_k G[a][8 ti + r][k], B[k][c] = G[b][8 tj + c][k]
         double acc[3][3][2];

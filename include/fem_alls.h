@@ -3,7 +3,7 @@
  *
  * A mesh (node coordinates, connectivity, element type Q4 / T3 / Hex20 / mixed
  * Q4+T3, per-element E and nu) goes in; a CSR matrix (row_ptr, col_idx sorted
- * within each row, FP64 values) comes out. Element stiffness, the atomic
+ * within each row, FP64 values) comes out. Element stiffness, the
  * row-list scatter and the list-to-CSR consolidation run as sm_100a CUDA
  * kernels; there is no CPU fallback.
  *
@@ -112,7 +112,7 @@ typedef struct fem_opts {
     int32_t precision;     /* FEM_PREC_FP64 */
     int32_t first_slots;   /* list slots in each node's first chunk; 0 = default */
     int32_t chunk_slots;   /* list slots per overflow chunk; 0 = default */
-    int32_t ctas_per_sm;   /* resident CTAs per SM of the scatter kernel's persistent grid
+    int32_t ctas_per_sm;   /* resident CTAs per SM of the 2-D row kernel's persistent grid
                               (capped at what fits); 0 = all that fit */
     double pool_factor;    /* overflow chunks per node in the pool; 0 = default */
     int32_t wait_limit_us; /* bound on a kernel's wait for its own tensor-core products
@@ -138,11 +138,11 @@ typedef struct fem_csr {
 /* Device-side result word of the last assembly in a workspace. */
 typedef struct fem_info {
     int64_t nnz;              /* CSR nonzeros */
-    int64_t list_entries;     /* list slots filled by the scatter (nnz/dof^2 + duplicates) */
+    int64_t list_entries;     /* list slots filled by the scatter (nnz/dof^2) */
     int32_t status_bits;      /* OR of (1 << FEM_ERR_*) raised on the device */
     int32_t overflow_chunks;  /* overflow chunks taken from the pool */
     int32_t pool_chunks;      /* overflow chunk capacity of the pool */
-    int32_t max_row_entries;  /* longest row list (node granularity, duplicates included) */
+    int32_t max_row_entries;  /* longest row list (node granularity) */
 } fem_info;
 
 /* ---- workspace ------------------------------------------------------------ */
@@ -159,8 +159,8 @@ FEM_API fem_status fem_alls_workspace_size(const fem_mesh* mesh, const fem_opts*
 FEM_API fem_status fem_alls_scatter(const fem_mesh* mesh, const fem_opts* opts, void* workspace,
                             size_t workspace_bytes, void* stream);
 
-/* Consolidates the lists into CSR: per row sort + duplicate merge, device scan
- * for row_ptr, coalesced writes of col_idx/values. Replaces the host
+/* Consolidates the lists into CSR: device scan for row_ptr, coalesced writes of
+ * col_idx/values (Hex20: summed from the element matrices as they are written). Replaces the host
  * buildCSRStructure and convertALLStoCSRKernel. row_ptr is always written; if
  * capacity < nnz nothing else is written and the device info gets
  * FEM_ERR_CAPACITY (the lists stay intact, so it can be re-run with larger
@@ -319,9 +319,11 @@ FEM_API fem_status fem_autotune_batched(const fem_mesh* meshes, int32_t n, const
  * has no such path: every assembly repeats the list build and the host pattern
  * (ALLS_Quad2D_Assembly_Accuracy_Analysis.cu:394-501,605-645). A scatter map,
  * built once from the CSR pattern of a full assembly, holds the CSR position
- * of every element node block; re-assembly then adds each element's blocks at
- * those positions with FP64 atomics, with no list, no pattern build and no
- * sort. The map buffer also holds the element visit order and a status word. */
+ * of every element node block (Hex20 and smaller 2-D meshes), where re-assembly
+ * adds each element's blocks with FP64 atomics, or, row node by row node, the
+ * elements and the places of their blocks in the node's rows (larger 2-D
+ * meshes), which re-assembly sums and writes once. No list, no pattern build
+ * and no sort. The map buffer also holds the element visit order and a status word. */
 
 /* Bytes of the scatter-map buffer (device, 256-byte aligned) for this mesh:
  * 4 * num_elems * npe^2 (npe 4 for Q4 and mixed, 3 for T3, 20 for Hex20) plus
@@ -336,8 +338,7 @@ FEM_API fem_status fem_scatter_map_build(const fem_mesh* mesh, const int32_t* ro
                                          void* map, size_t map_bytes, void* stream);
 
 /* values[0, nnz) = the assembled FP64 values of the mesh's current
- * coordinates and materials, in the pattern the map was built for (zeroed,
- * then every element block added). opts->precision as fem_alls_scatter.
+ * coordinates and materials, in the pattern the map was built for. opts->precision as fem_alls_scatter.
  * Values are not bitwise reproducible run to run (atomic order). Asynchronous. */
 FEM_API fem_status fem_reassemble_values(const fem_mesh* mesh, const fem_opts* opts, const void* map,
                                          size_t map_bytes, const int32_t* row_ptr, double* values, int64_t nnz,

@@ -79,9 +79,9 @@ def test_fp32_reassembly(fem, oracle_mod, cuda_device, name):
 
 
 @pytest.mark.parametrize("count", [1, 591, 592, 593, 800])
-def test_hex20_drawn_elements(fem, oracle_mod, cuda_device, count):
-    # around the launch's first elements (4 CTAs on each of 148 SMs), past which they are drawn from a counter;
-    # a second call draws again, and elements that went bad (the first, one of the middle, the last) add nothing
+def test_hex20_element_counts(fem, oracle_mod, cuda_device, count):
+    # around the resident CTAs (4 on each of 148 SMs), past which a CTA takes several elements, on a first and a
+    # second call; elements that went bad (the first, one of the middle, the last) add nothing
     import copy
     import torch
     import meshgen as mg
@@ -112,3 +112,21 @@ def test_hex20_drawn_elements(fem, oracle_mod, cuda_device, count):
     got = vals[:-1].cpu().numpy()
     scale = value_errors(orp, oci, ov, ov + (got - ov2))[1]  # on the scale of the whole matrix
     assert scale <= RTOL
+
+
+@pytest.mark.parametrize("count", [4736, 4737, 4913])
+def test_hex20_second_wave(fem, cuda_device, count):
+    # past 8 elements for each resident CTA the order is cut into waves; against the values of the assembly
+    import torch
+    import meshgen as mg
+    m = mg.hex20_grid(17, 17, 17, seed=3)
+    m.conn = m.conn[:count].copy()
+    asm = fem.Assembler(m)
+    rp, ci, v, info = asm.assemble()
+    nnz = int(info.nnz)
+    re = fem.Reassembler(asm)
+    re.build(nnz)
+    vals = torch.full((nnz,), 7.0, dtype=torch.float64, device="cuda")
+    re.reassemble(vals)
+    assert re.read_info() == 0
+    assert value_errors(rp.cpu().numpy(), ci.cpu().numpy()[:nnz], v.cpu().numpy()[:nnz], vals.cpu().numpy())[1] <= RTOL
