@@ -1,5 +1,5 @@
 // Device code of the list -> CSR consolidation (consolidate.cu), shared with
-// the batched persistent kernel (batched.cu): tile-level scan steps and the
+// the batch's merged launches (batched.cu): tile-level scan steps and the
 // sorted write of a range of row-node batches. See consolidate.cu for the
 // algorithm and the reference steps it replaces.
 #pragma once

@@ -628,8 +628,8 @@ def reassembly(fem, torch, asm, mesh, nnz, args, flush, stream) -> dict:
     torch.cuda.empty_cache()
     return {"value": mesh.num_elems / (ms / 1e3), "unit": "elements/s", "ms_per_step": ms, "map_build_ms": build_ms,
             "max_rel_diff_vs_alls_nonzero": diff,
-            "what": "fem_reassemble_values: values zeroed, element blocks added at scatter-map positions (FP64 "
-                    "atomics); no lists, no pattern build"}
+            "what": "fem_reassemble_values: element blocks added at scatter-map positions (FP64 atomics), or summed row "
+                    "node by row node (larger 2-D meshes); no lists, no pattern build"}
 
 
 def colour_baseline(fem, torch, asm, mesh, nnz, args, flush, stream) -> dict:
