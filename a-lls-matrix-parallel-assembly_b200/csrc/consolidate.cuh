@@ -262,6 +262,16 @@ __device__ void long_row_write_upper(const ListLayout& L, int n, int u, const in
 
 enum : int { kOutCsr = 0, kOutBsr = 1, kOutUpper = 2 };
 
+// Whether the output is written: its entries fit the caller's buffers, and its row pointers (entries; kOutBsr: blocks)
+// fit int32. Past either, FEM_ERR_CAPACITY / FEM_ERR_RANGE is raised already (row_ptr_rows) and nothing is stored: a
+// wrapped row pointer would place rows in front of the buffers, whatever their capacity.
+template <int DPN, int kMode>
+__device__ __forceinline__ bool output_fits(const DevInfo* info, long long capacity) {
+    constexpr long long kMost = 0x7FFFFFFFll * (kMode == kOutBsr ? DPN * DPN : 1);
+    const long long nnz = __ldcg(&info->nnz);
+    return nnz <= capacity && nnz <= kMost;
+}
+
 // Next link and slot words (kPre per lane of a G-lane group) of a node's first chunk.
 template <int G, int kPre>
 __device__ __forceinline__ void prefetch_first_chunk(const ListLayout& L, long long node, int glane, int (&w)[kPre],
@@ -309,7 +319,7 @@ __device__ __forceinline__ void write_batches(const ListLayout& L, const int* __
     constexpr int kPre = (DPN == 2 ? 16 : 96) / G;
     auto& s_keys = sm.keys;
     auto& s_vals = sm.vals;
-    if (__ldcg(&L.info->nnz) > capacity) return;  // FEM_ERR_CAPACITY already raised; write nothing
+    if (!output_fits<DPN, kMode>(L.info, capacity)) return;
     const int tid = threadIdx.x;
     const int grp = tid / G, glane = tid % G;
     const unsigned gmask = group_mask<G>((tid & 31) / G);
@@ -575,7 +585,7 @@ __device__ __forceinline__ void write_sorted_2d(const ListLayout& L, const int* 
     constexpr int G = 16, NPB = kBlockThreads / G;
     int* const s_sum = s_stat;
     int* const s_max = s_stat + kBlockThreads / 32;
-    if (__ldg(&L.info->nnz) > capacity) return;  // FEM_ERR_CAPACITY already raised; write nothing
+    if (!output_fits<2, kOutCsr>(L.info, capacity)) return;
     const int tid = threadIdx.x, grp = tid / G, lane = tid % G, i = lane & 1;
     const unsigned gmask = 0xFFFFu << (((tid & 31) / G) * G);
     int t_sum = 0, t_max = 0;

@@ -84,7 +84,7 @@ __device__ __forceinline__ void write_hex20(const ListLayout& L, const HexRows& 
     int* const s_max = cta.max;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     WriteHexSmem& sm = cta.w[warp];
-    if (__ldg(&L.info->nnz) > capacity) return;  // FEM_ERR_CAPACITY already raised; write nothing
+    if (!output_fits<3, kMode>(L.info, capacity)) return;
     for (int k = threadIdx.x; k < 20 * 32 * kItems; k += kWriteThreads) {
         const int a = k / (32 * kItems), x = k - a * 32 * kItems, b = min(x / 9, 19), v = x - 9 * (x / 9);
         (&cta.src[0][0])[k] =
