@@ -59,7 +59,8 @@ __device__ __forceinline__ int npe_of(const MeshView& m, int e) {
 }
 
 // One thread per (element, block): binary search of the block's first column
-// in its first row. Blocks past the element's nodes (T3 in a mixed mesh) get -1.
+// in its first row. Blocks past the element's nodes (T3 in a mixed mesh) get -1, and so do all blocks of an element
+// with a bad node id: it takes no part, and the re-assembly reads the coordinates of every node of an element that does.
 __global__ void k_build_map(MeshView m, int dpn, int npe_max, const int* __restrict__ row_ptr,
                             const int* __restrict__ col_idx, int* __restrict__ map, int* __restrict__ status) {
     const int G = npe_max * npe_max;
@@ -71,10 +72,15 @@ __global__ void k_build_map(MeshView m, int dpn, int npe_max, const int* __restr
         const int npe = npe_of(m, e);
         int pos = -1;
         if (a < npe && b < npe) {
-            const int na = __ldg(m.conn + (size_t)e * m.stride + a), nb = __ldg(m.conn + (size_t)e * m.stride + b);
-            if (na < 0 || na >= m.N || nb < 0 || nb >= m.N) {
+            bool bad = false;
+            for (int k = 0; k < npe; k++) {
+                const int n = __ldg(m.conn + (size_t)e * m.stride + k);
+                bad |= n < 0 || n >= m.N;
+            }
+            if (bad) {
                 atomicOr(status, 1 << FEM_ERR_BAD_MESH);
             } else {
+                const int na = __ldg(m.conn + (size_t)e * m.stride + a), nb = __ldg(m.conn + (size_t)e * m.stride + b);
                 pos = find_col(row_ptr, col_idx, dpn * na, dpn * nb);
                 if (pos < 0) atomicOr(status, 1 << FEM_ERR_INTERNAL);  // the pattern lacks the block
             }
