@@ -718,8 +718,9 @@ namespace {
 struct MapHostLayout {
     int G;  // map entries per element
     size_t off_info, off_pos, off_perm, off_ranges, off_hist, off_bbox, total;
-    // 2-D meshes of at least min_row_nodes nodes, whose occurrences fit in the same bytes (all but mostly unconnected
-    // triangles): by row nodes instead
+    // 2-D meshes of at least min_row_nodes nodes, whose occurrences fit in the positions' bytes (all but mostly
+    // unconnected triangles): by row nodes instead, unless the pattern turns out not to be one of node blocks with
+    // rows of at most 65,536 columns (known on the device only: RowsMap::blocks), when the positions take their place
     bool rows;
     size_t off_off, off_occ, off_ranks;
 };
@@ -739,7 +740,7 @@ MapHostLayout map_layout(const fem_mesh* m) {
                                                  : (size_t)2 * reorder_buckets(m->num_nodes);
     size_t off = 0;
     h.off_info = off;
-    off += align_up(sizeof(DevInfo));
+    off += align_up(sizeof(DevInfo) + sizeof(int));  // the info word; by rows: RowsMap::blocks behind it
     h.off_pos = off;
     off += align_up(E * h.G * sizeof(int));
     h.off_perm = off;
@@ -759,14 +760,15 @@ MapHostLayout map_layout(const fem_mesh* m) {
         // the ranks, or, while the map is built, the counters and scan partials in their place
         const size_t end = h.off_ranks + std::max(align_up(E * npe * npe * sizeof(unsigned short)),
                                                   align_up(N * sizeof(int)) + row_tiles(m->num_nodes) * sizeof(long long));
-        h.rows = N >= min_row_nodes(m->kind) && end <= h.total && E < ((size_t)1 << 29) && E > 0;
+        h.rows = N >= min_row_nodes(m->kind) && end <= h.off_perm && E < ((size_t)1 << 29) && E > 0;
     }
     return h;
 }
 
 RowsMap rows_map(const MapHostLayout& h, unsigned char* b) {
     return RowsMap{reinterpret_cast<int*>(b + h.off_off), reinterpret_cast<unsigned*>(b + h.off_occ),
-                   reinterpret_cast<unsigned short*>(b + h.off_ranks)};
+                   reinterpret_cast<unsigned short*>(b + h.off_ranks),
+                   reinterpret_cast<int*>(b + h.off_info + sizeof(DevInfo))};
 }
 
 fem_status check_map(const fem_mesh* mesh, const void* map, size_t map_bytes, MapHostLayout& h) {
@@ -802,14 +804,17 @@ fem_status fem_scatter_map_build(const fem_mesh* mesh, const int32_t* row_ptr, c
     int* perm = reinterpret_cast<int*>(b + h.off_perm);
     int* ranges = reinterpret_cast<int*>(b + h.off_ranges);
     int* hist = reinterpret_cast<int*>(b + h.off_hist);
-    cudaError_t err = cudaMemsetAsync(info, 0, sizeof(DevInfo), s);
+    int* pos = reinterpret_cast<int*>(b + h.off_pos);
+    cudaError_t err = cudaMemsetAsync(info, 0, sizeof(DevInfo) + sizeof(int), s);
     if (!err && h.rows) {
         int* cnt = reinterpret_cast<int*>(b + h.off_ranks);
         long long* tiles = reinterpret_cast<long long*>(b + h.off_ranks + align_up((size_t)m.N * sizeof(int)));
-        err = launch_build_rows_map(m, mesh->kind, row_ptr, col_idx, rows_map(h, b), cnt, tiles, info, s);
+        const RowsMap r = rows_map(h, b);
+        err = launch_build_rows_map(m, mesh->kind, row_ptr, col_idx, r, cnt, tiles, info, s);
+        if (!err) err = launch_build_map(m, mesh->kind, row_ptr, col_idx, pos, &info->status_bits, s, r.blocks);
+        if (!err) err = launch_reorder(m, hist, ranges, perm, sm_count(), s, r.blocks);
     } else if (!err && mesh->num_elems > 0) {
-        err = launch_build_map(m, mesh->kind, row_ptr, col_idx, reinterpret_cast<int*>(b + h.off_pos),
-                               &info->status_bits, s);
+        err = launch_build_map(m, mesh->kind, row_ptr, col_idx, pos, &info->status_bits, s);
         // the element visit order of the A-LLS scatter, for the locality of the adds
         if (!err && mesh->kind == FEM_HEX20)
             err = launch_reorder_3d(m, hist, ranges, perm, reinterpret_cast<unsigned long long*>(b + h.off_bbox),
@@ -839,9 +844,13 @@ fem_status fem_reassemble_values(const fem_mesh* mesh, const fem_opts* opts, con
     if (!err && nnz > 0 && !h.rows) err = cudaMemsetAsync(values, 0, (size_t)nnz * sizeof(double), s);
     if (!err && mesh->num_elems > 0) {
         const MeshView m = mesh_view(mesh);
-        if (h.rows)
-            err = launch_rows_values_2d(m, mesh->kind, precision, rows_map(h, b), row_ptr, values, &info->status_bits, s);
-        else if (mesh->kind == FEM_HEX20)
+        if (h.rows) {
+            const RowsMap r = rows_map(h, b);
+            err = launch_rows_values_2d(m, mesh->kind, precision, r, row_ptr, values, nnz, &info->status_bits, s);
+            if (!err)
+                err = launch_reassemble_2d(m, precision, pos, h.G, perm, ranges, row_ptr, values, &info->status_bits, s,
+                                           r.blocks);
+        } else if (mesh->kind == FEM_HEX20)
             err = launch_reassemble_hex20(m, precision, perm, MapTarget{pos, row_ptr, values, nullptr}, info, s);
         else
             err = launch_reassemble_2d(m, precision, pos, h.G, perm, ranges, row_ptr, values, &info->status_bits, s);

@@ -61,7 +61,9 @@ cudaError_t launch_rows_2d(const MeshView& m, const ListLayout& L, int* queue, i
                            int ctas_per_sm, cudaStream_t s);
 // Node-local element order (perm) and the element ranges {q4 begin, q4 end, t3 begin, t3 end}.
 int reorder_buckets(int num_nodes);
-cudaError_t launch_reorder(const MeshView& m, int* hist, int* ranges, int* perm, int sms, cudaStream_t s);
+// gate: NULL, or a device word; 0 there when the sort's kernels run leaves the order as it is.
+cudaError_t launch_reorder(const MeshView& m, int* hist, int* ranges, int* perm, int sms, cudaStream_t s,
+                           const int* gate = nullptr);
 int sm_count();
 // Packed symmetric element stiffness (fem_element_stiffness): doubles per element.
 constexpr int kPackedHex20 = 210 * 9;  // 210 upper 3x3 node blocks
@@ -89,24 +91,28 @@ struct MapTarget {
     const int* col_idx;  // CSR columns (the colouring baseline searches them)
 };
 
-// Scatter map of a mesh into a CSR pattern; status gets 1 << FEM_ERR_* bits.
+// Scatter map of a mesh into a CSR pattern; status gets 1 << FEM_ERR_* bits. gate as launch_reorder's.
 cudaError_t launch_build_map(const MeshView& m, int kind, const int* row_ptr, const int* col_idx, int* map,
-                             int* status, cudaStream_t s);
+                             int* status, cudaStream_t s, const int* gate = nullptr);
 // Value-only re-assembly (atomics into values): 2-D kinds over perm ranges
 // {q4 begin, q4 end, t3 begin, t3 end}; Hex20 over perm (status bits in info).
 cudaError_t launch_reassemble_2d(const MeshView& m, int precision, const int* map, int G, const int* perm,
-                                 const int* ranges, const int* row_ptr, double* values, int* status, cudaStream_t s);
+                                 const int* ranges, const int* row_ptr, double* values, int* status, cudaStream_t s,
+                                 const int* gate = nullptr);
 // The same by row nodes (2-D): each node's occurrences (element << 2 | position) and the ranks of their nodes in its row.
 struct RowsMap {
     int* off;               // [N + 1]
     unsigned* occ;          // [npe * E]
     unsigned short* ranks;  // [npe * npe * E]
+    int* blocks;            // not 0: the pattern does not take this form, the map is the block positions
 };
-// cnt (N ints) and tiles (row_tiles(N) partials): scratch.
+// cnt (N ints) and tiles (row_tiles(N) partials): scratch. *r.blocks (0 before) is set when the pattern is not one of
+// node blocks that holds all of the mesh's, with rows of at most 65,536 columns.
 cudaError_t launch_build_rows_map(const MeshView& m, int kind, const int* row_ptr, const int* col_idx, const RowsMap& r,
                                   int* cnt, long long* tiles, DevInfo* info, cudaStream_t s);
+// values[0, nnz): the rows and zeros behind them; all zeros where *r.blocks is set.
 cudaError_t launch_rows_values_2d(const MeshView& m, int kind, int precision, const RowsMap& r, const int* row_ptr,
-                                  double* values, int* status, cudaStream_t s);
+                                  double* values, long long nnz, int* status, cudaStream_t s);
 // The tensor-core form of the Hex20 value-only re-assembly (ke_tcgen05.cu).
 cudaError_t launch_reassemble_hex20_tc(const MeshView& m, const int* perm, const MapTarget& t, DevInfo* info,
                                        cudaStream_t s);

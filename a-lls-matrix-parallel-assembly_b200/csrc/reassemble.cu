@@ -62,7 +62,9 @@ __device__ __forceinline__ int npe_of(const MeshView& m, int e) {
 // in its first row. Blocks past the element's nodes (T3 in a mixed mesh) get -1, and so do all blocks of an element
 // with a bad node id: it takes no part, and the re-assembly reads the coordinates of every node of an element that does.
 __global__ void k_build_map(MeshView m, int dpn, int npe_max, const int* __restrict__ row_ptr,
-                            const int* __restrict__ col_idx, int* __restrict__ map, int* __restrict__ status) {
+                            const int* __restrict__ col_idx, int* __restrict__ map, int* __restrict__ status,
+                            const int* gate) {
+    if (gate && __ldcg(gate) == 0) return;
     const int G = npe_max * npe_max;
     const long long total = (long long)m.E_count * G;
     for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total;
@@ -95,7 +97,9 @@ template <int NPE, typename T>
 __global__ void __launch_bounds__(kThreads) k_reassemble_2d(MeshView m, const int* __restrict__ map, int G,
                                                             const int* __restrict__ perm, const int* __restrict__ range,
                                                             const int* __restrict__ row_ptr,
-                                                            double* __restrict__ values, int* __restrict__ status) {
+                                                            double* __restrict__ values, int* __restrict__ status,
+                                                            const int* gate) {
+    if (gate && __ldcg(gate) == 0) return;
     constexpr int GL = NPE * NPE, EPW = 32 / GL;
     const int lane = threadIdx.x & 31;
     const int eslot = lane / GL, sub = lane - eslot * GL, a = sub / NPE, b = sub - (sub / NPE) * NPE;
@@ -191,27 +195,34 @@ __global__ void __launch_bounds__(kThreads) k_map_fill(MeshView m, const int* __
 }
 
 // ranks[NPE * j + k]: rank in the row of occurrence j's node of the element's node k positions after it.
+// blocks: set when a node's two rows differ in length or are odd, a column node's pair starts at an odd place, a rank
+// passes 16 bits or the pattern lacks a block (a caller's own pattern: with further columns, or too small).
 template <int KIND>
 __global__ void __launch_bounds__(kThreads) k_map_ranks(MeshView m, const int* __restrict__ off,
                                                         const unsigned* __restrict__ occ,
                                                         const int* __restrict__ row_ptr,
                                                         const int* __restrict__ col_idx,
-                                                        unsigned short* __restrict__ ranks, int* __restrict__ status) {
+                                                        unsigned short* __restrict__ ranks, int* __restrict__ blocks) {
     constexpr int NPE = KIND == FEM_T3 ? 3 : 4;
     const int total = __ldg(off + m.N);
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < total; j += gridDim.x * blockDim.x) {
+    bool other = false;
+    for (long long n = blockIdx.x * blockDim.x + threadIdx.x; n < m.N; n += gridDim.x * blockDim.x) {
+        const int r0 = __ldg(row_ptr + 2 * n), r1 = __ldg(row_ptr + 2 * n + 1), r2 = __ldg(row_ptr + 2 * n + 2);
+        other |= r2 - r1 != r1 - r0 || ((r1 - r0) & 1);
+    }
+    for (long long j = blockIdx.x * blockDim.x + threadIdx.x; j < total; j += gridDim.x * blockDim.x) {
         const unsigned w = __ldg(occ + j);
         const int e = (int)(w >> 2), a = (int)(w & 3u), npe = elem_nodes<KIND>(m, e);
         const int n = __ldg(m.conn + (size_t)e * m.stride + a);
         for (int k = 0; k < npe; k++) {
             const int b = a + k < npe ? a + k : a + k - npe;
             const int p = find_col(row_ptr, col_idx, 2 * n, 2 * __ldg(m.conn + (size_t)e * m.stride + b));
-            if (p < 0) atomicOr(status, 1 << FEM_ERR_INTERNAL);  // the pattern lacks the block
-            const int r = p < 0 ? 0 : (p - __ldg(row_ptr + 2 * n)) / 2;
-            if (r > 0xFFFF) atomicOr(status, 1 << FEM_ERR_RANGE);
-            ranks[(size_t)NPE * j + k] = (unsigned short)r;
+            const int r = p - __ldg(row_ptr + 2 * n);
+            other |= p < 0 || (r & 1) || r / 2 > 0xFFFF;
+            ranks[(size_t)NPE * j + k] = (unsigned short)(r / 2);
         }
     }
+    if (other) *blocks = 1;
 }
 
 constexpr int kRowThreads = 64;
@@ -289,11 +300,18 @@ template <int KIND, typename T>
 __global__ void __launch_bounds__(kRowThreads, RowsShape<KIND>::kCtas)
     k_rows_values_2d(MeshView m, const int* __restrict__ off, const unsigned* __restrict__ occ,
                      const unsigned short* __restrict__ ranks, const int* __restrict__ row_ptr,
-                     double* __restrict__ values, bool wide, int* __restrict__ status) {
+                     double* __restrict__ values, long long nnz, bool wide, int* __restrict__ status,
+                     const int* __restrict__ blocks) {
     constexpr int NPE = KIND == FEM_T3 ? 3 : 4, kRowCols = RowsShape<KIND>::kCols;
     constexpr unsigned kFull = 0xFFFFFFFFu;
     __shared__ double acc[kRowCols][4][kRowPad];
     const int tid = threadIdx.x, lane = tid & 31, warp0 = tid & ~31;
+    // entries that no row of the mesh covers: behind the rows, or, for a pattern that is not in this form, all of them
+    const bool other = __ldg(blocks) != 0;
+    for (long long i = (other ? 0 : __ldg(row_ptr + 2 * (size_t)m.N)) + (long long)blockIdx.x * kRowThreads + tid; i < nnz;
+         i += (long long)gridDim.x * kRowThreads)
+        values[i] = 0.0;
+    if (other) return;  // k_reassemble_2d adds the blocks
     for (long long tile = blockIdx.x; tile * kRowThreads < m.N; tile += gridDim.x) {
         const long long n = tile * kRowThreads + tid;
         int base = 0, u = 0, lo = 0, d = 0;
@@ -425,13 +443,13 @@ cudaError_t build_rows_map(const MeshView& m, const int* row_ptr, const int* col
     k_map_offsets<<<ntiles, kScanThreads, 0, s>>>(cnt, m.N, tiles, r.off, info);
     k_map_fill<KIND><<<grid, kThreads, 0, s>>>(m, r.off, cnt, r.occ);
     k_map_ranks<KIND><<<(int)std::min<long long>(3ll * grid, (long long)sm_count() * 16), kThreads, 0, s>>>(
-        m, r.off, r.occ, row_ptr, col_idx, r.ranks, status);
+        m, r.off, r.occ, row_ptr, col_idx, r.ranks, r.blocks);
     return cudaGetLastError();
 }
 
 template <int KIND, typename T>
-cudaError_t rows_values(const MeshView& m, const RowsMap& r, const int* row_ptr, double* values, int* status,
-                        cudaStream_t s) {
+cudaError_t rows_values(const MeshView& m, const RowsMap& r, const int* row_ptr, double* values, long long nnz,
+                        int* status, cudaStream_t s) {
     static DeviceCache cache;
     int per_sm = 0;
     const cudaError_t err = per_device(cache, [](int& v) {
@@ -440,51 +458,52 @@ cudaError_t rows_values(const MeshView& m, const RowsMap& r, const int* row_ptr,
     if (err) return err;
     const long long tiles = ((long long)m.N + kRowThreads - 1) / kRowThreads;
     k_rows_values_2d<KIND, T><<<(int)std::min<long long>(tiles, (long long)per_sm * sm_count()), kRowThreads, 0, s>>>(
-        m, r.off, r.occ, r.ranks, row_ptr, values, reinterpret_cast<uintptr_t>(values) % 16 == 0, status);
+        m, r.off, r.occ, r.ranks, row_ptr, values, nnz, reinterpret_cast<uintptr_t>(values) % 16 == 0, status, r.blocks);
     return cudaGetLastError();
 }
 
 template <typename T>
 cudaError_t rows_values_kind(const MeshView& m, int kind, const RowsMap& r, const int* row_ptr, double* values,
-                             int* status, cudaStream_t s) {
-    if (kind == FEM_T3) return rows_values<FEM_T3, T>(m, r, row_ptr, values, status, s);
-    if (kind == FEM_Q4) return rows_values<FEM_Q4, T>(m, r, row_ptr, values, status, s);
-    return rows_values<FEM_MIXED_2D, T>(m, r, row_ptr, values, status, s);
+                             long long nnz, int* status, cudaStream_t s) {
+    if (kind == FEM_T3) return rows_values<FEM_T3, T>(m, r, row_ptr, values, nnz, status, s);
+    if (kind == FEM_Q4) return rows_values<FEM_Q4, T>(m, r, row_ptr, values, nnz, status, s);
+    return rows_values<FEM_MIXED_2D, T>(m, r, row_ptr, values, nnz, status, s);
 }
 
 }  // namespace
 
 cudaError_t launch_build_map(const MeshView& m, int kind, const int* row_ptr, const int* col_idx, int* map,
-                             int* status, cudaStream_t s) {
+                             int* status, cudaStream_t s, const int* gate) {
     const int npe_max = kind == FEM_HEX20 ? 20 : (kind == FEM_T3 ? 3 : 4);
     const int dpn = kind == FEM_HEX20 ? 3 : 2;
     const long long total = (long long)m.E_count * npe_max * npe_max;
     if (total == 0) return cudaSuccess;
     const int grid = (int)std::min<long long>((total + kThreads - 1) / kThreads, (long long)sm_count() * 16);
-    k_build_map<<<grid, kThreads, 0, s>>>(m, dpn, npe_max, row_ptr, col_idx, map, status);
+    k_build_map<<<grid, kThreads, 0, s>>>(m, dpn, npe_max, row_ptr, col_idx, map, status, gate);
     return cudaGetLastError();
 }
 
 template <typename T>
 void reassemble_2d_t(const MeshView& m, const int* map, int G, const int* perm, const int* ranges, const int* row_ptr,
-                     double* values, int* status, cudaStream_t s) {
+                     double* values, int* status, cudaStream_t s, const int* gate) {
     const bool has_q4 = m.types || m.stride == 4, has_t3 = m.types || m.stride == 3;
     const long long warps = ((long long)m.E_count + 1) / 2;
     const int grid = (int)std::min<long long>((warps * 32 + kThreads - 1) / kThreads, (long long)sm_count() * 8);
     if (has_q4)
         k_reassemble_2d<4, T><<<grid > 0 ? grid : 1, kThreads, 0, s>>>(m, map, G, perm, ranges + 0, row_ptr, values,
-                                                                      status);
+                                                                      status, gate);
     if (has_t3)
         k_reassemble_2d<3, T><<<grid > 0 ? grid : 1, kThreads, 0, s>>>(m, map, G, perm, ranges + 2, row_ptr, values,
-                                                                      status);
+                                                                      status, gate);
 }
 
 cudaError_t launch_reassemble_2d(const MeshView& m, int precision, const int* map, int G, const int* perm,
-                                 const int* ranges, const int* row_ptr, double* values, int* status, cudaStream_t s) {
+                                 const int* ranges, const int* row_ptr, double* values, int* status, cudaStream_t s,
+                                 const int* gate) {
     if (precision == FEM_PREC_FP32)
-        reassemble_2d_t<float>(m, map, G, perm, ranges, row_ptr, values, status, s);
+        reassemble_2d_t<float>(m, map, G, perm, ranges, row_ptr, values, status, s, gate);
     else
-        reassemble_2d_t<double>(m, map, G, perm, ranges, row_ptr, values, status, s);
+        reassemble_2d_t<double>(m, map, G, perm, ranges, row_ptr, values, status, s, gate);
     return cudaGetLastError();
 }
 
@@ -496,9 +515,9 @@ cudaError_t launch_build_rows_map(const MeshView& m, int kind, const int* row_pt
 }
 
 cudaError_t launch_rows_values_2d(const MeshView& m, int kind, int precision, const RowsMap& r, const int* row_ptr,
-                                  double* values, int* status, cudaStream_t s) {
-    return precision == FEM_PREC_FP32 ? rows_values_kind<float>(m, kind, r, row_ptr, values, status, s)
-                                      : rows_values_kind<double>(m, kind, r, row_ptr, values, status, s);
+                                  double* values, long long nnz, int* status, cudaStream_t s) {
+    return precision == FEM_PREC_FP32 ? rows_values_kind<float>(m, kind, r, row_ptr, values, nnz, status, s)
+                                      : rows_values_kind<double>(m, kind, r, row_ptr, values, nnz, status, s);
 }
 
 }  // namespace fem

@@ -48,14 +48,19 @@ __device__ __forceinline__ int element_key(const MeshView& m, int e, int NB) {
     return (m.types && t3 ? NB : 0) + (lo >> kBucketShift);
 }
 
-__global__ void k_bucket_count(MeshView m, int NB, int* __restrict__ hist) {
+// A gate (or NULL: open) is a device word that a sort waits for: 0 when its kernels reach it leaves them nothing to do.
+__device__ __forceinline__ bool closed(const int* gate) { return gate && __ldcg(gate) == 0; }
+
+__global__ void k_bucket_count(MeshView m, int NB, int* __restrict__ hist, const int* gate) {
+    if (closed(gate)) return;
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < m.E_count; e += gridDim.x * blockDim.x)
         atomicAdd(hist + element_key(m, e, NB), 1);
 }
 
 // Exclusive scan of hist[0..nkeys) in place; ranges = {q4 begin, q4 end, t3 begin, t3 end}.
 __global__ void __launch_bounds__(1024) k_bucket_scan(int* __restrict__ hist, int nkeys, int NB, int mixed,
-                                                      int* __restrict__ ranges) {
+                                                      int* __restrict__ ranges, const int* gate) {
+    if (closed(gate)) return;
     __shared__ int s_warp[33];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int carry = 0;
@@ -102,7 +107,8 @@ __global__ void __launch_bounds__(1024) k_bucket_scan(int* __restrict__ hist, in
     }
 }
 
-__global__ void k_bucket_scatter(MeshView m, int NB, int* __restrict__ offsets, int* __restrict__ perm) {
+__global__ void k_bucket_scatter(MeshView m, int NB, int* __restrict__ offsets, int* __restrict__ perm, const int* gate) {
+    if (closed(gate)) return;
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < m.E_count; e += gridDim.x * blockDim.x)
         perm[atomicAdd(offsets + element_key(m, e, NB), 1)] = e;
 }
@@ -238,8 +244,10 @@ constexpr int kSmThreads = 1024;
 constexpr int kMaxSmemKeys = 160 * 1024 / 4;
 
 template <typename Key>
-__global__ void __launch_bounds__(kSmThreads) k_key_count_sm(Key key, int E, int nkeys, int* __restrict__ hist) {
+__global__ void __launch_bounds__(kSmThreads) k_key_count_sm(Key key, int E, int nkeys, int* __restrict__ hist,
+                                                             const int* gate) {
     extern __shared__ int s_cnt[];
+    if (closed(gate)) return;
     for (int k = threadIdx.x; k < nkeys; k += blockDim.x) s_cnt[k] = 0;
     __syncthreads();
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < E; e += gridDim.x * blockDim.x)
@@ -254,8 +262,9 @@ __global__ void __launch_bounds__(kSmThreads) k_key_count_sm(Key key, int E, int
 // and places its elements inside the ranges with shared-memory atomics.
 template <typename Key>
 __global__ void __launch_bounds__(kSmThreads) k_key_scatter_sm(Key key, int E, int nkeys, int* __restrict__ offsets,
-                                                               int* __restrict__ perm) {
+                                                               int* __restrict__ perm, const int* gate) {
     extern __shared__ int s_pos[];
+    if (closed(gate)) return;
     for (int k = threadIdx.x; k < nkeys; k += blockDim.x) s_pos[k] = 0;
     __syncthreads();
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < E; e += gridDim.x * blockDim.x)
@@ -290,21 +299,22 @@ cudaError_t smem_kernels_ready() {
 // Counting sort of the elements by key: histogram, scan (ranges), scatter.
 template <typename Key, typename CountK, typename ScatterK>
 cudaError_t counting_sort(const Key& key, int E, int nkeys, int NB, int mixed, int* hist, int* ranges, int* perm,
-                          int sms, CountK count_global, ScatterK scatter_global, cudaStream_t s) {
+                          int sms, CountK count_global, ScatterK scatter_global, cudaStream_t s,
+                          const int* gate = nullptr) {
     if (nkeys <= kMaxSmemKeys) {
         cudaError_t err = smem_kernels_ready<Key>();
         if (err) return err;
         const long long want = ((long long)E + kSmThreads - 1) / kSmThreads;
         const int grid = (int)std::min<long long>(want > 0 ? want : 1, (long long)sms);
         const size_t smem = (size_t)nkeys * sizeof(int);
-        k_key_count_sm<Key><<<grid, kSmThreads, smem, s>>>(key, E, nkeys, hist);
-        k_bucket_scan<<<1, 1024, 0, s>>>(hist, nkeys, NB, mixed, ranges);
-        k_key_scatter_sm<Key><<<grid, kSmThreads, smem, s>>>(key, E, nkeys, hist, perm);
+        k_key_count_sm<Key><<<grid, kSmThreads, smem, s>>>(key, E, nkeys, hist, gate);
+        k_bucket_scan<<<1, 1024, 0, s>>>(hist, nkeys, NB, mixed, ranges, gate);
+        k_key_scatter_sm<Key><<<grid, kSmThreads, smem, s>>>(key, E, nkeys, hist, perm, gate);
     } else {
         const long long want = ((long long)E + kThreads - 1) / kThreads;
         const int grid = (int)std::min<long long>(want > 0 ? want : 1, (long long)sms * 8);
         count_global(grid);
-        k_bucket_scan<<<1, 1024, 0, s>>>(hist, nkeys, NB, mixed, ranges);
+        k_bucket_scan<<<1, 1024, 0, s>>>(hist, nkeys, NB, mixed, ranges, gate);
         scatter_global(grid);
     }
     return cudaGetLastError();
@@ -349,15 +359,16 @@ cudaError_t launch_node_order(const MeshView& m, int* hist, int* ranges, int* or
                          [](int) {}, [](int) {}, s);
 }
 
-cudaError_t launch_reorder(const MeshView& m, int* hist, int* ranges, int* perm, int sms, cudaStream_t s) {
+cudaError_t launch_reorder(const MeshView& m, int* hist, int* ranges, int* perm, int sms, cudaStream_t s,
+                           const int* gate) {
     const int NB = reorder_buckets(m.N);
     const int nkeys = (m.types ? 2 : 1) * NB;
     cudaError_t err = cudaMemsetAsync(hist, 0, (size_t)nkeys * sizeof(int), s);
     if (err) return err;
     return counting_sort(
         BucketKey{m, NB}, m.E_count, nkeys, NB, m.types ? 1 : 0, hist, ranges, perm, sms,
-        [&](int grid) { k_bucket_count<<<grid, kThreads, 0, s>>>(m, NB, hist); },
-        [&](int grid) { k_bucket_scatter<<<grid, kThreads, 0, s>>>(m, NB, hist, perm); }, s);
+        [&](int grid) { k_bucket_count<<<grid, kThreads, 0, s>>>(m, NB, hist, gate); },
+        [&](int grid) { k_bucket_scatter<<<grid, kThreads, 0, s>>>(m, NB, hist, perm, gate); }, s, gate);
 }
 
 }  // namespace fem

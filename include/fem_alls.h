@@ -322,7 +322,7 @@ FEM_API fem_status fem_autotune_batched(const fem_mesh* meshes, int32_t n, const
  * of every element node block (Hex20 and smaller 2-D meshes), where re-assembly
  * adds each element's blocks with FP64 atomics, or, row node by row node, the
  * elements and the places of their blocks in the node's rows (larger 2-D
- * meshes), which re-assembly sums and writes once. No list, no pattern build
+ * meshes in a pattern of node blocks), which re-assembly sums and writes once. No list, no pattern build
  * and no sort. The map buffer also holds the element visit order and a status word. */
 
 /* Bytes of the scatter-map buffer (device, 256-byte aligned) for this mesh:
@@ -338,7 +338,8 @@ FEM_API fem_status fem_scatter_map_build(const fem_mesh* mesh, const int32_t* ro
                                          void* map, size_t map_bytes, void* stream);
 
 /* values[0, nnz) = the assembled FP64 values of the mesh's current
- * coordinates and materials, in the pattern the map was built for. opts->precision as fem_alls_scatter.
+ * coordinates and materials, in the pattern the map was built for; entries that no
+ * element block reaches, and those behind the pattern's last row, become zero. opts->precision as fem_alls_scatter.
  * Values are not bitwise reproducible run to run (atomic order). Asynchronous. */
 FEM_API fem_status fem_reassemble_values(const fem_mesh* mesh, const fem_opts* opts, const void* map,
                                          size_t map_bytes, const int32_t* row_ptr, double* values, int64_t nnz,

@@ -1,6 +1,8 @@
 """What a scatter map takes in (fem_scatter_map_build, fem_reassemble_values),
-through the C ABI: elements with a bad node id, in both forms of the map (by
-element blocks, small 2-D meshes and Hex20; by row nodes, larger 2-D meshes).
+through the C ABI: elements with a bad node id, and a caller's own patterns
+(further columns and rows, missing blocks, a row of more than 65,536 columns), in
+both forms of the map (by element blocks, small 2-D meshes and Hex20; by row
+nodes, larger 2-D meshes).
 Values within 1e-12 of max(|K_ij|, sqrt(|K_ii K_jj|)) of the oracle's assembly."""
 import copy
 
@@ -65,3 +67,106 @@ def test_elements_with_a_bad_node_take_no_part(fem, oracle_mod, cuda_device, nam
     ov = oracle_mod.assemble(m2)[2]
     scale = np.maximum(np.abs(full), diag_scale(orp, oci, full))
     assert np.all(np.abs(vals.cpu().numpy() - ov) <= RTOL * scale)
+
+
+def _extended(rp, ci, lead, tail, rows):
+    """The pattern (rp, ci) with `lead` further columns in front of every row, `tail` behind it (the columns move up by
+    `lead`) and `rows` further rows of one entry at the end; and where each old entry went."""
+    n = rp.size - 1
+    length = np.diff(rp)
+    rp2 = np.concatenate([[0], np.cumsum(length + lead + tail), rp[-1] + n * (lead + tail) + 1 + np.arange(rows)])
+    ci2 = np.zeros(rp2[-1], np.int32)
+    at = np.repeat(rp2[:n] + lead - rp[:-1], length) + np.arange(rp[-1])
+    ci2[at] = ci
+    for k in range(lead):
+        ci2[rp2[:n] + k] = k - lead
+    for k in range(tail):
+        ci2[rp2[1:n + 1] - tail + k] = n + k
+    return rp2.astype(np.int32), ci2, at
+
+
+def _with_pattern(asm, rp, ci):
+    import torch
+    asm.row_ptr = torch.from_numpy(np.ascontiguousarray(rp, np.int32)).cuda()
+    asm.col_idx = torch.from_numpy(np.ascontiguousarray(ci, np.int32)).cuda()
+    return torch.full((ci.size,), 7.0, dtype=torch.float64, device="cuda")
+
+
+@pytest.mark.parametrize("name", list(MESHES))
+@pytest.mark.parametrize("lead,tail,rows", [(0, 1, 1), (1, 0, 0), (2, 1, 0), (2, 0, 3), (0, 2, 2)])
+def test_patterns_with_further_entries(fem, oracle_mod, cuda_device, name, lead, tail, rows):
+    # the mesh's entries get the assembled values, all others are zero
+    m = _mesh(name)
+    orp, oci, ov = oracle_mod.assemble(m)
+    rp, ci, at = _extended(orp, oci, lead, tail, rows)
+    asm = fem.Assembler(m)
+    vals = _with_pattern(asm, rp, ci)
+    re = _build(fem, asm, ci.size, 0)
+    for _ in range(2):
+        vals.fill_(7.0)
+        re.reassemble(vals)
+        assert re.read_info() == 0
+        got = vals.cpu().numpy()
+        _close(orp, oci, ov, got[at])
+        assert np.all(np.delete(got, at) == 0.0)
+
+
+@pytest.mark.parametrize("name", list(MESHES))
+def test_patterns_without_some_blocks(fem, oracle_mod, cuda_device, name):
+    # the last column node of every 50th row node left out: reported when the map is built, the others are right
+    m = _mesh(name)
+    orp, oci, ov = oracle_mod.assemble(m)
+    keep = np.ones(oci.size, bool)
+    nodes = np.arange(0, m.num_nodes, 50)
+    for r in (2 * nodes, 2 * nodes + 1):
+        keep[orp[r + 1] - 1] = keep[orp[r + 1] - 2] = False
+    rp = np.concatenate([[0], np.cumsum(keep)[orp[1:] - 1]])
+    asm = fem.Assembler(m)
+    vals = _with_pattern(asm, rp, oci[keep])
+    re = _build(fem, asm, int(keep.sum()), fem.FEM_ERR_INTERNAL)
+    re.reassemble(vals)
+    scale = np.maximum(np.abs(ov), diag_scale(orp, oci, ov))
+    assert np.all(np.abs(vals.cpu().numpy() - ov[keep]) <= RTOL * scale[keep])
+
+
+def _t3_stiffness(m):
+    """The CSR of a T3 mesh from its constant-strain element matrices (numpy): a row of tens of thousands of columns takes
+    the oracle's linear search too long."""
+    import scipy.sparse as sp
+    c = m.conn
+    x, y = m.x[c], m.y[c]
+    X = np.stack([y[:, 1] - y[:, 2], y[:, 2] - y[:, 0], y[:, 0] - y[:, 1]], 1)
+    Y = np.stack([x[:, 2] - x[:, 1], x[:, 0] - x[:, 2], x[:, 1] - x[:, 0]], 1)
+    det = Y[:, 2] * X[:, 1] - Y[:, 1] * X[:, 2]
+    B = np.zeros((c.shape[0], 3, 6))
+    B[:, 0, 0::2], B[:, 1, 1::2], B[:, 2, 0::2], B[:, 2, 1::2] = X, Y, Y, X
+    D = m.E0 / (1 - m.nu0 ** 2) * np.array([[1, m.nu0, 0], [m.nu0, 1, 0], [0, 0, (1 - m.nu0) / 2]])
+    ke = np.einsum("eki,kl,elj->eij", B, D, B) * (0.5 * m.thickness / det)[:, None, None]
+    dof = (2 * c[:, :, None] + np.arange(2)).reshape(c.shape[0], 6)
+    a = sp.coo_matrix((ke.ravel(), (np.repeat(dof, 6, axis=1).ravel(), np.tile(dof, (1, 6)).ravel())),
+                      shape=(m.num_dofs, m.num_dofs)).tocsr()
+    a.sort_indices()
+    return a.indptr.astype(np.int32), a.indices.astype(np.int32), a.data
+
+
+@pytest.mark.parametrize("cols", [65535, 65536, 65537, 70001])
+def test_rows_past_16_bit_ranks(fem, cuda_device, cols):
+    # a closed fan: its hub's row has a column per triangle and its own
+    import meshgen as mg
+    k = cols - 1
+    ang = np.linspace(0, 2 * np.pi, k, endpoint=False)
+    conn = np.stack([np.full(k, k // 2), np.arange(k), (np.arange(k) + 1) % k], 1)
+    conn[:, 1:] += conn[:, 1:] >= k // 2  # the hub's id in the middle
+    xy = np.insert(np.stack([np.cos(ang), np.sin(ang)], 1), k // 2, 0.0, axis=0)
+    conn = np.random.default_rng(1).permutation(conn).astype(np.int32)
+    m = mg.Mesh(mg.T3, xy[:, 0].copy(), xy[:, 1].copy(), None, np.ascontiguousarray(conn), None, None, None, E0=1.0, nu0=0.3)
+    rp, ci, v = _t3_stiffness(m)
+    assert np.diff(rp).max() == 2 * cols
+    asm = fem.Assembler(m)
+    vals = _with_pattern(asm, rp, ci)
+    re = _build(fem, asm, ci.size, 0)
+    re.reassemble(vals)
+    assert re.read_info() == 0
+    # the hub's entries are sums of up to 70,001 terms: 1e-10 of its diagonal covers their order
+    scale = np.maximum(np.abs(v), diag_scale(rp, ci, v))
+    assert np.all(np.abs(vals.cpu().numpy() - v) <= 1e-10 * scale)
