@@ -840,20 +840,20 @@ fem_status fem_reassemble_values(const fem_mesh* mesh, const fem_opts* opts, con
     const int* pos = reinterpret_cast<const int*>(b + h.off_pos);
     const int* perm = reinterpret_cast<const int*>(b + h.off_perm);
     const int* ranges = reinterpret_cast<const int*>(b + h.off_ranges);
-    cudaError_t err = cudaMemsetAsync(info, 0, sizeof(DevInfo), s);
-    if (!err && nnz > 0 && !h.rows) err = cudaMemsetAsync(values, 0, (size_t)nnz * sizeof(double), s);
+    const MeshView m = mesh_view(mesh);
+    const BlocksMap blocks{pos, h.G, perm, ranges};
+    cudaError_t err = cudaSuccess;
+    if (h.rows) {
+        err = launch_rows_values_2d(m, mesh->kind, precision, rows_map(h, b), blocks, row_ptr, values, nnz, info, s);
+        return err ? cuda_fail(err) : FEM_OK;
+    }
+    err = cudaMemsetAsync(info, 0, sizeof(DevInfo), s);
+    if (!err && nnz > 0) err = cudaMemsetAsync(values, 0, (size_t)nnz * sizeof(double), s);
     if (!err && mesh->num_elems > 0) {
-        const MeshView m = mesh_view(mesh);
-        if (h.rows) {
-            const RowsMap r = rows_map(h, b);
-            err = launch_rows_values_2d(m, mesh->kind, precision, r, row_ptr, values, nnz, &info->status_bits, s);
-            if (!err)
-                err = launch_reassemble_2d(m, precision, pos, h.G, perm, ranges, row_ptr, values, &info->status_bits, s,
-                                           r.blocks);
-        } else if (mesh->kind == FEM_HEX20)
+        if (mesh->kind == FEM_HEX20)
             err = launch_reassemble_hex20(m, precision, perm, MapTarget{pos, row_ptr, values, nullptr}, info, s);
         else
-            err = launch_reassemble_2d(m, precision, pos, h.G, perm, ranges, row_ptr, values, &info->status_bits, s);
+            err = launch_reassemble_2d(m, precision, blocks, row_ptr, values, &info->status_bits, s);
     }
     return err ? cuda_fail(err) : FEM_OK;
 }

@@ -96,9 +96,14 @@ cudaError_t launch_build_map(const MeshView& m, int kind, const int* row_ptr, co
                              int* status, cudaStream_t s, const int* gate = nullptr);
 // Value-only re-assembly (atomics into values): 2-D kinds over perm ranges
 // {q4 begin, q4 end, t3 begin, t3 end}; Hex20 over perm (status bits in info).
-cudaError_t launch_reassemble_2d(const MeshView& m, int precision, const int* map, int G, const int* perm,
-                                 const int* ranges, const int* row_ptr, double* values, int* status, cudaStream_t s,
-                                 const int* gate = nullptr);
+struct BlocksMap {
+    const int* pos;     // [E * G] positions, -1: no block
+    int G;              // npe^2
+    const int* perm;    // element order
+    const int* ranges;
+};
+cudaError_t launch_reassemble_2d(const MeshView& m, int precision, const BlocksMap& b, const int* row_ptr,
+                                 double* values, int* status, cudaStream_t s);
 // The same by row nodes (2-D): each node's occurrences (element << 2 | position) and the ranks of their nodes in its row.
 struct RowsMap {
     int* off;               // [N + 1]
@@ -110,9 +115,9 @@ struct RowsMap {
 // node blocks that holds all of the mesh's, with rows of at most 65,536 columns.
 cudaError_t launch_build_rows_map(const MeshView& m, int kind, const int* row_ptr, const int* col_idx, const RowsMap& r,
                                   int* cnt, long long* tiles, DevInfo* info, cudaStream_t s);
-// values[0, nnz): the rows and zeros behind them; all zeros where *r.blocks is set.
-cudaError_t launch_rows_values_2d(const MeshView& m, int kind, int precision, const RowsMap& r, const int* row_ptr,
-                                  double* values, long long nnz, int* status, cudaStream_t s);
+// Clears the info word; values[0, nnz): the rows and zeros behind them; by the block positions b where *r.blocks is set.
+cudaError_t launch_rows_values_2d(const MeshView& m, int kind, int precision, const RowsMap& r, const BlocksMap& b,
+                                  const int* row_ptr, double* values, long long nnz, DevInfo* info, cudaStream_t s);
 // The tensor-core form of the Hex20 value-only re-assembly (ke_tcgen05.cu).
 cudaError_t launch_reassemble_hex20_tc(const MeshView& m, const int* perm, const MapTarget& t, DevInfo* info,
                                        cudaStream_t s);

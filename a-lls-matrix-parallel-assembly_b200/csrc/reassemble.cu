@@ -94,12 +94,9 @@ __global__ void k_build_map(MeshView m, int dpn, int npe_max, const int* __restr
 // 2-D value-only assembly: one lane per element block (NPE^2 lanes per
 // element), elements perm[range[0], range[1]), FP64 red.add into the values.
 template <int NPE, typename T>
-__global__ void __launch_bounds__(kThreads) k_reassemble_2d(MeshView m, const int* __restrict__ map, int G,
-                                                            const int* __restrict__ perm, const int* __restrict__ range,
-                                                            const int* __restrict__ row_ptr,
-                                                            double* __restrict__ values, int* __restrict__ status,
-                                                            const int* gate) {
-    if (gate && __ldcg(gate) == 0) return;
+__device__ __forceinline__ void add_blocks_2d(const MeshView& m, const BlocksMap& b2, const int* __restrict__ range,
+                                              const int* __restrict__ row_ptr, double* __restrict__ values,
+                                              int* __restrict__ status) {
     constexpr int GL = NPE * NPE, EPW = 32 / GL;
     const int lane = threadIdx.x & 31;
     const int eslot = lane / GL, sub = lane - eslot * GL, a = sub / NPE, b = sub - (sub / NPE) * NPE;
@@ -108,8 +105,8 @@ __global__ void __launch_bounds__(kThreads) k_reassemble_2d(MeshView m, const in
     const long long stride = (((long long)gridDim.x * blockDim.x) >> 5) * EPW;
     for (long long i = warp_id * EPW + eslot; i - eslot < count; i += stride) {
         if (eslot >= EPW || i >= count) continue;
-        const int e = __ldg(perm + begin + i);
-        const int p = __ldg(map + (size_t)e * G + a * (G == 16 ? 4 : NPE) + b);
+        const int e = __ldg(b2.perm + begin + i);
+        const int p = __ldg(b2.pos + (size_t)e * b2.G + a * (b2.G == 16 ? 4 : NPE) + b);
         if (p < 0) continue;  // bad node (reported when the map was built)
         int nodes[NPE];
 #pragma unroll
@@ -134,6 +131,13 @@ __global__ void __launch_bounds__(kThreads) k_reassemble_2d(MeshView m, const in
         atomicAdd(values + p + len, kv[2]);
         atomicAdd(values + p + len + 1, kv[3]);
     }
+}
+
+template <int NPE, typename T>
+__global__ void __launch_bounds__(kThreads) k_reassemble_2d(MeshView m, BlocksMap b2, const int* __restrict__ range,
+                                                            const int* __restrict__ row_ptr,
+                                                            double* __restrict__ values, int* __restrict__ status) {
+    add_blocks_2d<NPE, T>(m, b2, range, row_ptr, values, status);
 }
 
 // ---- 2-D rows ---------------------------------------------------------------------
@@ -296,22 +300,33 @@ __device__ __forceinline__ double occ_blocks(const OccData<NPE>& d, double t, do
     }
 }
 
+// Clears the call's info word and the entries that no row of the mesh covers: those behind the rows or, for a pattern
+// that is not in the form of rows, all of them.
+__global__ void __launch_bounds__(kThreads) k_rows_begin_2d(DevInfo* info, const int* __restrict__ blocks,
+                                                            const int* __restrict__ end, double* __restrict__ values,
+                                                            long long nnz) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) *info = DevInfo{};
+    const long long first = __ldg(end), all = __ldg(blocks);
+    for (long long i = (all ? 0 : first) + (long long)blockIdx.x * kThreads + threadIdx.x; i < nnz;
+         i += (long long)gridDim.x * kThreads)
+        values[i] = 0.0;
+}
+
 template <int KIND, typename T>
 __global__ void __launch_bounds__(kRowThreads, RowsShape<KIND>::kCtas)
     k_rows_values_2d(MeshView m, const int* __restrict__ off, const unsigned* __restrict__ occ,
                      const unsigned short* __restrict__ ranks, const int* __restrict__ row_ptr,
-                     double* __restrict__ values, long long nnz, bool wide, int* __restrict__ status,
-                     const int* __restrict__ blocks) {
+                     double* __restrict__ values, bool wide, int* __restrict__ status,
+                     const int* __restrict__ blocks, BlocksMap b2) {
     constexpr int NPE = KIND == FEM_T3 ? 3 : 4, kRowCols = RowsShape<KIND>::kCols;
     constexpr unsigned kFull = 0xFFFFFFFFu;
     __shared__ double acc[kRowCols][4][kRowPad];
     const int tid = threadIdx.x, lane = tid & 31, warp0 = tid & ~31;
-    // entries that no row of the mesh covers: behind the rows, or, for a pattern that is not in this form, all of them
-    const bool other = __ldg(blocks) != 0;
-    for (long long i = (other ? 0 : __ldg(row_ptr + 2 * (size_t)m.N)) + (long long)blockIdx.x * kRowThreads + tid; i < nnz;
-         i += (long long)gridDim.x * kRowThreads)
-        values[i] = 0.0;
-    if (other) return;  // k_reassemble_2d adds the blocks
+    if (__ldg(blocks)) {  // the pattern is not in this form; the values are zero (k_rows_begin_2d)
+        if constexpr (KIND != FEM_T3) add_blocks_2d<4, T>(m, b2, b2.ranges, row_ptr, values, status);
+        if constexpr (KIND != FEM_Q4) add_blocks_2d<3, T>(m, b2, b2.ranges + 2, row_ptr, values, status);
+        return;
+    }
     for (long long tile = blockIdx.x; tile * kRowThreads < m.N; tile += gridDim.x) {
         const long long n = tile * kRowThreads + tid;
         int base = 0, u = 0, lo = 0, d = 0;
@@ -448,7 +463,7 @@ cudaError_t build_rows_map(const MeshView& m, const int* row_ptr, const int* col
 }
 
 template <int KIND, typename T>
-cudaError_t rows_values(const MeshView& m, const RowsMap& r, const int* row_ptr, double* values, long long nnz,
+cudaError_t rows_values(const MeshView& m, const RowsMap& r, const BlocksMap& b2, const int* row_ptr, double* values,
                         int* status, cudaStream_t s) {
     static DeviceCache cache;
     int per_sm = 0;
@@ -458,16 +473,16 @@ cudaError_t rows_values(const MeshView& m, const RowsMap& r, const int* row_ptr,
     if (err) return err;
     const long long tiles = ((long long)m.N + kRowThreads - 1) / kRowThreads;
     k_rows_values_2d<KIND, T><<<(int)std::min<long long>(tiles, (long long)per_sm * sm_count()), kRowThreads, 0, s>>>(
-        m, r.off, r.occ, r.ranks, row_ptr, values, nnz, reinterpret_cast<uintptr_t>(values) % 16 == 0, status, r.blocks);
+        m, r.off, r.occ, r.ranks, row_ptr, values, reinterpret_cast<uintptr_t>(values) % 16 == 0, status, r.blocks, b2);
     return cudaGetLastError();
 }
 
 template <typename T>
-cudaError_t rows_values_kind(const MeshView& m, int kind, const RowsMap& r, const int* row_ptr, double* values,
-                             long long nnz, int* status, cudaStream_t s) {
-    if (kind == FEM_T3) return rows_values<FEM_T3, T>(m, r, row_ptr, values, nnz, status, s);
-    if (kind == FEM_Q4) return rows_values<FEM_Q4, T>(m, r, row_ptr, values, nnz, status, s);
-    return rows_values<FEM_MIXED_2D, T>(m, r, row_ptr, values, nnz, status, s);
+cudaError_t rows_values_kind(const MeshView& m, int kind, const RowsMap& r, const BlocksMap& b2, const int* row_ptr,
+                             double* values, int* status, cudaStream_t s) {
+    if (kind == FEM_T3) return rows_values<FEM_T3, T>(m, r, b2, row_ptr, values, status, s);
+    if (kind == FEM_Q4) return rows_values<FEM_Q4, T>(m, r, b2, row_ptr, values, status, s);
+    return rows_values<FEM_MIXED_2D, T>(m, r, b2, row_ptr, values, status, s);
 }
 
 }  // namespace
@@ -484,26 +499,23 @@ cudaError_t launch_build_map(const MeshView& m, int kind, const int* row_ptr, co
 }
 
 template <typename T>
-void reassemble_2d_t(const MeshView& m, const int* map, int G, const int* perm, const int* ranges, const int* row_ptr,
-                     double* values, int* status, cudaStream_t s, const int* gate) {
+void reassemble_2d_t(const MeshView& m, const BlocksMap& b2, const int* row_ptr, double* values, int* status,
+                     cudaStream_t s) {
     const bool has_q4 = m.types || m.stride == 4, has_t3 = m.types || m.stride == 3;
     const long long warps = ((long long)m.E_count + 1) / 2;
     const int grid = (int)std::min<long long>((warps * 32 + kThreads - 1) / kThreads, (long long)sm_count() * 8);
     if (has_q4)
-        k_reassemble_2d<4, T><<<grid > 0 ? grid : 1, kThreads, 0, s>>>(m, map, G, perm, ranges + 0, row_ptr, values,
-                                                                      status, gate);
+        k_reassemble_2d<4, T><<<grid > 0 ? grid : 1, kThreads, 0, s>>>(m, b2, b2.ranges, row_ptr, values, status);
     if (has_t3)
-        k_reassemble_2d<3, T><<<grid > 0 ? grid : 1, kThreads, 0, s>>>(m, map, G, perm, ranges + 2, row_ptr, values,
-                                                                      status, gate);
+        k_reassemble_2d<3, T><<<grid > 0 ? grid : 1, kThreads, 0, s>>>(m, b2, b2.ranges + 2, row_ptr, values, status);
 }
 
-cudaError_t launch_reassemble_2d(const MeshView& m, int precision, const int* map, int G, const int* perm,
-                                 const int* ranges, const int* row_ptr, double* values, int* status, cudaStream_t s,
-                                 const int* gate) {
+cudaError_t launch_reassemble_2d(const MeshView& m, int precision, const BlocksMap& b2, const int* row_ptr,
+                                 double* values, int* status, cudaStream_t s) {
     if (precision == FEM_PREC_FP32)
-        reassemble_2d_t<float>(m, map, G, perm, ranges, row_ptr, values, status, s, gate);
+        reassemble_2d_t<float>(m, b2, row_ptr, values, status, s);
     else
-        reassemble_2d_t<double>(m, map, G, perm, ranges, row_ptr, values, status, s, gate);
+        reassemble_2d_t<double>(m, b2, row_ptr, values, status, s);
     return cudaGetLastError();
 }
 
@@ -514,10 +526,13 @@ cudaError_t launch_build_rows_map(const MeshView& m, int kind, const int* row_pt
     return build_rows_map<FEM_MIXED_2D>(m, row_ptr, col_idx, r, cnt, tiles, info, s);
 }
 
-cudaError_t launch_rows_values_2d(const MeshView& m, int kind, int precision, const RowsMap& r, const int* row_ptr,
-                                  double* values, long long nnz, int* status, cudaStream_t s) {
-    return precision == FEM_PREC_FP32 ? rows_values_kind<float>(m, kind, r, row_ptr, values, nnz, status, s)
-                                      : rows_values_kind<double>(m, kind, r, row_ptr, values, nnz, status, s);
+cudaError_t launch_rows_values_2d(const MeshView& m, int kind, int precision, const RowsMap& r, const BlocksMap& b2,
+                                  const int* row_ptr, double* values, long long nnz, DevInfo* info, cudaStream_t s) {
+    const int grid = (int)std::min<long long>((nnz + 4 * kThreads - 1) / (4 * kThreads) + 1, 2ll * sm_count());
+    k_rows_begin_2d<<<grid, kThreads, 0, s>>>(info, r.blocks, row_ptr + 2 * (size_t)m.N, values, nnz);
+    int* status = &info->status_bits;
+    return precision == FEM_PREC_FP32 ? rows_values_kind<float>(m, kind, r, b2, row_ptr, values, status, s)
+                                      : rows_values_kind<double>(m, kind, r, b2, row_ptr, values, status, s);
 }
 
 }  // namespace fem
