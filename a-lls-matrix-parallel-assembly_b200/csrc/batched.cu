@@ -92,7 +92,7 @@ FEM_BATCH_KERNEL(kScanThreads) kb_occ_sums(const __grid_constant__ BatchRound<kM
 FEM_BATCH_KERNEL(kScanThreads) kb_occ_offsets(const __grid_constant__ BatchRound<kMax> r) {
     FEM_BATCH_MESH;
     __shared__ OccSmem sm;
-    occ_offsets(bm.cnt, bm.L.N, bm.tiles, bm.h.off, bm.L.info, block, nblocks, sm);
+    occ_offsets(bm.cnt, bm.L.N, bm.tiles, bm.h.off, block, nblocks, sm);
 }
 
 FEM_BATCH_KERNEL(kOccThreads) kb_occ_fill(const __grid_constant__ BatchRound<kMax> r) {
@@ -125,10 +125,14 @@ FEM_BATCH_KERNEL(kHexRowThreads, FEM_HEXR_CTAS) kb_rows_hex20(const __grid_const
 
 FEM_BATCH_KERNEL(kHexRowThreads) kb_long_rows_hex20(const __grid_constant__ BatchRound<kMax> r) {
     FEM_BATCH_MESH;
-    __shared__ int s_uniq[kHexRowWarps][kWideElems * 20];
+    __shared__ union {
+        int uniq[kHexRowWarps][kWideElems * 20];
+        LongHexSmem longs;
+    } sm;
     const int warp = threadIdx.x >> 5;
-    wide_rows_hex20(bm.m.conn, bm.L, bm.h, bm.queue, block * kHexRowWarps + warp, nblocks * kHexRowWarps, s_uniq[warp]);
-    long_rows_hex20(bm.m.conn, bm.L, bm.h, bm.queue, block, nblocks);
+    wide_rows_hex20(bm.m.conn, bm.L, bm.h, bm.queue, block * kHexRowWarps + warp, nblocks * kHexRowWarps, sm.uniq[warp]);
+    __syncthreads();
+    long_rows_hex20(bm.m.conn, bm.L, bm.h, bm.queue, block, nblocks, sm.longs);
 }
 
 FEM_BATCH_KERNEL(kKeThreads, 1) kb_ke_hex20(const __grid_constant__ BatchRound<kMax> r) {

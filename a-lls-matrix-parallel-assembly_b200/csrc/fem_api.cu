@@ -70,6 +70,7 @@ fem_status make_layout(const fem_mesh* m, const fem_opts* o, HostLayout& h) {
     h.B = h.dpn * h.dpn;
     h.N = m->num_nodes;
     h.E = m->num_elems;
+    if (h.kind == FEM_HEX20 && h.E > 0x7FFFFFFF / 20) return FEM_ERR_RANGE;  // occurrences are numbered 20 e + a
     if (h.dpn == 2) {
         // 2-D chunk rows are fixed at 16 words (the scatter reads them as 4 x 16 bytes).
         if ((o->first_slots && o->first_slots != k2DSlots) || (o->chunk_slots && o->chunk_slots != k2DSlots))
@@ -149,11 +150,12 @@ ListLayout device_layout(const HostLayout& h, void* ws) {
 // smaller ones (46 MB) stays in L2 whatever the order.
 constexpr int kOrderedElems = 3072;
 
-HexRows hex_rows(const HostLayout& h, void* ws) {
+HexRows hex_rows(const fem_mesh* mesh, const HostLayout& h, void* ws) {
     unsigned char* b = static_cast<unsigned char*>(ws);
     HexRows r{};
     if (h.kind != FEM_HEX20) return r;
     const size_t n = align_up((size_t)(h.N + 1) * sizeof(int));
+    r.conn = mesh->conn;
     r.ke = reinterpret_cast<double*>(b + h.off_vals);
     r.off = reinterpret_cast<int*>(b + h.off_inc + n);
     r.inc = reinterpret_cast<int*>(b + h.off_inc + 2 * n);
@@ -268,7 +270,7 @@ fem_status fem_alls_scatter(const fem_mesh* mesh, const fem_opts* opts, void* wo
         err = launch_rows_2d(m, L, queue, h.kind, precision, ctas, s);
         return err ? cuda_fail(err) : FEM_OK;
     }
-    const HexRows hex = hex_rows(h, workspace);
+    const HexRows hex = hex_rows(mesh, h, workspace);
     int* cnt = reinterpret_cast<int*>(b + h.off_inc);
     long long* tiles = reinterpret_cast<long long*>(b + h.off_tiles);  // free until the consolidation
     err = launch_rows_hex20(m, L, hex, cnt, tiles, queue, s);
@@ -294,7 +296,7 @@ fem_status fem_alls_consolidate(const fem_mesh* mesh, const fem_opts* opts, void
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     ListLayout L = device_layout(h, workspace);
     long long* tiles = reinterpret_cast<long long*>(static_cast<unsigned char*>(workspace) + h.off_tiles);
-    cudaError_t err = launch_consolidate(L, h.dpn, hex_rows(h, workspace), row_ptr, col_idx, values, capacity, tiles, s);
+    cudaError_t err = launch_consolidate(L, h.dpn, hex_rows(mesh, h, workspace), row_ptr, col_idx, values, capacity, tiles, s);
     return err ? cuda_fail(err) : FEM_OK;
 }
 
@@ -310,7 +312,7 @@ fem_status fem_alls_consolidate_bsr(const fem_mesh* mesh, const fem_opts* opts, 
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     ListLayout L = device_layout(h, workspace);
     long long* tiles = reinterpret_cast<long long*>(static_cast<unsigned char*>(workspace) + h.off_tiles);
-    cudaError_t err = launch_consolidate_bsr(L, h.dpn, hex_rows(h, workspace), block_row_ptr, block_col_idx, block_values, capacity_blocks,
+    cudaError_t err = launch_consolidate_bsr(L, h.dpn, hex_rows(mesh, h, workspace), block_row_ptr, block_col_idx, block_values, capacity_blocks,
                                              tiles, s);
     return err ? cuda_fail(err) : FEM_OK;
 }
@@ -329,7 +331,7 @@ fem_status fem_alls_consolidate_upper(const fem_mesh* mesh, const fem_opts* opts
     long long* tiles = reinterpret_cast<long long*>(b + h.off_tiles);
     int* ucounts = reinterpret_cast<int*>(b + h.off_ucounts);
     cudaError_t err =
-        launch_consolidate_upper(L, h.dpn, hex_rows(h, workspace), ucounts, row_ptr, col_idx, values, capacity, tiles, s);
+        launch_consolidate_upper(L, h.dpn, hex_rows(mesh, h, workspace), ucounts, row_ptr, col_idx, values, capacity, tiles, s);
     return err ? cuda_fail(err) : FEM_OK;
 }
 
@@ -515,7 +517,7 @@ fem_status fem_assemble_batched(const fem_mesh* meshes, int32_t n, const fem_opt
         bm = BatchMesh{};
         bm.m = mesh_view(&meshes[i]);
         bm.L = device_layout(h, ws);
-        bm.h = hex_rows(h, ws);
+        bm.h = hex_rows(&meshes[i], h, ws);
         bm.cnt = reinterpret_cast<int*>(ws + h.off_inc);
         bm.queue = reinterpret_cast<int*>(ws + h.off_ucounts);
         bm.tiles = reinterpret_cast<long long*>(ws + h.off_tiles);

@@ -6,7 +6,8 @@
 // the consolidation sums each row's element blocks where it writes them. An
 // element's block (a, b) meets its row through two tables: the node's
 // occurrences (node -> element e and local position a, as o = 20 e + a) and
-// the rank of column node b in row node a's sorted list, map[20 o + b].
+// the rank of column node b in row node a's sorted list, map[20 o + b] (its low
+// 16 bits: in a row of more than 65,536 columns the gather compares the columns).
 #pragma once
 
 #include "launch.h"
@@ -14,7 +15,7 @@
 namespace fem {
 namespace {
 
-constexpr int kMaxRank = 0xFFFF;  // columns of a row that the rank map can number
+constexpr int kRankRange = 0x10000;  // columns of a row that the rank map tells apart
 
 __device__ __forceinline__ unsigned occ_of(int word) { return (unsigned)word & ~kOccRepeats; }
 

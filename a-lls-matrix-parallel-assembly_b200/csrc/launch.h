@@ -142,6 +142,7 @@ struct HexRows {
     int* inc;             // occurrences 20 e + a (bit 31: kOccRepeats)
     const int* order;     // [N] node visit order of the consolidation, or NULL: as numbered
     unsigned short* map;  // [E * 400] rank of column node b in row node a's list, at 20 (20 e + a) + b
+    const int* conn;      // the mesh's connectivity (rows longer than a rank of the map)
 };
 // The info word, the occurrences (off / inc, of the elements without a bad node id), the sorted row lists and the
 // rank map; cnt, queue: N ints, tiles: row_tiles(N) partials of scratch.

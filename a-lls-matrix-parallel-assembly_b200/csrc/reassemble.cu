@@ -179,9 +179,9 @@ __global__ void __launch_bounds__(kScanThreads) k_map_sums(const int* __restrict
 
 __global__ void __launch_bounds__(kScanThreads) k_map_offsets(const int* __restrict__ cnt, int N,
                                                               const long long* __restrict__ tiles,
-                                                              int* __restrict__ off, DevInfo* info) {
+                                                              int* __restrict__ off) {
     __shared__ OccSmem sm;
-    occ_offsets(cnt, N, tiles, off, info, blockIdx.x, gridDim.x, sm);
+    occ_offsets(cnt, N, tiles, off, blockIdx.x, gridDim.x, sm);
 }
 
 // The occurrences of every node (cnt counts down to zero).
@@ -455,7 +455,7 @@ cudaError_t build_rows_map(const MeshView& m, const int* row_ptr, const int* col
     int* status = &info->status_bits;
     k_map_count<KIND><<<grid, kThreads, 0, s>>>(m, cnt, status);
     k_map_sums<<<ntiles, kScanThreads, 0, s>>>(cnt, m.N, tiles);
-    k_map_offsets<<<ntiles, kScanThreads, 0, s>>>(cnt, m.N, tiles, r.off, info);
+    k_map_offsets<<<ntiles, kScanThreads, 0, s>>>(cnt, m.N, tiles, r.off);
     k_map_fill<KIND><<<grid, kThreads, 0, s>>>(m, r.off, cnt, r.occ);
     k_map_ranks<KIND><<<(int)std::min<long long>(3ll * grid, (long long)sm_count() * 16), kThreads, 0, s>>>(
         m, r.off, r.occ, row_ptr, col_idx, r.ranks, r.blocks);

@@ -20,9 +20,9 @@ __global__ void __launch_bounds__(kScanThreads) k_occ_sums(const int* __restrict
 
 __global__ void __launch_bounds__(kScanThreads) k_occ_offsets(const int* __restrict__ cnt, int N,
                                                               const long long* __restrict__ tiles,
-                                                              int* __restrict__ off, DevInfo* info) {
+                                                              int* __restrict__ off) {
     __shared__ OccSmem sm;
-    occ_offsets(cnt, N, tiles, off, info, blockIdx.x, gridDim.x, sm);
+    occ_offsets(cnt, N, tiles, off, blockIdx.x, gridDim.x, sm);
 }
 
 __global__ void __launch_bounds__(kOccThreads) k_occ_fill(MeshView m, HexRows h) {
@@ -38,10 +38,14 @@ __global__ void __launch_bounds__(kHexRowThreads, FEM_HEXR_CTAS)
 // Nodes with more than 8 elements: a warp each, or a CTA.
 __global__ void __launch_bounds__(kHexRowThreads) k_long_rows_hex20(const int* __restrict__ conn, ListLayout L,
                                                                     HexRows h, const int* __restrict__ queue) {
-    __shared__ int s_uniq[kHexRowWarps][kWideElems * 20];
+    __shared__ union {
+        int uniq[kHexRowWarps][kWideElems * 20];
+        LongHexSmem longs;
+    } sm;
     const int warp = threadIdx.x >> 5;
-    wide_rows_hex20(conn, L, h, queue, blockIdx.x * kHexRowWarps + warp, gridDim.x * kHexRowWarps, s_uniq[warp]);
-    long_rows_hex20(conn, L, h, queue, blockIdx.x, gridDim.x);
+    wide_rows_hex20(conn, L, h, queue, blockIdx.x * kHexRowWarps + warp, gridDim.x * kHexRowWarps, sm.uniq[warp]);
+    __syncthreads();
+    long_rows_hex20(conn, L, h, queue, blockIdx.x, gridDim.x, sm.longs);
 }
 
 __global__ void __launch_bounds__(256) k_begin_hex20(ListLayout L, int* __restrict__ cnt) {
@@ -58,6 +62,7 @@ __global__ void __launch_bounds__(kHexRowThreads, FEM_HEXR_CTAS)
         HexRowSmem rows[kHexRowWarps];
         OccSmem occ;
         int uniq[kHexRowWarps][kWideElems * 20];
+        LongHexSmem longs;
         __device__ Smem() {}
     } sm;
     const cooperative_groups::grid_group grid = cooperative_groups::this_grid();
@@ -66,14 +71,15 @@ __global__ void __launch_bounds__(kHexRowThreads, FEM_HEXR_CTAS)
     grid.sync();
     occ_count(m, h, cnt, L.info, block, nblocks);
     grid.sync();
-    for (int t = block; t < tiles; t += nblocks) occ_offsets(cnt, L.N, nullptr, h.off, L.info, t, tiles, sm.occ);
+    for (int t = block; t < tiles; t += nblocks) occ_offsets(cnt, L.N, nullptr, h.off, t, tiles, sm.occ);
     grid.sync();
     occ_fill(m, h, block, nblocks);
     grid.sync();
     rows_hex20(m.conn, L, h, queue, block, nblocks, sm.rows);
     grid.sync();
     wide_rows_hex20(m.conn, L, h, queue, block * kHexRowWarps + warp, nblocks * kHexRowWarps, sm.uniq[warp]);
-    long_rows_hex20(m.conn, L, h, queue, block, nblocks);
+    __syncthreads();
+    long_rows_hex20(m.conn, L, h, queue, block, nblocks, sm.longs);
 }
 
 }  // namespace
@@ -112,7 +118,7 @@ cudaError_t launch_rows_hex20(const MeshView& m, const ListLayout& L, const HexR
     k_begin_hex20<<<blocks(m.N, 1024, 4), 256, 0, s>>>(L, cnt);
     if (m.E_count > 0) k_occ_count<<<blocks(m.E_count, kOccThreads, 8), kOccThreads, 0, s>>>(m, h, cnt, L.info);
     k_occ_sums<<<ntiles, kScanThreads, 0, s>>>(cnt, m.N, tiles);
-    k_occ_offsets<<<ntiles, kScanThreads, 0, s>>>(cnt, m.N, tiles, h.off, L.info);
+    k_occ_offsets<<<ntiles, kScanThreads, 0, s>>>(cnt, m.N, tiles, h.off);
     if (m.E_count > 0) k_occ_fill<<<blocks(20ll * m.E_count, kOccThreads, 16), kOccThreads, 0, s>>>(m, h);
     k_rows_hex20<<<blocks(m.N, kHexRowWarps, per_sm), kHexRowThreads, 0, s>>>(m.conn, L, h, queue);
     k_long_rows_hex20<<<blocks(m.N, kHexRowWarps, 1), kHexRowThreads, 0, s>>>(m.conn, L, h, queue);

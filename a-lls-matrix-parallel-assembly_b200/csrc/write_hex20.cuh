@@ -173,7 +173,12 @@ __device__ __forceinline__ void write_hex20(const ListLayout& L, const HexRows& 
             __syncwarp();
             for (int t = 0; t < d; t++) {
                 // where column node `lane`'s block goes: its rank in the window, or the bin
-                int to = lane < 20 && rk - (unsigned)w0 < (unsigned)uw ? (int)(rk - (unsigned)w0) * 9 : kBin;
+                const int place = (int)((rk - (unsigned)w0) & (kRankRange - 1));
+                int to = lane < 20 && place < uw ? place * 9 : kBin;
+                if (u > kRankRange && to != kBin &&  // the rank is known up to a multiple of kRankRange only
+                    __ldg(hex_col_word(L, n, next, w0 + place)) - 1 !=
+                        __ldg(h.conn + (size_t)(occ_of(word) / 20) * 20 + lane))
+                    to = kBin;
                 unsigned later = 0;  // column nodes that the element has at an earlier position too
                 const int again = to;
                 if (word < 0) {
