@@ -143,6 +143,9 @@ ListLayout device_layout(const HostLayout& h, void* ws) {
     L.vals = reinterpret_cast<double*>(b + h.off_vals);
     L.counts = reinterpret_cast<int*>(b + h.off_counts);
     L.info = reinterpret_cast<DevInfo*>(b + h.off_info);
+    // 2-D: an int per element in the place of the element order, which the 2-D scatter does not need
+    L.spill = reinterpret_cast<unsigned*>(b + h.off_elist);
+    L.spill_cap = h.dpn == 2 && h.E < (1 << 29) ? h.E : 0;  // 4 element + position, and 4 E entries, fit 32 bits
     return L;
 }
 

@@ -43,7 +43,9 @@ struct DevInfo {
     int max_row_entries;
     int long_rows;         // rows queued for the long-row kernels
     int ticket;            // consolidation: next row node to write
-    long long pad1[3];
+    int spilled;           // 2-D: entries of the spill list (may overshoot its capacity)
+    int pad0;
+    long long pad1[2];
 };
 static_assert(sizeof(DevInfo) == 64, "DevInfo size");
 static_assert(offsetof(DevInfo, max_row_entries) == offsetof(fem_info, max_row_entries), "fem_info layout");
@@ -58,6 +60,8 @@ struct ListLayout {
     int* meta2;     // [cap2 * H2]
     double* vals;   // 2-D: [(N*S1 + cap2*S2) * B]
     int* counts;    // [N] list entries of each row node (2-D: elements of the node until its row is built)
+    unsigned* spill;  // 2-D: [spill_cap] elements past those that a node's own list storage keeps (4 element + position)
+    int spill_cap;    // 0: none
     DevInfo* info;
 };
 
@@ -110,20 +114,14 @@ __device__ __forceinline__ int probe_start(int key, int S) {
     return (int)__umulhi((unsigned)key * 2654435761u, (unsigned)S);
 }
 
-// Appends a chunk to the end of row node n's chain (one thread). Returns false
-// on pool overflow (status raised).
-__device__ __forceinline__ bool append_chunk(const ListLayout& L, int n) {
-    int c = n;
-    for (int step = 0; step < kMaxChainSteps; step++) {
-        const int nx = ld_cg(chunk_meta(L, c) + 1);
-        if (nx == 0) break;
-        c = nx - 1;
-    }
-    const int nc = alloc_chunk(L);
-    if (nc < 0) return false;
+// Appends a chunk to a row's chain, whose last chunk is `tail` (one thread). Returns its id, or -1 on pool overflow
+// (status raised).
+__device__ __forceinline__ int append_chunk(const ListLayout& L, int tail) {
+    const int c = alloc_chunk(L);
+    if (c < 0) return -1;
     __threadfence();  // the zeroed meta row is visible before the link
-    atomicExch(chunk_meta(L, c) + 1, nc + 1);
-    return true;
+    atomicExch(chunk_meta(L, tail) + 1, c + 1);
+    return c;
 }
 
 // Host-side layout description (sizes in bytes, offsets from the workspace base).

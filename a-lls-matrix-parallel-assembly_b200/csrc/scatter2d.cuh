@@ -27,22 +27,17 @@ __device__ __forceinline__ unsigned rot14(unsigned m, int h) {
 }
 
 // Finds or claims the slot of column key `key` in the row list of node `row`.
-// Returns the slot state (kFound, kClaimed, or kSkip on pool overflow); gid is
-// the slot's global id.
-// view: the row's first chunk, loaded by the caller (possibly some time ago:
-// a stale view only costs failed CASes, never a wrong slot).
-// A column that needs a further chunk is left kUnresolved.
-__device__ __forceinline__ int resolve_2d(const ListLayout& L, int row, int key, const int4 (&view)[4], unsigned& gid) {
-    int c = row;
+// Returns the slot state (kFound or kClaimed; kSkip: the chain has no end); gid is
+// the slot's global id. A column that needs a further chunk is left
+// kUnresolved, and `last` is then the chain's last chunk + 1 (0 before the first
+// call): the chunks up to it are full of other columns for good, so the next call
+// goes on behind it.
+__device__ __forceinline__ int resolve_2d(const ListLayout& L, int row, int key, int& last, unsigned& gid) {
+    int c = last ? ld_cg(chunk_meta(L, last - 1) + 1) - 1 : row;
+    if (c < 0) return kUnresolved;
     for (int step = 0; step < kMaxChainSteps; step++) {
         int* meta = chunk_meta(L, c);
-        int4 w0 = view[0], w1 = view[1], w2 = view[2], w3 = view[3];
-        if (step > 0) {
-            w0 = ld_cg4(meta);
-            w1 = ld_cg4(meta + 4);
-            w2 = ld_cg4(meta + 8);
-            w3 = ld_cg4(meta + 12);
-        }
+        const int4 w0 = ld_cg4(meta), w1 = ld_cg4(meta + 4), w2 = ld_cg4(meta + 8), w3 = ld_cg4(meta + 12);
         const int cols[k2DSlots] = {w0.z, w0.w, w1.x, w1.y, w1.z, w1.w, w2.x,
                                     w2.y, w2.z, w2.w, w3.x, w3.y, w3.z, w3.w};
         unsigned empty = 0, match = 0;
@@ -78,6 +73,7 @@ __device__ __forceinline__ int resolve_2d(const ListLayout& L, int row, int key,
             gid = slot_gid(L, c, pos);
             return state;
         }
+        last = c + 1;
         c = ld_cg(meta + 1) - 1;
         if (c < 0) return kUnresolved;
     }

@@ -89,3 +89,71 @@ def test_hex20_star_that_overflows_the_pool(fem, cuda_device, k):
 @pytest.mark.parametrize("k", [3449, 3450])
 def test_hex20_rows_past_16_bit_ranks(fem, oracle_mod, cuda_device, k):
     _check(fem, oracle_mod, _star(k), k, forms=False)
+
+
+def _quad_fan(k):
+    """k quadrilaterals around one node (2 k + 1 columns in its row), node ids shuffled."""
+    import meshgen as mg
+    ang = np.linspace(0, 2 * np.pi, 2 * k, endpoint=False)
+    r = np.where(np.arange(2 * k) % 2 == 0, 1.0, 1.0 / np.cos(np.pi / (2 * k)))  # the quads stay convex
+    x, y = np.concatenate([[0.0], r * np.cos(ang)]), np.concatenate([[0.0], r * np.sin(ang)])
+    i = np.arange(k)
+    conn = np.stack([np.zeros(k, int), 1 + 2 * i, 2 + 2 * i, 1 + (2 * i + 2) % (2 * k)], 1)
+    return _shuffled(mg.Mesh(mg.Q4, x, y, None, conn, None, None, None, E0=1.0, nu0=0.3))
+
+
+def _book(k):
+    """k triangles on one common edge: two hubs, the list of further elements (2 (k - 126) of them) longer than k from k = 253 on."""
+    import meshgen as mg
+    x = np.concatenate([[0.0, 1.0], np.linspace(0.1, 0.9, k)])
+    y = np.concatenate([[0.0, 0.0], 1.0 + 0.1 * np.sin(np.arange(k))])
+    conn = np.stack([np.zeros(k, int), np.ones(k, int), 2 + np.arange(k)], 1)
+    conn = np.stack([np.roll(c, s) for s, c in zip(np.arange(k) % 3, conn)])
+    return _shuffled(mg.Mesh(mg.T3, x, y, None, conn, None, None, None, E0=1.0, nu0=0.3))
+
+
+def _mixed_fan(k):
+    """A fan of k triangles whose every other element is a quadrilateral of two neighbouring rim edges."""
+    import meshgen as mg
+    m = _quad_fan(k)
+    m.kind = mg.MIXED_2D
+    m.types = np.where(np.arange(k) % 2 == 0, mg.Q4, mg.T3).astype(np.uint8)
+    return m
+
+
+def _shuffled(m):
+    rng = np.random.default_rng(m.num_elems)
+    p = rng.permutation(m.num_nodes)
+    inv = np.argsort(p)
+    m.x, m.y = m.x[inv], m.y[inv]
+    m.conn = np.ascontiguousarray(rng.permutation(p[m.conn]).astype(np.int32))
+    return m
+
+
+# a row's own storage keeps 126 elements; a CTA takes 64 at a time and searches the further ones 1,024 at a time
+@pytest.mark.parametrize("name,k", [("t3", 126), ("t3", 127), ("t3", 360), ("t3", 1150), ("t3", 1151), ("t3", 2300),
+                                    ("q4", 63), ("q4", 126), ("q4", 127), ("q4", 400), ("mixed", 126), ("mixed", 300),
+                                    ("book", 126), ("book", 127), ("book", 252), ("book", 253), ("book", 1500)])
+@pytest.mark.parametrize("beside", [False, True])
+def test_2d_hubs(fem, oracle_mod, cuda_device, name, k, beside):
+    import meshgen as mg
+    from test_gpu_rows2d import _fan
+    m = {"t3": lambda: _shuffled(_fan(k, True)), "q4": lambda: _quad_fan(k), "mixed": lambda: _mixed_fan(k),
+         "book": lambda: _book(k)}[name]()
+    if beside:
+        g = {"q4": mg.q4_grid, "mixed": mg.mixed_grid}.get(name, mg.t3_grid)(131, 130, seed=5)
+        g.E = g.nu = None
+        m = _beside(m, g)
+    info = _check(fem, oracle_mod, m, k, fem.opts(pool_factor=1.0))
+    if not beside:
+        rows = np.diff(oracle_mod.pattern(m)[0])[::2] // 2
+        assert info.overflow_chunks == np.maximum(0, -(-(rows - 14) // 14)).sum()
+
+
+def test_2d_hubs_that_share_elements_and_many_of_them(fem, oracle_mod, cuda_device):
+    # fans of different sizes beside one another: their further elements share one list
+    from test_gpu_rows2d import _fan
+    m = _fan(130, True)
+    for k in (127, 500, 14, 200, 360):
+        m = _beside(_fan(k, k != 200), m)
+    _check(fem, oracle_mod, m, 500, fem.opts(pool_factor=1.0))
