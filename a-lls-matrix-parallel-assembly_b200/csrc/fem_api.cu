@@ -54,9 +54,8 @@ fem_status check_mesh(const fem_mesh* m, bool device_pointers_needed = true) {
     return FEM_OK;
 }
 
-// Bytes per Hex20 element of the region that holds the rank map (800 bytes an
-// element): the workspace sizes that callers have been given, from 20,880-byte
-// records per 8 elements of at most `wave`.
+// Room that workspaces have had for Hex20 meshes: a record of 20,880 bytes for every 8 of at most `wave` elements. It
+// is kept, so that workspace sizes that callers saved stay valid, and is part of what make_layout shares out.
 size_t hex20_record_bytes(int E, int wave) { return ((size_t)std::min(E, wave) + 7) / 8 * 20880; }
 
 fem_status make_layout(const fem_mesh* m, const fem_opts* o, HostLayout& h) {
@@ -99,31 +98,35 @@ fem_status make_layout(const fem_mesh* m, const fem_opts* o, HostLayout& h) {
     off += align_up(h.meta1_bytes);
     h.off_meta2 = off;
     off += align_up((size_t)h.cap2 * h.H2 * sizeof(int));
-    // 2-D: the slots' value blocks; Hex20: the packed Ke of the elements, which take less (15.1 KB an element,
-    // about 4 nodes of 7.8 KB) unless elements overlap
-    h.off_vals = off;
-    size_t vals_bytes = (size_t)slots * h.B * sizeof(double);
-    if (h.kind == FEM_HEX20) vals_bytes = std::max(vals_bytes, (size_t)h.E * kPackedHex20 * sizeof(double));
-    off += align_up(vals_bytes);
     h.off_counts = off;
     off += align_up((size_t)h.N * sizeof(int));
     h.off_ucounts = off;  // upper-triangle column counts (fem_alls_consolidate_upper)
     off += align_up((size_t)h.N * sizeof(int));
-    h.off_tiles = off;  // scan partials of kRowTile nodes (2-D: running on into the next region)
-    off += align_up((size_t)(h.dpn == 2 ? h.num_tiles : row_tiles(h.N)) * sizeof(long long));
+    h.off_tiles = off;  // 2-D: scan partials of kRowTile nodes, running on into the next region
+    off += align_up((size_t)h.num_tiles * sizeof(long long));
     h.off_elist = off;  // visit order of the elements (perm), ranges, bucket histogram (+ bbox)
     {
         const size_t nbuckets = h.dpn == 2 ? (size_t)2 * reorder_buckets(h.N) : (size_t)1 << (3 * morton_bits(h.E));
         off += align_up((size_t)h.E * sizeof(int)) + align_up(4 * sizeof(int)) + align_up(nbuckets * sizeof(int)) +
                align_up(6 * sizeof(unsigned long long));
     }
-    // Hex20: node -> occurrences (counts, offsets, lists) and the rank map of the rows
+    // Hex20: node -> occurrences (counts, offsets, lists)
     h.off_inc = off;
     if (h.kind == FEM_HEX20)
         off += 2 * align_up((size_t)(h.N + 1) * sizeof(int)) + align_up((size_t)h.E * 20 * sizeof(int));
-    h.off_map = off;
-    if (h.kind == FEM_HEX20)
-        off += align_up(std::max(hex20_record_bytes(h.E, 32768), (size_t)h.E * 400 * sizeof(unsigned short)));
+    // 2-D: the slots' value blocks. Hex20: in the bytes that these and the records would take (7.8 KB a node and up to
+    // 2.6 KB an element), the packed Ke of the elements, the rank map (15.9 KB an element together) and the scan
+    // partials. They fit unless there are more than about half as many elements as nodes (a regular mesh has a
+    // quarter), when the workspace grows by what is missing.
+    h.off_vals = off;
+    size_t room = align_up((size_t)slots * h.B * sizeof(double));
+    if (h.kind == FEM_HEX20) {
+        room += align_up(hex20_record_bytes(h.E, 32768));
+        h.off_map = off + align_up((size_t)h.E * kPackedHex20 * sizeof(double));
+        h.off_tiles = h.off_map + align_up((size_t)h.E * 400 * sizeof(unsigned short));
+        room = std::max(room, h.off_tiles - off + align_up(row_tiles(h.N) * sizeof(long long)));
+    }
+    off += room;
     h.total = off;
     return FEM_OK;
 }
