@@ -127,13 +127,15 @@ __device__ int long_row_next_col(const ListLayout& L, int n, int after, int glan
     return best;
 }
 
+// Returns whether the row has u columns.
 template <int DPN, int G>
-__device__ void long_row_write(const ListLayout& L, int n, int u, long long base, int glane, unsigned mask,
+__device__ bool long_row_write(const ListLayout& L, int n, int u, long long base, int glane, unsigned mask,
                                int* __restrict__ col_idx, double* __restrict__ values) {
     constexpr int B = DPN * DPN;
     int last = -1;
-    for (int k = 0; k < u; k++) {
+    for (int k = 0;; k++) {
         const int col = long_row_next_col<G>(L, n, last, glane, mask);
+        if (k == u || col == 0x7FFFFFFF) return k == u && col == 0x7FFFFFFF;
         last = col;
         double sum[B];
 #pragma unroll
@@ -577,7 +579,8 @@ __device__ __forceinline__ void row_ptr_rows(const int* __restrict__ counts, int
 // lanes per node, lane 2k + i on row i of block k. A lane moves 16 bytes of
 // values (a warp's loads are consecutive, its stores two runs per node) and 8
 // bytes of columns; four nodes of a group are in flight. Hashed rows (fans)
-// take the exact slow path.
+// take the exact slow path, and so do rows whose header has another number of
+// columns than the row pointers; a list without them raises FEM_ERR_INTERNAL.
 constexpr int kCopyNodes = 4;
 __device__ __forceinline__ void write_sorted_2d(const ListLayout& L, const int* __restrict__ row_ptr,
                                                 int* __restrict__ col_idx, double* __restrict__ values,
@@ -589,6 +592,7 @@ __device__ __forceinline__ void write_sorted_2d(const ListLayout& L, const int* 
     const int tid = threadIdx.x, grp = tid / G, lane = tid % G, i = lane & 1;
     const unsigned gmask = 0xFFFFu << (((tid & 31) / G) * G);
     int t_sum = 0, t_max = 0;
+    int lowest = 1;  // lowest column word met; 0: a row whose list does not have the columns it is counted with
     for (long long nb = (long long)block * NPB * kCopyNodes; nb < L.N; nb += (long long)nblocks * NPB * kCopyNodes) {
         int base[kCopyNodes], u[kCopyNodes], head[kCopyNodes];
 #pragma unroll
@@ -610,7 +614,7 @@ __device__ __forceinline__ void write_sorted_2d(const ListLayout& L, const int* 
 #pragma unroll
             for (int h = 0; h < 2; h++) {
                 const int p = lane + h * G;
-                if (head[q] == kRowSorted && p < 2 * u[q]) {
+                if (head[q] == kRowSorted + u[q] && p < 2 * u[q]) {
                     v[q][h] = __ldg(reinterpret_cast<const double2*>(L.vals + n * (k2DSlots * 4)) + p);
                     c[q][h] = __ldg(L.meta1 + n * (k2DSlots + 2) + 2 + (p >> 1));
                 }
@@ -621,21 +625,23 @@ __device__ __forceinline__ void write_sorted_2d(const ListLayout& L, const int* 
             const long long n = nb + q * NPB + grp;
             t_sum += u[q];
             t_max = max(t_max, u[q]);
-            if (head[q] == kRowSorted) {
+            if (head[q] == kRowSorted + u[q]) {
 #pragma unroll
                 for (int h = 0; h < 2; h++) {
                     const int k = (lane + h * G) >> 1;
                     if (k < u[q]) {
+                        lowest = min(lowest, c[q][h]);
                         const long long p = base[q] + 2ll * i * u[q] + 2 * k;
                         *reinterpret_cast<double2*>(values + p) = v[q][h];
                         *reinterpret_cast<int2*>(col_idx + p) = make_int2(2 * c[q][h] - 2, 2 * c[q][h] - 1);
                     }
                 }
             } else {
-                long_row_write<2, G>(L, (int)n, u[q], base[q], lane, gmask, col_idx, values);
+                if (!long_row_write<2, G>(L, (int)n, u[q], base[q], lane, gmask, col_idx, values)) lowest = 0;
             }
         }
     }
+    if (lowest <= 0) raise_status(L.info, FEM_ERR_INTERNAL);
     // list statistics (one atomic pair per CTA)
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) {

@@ -8,7 +8,7 @@
 // one column NODE of a row node, so the dpn rows of a node share one list.
 //
 // Chunk metadata is a row of H = S + 2 int32 words:
-//     word 0 = kRowSorted for a 2-D row stored sorted and compact, else 0
+//     word 0 = kRowSorted + columns for a 2-D row stored sorted and compact, else 0
 //     word 1 = next  (chunk id + 1 of the next chunk, 0 = none)
 //     word 2+s = slot s: 0 = empty, col+1 = column node col
 // A row belongs to the thread, warp or CTA that builds it (rows2d.cuh,
@@ -104,9 +104,8 @@ constexpr int kMaxChainSteps = 1 << 20;
 
 constexpr int kColMask = 0x7FFFFFFF;
 
-// Header word (word 0) of a 2-D first chunk whose row is complete in it: its
-// columns fill the first slots in increasing order (no next chunk). 0: the
-// row is hashed (fans, and the batched kernel's rows).
+// Header word (word 0) of a 2-D first chunk whose row is complete in it: this plus the number of columns, which fill
+// the first slots in increasing order (no next chunk). 0: the row is hashed (fans).
 constexpr int kRowSorted = 1;
 
 // Start of the probe sequence of column key `key` (col + 1) in a chunk of S slots.

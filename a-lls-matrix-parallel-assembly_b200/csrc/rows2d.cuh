@@ -24,7 +24,7 @@
 //              conflicts), the diagonal block in registers; further columns
 //              (up to the chunk's 14) in the row's own value blocks. The row
 //              leaves the thread once, sorted by column and compact: its slot
-//              words (header word kRowSorted) and its blocks as 32-byte
+//              words (header word kRowSorted + columns) and its blocks as 32-byte
 //              stores, whole sectors.
 // No value is ever added in global memory, so nothing is zeroed first, no
 // element order is needed and the value blocks are written once.
@@ -547,7 +547,7 @@ __device__ __forceinline__ void rows_2d(const MeshView& m, const ListLayout& L, 
 #pragma unroll
                     for (int k = 0; k < 4; k++) {
                         const int s = 4 * q + k - 2;
-                        w[k] = s == -2 ? kRowSorted : (s >= 0 && s < total ? sm.words[4 * q + k][tid] : 0);
+                        w[k] = s == -2 ? kRowSorted + total : (s >= 0 && s < total ? sm.words[4 * q + k][tid] : 0);
                     }
                     reinterpret_cast<int4*>(meta)[q] = make_int4(w[0], w[1], w[2], w[3]);
                 }

@@ -100,6 +100,7 @@ __device__ __forceinline__ void write_hex20(const ListLayout& L, const HexRows& 
         sv[i] = x - 9 * sb[i];
     }
     int t_sum = 0, t_max = 0;
+    bool bad = false;  // a row whose list lacks a column, or that an element has a further column for
     // The warps draw their nodes one by one from one counter, so that the rows in flight stay close in the visit order
     // however unevenly the SMs run (a fixed stride let them drift apart: Ke read 2.1 times from DRAM, 1.4 so). The
     // draws, the node ids and the headers of the next rows are in flight while a row is summed.
@@ -153,6 +154,7 @@ __device__ __forceinline__ void write_hex20(const ListLayout& L, const HexRows& 
             for (int q = 0; q < kWindow / 32; q++) {
                 const int k = lane + 32 * q;
                 col[q] = k < uw ? __ldg(hex_col_word(L, n, next, w0 + k)) - 1 : 0;
+                bad |= (unsigned)col[q] >= (unsigned)L.N;
             }
             double val[kItems];
             unsigned rk = 0;  // lane b < 20: rank of the occurrence's column node b
@@ -175,6 +177,7 @@ __device__ __forceinline__ void write_hex20(const ListLayout& L, const HexRows& 
                 // where column node `lane`'s block goes: its rank in the window, or the bin
                 const int place = (int)((rk - (unsigned)w0) & (kRankRange - 1));
                 int to = lane < 20 && place < uw ? place * 9 : kBin;
+                bad |= lane < 20 && rk >= (unsigned)u && u != L.S1;  // S1 columns: cut when the pool overflowed
                 if (u > kRankRange && to != kBin &&  // the rank is known up to a multiple of kRankRange only
                     __ldg(hex_col_word(L, n, next, w0 + place)) - 1 !=
                         __ldg(h.conn + (size_t)(occ_of(word) / 20) * 20 + lane))
@@ -244,6 +247,7 @@ __device__ __forceinline__ void write_hex20(const ListLayout& L, const HexRows& 
         }
         cur = nxt;
     }
+    if (bad) raise_status(L.info, FEM_ERR_INTERNAL);
     // list statistics (one atomic pair per CTA)
     if (lane == 0) {
         s_sum[warp] = t_sum;
