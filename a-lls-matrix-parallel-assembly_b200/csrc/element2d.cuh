@@ -118,8 +118,10 @@ __device__ __forceinline__ double ke_block_2d(const double (&xd)[NPE], const dou
 // ke_block_2d with the gradients left unnormalised (X = j3 dN/dxi - j1
 // dN/deta, Y = j0 dN/deta - j2 dN/dxi, the true gradient times detJ), so one
 // division per Gauss point carries the weight and both 1/detJ factors, and a
-// T3 needs a single one. Returns detJ (Q4: the smallest over the Gauss
-// points).
+// T3 needs a single one. In FP32 the division is of one and the material comes
+// in after the first gradient: E / detJ passes FP32's range for elements of
+// 1e-14 and less (in FP64's range both forms are far from it). Returns detJ
+// (Q4: the smallest over the Gauss points).
 template <int NPE, typename T = double>
 __device__ __forceinline__ double ke_row_2d(const double (&xd)[NPE], const double (&yd)[NPE], double Ed, double nud,
                                             double td, double (&kv)[NPE][4]) {
@@ -135,8 +137,9 @@ __device__ __forceinline__ double ke_row_2d(const double (&xd)[NPE], const doubl
         const T X[3] = {y[1] - y[2], y[2] - y[0], y[0] - y[1]};
         const T Y[3] = {x[2] - x[1], x[0] - x[2], x[1] - x[0]};
         const T det = Y[2] * X[1] - Y[1] * X[2];
-        const T s = T(0.5) * t * E / (one_nu2 * det);
-        const T sx = s * X[0], sy = s * Y[0], hx = h * sx, hy = h * sy, nx = nu * sx, ny = nu * sy;
+        const T f = sizeof(T) == 8 ? T(1) : T(0.5) * t * E / one_nu2;
+        const T s = sizeof(T) == 8 ? T(0.5) * t * E / (one_nu2 * det) : T(1) / det;
+        const T sx = f * (s * X[0]), sy = f * (s * Y[0]), hx = h * sx, hy = h * sy, nx = nu * sx, ny = nu * sy;
 #pragma unroll
         for (int b = 0; b < 3; b++) {
             kv[b][0] = double(fma(sx, X[b], hy * Y[b]));
@@ -169,14 +172,14 @@ __device__ __forceinline__ double ke_row_2d(const double (&xd)[NPE], const doubl
                 const T det = j0 * j3 - j1 * j2;
                 min_det = fmin(min_det, det);
                 const T dxi[4] = {-em, em, ep, -ep}, deta[4] = {-xm, -xp, xp, xm};
-                const T r = f / det;
+                const T r = (sizeof(T) == 8 ? f : T(1)) / det, m = sizeof(T) == 8 ? T(1) : f;
                 T X[4], Y[4];
 #pragma unroll
                 for (int b = 0; b < 4; b++) {
                     X[b] = fma(j3, dxi[b], -j1 * deta[b]);
                     Y[b] = fma(j0, deta[b], -j2 * dxi[b]);
                 }
-                const T sx = r * X[0], sy = r * Y[0], hx = h * sx, hy = h * sy, nx = nu * sx, ny = nu * sy;
+                const T sx = m * (r * X[0]), sy = m * (r * Y[0]), hx = h * sx, hy = h * sy, nx = nu * sx, ny = nu * sy;
 #pragma unroll
                 for (int b = 0; b < 4; b++) {
                     k[b][0] = fma(sx, X[b], fma(hy, Y[b], k[b][0]));
