@@ -6,17 +6,19 @@
 // are assembled in rounds of `slots` (the workspace holds that many meshes'
 // lists at once), and a round runs phase by phase: one launch per phase covers
 // all of the round's meshes (begin; 2-D fill and Hex20 occurrences; rows; Hex20
-// Ke; row pointers; writes; finish), its blocks dealt to the meshes in
+// Ke; row pointers; writes), its blocks dealt to the meshes in
 // proportion to their work, each block running the device code of the
 // single-mesh kernels. Phases follow each other in stream order, so nothing
 // waits inside a kernel, small meshes share their launches, and large ones get
 // the same kernels as on their own. A round's mesh descriptors travel as kernel
 // parameters, so a captured CUDA graph holds them.
 //
-// What bounds it: the single-mesh kernels; a round costs up to 15 launches
-// whatever its number of meshes. B200, 16 meshes of 1,000 to 50,000 elements of
-// all kinds in 4 slots: 1.69 ms, where one persistent kernel of dependent work
-// items (CAS claims, element-wise atomics, no spatial order) took 8.0 ms.
+// What bounds it: the single-mesh kernels. A round costs 14 merged launches
+// (two more if some outputs are not aligned or have no room) and, for each of its
+// Hex20 meshes of 3,072 elements or more, a node order: a memset and five small
+// kernels. B200, 16 meshes of 1,000 to 50,000 elements of all kinds in 4 slots:
+// 1.69 ms, where one persistent kernel of dependent work items (CAS claims,
+// element-wise atomics, no spatial order) took 8.0 ms.
 #include <algorithm>
 #include <numeric>
 #include <vector>
@@ -157,10 +159,30 @@ FEM_BATCH_KERNEL(kScanThreads) kb_row_ptr(const __grid_constant__ BatchRound<kMa
         row_ptr_rows<2, kOutCsr>(bm.L.counts, bm.L.N, bm.tiles, bm.row_ptr, bm.L.info, bm.capacity, block, nblocks, sm);
 }
 
+// The info word to the caller's array and the completion stamp (one thread).
+__device__ __forceinline__ void finish_mesh(const BatchMesh& bm) {
+    static_assert(sizeof(fem_info) % 8 == 0, "copied in 8-byte words");
+    for (int w = 0; w < (int)(sizeof(fem_info) / 8); w++)
+        reinterpret_cast<unsigned long long*>(bm.info_out)[w] =
+            __ldcg(reinterpret_cast<const unsigned long long*>(bm.L.info) + w);
+    if (bm.stamp) *bm.stamp = global_timer();
+}
+
+// The end of a write block; the mesh's last one finishes the mesh.
+__device__ __forceinline__ void write_done(const BatchMesh& bm, int nblocks) {
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    __threadfence();  // the block's entries and statistics before its count
+    if (atomicAdd(&bm.L.info->done, 1) != nblocks - 1) return;
+    __threadfence();
+    finish_mesh(bm);
+}
+
 FEM_BATCH_KERNEL(kBlockThreads) kb_write_2d(const __grid_constant__ BatchRound<kMax> r) {
     FEM_BATCH_MESH;
     __shared__ int s_stat[2 * (kBlockThreads / 32)];
     write_sorted_2d(bm.L, bm.row_ptr, bm.col_idx, bm.values, bm.capacity, block, nblocks, s_stat);
+    write_done(bm, nblocks);
 }
 
 // The 2-D meshes whose outputs are not aligned for write_sorted_2d.
@@ -170,6 +192,7 @@ FEM_BATCH_KERNEL(kBlockThreads) kb_write_2d_entries(const __grid_constant__ Batc
     constexpr int NPB = kBlockThreads / 8;
     write_batches<2, 8, 2, kOutCsr>(bm.L, bm.row_ptr, bm.col_idx, bm.values, bm.capacity, nullptr,
                                     (long long)block * NPB, (long long)nblocks * NPB, bm.L.N, sm);
+    write_done(bm, nblocks);
 }
 
 FEM_BATCH_KERNEL(kWriteThreads, FEM_HEXW_CTAS) kb_write_hex20(const __grid_constant__ BatchRound<kMax> r) {
@@ -177,15 +200,13 @@ FEM_BATCH_KERNEL(kWriteThreads, FEM_HEXW_CTAS) kb_write_hex20(const __grid_const
     FEM_BATCH_MESH;
     write_hex20<kOutCsr>(bm.L, bm.h, nullptr, bm.row_ptr, bm.col_idx, bm.values, bm.capacity, block, nblocks,
                          *reinterpret_cast<WriteHexCta*>(smem_raw));
+    write_done(bm, nblocks);
 }
 
-// One block per mesh: the info word to the caller's array, the completion stamp.
+// The meshes without an output, one block each.
 FEM_BATCH_KERNEL(32) kb_finish(const __grid_constant__ BatchRound<kMax> r) {
     FEM_BATCH_MESH;
-    if (threadIdx.x < (int)(sizeof(fem_info) / 8))
-        reinterpret_cast<unsigned long long*>(bm.info_out)[threadIdx.x] =
-            reinterpret_cast<const unsigned long long*>(bm.L.info)[threadIdx.x];
-    if (threadIdx.x == 0 && bm.stamp) *bm.stamp = global_timer();
+    if (threadIdx.x == 0) finish_mesh(bm);
 }
 
 template <int kMax>
@@ -269,7 +290,7 @@ cudaError_t launch_round(const BatchMesh* meshes, int n, unsigned long long* sta
     });
     l.run(kb_write_hex20<kMax>, kWriteThreads, sizeof(WriteHexCta), FEM_HEXW_CTAS * sms,
           [&](M b) { return hex(b) && b.capacity > 0 ? blocks_of(b.L.N, kWriteWarps) : 0; });
-    l.run(kb_finish<kMax>, 32, 0, 0, [](M) { return 1ll; });
+    l.run(kb_finish<kMax>, 32, 0, 0, [](M b) { return b.capacity > 0 ? 0ll : 1ll; });
     return l.err;
 }
 

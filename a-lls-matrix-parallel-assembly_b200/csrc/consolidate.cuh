@@ -571,6 +571,7 @@ __device__ __forceinline__ void row_ptr_rows(const int* __restrict__ counts, int
         info->list_entries = 0;
         info->max_row_entries = 0;
         info->ticket = 0;
+        info->done = 0;
         row_ptr[(long long)N * R] = (int)(nnz / (kMode == kOutBsr ? B : 1));
     }
 }

@@ -44,7 +44,7 @@ struct DevInfo {
     int long_rows;         // rows queued for the long-row kernels
     int ticket;            // consolidation: next row node to write
     int spilled;           // 2-D: entries of the spill list (may overshoot its capacity)
-    int pad0;
+    int done;              // batch: blocks of the mesh's write that are done
     long long pad1[2];
 };
 static_assert(sizeof(DevInfo) == 64, "DevInfo size");

@@ -804,8 +804,8 @@ def batch_launches(meshes, slots: int) -> int:
         for i in range(0, len(part), ROUND_LARGE):
             ms = part[i:i + ROUND_LARGE]
             hexes = [m for m in ms if m.kind == 2]
-            # begin, fill, tile entries, row pointers, finish; occurrences (3), rows (2), Ke, write; 2-D rows (2), write
-            total += 5 + 7 * bool(hexes) + 3 * (len(hexes) < len(ms))
+            # begin, fill, tile entries, row pointers; occurrences (3), rows (2), Ke, write; 2-D rows (2), write
+            total += 4 + 7 * bool(hexes) + 3 * (len(hexes) < len(ms))
             total += 5 * sum(m.num_elems >= ORDERED_ELEMS for m in hexes)
     return total
 

@@ -278,7 +278,7 @@ FEM_API fem_status fem_batched_workspace_size(const fem_mesh* meshes, int32_t n,
  * row_ptr and FEM_ERR_CAPACITY in its info). infos: DEVICE array [n] that
  * receives each mesh's fem_info (nnz, status bits, ...). stamps: optional
  * DEVICE array [n + 1] of GPU global-timer nanoseconds: stamps[0] at the start,
- * stamps[1 + i] when mesh i's round is done. outs[i].n_rows is set. Asynchronous. */
+ * stamps[1 + i] when mesh i is done. outs[i].n_rows is set. Asynchronous. */
 FEM_API fem_status fem_assemble_batched(const fem_mesh* meshes, int32_t n, const fem_opts* opts,
                                         int32_t concurrency, void* workspace, size_t workspace_bytes,
                                         fem_csr* outs, fem_info* infos, unsigned long long* stamps, void* stream);
