@@ -570,28 +570,24 @@ fem_status fem_assemble_batched(const fem_mesh* meshes, int32_t n, const fem_opt
 
 namespace {
 
-// Candidate options for one mesh: the scatter grid (all resident CTAs, or
-// 1..3 per SM) and, for Hex20, the list shape (first chunk 94 / 62 / 46
-// slots, overflow chunks of 30; a pool of one overflow chunk per node for the
-// smaller first chunks, whose corner-node rows spill).
+// Candidate options for one mesh. 2-D: the grid of the row kernel (all resident
+// CTAs, or 1..3 per SM). Hex20: the list shape (first chunk 94 / 62 / 46 slots,
+// overflow chunks of 30; a pool of one overflow chunk per node for the smaller
+// first chunks, whose corner-node rows spill).
 std::vector<fem_opts> tune_candidates(const fem_mesh* m, const fem_opts* base) {
     fem_opts b{};
     if (base) b = *base;
     std::vector<fem_opts> out;
-    const int ctas[] = {0, 1, 2, 3};
     if (m->kind == FEM_HEX20) {
-        const int first[] = {94, 62, 46};
-        for (int f : first)
-            for (int c : ctas) {
-                fem_opts o = b;
-                o.first_slots = f;
-                o.chunk_slots = 30;
-                if (f < 94) o.pool_factor = std::max(o.pool_factor, 1.0);
-                o.ctas_per_sm = c;
-                out.push_back(o);
-            }
+        for (int f : {94, 62, 46}) {
+            fem_opts o = b;
+            o.first_slots = f;
+            o.chunk_slots = 30;
+            if (f < 94) o.pool_factor = std::max(o.pool_factor, 1.0);
+            out.push_back(o);
+        }
     } else {
-        for (int c : ctas) {
+        for (int c : {0, 1, 2, 3}) {
             fem_opts o = b;
             o.first_slots = o.chunk_slots = 0;
             o.ctas_per_sm = c;
@@ -697,7 +693,7 @@ fem_status fem_autotune_batched(const fem_mesh* meshes, int32_t n, const fem_opt
         auto run = [&] {
             return fem_assemble_batched(meshes, n, opts, k, workspace, workspace_bytes, outs, infos, nullptr, stream);
         };
-        if ((st = run())) return st;  // untimed (creates the slot streams)
+        if ((st = run())) return st;  // untimed
         float ms = 0.0f;
         if ((st = time_calls(s, repeats, run, ms))) return st;
         if (!found || ms < best_t) {

@@ -666,7 +666,7 @@ def colour_baseline(fem, torch, asm, mesh, nnz, args, flush, stream) -> dict:
 def autotune_leg(asm, ms) -> dict:
     t0 = time.perf_counter()
     best, best_ms = asm.autotune(repeats=3)
-    return {"api": "fem_autotune (scatter grid CTAs/SM; Hex20 also first/overflow chunk slots)",
+    return {"api": "fem_autotune (2-D: row kernel CTAs/SM; Hex20: first/overflow chunk slots)",
             "best": {"ctas_per_sm": best.ctas_per_sm, "first_slots": best.first_slots,
                      "chunk_slots": best.chunk_slots, "pool_factor": best.pool_factor},
             "best_ms": best_ms, "default_ms": ms, "tuning_s": time.perf_counter() - t0,

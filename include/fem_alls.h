@@ -294,9 +294,9 @@ FEM_API fem_status fem_assemble_batched(const fem_mesh* meshes, int32_t n, const
 /* Bytes of workspace that every candidate of fem_autotune fits in. */
 FEM_API fem_status fem_autotune_workspace_size(const fem_mesh* mesh, const fem_opts* opts, size_t* bytes);
 
-/* One mesh: the scatter grid (opts.ctas_per_sm: all that fit, 1, 2 or 3) and,
- * for Hex20, the list shape (first_slots 94, 62 or 46 with chunk_slots 30; pool
- * factor at least 1 for the smaller first chunks). The precision of opts is
+/* One mesh: the grid of the 2-D row kernel (opts.ctas_per_sm: all that fit, 1,
+ * 2 or 3) or, for Hex20, the list shape (first_slots 94, 62 or 46 with chunk_slots
+ * 30; pool factor at least 1 for the smaller first chunks). The other options are
  * kept. out: as for fem_assemble, with capacity >= nnz; on return it holds the
  * assembly with the chosen options (status as fem_assemble's). *best: the
  * fastest options; *best_ms (may be NULL): their mean time per assembly.
