@@ -129,28 +129,8 @@ def test_patterns_without_some_blocks(fem, oracle_mod, cuda_device, name):
     assert np.all(np.abs(vals.cpu().numpy() - ov[keep]) <= RTOL * scale[keep])
 
 
-def _t3_stiffness(m):
-    """The CSR of a T3 mesh from its constant-strain element matrices (numpy): a row of tens of thousands of columns takes
-    the oracle's linear search too long."""
-    import scipy.sparse as sp
-    c = m.conn
-    x, y = m.x[c], m.y[c]
-    X = np.stack([y[:, 1] - y[:, 2], y[:, 2] - y[:, 0], y[:, 0] - y[:, 1]], 1)
-    Y = np.stack([x[:, 2] - x[:, 1], x[:, 0] - x[:, 2], x[:, 1] - x[:, 0]], 1)
-    det = Y[:, 2] * X[:, 1] - Y[:, 1] * X[:, 2]
-    B = np.zeros((c.shape[0], 3, 6))
-    B[:, 0, 0::2], B[:, 1, 1::2], B[:, 2, 0::2], B[:, 2, 1::2] = X, Y, Y, X
-    D = m.E0 / (1 - m.nu0 ** 2) * np.array([[1, m.nu0, 0], [m.nu0, 1, 0], [0, 0, (1 - m.nu0) / 2]])
-    ke = np.einsum("eki,kl,elj->eij", B, D, B) * (0.5 * m.thickness / det)[:, None, None]
-    dof = (2 * c[:, :, None] + np.arange(2)).reshape(c.shape[0], 6)
-    a = sp.coo_matrix((ke.ravel(), (np.repeat(dof, 6, axis=1).ravel(), np.tile(dof, (1, 6)).ravel())),
-                      shape=(m.num_dofs, m.num_dofs)).tocsr()
-    a.sort_indices()
-    return a.indptr.astype(np.int32), a.indices.astype(np.int32), a.data
-
-
 @pytest.mark.parametrize("cols", [65535, 65536, 65537, 70001])
-def test_rows_past_16_bit_ranks(fem, cuda_device, cols):
+def test_rows_past_16_bit_ranks(fem, oracle_mod, cuda_device, cols):
     # a closed fan: its hub's row has a column per triangle and its own
     import meshgen as mg
     k = cols - 1
@@ -160,7 +140,7 @@ def test_rows_past_16_bit_ranks(fem, cuda_device, cols):
     xy = np.insert(np.stack([np.cos(ang), np.sin(ang)], 1), k // 2, 0.0, axis=0)
     conn = np.random.default_rng(1).permutation(conn).astype(np.int32)
     m = mg.Mesh(mg.T3, xy[:, 0].copy(), xy[:, 1].copy(), None, np.ascontiguousarray(conn), None, None, None, E0=1.0, nu0=0.3)
-    rp, ci, v = _t3_stiffness(m)
+    rp, ci, v = oracle_mod.assemble(m)
     assert np.diff(rp).max() == 2 * cols
     asm = fem.Assembler(m)
     vals = _with_pattern(asm, rp, ci)
@@ -170,3 +150,28 @@ def test_rows_past_16_bit_ranks(fem, cuda_device, cols):
     # the hub's entries are sums of up to 70,001 terms: 1e-10 of its diagonal covers their order
     scale = np.maximum(np.abs(v), diag_scale(rp, ci, v))
     assert np.all(np.abs(vals.cpu().numpy() - v) <= 1e-10 * scale)
+
+
+# columns that a thread sums in shared memory: 10 (T3), 14 (Q4, mixed); longer rows are added with atomics
+@pytest.mark.parametrize("kind,k", [("t3", 8), ("t3", 9), ("t3", 10), ("t3", 40), ("q4", 6), ("q4", 7), ("q4", 30), ("mixed", 6),
+                                    ("mixed", 7), ("mixed", 30)])
+@pytest.mark.parametrize("precision", [0, 3])
+def test_rows_around_the_sums_of_a_thread(fem, oracle_mod, cuda_device, kind, k, precision):
+    # fans of k triangles (k + 1 columns) or quadrilaterals (2 k + 1), one beside another and a grid by row nodes
+    import torch
+    import meshgen as mg
+    from test_gpu_hubs import _beside, _mixed_fan, _quad_fan, _shuffled
+    from test_gpu_rows2d import _fan
+    fan = {"t3": lambda: _shuffled(_fan(k, True)), "q4": lambda: _quad_fan(k), "mixed": lambda: _mixed_fan(k)}[kind]
+    g = _mesh(kind + "_large")
+    g.E = g.nu = None
+    m = _beside(fan(), _beside(fan(), g))
+    asm = fem.Assembler(m)
+    rp, ci, v, info = asm.assemble()
+    re = _build(fem, asm, int(info.nnz), 0)
+    vals = torch.full((int(info.nnz),), 7.0, dtype=torch.float64, device="cuda")
+    re.reassemble(vals, fem.opts(precision=precision))
+    assert re.read_info() == 0
+    orp, oci, ov = oracle_mod.assemble(m)
+    scale = np.maximum(np.abs(ov), diag_scale(orp, oci, ov))
+    assert np.all(np.abs(vals.cpu().numpy() - ov) <= (1e-5 if precision else RTOL) * scale)
