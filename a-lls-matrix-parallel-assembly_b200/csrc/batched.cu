@@ -188,9 +188,9 @@ FEM_BATCH_KERNEL(kBlockThreads) kb_write_2d(const __grid_constant__ BatchRound<k
 // The 2-D meshes whose outputs are not aligned for write_sorted_2d.
 FEM_BATCH_KERNEL(kBlockThreads) kb_write_2d_entries(const __grid_constant__ BatchRound<kMax> r) {
     FEM_BATCH_MESH;
-    __shared__ WriteSmem<2, 8, 2> sm;
+    __shared__ WriteSmem<8, 2> sm;
     constexpr int NPB = kBlockThreads / 8;
-    write_batches<2, 8, 2, kOutCsr>(bm.L, bm.row_ptr, bm.col_idx, bm.values, bm.capacity, nullptr,
+    write_batches<8, 2, kOutCsr>(bm.L, bm.row_ptr, bm.col_idx, bm.values, bm.capacity, nullptr,
                                     (long long)block * NPB, (long long)nblocks * NPB, bm.L.N, sm);
     write_done(bm, nblocks);
 }

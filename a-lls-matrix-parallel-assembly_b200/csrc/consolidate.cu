@@ -52,13 +52,13 @@ __global__ void __launch_bounds__(kScanThreads) k_row_ptr(const int* __restrict_
     row_ptr_rows<DPN, kMode>(counts, N, tile_sums, row_ptr, info, capacity, blockIdx.x, gridDim.x, sm);
 }
 
-template <int DPN, int G, int KPL, int kMode>
+template <int G, int KPL, int kMode>
 __global__ void __launch_bounds__(kBlockThreads, FEM_WRITE_MIN_CTAS_2D)
     k_write(ListLayout L, const int* __restrict__ row_ptr, int* __restrict__ col_idx, double* __restrict__ values,
             long long capacity, const int* __restrict__ ucounts) {
     constexpr int NPB = kBlockThreads / G;  // nodes per batch
-    __shared__ WriteSmem<DPN, G, KPL> sm;
-    write_batches<DPN, G, KPL, kMode>(L, row_ptr, col_idx, values, capacity, ucounts, (long long)blockIdx.x * NPB,
+    __shared__ WriteSmem<G, KPL> sm;
+    write_batches<G, KPL, kMode>(L, row_ptr, col_idx, values, capacity, ucounts, (long long)blockIdx.x * NPB,
                                       (long long)gridDim.x * NPB, L.N, sm);
 }
 
@@ -70,12 +70,12 @@ __global__ void __launch_bounds__(kBlockThreads) k_write_sorted_2d(ListLayout L,
 }
 
 // Persistent grid of k_write: the CTAs that fit on the GPU at once.
-template <int DPN, int G, int KPL, int kMode>
+template <int G, int KPL, int kMode>
 long long write_grid(long long batches) {
     static DeviceCache cache;
     int per_sm = 0;
     if (per_device(cache, [](int& v) {
-            return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, k_write<DPN, G, KPL, kMode>, kBlockThreads, 0);
+            return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, k_write<G, KPL, kMode>, kBlockThreads, 0);
         }, per_sm))
         per_sm = 1;
     return std::max<long long>(1, std::min<long long>(batches, (long long)per_sm * sm_count()));
@@ -108,7 +108,7 @@ cudaError_t launch_mode(const ListLayout& L, const HexRows& hex, const int* coun
         } else {
             constexpr int G = 8, NPB = kBlockThreads / G;
             const long long batches = ((long long)L.N + NPB - 1) / NPB;
-            k_write<DPN, G, 2, kMode><<<(int)write_grid<DPN, G, 2, kMode>(batches), kBlockThreads, 0, s>>>(
+            k_write<G, 2, kMode><<<(int)write_grid<G, 2, kMode>(batches), kBlockThreads, 0, s>>>(
                 L, row_ptr, col_idx, values, capacity, counts);
         }
         return cudaGetLastError();

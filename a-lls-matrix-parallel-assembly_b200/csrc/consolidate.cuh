@@ -52,7 +52,7 @@ __global__ void __launch_bounds__(kBlockThreads) k_count_upper(ListLayout L, int
                 const int cap = chunk_cap(L, c);
                 const int next = __ldg(meta + 1);
                 for (int s = glane; s < cap; s += G) {
-                    const int col = (__ldg(meta + 2 + s) & kColMask) - 1;
+                    const int col = __ldg(meta + 2 + s) - 1;
                     cnt += col >= n;
                 }
                 if (next == 0) break;
@@ -116,7 +116,7 @@ __device__ int long_row_next_col(const ListLayout& L, int n, int after, int glan
         const int cap = chunk_cap(L, c);
         const int next = __ldg(meta + 1);
         for (int s = glane; s < cap; s += G) {
-            const int col = (__ldg(meta + 2 + s) & kColMask) - 1;
+            const int col = __ldg(meta + 2 + s) - 1;
             if (col > after && col < best) best = col;
         }
         if (next == 0) break;
@@ -128,10 +128,10 @@ __device__ int long_row_next_col(const ListLayout& L, int n, int after, int glan
 }
 
 // Returns whether the row has u columns.
-template <int DPN, int G>
+template <int G>
 __device__ bool long_row_write(const ListLayout& L, int n, int u, long long base, int glane, unsigned mask,
                                int* __restrict__ col_idx, double* __restrict__ values) {
-    constexpr int B = DPN * DPN;
+    constexpr int DPN = 2, B = DPN * DPN;
     int last = -1;
     for (int k = 0;; k++) {
         const int col = long_row_next_col<G>(L, n, last, glane, mask);
@@ -146,7 +146,7 @@ __device__ bool long_row_write(const ListLayout& L, int n, int u, long long base
             const int cap = chunk_cap(L, c);
             const int next = __ldg(meta + 1);
             for (int s = glane; s < cap; s += G) {
-                if ((__ldg(meta + 2 + s) & kColMask) - 1 == col) {
+                if (__ldg(meta + 2 + s) - 1 == col) {
                     const double* p = L.vals + (size_t)slot_gid(L, c, s) * B;
 #pragma unroll
                     for (int v = 0; v < B; v++) sum[v] += __ldg(p + v);
@@ -174,10 +174,10 @@ __device__ bool long_row_write(const ListLayout& L, int n, int u, long long base
 }
 
 // Long-row slow path of the block (BSR) output: block k of the node's block row.
-template <int DPN, int G>
+template <int G>
 __device__ void long_row_write_bsr(const ListLayout& L, int n, int u, long long base, int glane, unsigned mask,
                                    int* __restrict__ col_idx, double* __restrict__ values) {
-    constexpr int B = DPN * DPN;
+    constexpr int DPN = 2, B = DPN * DPN;
     int last = -1;
     for (int k = 0; k < u; k++) {
         const int col = long_row_next_col<G>(L, n, last, glane, mask);
@@ -191,7 +191,7 @@ __device__ void long_row_write_bsr(const ListLayout& L, int n, int u, long long 
             const int cap = chunk_cap(L, c);
             const int next = __ldg(meta + 1);
             for (int s = glane; s < cap; s += G) {
-                if ((__ldg(meta + 2 + s) & kColMask) - 1 == col) {
+                if (__ldg(meta + 2 + s) - 1 == col) {
                     const double* p = L.vals + (size_t)slot_gid(L, c, s) * B;
 #pragma unroll
                     for (int v = 0; v < B; v++) sum[v] += __ldg(p + v);
@@ -215,10 +215,10 @@ __device__ void long_row_write_bsr(const ListLayout& L, int n, int u, long long 
 
 // Long-row slow path of the upper-triangle output: the node's u column nodes
 // >= n in increasing order (the first is n itself).
-template <int DPN, int G>
+template <int G>
 __device__ void long_row_write_upper(const ListLayout& L, int n, int u, const int* __restrict__ row_ptr, int glane,
                                      unsigned mask, int* __restrict__ col_idx, double* __restrict__ values) {
-    constexpr int B = DPN * DPN;
+    constexpr int DPN = 2, B = DPN * DPN;
     int last = n - 1;
     for (int k = 0; k < u; k++) {
         const int col = long_row_next_col<G>(L, n, last, glane, mask);
@@ -232,7 +232,7 @@ __device__ void long_row_write_upper(const ListLayout& L, int n, int u, const in
             const int cap = chunk_cap(L, c);
             const int next = __ldg(meta + 1);
             for (int s = glane; s < cap; s += G) {
-                if ((__ldg(meta + 2 + s) & kColMask) - 1 == col) {
+                if (__ldg(meta + 2 + s) - 1 == col) {
                     const double* p = L.vals + (size_t)slot_gid(L, c, s) * B;
 #pragma unroll
                     for (int v = 0; v < B; v++) sum[v] += __ldg(p + v);
@@ -295,33 +295,32 @@ __device__ __forceinline__ void prefetch_first_chunk(const ListLayout& L, long l
 #define FEM_WRITE_MIN_CTAS_2D 5
 #endif
 
-// Shared memory of the sorted write: each group's sort keys and (2-D) the
-// node's sorted 2x2 blocks, loaded together before the rows are written.
-template <int DPN, int G, int KPL>
+// Shared memory of the sorted write: each group's sort keys and the node's
+// sorted 2x2 blocks, loaded together before the rows are written.
+template <int G, int KPL>
 struct WriteSmem {
     unsigned long long keys[kBlockThreads / G][G * KPL];
-    double2 vals[DPN == 2 ? kBlockThreads / G : 1][DPN == 2 ? G * KPL : 1][2];
+    double2 vals[kBlockThreads / G][G * KPL][2];
 };
 
-// The sorted write of the row nodes of batches nb = nb_first, nb_first +
+// The sorted write of the 2-D row nodes of batches nb = nb_first, nb_first +
 // nb_stride, ... below nb_end (a batch: kBlockThreads / G consecutive nodes,
 // one G-lane group each). Every thread of the CTA (kBlockThreads) calls it.
 // kMode kOutBsr: block (BSR) output, one block row per node: block_col_idx =
 // column node, block values dpn x dpn row-major; row_ptr is then the block row
 // pointer. kOutUpper: the upper triangle in CSR (ucounts: columns >= n).
-template <int DPN, int G, int KPL, int kMode>
+template <int G, int KPL, int kMode>
 __device__ __forceinline__ void write_batches(const ListLayout& L, const int* __restrict__ row_ptr,
                                               int* __restrict__ col_idx, double* __restrict__ values,
                                               long long capacity, const int* __restrict__ ucounts, long long nb_first,
-                                              long long nb_stride, long long nb_end, WriteSmem<DPN, G, KPL>& sm) {
+                                              long long nb_stride, long long nb_end, WriteSmem<G, KPL>& sm) {
     constexpr bool kBsr = kMode == kOutBsr;
     constexpr int NK = G * KPL;             // sort capacity per node
-    constexpr int B = DPN * DPN;
-    // slot words of a node's first chunk per lane (2-D: 14 slots; Hex20: at most 94)
-    constexpr int kPre = (DPN == 2 ? 16 : 96) / G;
+    constexpr int DPN = 2, B = DPN * DPN;
+    constexpr int kPre = 16 / G;  // slot words of a node's first chunk per lane (14 slots)
     auto& s_keys = sm.keys;
     auto& s_vals = sm.vals;
-    if (!output_fits<DPN, kMode>(L.info, capacity)) return;
+    if (!output_fits<2, kMode>(L.info, capacity)) return;
     const int tid = threadIdx.x;
     const int grp = tid / G, glane = tid % G;
     const unsigned gmask = group_mask<G>((tid & 31) / G);
@@ -355,7 +354,7 @@ __device__ __forceinline__ void write_batches(const ListLayout& L, const int* __
             for (int q = 0; q < kPre; q++) {
                 if (q * G < L.S1) {
                     const int s = q * G + glane;
-                    const int col = s < L.S1 ? (pre_w[q] & kColMask) : 0;
+                    const int col = s < L.S1 ? pre_w[q] : 0;
                     const unsigned used = (__ballot_sync(gmask, col != 0) >> gshift) & gmask >> gshift;
                     const int e = T + __popc(used & ((1u << glane) - 1u));
                     if (col != 0 && e < NK)
@@ -371,7 +370,7 @@ __device__ __forceinline__ void write_batches(const ListLayout& L, const int* __
                 next = __ldg(meta + 1);
                 for (int s0 = 0; s0 < cap; s0 += G) {
                     const int s = s0 + glane;
-                    const int col = s < cap ? (__ldg(meta + 2 + s) & kColMask) : 0;
+                    const int col = s < cap ? __ldg(meta + 2 + s) : 0;
                     const unsigned used = (__ballot_sync(gmask, col != 0) >> gshift) & gmask >> gshift;
                     const int e = T + __popc(used & ((1u << glane) - 1u));
                     if (col != 0 && e < NK)
@@ -399,24 +398,19 @@ __device__ __forceinline__ void write_batches(const ListLayout& L, const int* __
 #pragma unroll
         for (int i = 0; i < KPL; i++) s_keys[grp][glane * KPL + i] = keys[i];
         __syncwarp();
-        if constexpr (DPN == 2) {
-            // all of the node's blocks in flight at once (two 16-byte loads each)
-            for (int k = glane; k < Ts; k += G) {
-                const double2* p = reinterpret_cast<const double2*>(L.vals + (size_t)(unsigned)s_keys[grp][k] * B);
-                s_vals[grp][k][0] = __ldg(p);
-                s_vals[grp][k][1] = __ldg(p + 1);
-            }
-            __syncwarp();
+        // all of the node's blocks in flight at once (two 16-byte loads each)
+        for (int k = glane; k < Ts; k += G) {
+            const double2* p = reinterpret_cast<const double2*>(L.vals + (size_t)(unsigned)s_keys[grp][k] * B);
+            s_vals[grp][k][0] = __ldg(p);
+            s_vals[grp][k][1] = __ldg(p + 1);
         }
+        __syncwarp();
         // entry v of the node's k-th sorted block
-        auto block_value = [&](int k, int v) -> double {
-            if constexpr (DPN == 2) return reinterpret_cast<const double*>(&s_vals[grp][k][0])[v];
-            return __ldg(L.vals + (size_t)(unsigned)s_keys[grp][k] * B + v);
-        };
+        auto block_value = [&](int k, int v) { return reinterpret_cast<const double*>(&s_vals[grp][k][0])[v]; };
         // 3. write the dpn rows of the node (or its block row, or its upper rows)
         if (valid && kMode == kOutUpper) {
             if (long_row) {
-                long_row_write_upper<DPN, G>(L, n, u, row_ptr, glane, gmask, col_idx, values);
+                long_row_write_upper<G>(L, n, u, row_ptr, glane, gmask, col_idx, values);
             } else if (u > 0 && u <= Ts) {
                 const int k0 = Ts - u;  // the sorted row's first column >= n (n itself)
                 for (int a = 0; a < DPN; a++) {
@@ -440,7 +434,7 @@ __device__ __forceinline__ void write_batches(const ListLayout& L, const int* __
             }
         } else if (valid && kBsr) {
             if (long_row) {
-                long_row_write_bsr<DPN, G>(L, n, u, base, glane, gmask, col_idx, values);
+                long_row_write_bsr<G>(L, n, u, base, glane, gmask, col_idx, values);
             } else {
                 for (int k = glane; k < Ts; k += G) col_idx[base + k] = (int)(s_keys[grp][k] >> 32);
                 for (int idx = glane; idx < Ts * B; idx += G) {
@@ -450,7 +444,7 @@ __device__ __forceinline__ void write_batches(const ListLayout& L, const int* __
             }
         } else if (valid) {
             if (long_row) {
-                long_row_write<DPN, G>(L, n, u, base, glane, gmask, col_idx, values);
+                long_row_write<G>(L, n, u, base, glane, gmask, col_idx, values);
             } else {
                 const int row_len = DPN * Ts;
                 for (int a = 0; a < DPN; a++) {
@@ -638,7 +632,7 @@ __device__ __forceinline__ void write_sorted_2d(const ListLayout& L, const int* 
                     }
                 }
             } else {
-                if (!long_row_write<2, G>(L, (int)n, u[q], base[q], lane, gmask, col_idx, values)) lowest = 0;
+                if (!long_row_write<G>(L, (int)n, u[q], base[q], lane, gmask, col_idx, values)) lowest = 0;
             }
         }
     }

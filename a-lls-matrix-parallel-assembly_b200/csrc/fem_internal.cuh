@@ -99,10 +99,8 @@ __device__ __forceinline__ int alloc_chunk(const ListLayout& L) {
     return L.N + k;
 }
 
-// Bound on retry loops (chunk chains, claims); hitting it raises FEM_ERR_TIMEOUT.
+// Bound on the walk along a chunk chain; hitting it raises FEM_ERR_TIMEOUT.
 constexpr int kMaxChainSteps = 1 << 20;
-
-constexpr int kColMask = 0x7FFFFFFF;
 
 // Header word (word 0) of a 2-D first chunk whose row is complete in it: this plus the number of columns, which fill
 // the first slots in increasing order (no next chunk). 0: the row is hashed (fans).

@@ -57,7 +57,7 @@ constexpr int kThreads = kValueWarps * 32;
 // row e; kToCsrColour: the elements perm[range[0], range[1]) of one colour).
 template <int kOut>
 __global__ void __launch_bounds__(kThreads, FEM_VALUES_CTAS)
-    k_values_hex20(MeshView m, const int* __restrict__ perm, int i0, int i1, const int* __restrict__ range,
+    k_values_hex20(MeshView m, const int* __restrict__ perm, [[maybe_unused]] int i0, int i1, const int* __restrict__ range,
                    ValuesTarget t, int group, int run) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     ValuesSmem& sm = *reinterpret_cast<ValuesSmem*>(smem_raw);

@@ -66,17 +66,15 @@ __device__ __forceinline__ void values_init(ValuesSmem& sm) {
 }
 
 // The value pass of the elements at positions i = i_first, i_first +
-// i_stride, ... below i1 of the visit order perm (perm NULL: element i) by
-// one CTA of at least kValueWarps warps (warps beyond them help with the
-// per-element tables only). Every thread of the CTA calls it.
+// i_stride, ... below i1 of the visit order perm by one CTA of kValueWarps
+// warps. Every thread of the CTA calls it.
 template <int kOut>
 __device__ __forceinline__ void values_cta(const MeshView& m, const int* __restrict__ perm, long long i_first,
                                            long long i_stride, int i1, const ValuesTarget& t, ValuesSmem& sm) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nt = blockDim.x;
-    const bool tile_warp = warp < kValueWarps;
     const int ti = tile_ti(warp), tj = tile_tj(warp);
     const int fr = lane >> 2, fc = lane & 3;
-    auto elem = [&](long long i) -> int { return perm ? __ldg(perm + i) : (int)i; };
+    auto elem = [&](long long i) { return __ldg(perm + i); };
     // node id and coordinates of the next element
     int pre_n = 0;
     double pre_x = 0.0, pre_y = 0.0, pre_z = 0.0;
@@ -168,7 +166,6 @@ __device__ __forceinline__ void values_cta(const MeshView& m, const int* __restr
             pre_y = __ldg(m.y + pre_n);
             pre_z = __ldg(m.z + pre_n);
         }
-        if (!tile_warp) continue;  // the remaining warps wait at the next element's first barrier
         // M^{ab} tiles (ti, tj): A[r][k] = w_k G[a][8 ti + r][k], B[k][c] = G[b][8 tj + c][k]
         double acc[3][3][2];
 #pragma unroll
