@@ -112,7 +112,7 @@ struct RowsMap {
     int* blocks;            // not 0: the pattern does not take this form, the map is the block positions
 };
 // cnt (N ints) and tiles (row_tiles(N) partials): scratch. *r.blocks (0 before) is set when the pattern is not one of
-// node blocks that holds all of the mesh's, with rows of at most 65,536 columns.
+// node blocks that holds all of the mesh's, from entry 0 on, with rows of at most 65,536 columns.
 cudaError_t launch_build_rows_map(const MeshView& m, int kind, const int* row_ptr, const int* col_idx, const RowsMap& r,
                                   int* cnt, long long* tiles, DevInfo* info, cudaStream_t s);
 // Clears the info word; values[0, nnz): the rows and zeros behind them; by the block positions b where *r.blocks is set.

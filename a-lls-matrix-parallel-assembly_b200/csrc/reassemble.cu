@@ -199,8 +199,9 @@ __global__ void __launch_bounds__(kThreads) k_map_fill(MeshView m, const int* __
 }
 
 // ranks[NPE * j + k]: rank in the row of occurrence j's node of the element's node k positions after it.
-// blocks: set when a node's two rows differ in length or are odd, a column node's pair starts at an odd place, a rank
-// passes 16 bits or the pattern lacks a block (a caller's own pattern: with further columns, or too small).
+// blocks: set when the first row does not start at entry 0 (the rows would not cover the entries before it, and could
+// start at odd places), a node's two rows differ in length or are odd, a column node's pair starts at an odd place, a
+// rank passes 16 bits or the pattern lacks a block (a caller's own pattern: with further columns, or too small).
 template <int KIND>
 __global__ void __launch_bounds__(kThreads) k_map_ranks(MeshView m, const int* __restrict__ off,
                                                         const unsigned* __restrict__ occ,
@@ -212,7 +213,7 @@ __global__ void __launch_bounds__(kThreads) k_map_ranks(MeshView m, const int* _
     bool other = false;
     for (long long n = blockIdx.x * blockDim.x + threadIdx.x; n < m.N; n += gridDim.x * blockDim.x) {
         const int r0 = __ldg(row_ptr + 2 * n), r1 = __ldg(row_ptr + 2 * n + 1), r2 = __ldg(row_ptr + 2 * n + 2);
-        other |= r2 - r1 != r1 - r0 || ((r1 - r0) & 1);
+        other |= r2 - r1 != r1 - r0 || ((r1 - r0) & 1) || (n == 0 && r0 != 0);
     }
     for (long long j = blockIdx.x * blockDim.x + threadIdx.x; j < total; j += gridDim.x * blockDim.x) {
         const unsigned w = __ldg(occ + j);

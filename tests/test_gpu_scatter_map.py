@@ -129,6 +129,22 @@ def test_patterns_without_some_blocks(fem, oracle_mod, cuda_device, name):
     assert np.all(np.abs(vals.cpu().numpy() - ov[keep]) <= RTOL * scale[keep])
 
 
+@pytest.mark.parametrize("name", list(MESHES))
+@pytest.mark.parametrize("first", [1, 2, 7])
+def test_patterns_that_start_behind_other_entries(fem, oracle_mod, cuda_device, name, first):
+    # the rows of one matrix among others: row_ptr[0] is not 0; the entries before it become zero, as those behind the rows
+    m = _mesh(name)
+    orp, oci, ov = oracle_mod.assemble(m)
+    asm = fem.Assembler(m)
+    vals = _with_pattern(asm, orp + first, np.concatenate([np.zeros(first, np.int32), oci]))
+    re = _build(fem, asm, vals.numel(), 0)
+    re.reassemble(vals)
+    assert re.read_info() == 0
+    got = vals.cpu().numpy()
+    assert np.all(got[:first] == 0.0)
+    _close(orp, oci, ov, got[first:])
+
+
 @pytest.mark.parametrize("cols", [65535, 65536, 65537, 70001])
 def test_rows_past_16_bit_ranks(fem, oracle_mod, cuda_device, cols):
     # a closed fan: its hub's row has a column per triangle and its own
