@@ -1143,8 +1143,8 @@ fem_status fem_assemble_host(fem_context* ctx, const fem_mesh* hm, const fem_opt
 // g_static_workspace is only a host-side stand-in, never a device address.
 //
 // All calls on a device share the one array, which keeps the last call's
-// contents. Each assembly clears what must start at zero (info word, first
-// chunk rows, row counters) and writes every value before reading it, so
+// contents. Each assembly clears what must start at zero (info word, row
+// counters) and writes every list word and value before reading it, so
 // consecutive calls are independent; calls whose work overlaps on the GPU
 // (different streams, or different host threads) race on the array and
 // corrupt each other's results.

@@ -1,5 +1,6 @@
 // Hex20 element definitions shared by the element-stiffness kernels
-// (element_stiffness.cu, ke_tcgen05.cu) and the two-pass A-LLS scatter (values_hex20.cuh).
+// (ke_hex20.cuh, element_stiffness.cu, ke_tcgen05.cu) and the element pass of
+// the re-assembly and the colouring (values_hex20.cuh).
 //
 // Element stiffness, in double. With the physical shape-function gradients
 // G_g (a 60-vector per Gauss point g, dof r = 3 node + dir) and

@@ -1,11 +1,12 @@
-// Element processing order for the scatter kernels.
+// Visit orders: of the elements for the re-assembly by block positions, of the
+// nodes for the Hex20 consolidation. (The scatter takes the elements as they come.)
 //
-// The scatter's cost is dominated by the L2 / HBM traffic of the row lists it
-// touches. Elements given in a shuffled order (the T3 and mixed benchmark
-// meshes) touch lists all over the pool at once; processing them grouped by
-// their lowest node id keeps the lists of a band of nodes hot in L2 while all
-// of their elements are scattered. The order is a stable-per-bucket counting
-// sort computed on the device every call:
+// The time of a re-assembly by block positions goes into the L2 / HBM traffic of
+// the CSR lines it adds to. Elements in a shuffled order (the T3 and mixed
+// benchmark meshes) touch lines all over the matrix at once; grouped by their
+// lowest node id, the rows of a band of nodes stay hot in L2 while all of their
+// elements are added. A stable-per-bucket counting sort on the device, part of
+// the map build:
 //   k_bucket_count    key = type * NB + (min node id >> kBucketShift); histogram
 //   k_bucket_scan     one CTA: exclusive scan of the histogram; the element
 //                     range of each element type (Q4 first, then T3)
@@ -13,13 +14,13 @@
 // When the key table fits in shared memory (up to 40 K keys), one CTA per SM
 // counts and places its elements with shared-memory atomics instead
 // (k_key_count_sm, k_key_scatter_sm), one global atomic per non-zero key.
-// The input arrays are not modified; only the order in which the scatter
-// visits elements changes (and with it the order of the FP64 atomic adds).
+// The input arrays are not modified; only the order of the visits changes (and
+// with it the order of the FP64 atomic adds).
 //
-// Hex20 meshes use a spatial order instead: a row node's elements (up to 8)
-// should be scattered close together in time, or its list lines are evicted
-// from L2 between their visits (in natural x-y-z order they are a whole z-layer
-// of elements apart). The key is the 3-D Morton code of the midpoint of each
+// Hex20 elements are re-assembled in a spatial order instead: a row node's
+// elements (up to 8) should be added close together in time, or its lines are
+// evicted from L2 between their visits (in natural x-y-z order they are a whole
+// z-layer of elements apart). The key is the 3-D Morton code of the midpoint of each
 // element's corner diagonal (nodes 0 and 6), quantized on a 2^b grid over the
 // node bounding box (k_bbox), counting-sorted the same way. The consolidation of
 // a large Hex20 mesh visits its nodes by the Morton code of their cell on a

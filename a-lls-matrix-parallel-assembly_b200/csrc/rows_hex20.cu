@@ -54,7 +54,7 @@ __global__ void __launch_bounds__(256) k_begin_hex20(ListLayout L, int* __restri
 
 // Everything up to the row lists of a small mesh (launch.h's kSmallNodes) in
 // one cooperative launch: seven launches at about 4 us of the caller's time
-// each become one and six grid barriers of 1 to 2 us.
+// each become one and five grid barriers of 1 to 2 us.
 static_assert(kOccThreads == kHexRowThreads && kScanThreads == kHexRowThreads, "one block shape");
 __global__ void __launch_bounds__(kHexRowThreads, FEM_HEXR_CTAS)
     k_small_hex20(MeshView m, ListLayout L, HexRows h, int* __restrict__ cnt, int* __restrict__ queue) {

@@ -16,9 +16,10 @@
 //                      registers: 64, 128 or 256 keys), written to the list
 //                      chunks, and their ranks go back through the table to
 //                      the rank map.
-//   k_wide_rows_hex20  nodes with up to 32 elements, one warp each: repeated
-//                      minimum over the candidates, which stay in registers.
-//   k_long_rows_hex20  longer rows, one CTA each: sorted in shared memory.
+//   k_long_rows_hex20  nodes with up to 32 elements, one warp each: repeated
+//                      minimum over the candidates, which stay in registers;
+//                      then nodes with more, one CTA each: sorted in shared
+//                      memory.
 // A row past its first chunk takes consecutive overflow chunks from the pool.
 //
 // What bounds it: instruction issue (660 warp instructions a node in hash, sort
@@ -363,7 +364,7 @@ __device__ __forceinline__ void wide_rows_hex20(const int* __restrict__ conn, co
     const int lane = threadIdx.x & 31, count = __ldcg(&L.info->long_rows);
     for (int k = warp; k < count; k += nwarps) {
         const int n = __ldcg(queue + k), lo = __ldcg(off + n), d = __ldcg(off + n + 1) - lo;
-        if (d > kWideElems) continue;  // k_long_rows_hex20's
+        if (d > kWideElems) continue;  // long_rows_hex20's
         const int o = lane < d ? (int)occ_of(__ldcg(inc + lo + lane)) : 0;
         int node[kWideCand];
 #pragma unroll

@@ -15,12 +15,14 @@
 // shuffles, the next occurrence's loads in flight meanwhile. An element names a
 // column node once, so the lanes' additions never meet; a repeated node's
 // further blocks are added one by one. Then the rows leave with consecutive
-// lanes on consecutive entries. No value is added atomically and the sums do
-// not depend on timing.
+// lanes on consecutive entries. No value is added atomically; a row's
+// occurrences come in the order in which the scatter's counters dealt their
+// places, so two runs differ in the sums' last bits.
 //
-// What bounds it: DRAM traffic and the latency of the slab loads together. A
-// 64^3 mesh has 4.0 GB of Ke to read and 6.7 GB of CSR to write (1.6 ms at the
-// measured copy rate). B200: 2.79 ms (4.02 ms with a fixed stride of nodes in
+// What bounds it: wavefronts of L1 and shared memory (six slab loads, table
+// reads, sums read and written back per lane and occurrence: 88 % of the LSU
+// data pipe at 32^3, DRAM 47 %). A 64^3 mesh has 4.0 GB of Ke to read and 6.7
+// GB of CSR to write (1.6 ms at the measured copy rate). B200: 2.79 ms (4.02 ms with a fixed stride of nodes in
 // their numbering, per-entry index arithmetic and no row headers in flight);
 // the value pass into list blocks (stores and FP64 atomics) and the copy out of
 // the lists that it replaces took 5.18 + 3.06 ms with the Ke computed inside.

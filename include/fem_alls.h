@@ -155,7 +155,10 @@ FEM_API fem_status fem_alls_workspace_size(const fem_mesh* mesh, const fem_opts*
 
 /* Resets the workspace lists and runs the fused element-stiffness + list
  * scatter kernel(s). Replaces the reference's pool resets and
- * assembleGlobalStiffnessKernelALLS / ...FixedArray launches. Asynchronous. */
+ * assembleGlobalStiffnessKernelALLS / ...FixedArray launches. Asynchronous.
+ * A small mesh (at most 16,384 nodes; elements: Hex20 as many, 2-D four times as
+ * many) is one cooperative launch, which starts when all of its blocks (at most
+ * those that the GPU holds at once) fit beside what runs on other streams. */
 FEM_API fem_status fem_alls_scatter(const fem_mesh* mesh, const fem_opts* opts, void* workspace,
                             size_t workspace_bytes, void* stream);
 
@@ -164,7 +167,9 @@ FEM_API fem_status fem_alls_scatter(const fem_mesh* mesh, const fem_opts* opts, 
  * buildCSRStructure and convertALLStoCSRKernel. row_ptr is always written; if
  * capacity < nnz nothing else is written and the device info gets
  * FEM_ERR_CAPACITY (the lists stay intact, so it can be re-run with larger
- * buffers). capacity 0 with NULL col_idx/values just counts. Asynchronous. */
+ * buffers). capacity 0 with NULL col_idx/values just counts. mesh: the one that was
+ * scattered, its conn unchanged (Hex20 rows of more than 65,536 column nodes read it
+ * again); the same holds for the two forms below. Asynchronous. */
 FEM_API fem_status fem_alls_consolidate(const fem_mesh* mesh, const fem_opts* opts, void* workspace,
                                 size_t workspace_bytes, int32_t* row_ptr, int32_t* col_idx,
                                 double* values, int64_t capacity, void* stream);
@@ -305,8 +310,8 @@ FEM_API fem_status fem_autotune_workspace_size(const fem_mesh* mesh, const fem_o
 FEM_API fem_status fem_autotune(const fem_mesh* mesh, const fem_opts* opts, void* workspace, size_t workspace_bytes,
                                 fem_csr* out, int32_t repeats, fem_opts* best, float* best_ms, void* stream);
 
-/* A batch: the concurrency of fem_assemble_batched (1, 2, 4, 8, 16 slots, at
- * most n; candidates whose workspace exceeds workspace_bytes are skipped).
+/* A batch: the concurrency of fem_assemble_batched (1, 2, 4, ... slots, at most
+ * n and 256; candidates whose workspace exceeds workspace_bytes are skipped).
  * outs / infos as for fem_assemble_batched; on return they hold the batch
  * assembled with *best_concurrency. */
 FEM_API fem_status fem_autotune_batched(const fem_mesh* meshes, int32_t n, const fem_opts* opts, void* workspace,
