@@ -36,3 +36,32 @@ def test_sizes(fem, oracle_mod, cuda_device, kind, nx, ny, scale):
     re.reassemble(vals, o)
     assert re.read_info() == 0
     assert np.all(np.abs(vals.cpu().numpy() - ov) <= most)
+
+
+def test_t3_blocks_that_fp32_holds(fem, oracle_mod, cuda_device):
+    # integer coordinates, nu = 0, thickness 2 and E = detJ: every factor and sum of a block is a whole number or a half
+    # below 2^24, so the FP32 form has no rounding to make (what is left is the oracle's: 1e-12, as in FP64)
+    import torch
+    import meshgen as mg
+    nx, ny = 185, 181
+    m = mg.t3_grid(nx, ny, seed=3)
+    r = np.random.default_rng(3)
+    at = np.arange(m.num_nodes)
+    m.x = 32.0 * (at % (nx + 1)) + r.integers(-7, 8, m.num_nodes)
+    m.y = 32.0 * (at // (nx + 1)) + r.integers(-7, 8, m.num_nodes)
+    x, y = m.x[m.conn], m.y[m.conn]
+    m.E = (x[:, 1] - x[:, 0]) * (y[:, 2] - y[:, 0]) - (x[:, 2] - x[:, 0]) * (y[:, 1] - y[:, 0])
+    assert m.E.min() > 0
+    m.nu, m.nu0, m.thickness = None, 0.0, 2.0
+    orp, oci, ov = oracle_mod.assemble(m)
+    o = fem.opts(precision=fem.FEM_PREC_FP32)
+    asm = fem.Assembler(m, o)
+    rp, ci, v, info = asm.assemble()
+    np.testing.assert_array_equal(ci.cpu().numpy(), oci)
+    most = 1e-12 * np.maximum(np.abs(ov), diag_scale(orp, oci, ov))
+    assert np.all(np.abs(v.cpu().numpy() - ov) <= most)
+    re = fem.Reassembler(asm)
+    re.build(int(info.nnz))
+    re.reassemble(v, o)
+    assert re.read_info() == 0
+    assert np.all(np.abs(v.cpu().numpy() - ov) <= most)
